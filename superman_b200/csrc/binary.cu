@@ -28,10 +28,10 @@ static double log2_perm_bound(const uint8_t* a, int n)
     return std::fmin(side(true), side(false));
 }
 
-// Limbs for the NW sum Sigma = 2^(n-1) perm: |Sigma| < 2^(32L-1).
-static int pick_limbs(double perm_bits, int n)
+// Limbs for a sum Sigma = 2^shift perm: |Sigma| < 2^(32L-1).
+static int pick_limbs(double perm_bits, int shift)
 {
-    const double bits = perm_bits + (n - 1) + 2;
+    const double bits = perm_bits + shift + 2;
     if (bits <= 128) return 4;
     if (bits <= 160) return 5;
     if (bits <= 192) return 6;
@@ -39,7 +39,40 @@ static int pick_limbs(double perm_bits, int n)
     return 12;
 }
 
-static int run(const uint8_t* a, int n, const spb_options* opt_in, uint32_t* limbs_out,
+// Rewrites the matrix for the expanded walk: the line with the fewest ones
+// becomes the last column (a row by transposing, which keeps the permanent) and
+// the rows with a one in it come first.  Returns their number m, or 0 when the
+// plain walk runs: n < 4 (no two walk columns besides the expanded one), an
+// empty line (permanent 0) or more ones than the kernel's halves hold.
+// Where it applies the expanded walk is the faster one at every n and m: it
+// takes half the subsets and at most 3/2 of the operations per subset.
+static int expand(std::vector<uint8_t>* m, int n)
+{
+    if (n < 4) return 0;
+    int best = n + 1, line = 0;  // line < n: column, else row line - n
+    for (int l = 0; l < 2 * n; ++l) {
+        int c = 0;
+        for (int i = 0; i < n; ++i) c += (l < n ? (*m)[i * n + l] : (*m)[(l - n) * n + i]) ? 1 : 0;
+        if (c < best) { best = c; line = l; }
+    }
+    if (best < 1 || best > kExpandHalves * half_rows(n)) return 0;
+    const std::vector<uint8_t> a = *m;
+    const int e = line % n;
+    const bool tr = line >= n;
+    auto at = [&](int r, int c) { return tr ? a[c * n + r] : a[r * n + c]; };
+    int to = 0;
+    for (int pass = 1; pass >= 0; --pass)
+        for (int r = 0; r < n; ++r) {
+            if ((at(r, e) ? 1 : 0) != pass) continue;
+            for (int c = 0, k = 0; c < n; ++c)
+                if (c != e) (*m)[to * n + k++] = at(r, c) ? 1 : 0;
+            (*m)[to * n + n - 1] = (uint8_t)pass;
+            ++to;
+        }
+    return best;
+}
+
+static int run(const uint8_t* a_in, int n, const spb_options* opt_in, uint32_t* limbs_out,
                spb_result* out)
 {
     double t_start = wall_seconds();
@@ -51,12 +84,13 @@ static int run(const uint8_t* a, int n, const spb_options* opt_in, uint32_t* lim
     std::memset(limbs_out, 0, sizeof(uint32_t) * 10);
     spb_options opt;
     if (opt_in) opt = *opt_in; else spb_default_options(&opt);
-    if (!a || n < 1 || n > kMaxN) {
+    if (!a_in || n < 1 || n > kMaxN) {
         spb_set_error("binary permanent needs a non-null matrix and 1 <= n <= %d (got n=%d)", kMaxN, n);
         return out->status = SPB_ERR_INVALID;
     }
     out->gray_steps = (uint64_t)n << (n - 1);
     if (n <= 2) {  // fewer than two walk columns: direct
+        const uint8_t* a = a_in;
         const unsigned v = n == 1 ? (a[0] ? 1u : 0u)
                                   : (unsigned)((a[0] && a[3]) ? 1 : 0) + ((a[1] && a[2]) ? 1 : 0);
         limbs_out[0] = v;
@@ -73,20 +107,24 @@ static int run(const uint8_t* a, int n, const spb_options* opt_in, uint32_t* lim
 
     Problem pb{};
     pb.n = n;
-    const double bits = log2_perm_bound(a, n);
-    pb.limbs = pick_limbs(bits < 0 ? 0.0 : bits, n);
-    // the NW walk runs over the n-1 columns other than the last
+    std::vector<uint8_t> a(a_in, a_in + (size_t)n * n);
+    const double bits = log2_perm_bound(a.data(), n);
+    pb.m = expand(&a, n);
+    // The NW walk takes the nc columns other than the expanded one (plain
+    // walk: all n), over the subsets of all but the last of them.
+    const int nc = pb.m > 0 ? n - 1 : n, nb = nc - 1;
+    pb.limbs = pick_limbs(bits < 0 ? 0.0 : bits, nb);
     int w = opt.unit_bits > 0 ? opt.unit_bits : 8;
     if (opt.unit_bits <= 0)
-        while (w > 2 && (((size_t)1 << w) * n * 4 > 32 * 1024 || n - 1 - w < 16)) --w;
+        while (w > 2 && (((size_t)1 << w) * n * 4 > 32 * 1024 || nb - w < 16)) --w;
     if (w > 12) w = 12;
-    if (w > n - 1) w = n - 1;
+    if (w > nb) w = nb;
     if (w < 2) w = 2;
     pb.w = w;
-    pb.units = 1ull << (n - 1 - w);
-    const int terms = 1 << w, ntop = n - 1 - w;
+    pb.units = 1ull << (nb - w);
+    const int terms = 1 << w, ntop = nb - w;
 
-    const int tmax = bin_max_threads(n, pb.limbs);
+    const int tmax = bin_max_threads(n, pb.limbs, pb.m > 0);
     int threads = opt.threads_per_block > 0 ? (opt.threads_per_block / 32) * 32 : tmax;
     if (threads > tmax) threads = tmax;
     if (threads < 32) threads = 32;
@@ -104,13 +142,13 @@ static int run(const uint8_t* a, int n, const spb_options* opt_in, uint32_t* lim
     if (blocks < 1) blocks = 1;
     pb.grid = blocks;
 
-    // host-built tables: x'_r = 2 a_{r,n-1} - rowsum_r, doubled low-column
-    // counts, doubled high columns
+    // host-built tables: x'_r = 2 a_{r,nc-1} - rowsum_r over the nc columns,
+    // doubled low-column counts, doubled high columns
     std::vector<int> x0(n);
     for (int r = 0; r < n; ++r) {
         int rs = 0;
-        for (int j = 0; j < n; ++j) rs += a[r * n + j] ? 1 : 0;
-        x0[r] = 2 * (a[r * n + n - 1] ? 1 : 0) - rs;
+        for (int j = 0; j < nc; ++j) rs += a[r * n + j] ? 1 : 0;
+        x0[r] = 2 * (a[r * n + nc - 1] ? 1 : 0) - rs;
     }
     std::vector<int> dei((size_t)terms * n);
     for (int d = 0; d < terms; ++d)
@@ -161,7 +199,7 @@ static int run(const uint8_t* a, int n, const spb_options* opt_in, uint32_t* lim
     SPB_CUDA_TRY(cudaEventElapsedTime(&ms_call, ctx->ev_call0, ctx->ev_call1));
 
     const int L = pb.limbs;
-    if (!(n & 1)) {  // perm = (+-) Sigma / 2^(n-1), + for odd n: negate mod 2^(32L)
+    if (!(nc & 1)) {  // perm = (+-) Sigma / 2^(nc-1), + for odd nc: negate mod 2^(32L)
         uint64_t c = 1;
         for (int l = 0; l < L; ++l) {
             uint64_t t = (uint64_t)(~res[l]) + c;
@@ -169,11 +207,11 @@ static int run(const uint8_t* a, int n, const spb_options* opt_in, uint32_t* lim
             c = t >> 32;
         }
     }
-    // arithmetic shift right by n-1 bits (Sigma is a multiple of 2^(n-1))
+    // arithmetic shift right by nc-1 bits (Sigma is a multiple of 2^(nc-1))
     const bool neg = (res[L - 1] >> 31) & 1u;
     uint32_t ext[kMaxLimbs + 2];
     for (int l = 0; l < kMaxLimbs + 2; ++l) ext[l] = l < L ? res[l] : (neg ? 0xffffffffu : 0u);
-    const int sh = n - 1, ws = sh / 32, bs = sh % 32;
+    const int sh = nc - 1, ws = sh / 32, bs = sh % 32;
     uint32_t shifted[kMaxLimbs];
     for (int l = 0; l < kMaxLimbs; ++l) {
         const uint32_t lo = l + ws < kMaxLimbs + 2 ? ext[l + ws] : (neg ? 0xffffffffu : 0u);

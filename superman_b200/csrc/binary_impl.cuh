@@ -23,6 +23,22 @@
 // bit widths so far can reach, and applies the sign (the xor of the words')
 // once.  Unit sums and the grid reduction are exact, so the result does not
 // depend on the launch shape.
+//
+// Expanded walk (walk_binary<N, L, true>).  The permanent is expanded along one
+// column c with m ones, whose rows the host puts first:
+//   perm(A) = sum_{r < m} perm(A without row r and column c).
+// All m minors share the columns, so one NW walk over the other n-1 columns
+// (2^(n-2) subsets, half of the plain walk's) evaluates them together: a term
+// is sum_{r < m} prod_{r' != r} x'_r', the first derivative of prod_r (x'_r + t)
+// over the rows r < m, times the other rows' product.  Per row below m that
+// takes one more multiply-add (q <- q x + p beside p <- p x), per row above m
+// nothing more, so two plain terms' work of 4 operations per row becomes 3 or 2.
+// The host picks the line (column, or row by transposing) with the fewest
+// ones.  Sigma = sum_S (-1)^|S| term = 2^(n-2) * (+-) perm(A) (+ for even n).
+// On one B200 at 1965 MHz, Bernoulli(0.5) entries with the identity: n=36
+// 203.0 -> 134.1 ms, n=32 11.25 -> 7.62 ms, n=28 0.668 -> 0.521 ms.  Bound, as the
+// plain walk, by the instructions it issues: with 32-bit words as there (a sign
+// and a magnitude per word) n=36 took 146 ms at 16 warps per SM and 183 ms at 8.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -38,10 +54,11 @@ constexpr int kMaxLimbs = 12;   // accumulator limbs (the result needs at most 1
 
 struct Problem {
     int n, w, limbs, grid;
-    unsigned long long units;  // 2^(n-1-w) Gray units of 2^w terms each
+    int m;                     // expanded walk: ones of the expanded column (rows 0..m-1); 0 = plain walk
+    unsigned long long units;  // 2^(n-1-w) Gray units of 2^w terms each (expanded walk: 2^(n-2-w))
     const int* x0;             // [n] 2 a_{r,n-1} - rowsum_r
     const int* dei;            // [2^w/4][n][4] twice the low-column row counts
-    const int8_t* mt;          // [n-1-w][n] high columns, doubled (0/2)
+    const int8_t* mt;          // [ntop][n] high columns, doubled (0/2)
     uint32_t* partials;        // [grid][limbs]
     unsigned* ticket;          // last-CTA election (reset by the kernel)
     uint32_t* result;          // [limbs] sum over subsets, mod 2^(32*limbs)
@@ -180,12 +197,212 @@ __device__ __forceinline__ void limb_add_masked(uint32_t (&a)[L], const uint32_t
     }
 }
 
-// Sum over one unit: sum_d (-1)^popc(d) prod_r (xt_r + DEI[d][r]).
-template <int N, int L>
-__device__ __forceinline__ void unit_sum_bin(const int (&xt)[N], const int* __restrict__ s_de, int nq,
+// ------------------------------------------------------- expanded walk ----
+// Rows multiply in halves of up to K rows, signed 32-bit integers, and two
+// halves make a signed 64-bit word (one 32x32->64 multiply), so that a term
+// takes a sign and a magnitude per 2K rows instead of one per K.  The words
+// with rows of the expanded column carry the derivative q beside the product.
+constexpr int kExpandHalves = 4;  // halves that may hold rows of the expanded column
+
+// Rows per half: the largest K with (n-1)^K < 2^31 and K (n-1)^(K-1) < 2^31 (the
+// half's product and its derivative; row values are at most n-1 in magnitude).
+__host__ __device__ constexpr int half_rows(int n)
+{
+    const unsigned long long b = (unsigned long long)(n - 1 > 1 ? n - 1 : 2);
+    int k = 1;
+    unsigned long long p = b;  // b^k
+    while (p * b < (1ull << 31) && (unsigned long long)(k + 1) * p < (1ull << 31) && k < 16) {
+        p *= b;
+        ++k;
+    }
+    return k;
+}
+__host__ __device__ constexpr int rows_in_half(int n, int h)
+{
+    const int left = n - h * half_rows(n);
+    return left <= 0 ? 0 : (left < half_rows(n) ? left : half_rows(n));
+}
+
+// Limbs that can be nonzero after words 0..g: a product of R rows is at most
+// (n-1)^R, a sum of m <= n products of R-1 rows at most n (n-1)^(R-1): one bit more.
+__host__ __device__ constexpr int expand_limbs_after(int n, int g, int L)
+{
+    int bits = 1;
+    for (int h = 0; h <= 2 * g + 1; ++h)
+        if (rows_in_half(n, h) > 0) bits += word_bits(n - 1, rows_in_half(n, h));
+    const int l = (bits + 31) / 32;
+    return l < L ? l : L;
+}
+
+// Half h: the product p of its rows' values.
+template <int N, int G, int h>
+__device__ __forceinline__ int half_plain(const int (&xt)[N], const int* __restrict__ de, int i)
+{
+    constexpr int r0 = h * half_rows(N), rows = rows_in_half(N, h);
+    int p = 1;
+#pragma unroll
+    for (int k = 0; k < rows; ++k) {
+        const int x = xt[r0 + k] + de[(r0 + k) * G + i];
+        p = k == 0 ? x : p * x;
+    }
+    return p;
+}
+
+// The same with its derivative q over the rows below m.  ALL: all of them are.
+template <int N, int G, int h, bool ALL>
+__device__ __forceinline__ void half_dual(const int (&xt)[N], const int* __restrict__ de, int i, int m, int& p, int& q)
+{
+    constexpr int r0 = h * half_rows(N), rows = rows_in_half(N, h);
+#pragma unroll
+    for (int k = 0; k < rows; ++k) {
+        const int x = xt[r0 + k] + de[(r0 + k) * G + i];
+        if (k == 0) {
+            p = x;
+            q = 1;  // the half holds a row below m
+        } else {
+            q = ALL && k == 1 ? x + p : q * x + (ALL || r0 + k < m ? p : 0);
+            p *= x;
+        }
+    }
+}
+
+template <int N, int G, int h>
+__device__ __forceinline__ void half_any(const int (&xt)[N], const int* __restrict__ de, int i, int m, int& p, int& q)
+{
+    if (m >= h * half_rows(N) + rows_in_half(N, h)) half_dual<N, G, h, true>(xt, de, i, m, p, q);
+    else half_dual<N, G, h, false>(xt, de, i, m, p, q);
+}
+
+// Word g: the product W of its rows, its derivative Q when it holds rows below m.
+template <int N, int G, int g>
+__device__ __forceinline__ long long word_plain(const int (&xt)[N], const int* __restrict__ de, int i)
+{
+    const long long a = half_plain<N, G, 2 * g>(xt, de, i);
+    if constexpr (rows_in_half(N, 2 * g + 1) == 0) return a;
+    else return a * (long long)half_plain<N, G, 2 * g + 1>(xt, de, i);
+}
+template <int N, int G, int g>
+__device__ __forceinline__ void word_dual(const int (&xt)[N], const int* __restrict__ de, int i, int m, long long& W,
+                                          long long& Q)
+{
+    int pa, qa;
+    half_any<N, G, 2 * g>(xt, de, i, m, pa, qa);
+    if constexpr (rows_in_half(N, 2 * g + 1) == 0) {
+        W = pa;
+        Q = qa;
+    } else {
+        int pb, qb;
+        if (m > (2 * g + 1) * half_rows(N)) {
+            half_any<N, G, 2 * g + 1>(xt, de, i, m, pb, qb);
+            // at most 2K (n-1)^(2K-1) < 2^63: 2K <= n rows, (n-1)^(2K) < 2^62
+            Q = (long long)qa * pb + (long long)pa * qb;
+        } else {
+            pb = half_plain<N, G, 2 * g + 1>(xt, de, i);
+            Q = (long long)qa * pb;
+        }
+        W = (long long)pa * pb;
+    }
+}
+
+__device__ __forceinline__ unsigned long long magnitude(long long v, uint32_t& sg)
+{
+    const long long s = v >> 63;
+    sg ^= (uint32_t)s;
+    return (unsigned long long)((v ^ s) - s);
+}
+
+// p (nb limbs) times w, into min(nb + 2, L) limbs (mod 2^(32L)).
+template <int L, int nb>
+__device__ __forceinline__ void fold64(uint32_t (&p)[L], unsigned long long w)
+{
+    const uint32_t w0 = (uint32_t)w, w1 = (uint32_t)(w >> 32);
+    uint32_t r[L];
+    uint64_t c = 0;
+#pragma unroll
+    for (int l = 0; l < nb; ++l) {
+        const uint64_t t = (uint64_t)p[l] * w0 + c;
+        r[l] = (uint32_t)t;
+        c = t >> 32;
+    }
+    if constexpr (nb < L) r[nb] = (uint32_t)c;
+    c = 0;
+#pragma unroll
+    for (int l = 0; l < nb && l + 1 < L; ++l) {
+        const uint64_t t = (uint64_t)p[l] * w1 + r[l + 1] + c;
+        r[l + 1] = (uint32_t)t;
+        c = t >> 32;
+    }
+    if constexpr (nb + 1 < L) r[nb + 1] = (uint32_t)c;
+#pragma unroll
+    for (int l = 0; l < nb + 2 && l < L; ++l) p[l] = r[l];
+}
+
+// Words g, g+1, ... of a term, none with rows of the expanded column.
+template <int N, int L, int G, int g>
+__device__ __forceinline__ void plain_words(const int (&xt)[N], const int* __restrict__ de, int i,
+                                            uint32_t (&p)[L], uint32_t& sg)
+{
+    if constexpr (rows_in_half(N, 2 * g) > 0) {
+        fold64<L, expand_limbs_after(N, g - 1, L)>(p, magnitude(word_plain<N, G, g>(xt, de, i), sg));
+        plain_words<N, L, G, g + 1>(xt, de, i, p, sg);
+    }
+}
+
+// |sum_{r < m} prod_{r' != r} x'_r'| mod 2^(32L) for one term into p; returns
+// a word whose bit 31 is its sign.  1 <= m <= kExpandHalves * K.  The branches
+// on m are the same for every thread of the grid.
+template <int N, int L, int G>
+__device__ __forceinline__ uint32_t term_expanded(const int (&xt)[N], const int* __restrict__ de, int i, int m,
+                                                  uint32_t (&p)[L])
+{
+#pragma unroll
+    for (int l = 0; l < L; ++l) p[l] = 0u;
+    uint32_t sg = 0u;
+    long long W0, Q0;
+    word_dual<N, G, 0>(xt, de, i, m, W0, Q0);
+    if constexpr (rows_in_half(N, 2) > 0) {
+        if (m > 2 * half_rows(N)) {
+            long long W1, Q1;
+            word_dual<N, G, 1>(xt, de, i, m, W1, Q1);
+            // Q0 W1 + W0 Q1, signed 128 bits (4K rows below (2^31)^4)
+            const unsigned long long a = (unsigned long long)Q0 * (unsigned long long)W1;
+            const unsigned long long b = (unsigned long long)W0 * (unsigned long long)Q1;
+            const unsigned long long lo = a + b;
+            const long long hi = (long long)((unsigned long long)__mul64hi(Q0, W1) +
+                                             (unsigned long long)__mul64hi(W0, Q1) + (lo < a ? 1ull : 0ull));
+            const unsigned long long s = (unsigned long long)(hi >> 63);
+            sg ^= (uint32_t)s;
+            const unsigned long long l0 = (lo ^ s) - s, h0 = ((unsigned long long)hi ^ s) + (s && l0 == 0 ? 1ull : 0ull);
+            p[0] = (uint32_t)l0;
+            p[1] = (uint32_t)(l0 >> 32);
+            p[2] = (uint32_t)h0;
+            p[3] = (uint32_t)(h0 >> 32);
+        } else {
+            const unsigned long long q = magnitude(Q0, sg);
+            p[0] = (uint32_t)q;
+            p[1] = (uint32_t)(q >> 32);
+            fold64<L, 2>(p, magnitude(word_plain<N, G, 1>(xt, de, i), sg));
+        }
+    } else {
+        const unsigned long long q = magnitude(Q0, sg);
+        p[0] = (uint32_t)q;
+        p[1] = (uint32_t)(q >> 32);
+    }
+    plain_words<N, L, G, 2>(xt, de, i, p, sg);
+    return sg;
+}
+
+// Sum over one unit: sum_d (-1)^popc(d) prod_r (xt_r + DEI[d][r]), or with X
+// the expanded walk's terms.
+template <int N, int L, bool X>
+__device__ __forceinline__ void unit_sum_bin(const int (&xt)[N], const int* __restrict__ s_de, int nq, int m,
                                              uint32_t (&acc)[L])
 {
     constexpr int G = 4;
+    auto term = [&](const int* de, int i, uint32_t (&p)[L]) {
+        if constexpr (X) return term_expanded<N, L, G>(xt, de, i, m, p);
+        else return term_product<N, L, G>(xt, de, i, p);
+    };
 #pragma unroll
     for (int l = 0; l < L; ++l) acc[l] = 0u;
 #pragma unroll 1
@@ -195,13 +412,13 @@ __device__ __forceinline__ void unit_sum_bin(const int (&xt)[N], const int* __re
         // pattern + - - + relative to popc(q); an all-ones mask subtracts
         const uint32_t flip = (__popc(q) & 1) ? 0x80000000u : 0u;
         uint32_t p[L];
-        uint32_t sg = term_product<N, L, G>(xt, de, 0, p);
+        uint32_t sg = term(de, 0, p);
         limb_add_masked<L>(acc, p, (uint32_t)((int32_t)(sg ^ flip) >> 31));
-        sg = term_product<N, L, G>(xt, de, 1, p);
+        sg = term(de, 1, p);
         limb_add_masked<L>(acc, p, (uint32_t)((int32_t)(sg ^ flip ^ 0x80000000u) >> 31));
-        sg = term_product<N, L, G>(xt, de, 2, p);
+        sg = term(de, 2, p);
         limb_add_masked<L>(acc, p, (uint32_t)((int32_t)(sg ^ flip ^ 0x80000000u) >> 31));
-        sg = term_product<N, L, G>(xt, de, 3, p);
+        sg = term(de, 3, p);
         limb_add_masked<L>(acc, p, (uint32_t)((int32_t)(sg ^ flip) >> 31));
     }
 }
@@ -215,16 +432,22 @@ __device__ __forceinline__ void shfl_add(uint32_t (&v)[L], int m)
     limb_add<L>(v, o);
 }
 
-// Threads per CTA: 512 (128 registers) keeps 4 limbs spill-free up to
-// n = 28; larger n or more limbs get 255 registers at 256 threads.
-__host__ __device__ constexpr int bin_max_threads(int n, int limbs) { return (limbs <= 4 && n <= 28) ? 512 : 256; }
+// Threads per CTA.  Plain walk: 512 (128 registers) keeps 4 limbs spill-free up
+// to n = 28; larger n or more limbs get 255 registers at 256 threads.  Expanded
+// walk, which holds fewer limbs at a time: 512 up to n = 36 (126 registers at
+// n = 36 with 5 limbs), 384 (168 registers) up to n = 44, then 256.
+__host__ __device__ constexpr int bin_max_threads(int n, int limbs, bool x)
+{
+    if (x) return n <= 36 ? 512 : (n <= 44 ? 384 : 256);
+    return (limbs <= 4 && n <= 28) ? 512 : 256;
+}
 
-template <int N, int L>
-__global__ void __launch_bounds__(bin_max_threads(N, L), 1) walk_binary(Problem pb)
+template <int N, int L, bool X>
+__global__ void __launch_bounds__(bin_max_threads(N, L, X), 1) walk_binary(Problem pb)
 {
     constexpr int G = 4;
     extern __shared__ __align__(16) int smem_i[];
-    const int w = pb.w, terms = 1 << w, nq = terms / G, ntop = N - 1 - w;
+    const int w = pb.w, terms = 1 << w, nq = terms / G, ntop = N - 1 - (X ? 1 : 0) - w;
     const int tid = threadIdx.x, bd = blockDim.x;
     int* s_de = smem_i;
     int8_t* s_mt = reinterpret_cast<int8_t*>(s_de + terms * N);
@@ -252,7 +475,7 @@ __global__ void __launch_bounds__(bin_max_threads(N, L), 1) walk_binary(Problem 
         unsigned long long u = u0;
         while (true) {
             uint32_t us[L];
-            unit_sum_bin<N, L>(xt, s_de, nq, us);
+            unit_sum_bin<N, L, X>(xt, s_de, nq, X ? pb.m : 0, us);
             if (u & 1ull) limb_sub<L>(tot, us);
             else limb_add<L>(tot, us);
             if (++u >= u1) break;
@@ -309,7 +532,7 @@ __global__ void __launch_bounds__(bin_max_threads(N, L), 1) walk_binary(Problem 
     }
 }
 
-// Launches walk_binary<pb.n, pb.limbs>; with per_sm set, launches nothing
+// Launches walk_binary<pb.n, pb.limbs, pb.m > 0>; with per_sm set, launches nothing
 // and stores the CTAs per SM that the launch shape allows.
 int launch_binary(const Problem& pb, int blocks, int threads, size_t smem, cudaStream_t s, int* per_sm = nullptr);
 
