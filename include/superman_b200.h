@@ -62,7 +62,9 @@ enum spb_precision {
 
 /* Walk used by spb_perm_sparse_f64. */
 enum spb_sparse_walk {
-    SPB_SPARSE_WALK_AUTO = 0,   /* row-compacted walk when its cost model wins   */
+    SPB_SPARSE_WALK_AUTO = 0,   /* row-by-row expansion, row-compacted walk or
+                                   dense walk, by their cost models (the
+                                   expansion only with automatic launch shapes)  */
     SPB_SPARSE_WALK_NEVER = 1,  /* always the dense walk                         */
     SPB_SPARSE_WALK_ALWAYS = 2  /* row-compacted walk whenever the pattern allows */
 };
@@ -107,13 +109,16 @@ typedef struct spb_result {
                               input copy (if any), kernels, result copy     */
     double err_est;        /* estimated relative error (statistical); for
                               spb_perm_approx the relative standard error */
-    uint64_t gray_steps;   /* Gray steps walked, n*2^(n-1) (every walk is
-                              Nijenhuis-Wilf); spb_perm_approx: samples    */
+    uint64_t gray_steps;   /* Gray steps of the Nijenhuis-Wilf formula,
+                              n*2^(n-1), whichever way the call evaluates
+                              it; spb_perm_approx: samples                  */
     uint64_t refined_units;/* units re-evaluated in double-double           */
     int status;            /* enum spb_status                               */
     int launches;          /* kernels launched by the call                  */
     int active_rows;       /* rows varying inside a Gray unit: n for the
-                              dense walk, fewer for the row-compacted walk  */
+                              dense walk, fewer for the row-compacted walk;
+                              for the row-by-row expansion the most columns
+                              open at a time                                */
 } spb_result;
 
 /* Fills *opt with the defaults (device 0, SPB_PREC_FP64, automatic shape). */
@@ -137,8 +142,9 @@ SPB_API int spb_device_count(void);
  * (Algorithms/GPU/Dense/dpSingleGPU.cuh:45-219) and its kernels
  * xRegisterMShared[Kahan] (Algorithms/GPU/Dense/DenseKernelDefinitions.cuh:
  * 189-264, 331-405).  a: n*n doubles, row-major.  A matrix with zeros may
- * run on the row-compacted walk of spb_perm_sparse_f64 when its cost model
- * wins (opt->sparse_walk; out->active_rows < n then). */
+ * run on the row-by-row expansion or the row-compacted walk of
+ * spb_perm_sparse_f64 when its cost model wins (opt->sparse_walk;
+ * out->active_rows < n then). */
 SPB_API int spb_perm_dense_f64(const double* a, int n, const spb_options* opt, spb_result* out);
 
 /* Sparse real permanent from compressed-column arrays, the layout of the
@@ -150,12 +156,16 @@ SPB_API int spb_perm_dense_f64(const double* a, int n, const spb_options* opt, s
  * per-matrix generated kernels (Algorithms/GPU/CodeGeneration/
  * KernelGenerator.cuh:114-176): rows and columns are permuted so that the
  * rows varying inside a Gray unit are few, and a walk compiled for that row
- * count runs (opt->sparse_walk; out->active_rows reports it). */
+ * count runs (opt->sparse_walk; out->active_rows reports it).  Where few columns
+ * are open at a time, i.e. have nonzeros both in rows already taken and in
+ * rows still to come, the permanent is instead expanded row by row over the
+ * sets of open columns, in double-double whatever opt->precision says. */
 SPB_API int spb_perm_sparse_f64(const int* cptrs, const int* rows, const double* cvals, int n,
                                 const spb_options* opt, spb_result* out);
 
-/* The plan spb_perm_sparse_f64 would run for a row-major n x n matrix under
- * sparse_walk `mode`, without running it: *na active rows (n = the dense
+/* The walk spb_perm_sparse_f64 would plan for a row-major n x n matrix under
+ * sparse_walk `mode` (whether or not the expansion takes its place), without
+ * running it: *na active rows (n = the dense
  * walk), *w low columns, and the row and column orders (new position ->
  * original index; either may be NULL).  In the permuted matrix rows
  * na..n-1 are zero in columns 0..w-1.  CPU only. */
@@ -208,10 +218,12 @@ SPB_API int spb_perm_dense_c128_dev(const double* d_a, int n, const spb_options*
 SPB_API int spb_perm_batch_dev(const double* d_mats, int n, int is_complex, int count,
                                double* d_out, void* stream);
 
-/* Exact permanent of a 0/1 matrix (a: n*n bytes, row-major, nonzero = 1) by
- * plain Ryser over all 2^n column subsets in wrap-around integer arithmetic
- * whose width (128, 192 or 320 bits) is chosen from a Bregman-Minc bound, so
- * the result is exact for every n <= 63.  limbs receives the permanent as a
+/* Exact permanent of a 0/1 matrix (a: n*n bytes, row-major, nonzero = 1): the
+ * line with the fewest ones is expanded and one Nijenhuis-Wilf walk over the
+ * other lines' 2^(n-2) subsets evaluates all its minors (where that line has
+ * too many ones, a walk over 2^(n-1) subsets of the whole matrix), in
+ * wrap-around integer arithmetic whose width (128 to 384 bits) is chosen from
+ * a Bregman-Minc bound, so the result is exact for every n <= 63.  limbs receives the permanent as a
  * 320-bit two's-complement integer in ten little-endian 32-bit words;
  * out->value is its nearest double.  Replaces the reference's 0/1 handling,
  * which reads the pattern (IO/IO.h:441-443) and runs the FP64 dense path

@@ -16,6 +16,9 @@
 // the low columns' support enter once per unit.  A cost model picks w (the
 // number of low columns) and whether the compacted walk beats the dense walk
 // at all; otherwise the dense walk runs.
+//
+// Before either walk, the automatic choice plans the row-by-row expansion
+// (frontier.cu) and runs it where its estimate is below any walk's.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -23,6 +26,7 @@
 
 #include "dense_host.h"
 #include "dense_launch.cuh"
+#include "frontier.h"
 #include "sparse_impl.cuh"
 
 namespace spb {
@@ -160,6 +164,38 @@ bool plan_compacted(const double* a, int n, int mode, const spb_options& opt, Ch
     return mode == SPB_SPARSE_WALK_ALWAYS || ch->cost < 0.8 * walk_cost(n, wd, n, 0.0, dd);
 }
 
+// Whether the row-by-row expansion can run, and its plan.  Only in the automatic
+// mode, with no launch shape or listing of the walks asked for, from n = 20 (the
+// size from which that mode looks for a compacted walk; below it a fused dense
+// call takes 20-40 us), and on finite entries: the walks turn any non-finite
+// entry into NaN, the expansion only those that a perfect matching uses.  A
+// zero column keeps the dense walk.
+bool plan_expansion(const double* a, int n, const spb_options& opt, frontier::Plan* plan)
+{
+    if (opt.sparse_walk != SPB_SPARSE_WALK_AUTO || n < 20 || n > kMaxN || opt.precision == SPB_PREC_FP32 ||
+        opt.unit_bits > 0 || opt.threads_per_block > 0 || opt.blocks > 0 || opt.replay_listing)
+        return false;
+    for (int c = 0; c < n; ++c) {
+        bool any = false;
+        for (int r = 0; r < n; ++r) {
+            if (!std::isfinite(a[(size_t)r * n + c])) return false;
+            any = any || a[(size_t)r * n + c] != 0.0;
+        }
+        if (!any) return false;
+    }
+    return frontier::make_plan(a, n, plan);
+}
+
+// Estimated wall time of the walk the automatic mode would take: FP64-pipe
+// operations at 1.3e13 a second, on top of what the call costs before its
+// first term (n=20: 132 us of wall time, 51 of them kernels, for the
+// row-compacted walk's five launches; 45 us for a fused dense call).
+double walk_seconds(int n, bool compacted, const Choice& ch)
+{
+    if (compacted) return 110e-6 + ch.cost / 1.3e13;
+    return (n <= 26 ? 40e-6 : 75e-6) + 1.5 * n * std::ldexp(1.0, n - 1) / 1.3e13;
+}
+
 }  // namespace
 
 int run_real_host(const double* a, int n, const spb_options* opt, spb_result* out, DeviceContext* ctx)
@@ -167,8 +203,20 @@ int run_real_host(const double* a, int n, const spb_options* opt, spb_result* ou
     if (a && n >= 1 && n <= kMaxN && opt->sparse_walk != SPB_SPARSE_WALK_NEVER) {
         bool has_zero = false;
         for (size_t i = 0; i < (size_t)n * n && !has_zero; ++i) has_zero = a[i] == 0.0;
+        // The expansion where it is the faster call: at once when it takes
+        // less than any walk's launches do, else by both estimates.
+        frontier::Plan fp;
+        const bool expand = has_zero && out && plan_expansion(a, n, *opt, &fp);
+        const double te = expand ? frontier::expansion_seconds(fp) + 20e-6 : INFINITY;
         Choice ch;
-        if (has_zero && plan_compacted(a, n, opt->sparse_walk, *opt, &ch)) {
+        const bool compacted = has_zero && te > 50e-6 && plan_compacted(a, n, opt->sparse_walk, *opt, &ch);
+        if (expand && (te <= 50e-6 || te < walk_seconds(n, compacted, ch))) {
+            std::memset(out, 0, sizeof(*out));
+            bool launched = false;
+            const int st = frontier::run(fp, opt, out, ctx, &launched);
+            if (st != SPB_OK || launched) return st;
+        }
+        if (compacted || (te <= 50e-6 && plan_compacted(a, n, opt->sparse_walk, *opt, &ch))) {
             std::vector<double> ap((size_t)n * n);
             for (int i = 0; i < n; ++i)
                 for (int j = 0; j < n; ++j) ap[(size_t)i * n + j] = a[(size_t)ch.rows[i] * n + ch.cols[j]];
