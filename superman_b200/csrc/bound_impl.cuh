@@ -10,7 +10,8 @@
 // f_r = |x_r + mid_r| + half_r with mid/half the centre and half-width of the
 // row's DE range, so the walk keeps y_r = x_r + mid_r.  Near a bin edge the
 // bin may differ from the walk's FP64 bin; that shifts the list length,
-// never the result.
+// never the result.  The derivative walk's bound sum_r prod_{r' != r} f_r' is
+// carried beside the product, both under the exponent of the larger.
 #pragma once
 
 #include "dense_impl.cuh"
@@ -42,12 +43,23 @@ __device__ __forceinline__ void bound_renorm(float& p, int& e)
     p = __int_as_float((bits & 0x007fffff) | 0x3f800000);
 }
 
+// Moves the binary exponent of q into e; q keeps [1, 2) and p is scaled alike.
+__device__ __forceinline__ void bound_renorm2(float& q, float& p, int& e)
+{
+    const int b = ((__float_as_int(q) >> 23) & 0xff) - 127;
+    e += b;
+    q = __int_as_float((__float_as_int(q) & 0x007fffff) | 0x3f800000);
+    p *= __int_as_float((127 - (b < 126 ? b : 126)) << 23);
+}
+
 template <int N, int C>
 __global__ void __launch_bounds__(256) bound_walk(Problem pb)
 {
+    const bool deriv = N >= (C == 1 ? kMinDerivReal : kMinDerivComplex) && deriv_on(pb);
+    if (eff_units(pb, deriv) <= pb.raw_cap / 2) return;  // every unit is listed (setup_kernel)
     extern __shared__ __align__(16) float fsm[];
     constexpr int S = bound_col_stride(N);
-    const int ntop = N - 1 - pb.w, ntp = ntop > 0 ? ntop : 0;
+    const int ntop = eff_ntop(pb, deriv), ntp = ntop > 0 ? ntop : 0;
     const int tid = threadIdx.x, bd = blockDim.x, lane = tid & 31;
     float* s_mt = fsm;                   // [C][ntop][S], rows 0..N-1 used
     float* s_b = s_mt + C * ntp * S;     // real [2][N] (mid, half), complex [N] (max |DE|)
@@ -67,7 +79,7 @@ __global__ void __launch_bounds__(256) bound_walk(Problem pb)
     const unsigned long long T = (unsigned long long)gridDim.x * bd;
     const unsigned long long t = (unsigned long long)blockIdx.x * bd + tid;
     unsigned long long u0, u1;
-    balanced_range(pb.units, T, t, &u0, &u1);
+    balanced_range(eff_units(pb, deriv), T, t, &u0, &u1);
     float x[C][N], hb[N];
     const unsigned long long g0 = gray_of(u0);
 #pragma unroll
@@ -92,7 +104,7 @@ __global__ void __launch_bounds__(256) bound_walk(Problem pb)
 #pragma unroll
                 for (int r = 0; r < N; ++r) x[c][r] = fmaf(sg, s_mt[(c * ntp + j) * S + r], x[c][r]);
         }
-        float p = 1.0f;
+        float p = 1.0f, q = 0.0f;
         int e = 0;
 #pragma unroll
         for (int r = 0; r < N; ++r) {
@@ -102,10 +114,16 @@ __global__ void __launch_bounds__(256) bound_walk(Problem pb)
                 const float m2 = fmaxf(fmaf(x[0][r], x[0][r], x[C - 1][r] * x[C - 1][r]), 0x1p-100f);
                 f = m2 * rsqrtf(m2) + hb[r];  // |x| to a few ulps: an estimate
             }
-            p *= fminf(fmaxf(f, 0x1p-24f), 0x1p24f);
-            if ((r & 3) == 3) bound_renorm(p, e);
+            f = fminf(fmaxf(f, 0x1p-24f), 0x1p24f);
+            if (deriv) q = fmaf(q, f, p);
+            p *= f;
+            if ((r & 3) == 3) {
+                if (deriv) bound_renorm2(q, p, e);
+                else bound_renorm(p, e);
+            }
         }
-        bound_renorm(p, e);
+        if (deriv) bound_renorm2(q, p, e);
+        else bound_renorm(p, e);
         int b = (e + 1024) >> 2;  // e = floor(log2 U), as ilogb in hist_bin
         b = b < 0 ? 0 : (b >= kHistBins ? kHistBins - 1 : b);
         const unsigned same = __match_any_sync(__activemask(), b);

@@ -42,8 +42,10 @@ namespace dense {
 // ------------------------------------------------------------ setup kernel --
 // Builds every table the walk kernels read, one CTA per row r (every value
 // below depends on its own row only, apart from the exponent sum, which
-// CTA 0 adds up).  Row r is staged in shared memory (CTA 0 stages the whole
-// matrix, n*n*comps doubles, for the exponents of every row).
+// CTA 0 adds up, and the pivot column).  Row r is staged in shared memory
+// (CTA 0, and every CTA of a call that may run the derivative walk, stages the
+// whole matrix, n*n*comps doubles: each picks the pivot column by itself, with
+// the same operations, rather than waiting for another).
 // Per part, one warp builds the row's subset sums DE[d][r] level by level
 // behind warp barriers (in shared memory with smem_tables, else in place in
 // the global table), another forms the NW start value, and the CTA then
@@ -55,12 +57,14 @@ __global__ void __launch_bounds__(128) setup_kernel(Problem pb, const double* __
     const int tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, wid = tid >> 5, r = blockIdx.x;
     const int terms = 1 << w;
     __shared__ int s_eall[kMaxN];
-    // CTA 0 stages the whole matrix (it also adds up every row's exponent),
-    // the others their row: row r is s_row[0 .. n*c) either way
-    extern __shared__ __align__(16) double s_row[];  // [rows][n][c], scaled after step 1; then [c][terms] hi, lo
-    double* th = s_row + ((n * n * c + 1) & ~1);
+    __shared__ double s_qh[2 * kMaxN], s_ql[2 * kMaxN];  // the row's walked columns, [column][c]
+    __shared__ int s_pivot;
+    extern __shared__ __align__(16) double s_mat[];  // [rows][n][c], scaled after step 1; then [c][terms] hi, lo
+    double* th = s_mat + ((n * n * c + 1) & ~1);
     double* tl = th + (size_t)c * terms;
-    const int nst = r == 0 ? n : 1;
+    const bool whole = r == 0 || pb.deriv != 0;
+    const int nst = whole ? n : 1, own = whole ? r : 0;
+    double* s_row = s_mat + (size_t)own * n * c;
 
     // 0. What the later kernels of the call accumulate into starts at zero.
     if (r == 0) {
@@ -72,49 +76,90 @@ __global__ void __launch_bounds__(128) setup_kernel(Problem pb, const double* __
                 pb.hist_cnt[i] = 0ull;
                 pb.pre_cnt[i] = 0u;
             }
-            if (tid == 0) {
-                *pb.raw_n = 0ull;
-                *pb.list_bin = pb.list_bin_init;
-            }
+            if (tid == 0) *pb.raw_n = 0ull;
         }
     }
-    for (int i = tid; i < nst * n * c; i += bd) s_row[i] = a_in[(size_t)r * n * c + i];
+    for (int i = tid; i < nst * n * c; i += bd) s_mat[i] = a_in[(size_t)(whole ? 0 : r) * n * c + i];
     __syncthreads();
     // 1. Row exponents: scale row q by 2^-e_q so that its largest |a_qj| lies
     //    in [0.5, 1); a warp per staged row (fmax does not depend on the
     //    order).  CTA 0 writes their sum.
     for (int q = wid; q < nst; q += bd >> 5) {
         double mx = 0.0;
-        for (int j = lane; j < n * c; j += 32) mx = fmax(mx, fabs(s_row[q * n * c + j]));
+        for (int j = lane; j < n * c; j += 32) mx = fmax(mx, fabs(s_mat[q * n * c + j]));
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-        if (lane == 0) {
-            int e = 0;
-            if (mx > 0.0 && isfinite(mx)) frexp(mx, &e);
-            s_eall[q] = e;
-        }
+        int e = 0;
+        if (mx > 0.0 && isfinite(mx)) frexp(mx, &e);
+        if (lane == 0) s_eall[q] = e;
+        if (q != own && pb.deriv == 0) continue;
+        for (int j = lane; j < n * c; j += 32) s_mat[q * n * c + j] = ldexp(s_mat[q * n * c + j], -e);
     }
+    if (tid == 0) s_pivot = -1;
     __syncthreads();
-    if (r == 0 && wid == 0) {
+    if (r == 0 && wid == 1) {
         int es = 0;
         for (int q = lane; q < n; q += 32) es += s_eall[q];
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) es += __shfl_xor_sync(0xffffffffu, es, off);
         if (lane == 0) *pb.exp_sum = es;
     }
-    const int er = s_eall[0];
-    for (int i = tid; i < n * c; i += bd) {
-        const double v = ldexp(s_row[i], -er);
-        s_row[i] = v;
-        pb.as[(size_t)r * n * c + i] = v;
+    if (pb.deriv != 0 && wid == 0) {
+        const int pv = c == 1 ? pick_pivot<1>(s_mat, n) : pick_pivot<2>(s_mat, n);
+        if (lane == 0) s_pivot = pv;
     }
     __syncthreads();
+    const int pivot = s_pivot;
+    const bool deriv = pivot >= 0;
+    const int nc = n - (deriv ? 1 : 0);  // walked columns
+    // 2. The row's walked columns: its entries, or their quotients by the pivot.
+    for (int j = tid; j < nc; j += bd) {
+        const int src = deriv && j >= pivot ? j + 1 : j;
+        if (!deriv) {
+            for (int p = 0; p < c; ++p) {
+                s_qh[j * c + p] = s_row[src * c + p];
+                s_ql[j * c + p] = 0.0;
+            }
+        } else if (c == 1) {
+            const dd v = quotient(s_row[src], s_row[pivot]);
+            s_qh[j] = v.hi;
+            s_ql[j] = v.lo;
+        } else {
+            const ddc v = quotient_c(s_row[2 * src], s_row[2 * src + 1], s_row[2 * pivot], s_row[2 * pivot + 1]);
+            s_qh[2 * j] = v.re.hi;
+            s_ql[2 * j] = v.re.lo;
+            s_qh[2 * j + 1] = v.im.hi;
+            s_ql[2 * j + 1] = v.im.lo;
+        }
+    }
+    __syncthreads();
+    if (r == 0 && wid == 3) {
+        DerivScale sc{};
+        if (deriv) {
+            auto get = [&](int q) {
+                const double* d = s_mat + ((size_t)q * n + pivot) * c;
+                return make_double2(d[0], d[c - 1]);
+            };
+            sc = c == 1 ? deriv_scale<1>(n, get) : deriv_scale<2>(n, get);
+        }
+        if (lane == 0) {
+            pb.rb->pivot = pivot;
+            pb.rb->scale[0] = sc.v.re;
+            pb.rb->scale[1] = sc.v.im;
+            pb.rb->scale_exp = sc.e;
+            // the walk's list bin: 0 lists every unit when all fit the list;
+            // kListNone lists none (the row-compacted walk, whose refinement goes
+            // through the scan); with a bound pass pick_list_bin overwrites it
+            if (pb.mode != 0) *pb.list_bin = pb.na == n && eff_units(pb, deriv) <= pb.raw_cap / 2 ? 0 : kListNone;
+        }
+    }
+    auto plus = [&](dd x, int i) { return deriv ? dd_step(x, s_qh[i], s_ql[i]) : dd_add_d(x, s_qh[i]); };
     // entry d of row r, part p, in the global table [c][terms/G][n][G]
     auto gpos = [&](int p, int d) {
         return (size_t)p * terms * n + (size_t)(d / G) * n * G + (size_t)r * G + (d % G);
     };
     if (wid < c) {
-        // 3. Low-column subset sums of part p = wid: the double-double sum
+        // 4. Low-column subset sums of part p = wid: the double-double sum
         //    of the selected columns added in ascending order, level by
         //    level: with k the highest bit of d, DE[d] = DE[d - 2^k] + a_k.
         const int p = wid;
@@ -128,9 +173,8 @@ __global__ void __launch_bounds__(128) setup_kernel(Problem pb, const double* __
             for (int k = 0; k < w; ++k) {
                 __syncwarp();  // level k reads the entries of levels < k
                 const int half = 1 << k;
-                const double ak = s_row[k * c + p];
                 for (int e = lane; e < half; e += 32) {
-                    const dd v = dd_add_d(dd{hh[e], ll[e]}, ak);
+                    const dd v = plus(dd{hh[e], ll[e]}, k * c + p);
                     hh[half + e] = v.hi;
                     ll[half + e] = v.lo;
                 }
@@ -143,38 +187,39 @@ __global__ void __launch_bounds__(128) setup_kernel(Problem pb, const double* __
             for (int k = 0; k < w; ++k) {
                 __syncwarp();
                 const int half = 1 << k;
-                const double ak = s_row[k * c + p];
                 for (int e = lane; e < half; e += 32) {
                     const size_t f = gpos(p, e), t = gpos(p, half + e);
-                    const dd v = dd_add_d(dd{pb.de_hi[f], pb.de_lo[f]}, ak);
+                    const dd v = plus(dd{pb.de_hi[f], pb.de_lo[f]}, k * c + p);
                     pb.de_hi[t] = v.hi;
                     pb.de_lo[t] = v.lo;
                 }
             }
         }
     } else if (wid == 2) {
-        // 2. NW start value in double-double: x0 = a'_{r,n-1} - rowsum'_r / 2.
+        // 3. NW start value in double-double: x0 = a'_{r,nc-1} - rowsum'_r / 2.
         if (lane < c) {
             const int p = lane;
             dd sm = {0.0, 0.0};
-            for (int j = 0; j < n; ++j) sm = dd_add_d(sm, s_row[j * c + p]);
+            for (int j = 0; j < nc; ++j) sm = plus(sm, j * c + p);
             dd h = {-0.5 * sm.hi, -0.5 * sm.lo};  // exact halving
-            dd x = dd_add_d(h, s_row[(n - 1) * c + p]);
+            dd x = plus(h, (nc - 1) * c + p);
             pb.x0_hi[p * n + r] = x.hi;
             pb.x0_lo[p * n + r] = x.lo;
         }
     } else if (wid == 3) {
-        // 4. High columns, column-major: mt[part][j][r] = a'_{r, w+j}.
-        const int ntop = n - 1 - w;
+        // 5. High columns, column-major: mt[part][j][r] = a'_{r, w+j}.
+        const int ntop = nc - 1 - w;
         for (int i = lane; i < ntop * c; i += 32) {
             const int p = i / ntop, j = i % ntop;
-            pb.mt[((size_t)p * ntop + j) * n + r] = s_row[(w + j) * c + p];
+            const size_t t = ((size_t)p * ntop + j) * n + r;
+            pb.mt[t] = s_qh[(w + j) * c + p];
+            if (deriv) pb.mt_lo[t] = s_ql[(w + j) * c + p];
         }
         // real row bound [sum_j min(0,a'_rj), sum_j max(0,a'_rj)] over the low columns
         if (c == 1 && lane == 0) {
             double lo = 0.0, hi = 0.0;
             for (int j = 0; j < w; ++j) {
-                const double v = s_row[j];
+                const double v = s_qh[j];
                 if (v < 0.0) lo += v; else hi += v;
             }
             pb.bnd[r] = lo;
@@ -278,7 +323,8 @@ int group_size(int n, int comps)
     return ComplexGroup(n);
 }
 
-int choose_unit_bits(int n, int comps, const spb_options* opt)
+// bits: walked columns less one, n-1 or, for the derivative walk, n-2.
+int choose_unit_bits(int n, int comps, const spb_options* opt, int bits)
 {
     int w;
     if (opt && opt->unit_bits > 0) {
@@ -287,13 +333,29 @@ int choose_unit_bits(int n, int comps, const spb_options* opt)
         // Table budget 64 KB per part; keep >= 2^16 units when n allows.
         w = 8;
         while (w > 2 && ((size_t)1 << w) * n * 8 * comps > (size_t)64 * 1024) --w;
-        while (w > 2 && (n - 1 - w) < 16 && w > (n - 1) - 16) --w;
+        while (w > 2 && bits - w < 16) --w;
     }
     if (w > n - 1) w = n - 1;
     const int g = group_size(n, comps);
     const int wmin = g == 4 ? 2 : (g == 2 ? 1 : 0);
     if (w < wmin) w = wmin;
     return w;
+}
+
+int choose_unit_bits(int n, int comps, const spb_options* opt) { return choose_unit_bits(n, comps, opt, n - 1); }
+
+// Whether the derivative walk may run, and the unit width to go with it: on
+// dense matrices of its sizes, where the units leave it a column to expand, and
+// not with FP32 products (n=27 complex 592 -> 541 us, but the error of a Haar
+// block against exact went from 2.6e-6 to 6.2e-6).  The setup kernel decides by the matrix (rb->pivot); `hint` false
+// (a host matrix known to have a zero in every column) only sizes the units
+// for the plain walk, which then runs.
+void choose_walk(Problem* pb, const spb_options* opt, bool hint)
+{
+    const int n = pb->n;
+    pb->deriv = pb->na == n && !pb->f32 && n >= (pb->comps == 1 ? kMinDerivReal : kMinDerivComplex) ? 1 : 0;
+    pb->w = choose_unit_bits(n, pb->comps, opt, n - 1 - (pb->deriv && hint ? 1 : 0));
+    if (pb->w > n - 2) pb->deriv = 0;
 }
 
 // Sizes the scratch arena and fills the device pointers of *pb.
@@ -307,7 +369,6 @@ size_t plan_layout(Problem* pb, char* base, size_t* in_offset)
         return o;
     };
     size_t o_in = take(sizeof(double) * n * n * c);
-    size_t o_as = take(sizeof(double) * n * n * c);
     size_t o_x0h = take(sizeof(double) * n * c);
     size_t o_x0l = take(sizeof(double) * n * c);
     size_t terms = (size_t)1 << pb->w;
@@ -315,7 +376,9 @@ size_t plan_layout(Problem* pb, char* base, size_t* in_offset)
     size_t o_del = take(sizeof(double) * terms * n * c);
     const bool f32 = pb->f32 != 0;
     size_t o_d32 = f32 ? take(sizeof(float) * terms * n * c) : 0;
-    size_t o_mt = take(sizeof(double) * (size_t)(n - 1 - pb->w > 0 ? n - 1 - pb->w : 1) * n * c);
+    const size_t top = (size_t)(n - 1 - pb->w > 0 ? n - 1 - pb->w : 1) * n * c;
+    size_t o_mt = take(sizeof(double) * top);
+    size_t o_ml = pb->deriv ? take(sizeof(double) * top) : 0;
     // two per CTA at least: the fused small call keeps its walk totals and its
     // corrections apart
     size_t o_part = take(sizeof(dd) * (size_t)pb->grid * (c > 2 ? c : 2));
@@ -343,13 +406,13 @@ size_t plan_layout(Problem* pb, char* base, size_t* in_offset)
         pb->bnd = reinterpret_cast<double*>(base + o_bnd);
         pb->hist_s2 = reinterpret_cast<double*>(base + o_hs);
         pb->hist_cnt = reinterpret_cast<unsigned long long*>(base + o_hc);
-        pb->as = reinterpret_cast<double*>(base + o_as);
         pb->x0_hi = reinterpret_cast<double*>(base + o_x0h);
         pb->x0_lo = reinterpret_cast<double*>(base + o_x0l);
         pb->de_hi = reinterpret_cast<double*>(base + o_deh);
         pb->de_lo = reinterpret_cast<double*>(base + o_del);
         pb->de32 = f32 ? reinterpret_cast<float*>(base + o_d32) : nullptr;
         pb->mt = reinterpret_cast<double*>(base + o_mt);
+        pb->mt_lo = pb->deriv ? reinterpret_cast<double*>(base + o_ml) : nullptr;
         pb->partials = reinterpret_cast<dd*>(base + o_part);
         pb->ticket = reinterpret_cast<unsigned*>(base + o_tick);
         pb->rb = reinterpret_cast<Readback*>(base + o_rbk);
@@ -366,7 +429,10 @@ size_t walk_smem_bytes(const Problem& pb, int threads)
     const int n = pb.n, c = pb.comps;
     if (pb.na < n) return sparse_smem_bytes(n, pb.na, pb.w, threads);
     size_t terms = (size_t)1 << pb.w;
+    // high columns: n-1-w, or with the derivative walk n-2-w with their low
+    // words; the call must fit whichever walk the matrix gets
     int ntop = n - 1 - pb.w;
+    if (pb.deriv && 2 * (ntop - 1) > ntop) ntop = 2 * (ntop - 1);
     return sizeof(double) * (terms * n * c + (size_t)(ntop > 0 ? ntop : 0) * n * c +
                              (size_t)n * c * threads) +
            kHistSmemBytes + bound_smem_bytes(n);
@@ -398,7 +464,6 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
     pb.n = n;
     pb.na = n;
     pb.comps = comps;
-    pb.w = choose_unit_bits(n, comps, &opt);
     if (opt.precision == SPB_PREC_FP32) {
         if (n > kMaxF32N || n < 3) {
             spb_set_error("FP32 products are offered for 3 <= n <= %d (got n=%d)", kMaxF32N, n);
@@ -407,6 +472,19 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
         pb.f32 = 1;
         plan = nullptr;  // the FP32 variant is the dense walk
     }
+    // a host matrix tells whether a column without zeros, a pivot, can exist
+    bool hint = true;
+    if (!a_on_device) {
+        hint = false;
+        for (int j = 0; j < n && !hint; ++j) {
+            hint = true;
+            for (int r = 0; r < n && hint; ++r) {
+                const double* e = a + ((size_t)r * n + j) * comps;
+                hint = e[0] != 0.0 || e[comps - 1] != 0.0;
+            }
+        }
+    }
+    choose_walk(&pb, &opt, hint);
     if (plan && plan->na < n) {
         if (comps != 1 || plan->na < 1 || plan->na > kMaxActive || plan->w < 2 || plan->w > n - 2) {
             spb_set_error("row-compacted walk: bad plan (n=%d, active rows %d, w=%d)", n, plan->na, plan->w);
@@ -414,9 +492,12 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
         }
         pb.na = plan->na;
         pb.w = plan->w;
+        pb.deriv = 0;
     }
     pb.g = group_size(n, comps);
     pb.units = 1ull << (n - 1 - pb.w);
+    // the units the launch is shaped for: half of them in the derivative walk
+    const unsigned long long units = pb.deriv && hint ? pb.units >> 1 : pb.units;
 
     auto smem_for = [&](int th) { return pb.f32 ? walk_f32_smem_bytes(pb, th) : walk_smem_bytes(pb, th); };
     int threads = opt.threads_per_block > 0 ? opt.threads_per_block : 0;
@@ -435,14 +516,14 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
         return out->status = SPB_ERR_INVALID;
     }
     // The fused small call (below) walks with fewer threads per CTA on every
-    // SM when the units would leave SMs idle at full CTAs (n = 19 .. 25:
-    // 2^15 or 2^16 units fill 64 or 128 CTAs of 512 threads; 147 CTAs of 448
-    // threads give each SM an eighth less to walk).
+    // SM when the units would leave SMs idle at full CTAs (n = 20 .. 26:
+    // 2^16 units fill 128 CTAs of 512 threads; 147 CTAs of 448 threads give
+    // each SM an eighth less to walk).
     const bool small_candidate = opt.small_call >= 0 && comps == 1 && pb.na == n && !pb.f32 && n >= 4 &&
                                  n <= kSmallCallMaxN && !opt.replay_listing;
     if (small_candidate && opt.threads_per_block <= 0 && opt.blocks <= 0) {
-        if (pb.units >= 256ull * (unsigned long long)ctx->sm_count) {
-            const unsigned long long per_sm = (pb.units + ctx->sm_count - 1) / ctx->sm_count;
+        if (units >= 256ull * (unsigned long long)ctx->sm_count) {
+            const unsigned long long per_sm = (units + ctx->sm_count - 1) / ctx->sm_count;
             const int t = (int)((per_sm + 31) / 32 * 32);
             if (t <= threads) threads = t;
         }
@@ -453,7 +534,7 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
     }
     int blocks = opt.blocks > 0 ? opt.blocks : ctx->sm_count;
     // never launch more threads than units
-    unsigned long long max_blocks = (pb.units + threads - 1) / threads;
+    unsigned long long max_blocks = (units + threads - 1) / threads;
     if ((unsigned long long)blocks > max_blocks) blocks = (int)max_blocks;
     if (blocks < 1) blocks = 1;
     pb.grid = blocks;
@@ -557,12 +638,6 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
     // after a replayed fused call whose count check failed, the call's device
     // span is timed from here (the graph records no ev_call0)
     if (graphed) SPB_CUDA_TRY(cudaEventRecord(ctx->ev_call0, stream));
-    // The walk's list bin, written by the setup kernel (which also zeroes the
-    // counters and histograms): 0 lists every unit when all fit the list;
-    // 0x7f7f7f7f, above every bin, lists none (the row-compacted walk, whose
-    // refinement goes through the scan); with a bound pass pick_list_bin
-    // overwrites it.
-    pb.list_bin_init = (pb.na == n && pb.units <= pb.raw_cap / 2) ? 0 : 0x7f7f7f7f;
     if ((st = launch_setup(pb, d_a, stream)) != SPB_OK) return out->status = st;
     SPB_CUDA_TRY(cudaGetLastError());
     SPB_CUDA_TRY(cudaEventRecord(ctx->ev_begin, stream));
@@ -686,9 +761,23 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
         }
     }
 
-    // perm = (4(n%2)-2) * total * 2^E ; the factor is +-2, an exact power of two.
-    const int e = exp_sum + 1;
-    const double sgn = (n % 2) ? 1.0 : -1.0;
+    // perm = (4(nc%2)-2) * total * 2^E over nc walked columns; the factor is
+    // +-2, an exact power of two.  The derivative walk's total is multiplied
+    // by the product of the pivots.
+    const bool deriv = hrb->pivot >= 0;
+    int e = exp_sum + 1;
+    if (deriv) {
+        const dd sr = hrb->scale[0], si = hrb->scale[1];
+        if (comps == 1) {
+            res[0] = dd_mul(res[0], sr);
+        } else {
+            const dd re = dd_add(dd_mul(res[0], sr), dd_neg(dd_mul(res[1], si)));
+            res[1] = dd_add(dd_mul(res[0], si), dd_mul(res[1], sr));
+            res[0] = re;
+        }
+        e += hrb->scale_exp;
+    }
+    const double sgn = ((n - (deriv ? 1 : 0)) % 2) ? 1.0 : -1.0;
     out->value = sgn * std::ldexp(res[0].hi, e);
     out->value_lo = sgn * std::ldexp(res[0].lo, e);
     if (comps == 2) {

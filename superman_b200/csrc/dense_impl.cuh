@@ -10,6 +10,11 @@ namespace spb {
 namespace dense {
 
 constexpr int kMaxN = 63;
+// Smallest n of the derivative walk in whole-GPU calls.  Below, picking the
+// pivot and dividing by it cost the call more than the walk saves (FP64 calls
+// on one B200, plain against derivative: real n=20 43.6 and 47.1 us, n=22 51.0 and
+// 52.0, n=24 75.5 and 70.5; complex n=21 95.4 and 97.4, n=23 133.5 and 130.9).
+constexpr int kMinDerivReal = 23, kMinDerivComplex = 22;
 
 // Everything the host reads back after a call, contiguous so that one copy
 // brings it over: a call costs one host round trip, the double-double
@@ -24,6 +29,9 @@ struct Readback {
     int thr;                    // refinement bin
     int from_list;              // 1: the walk's own list holds every unit at or above thr
     int exp_sum;                // sum of the row scaling exponents
+    int pivot;                  // derivative walk: the column the rows are divided by; -1: plain walk
+    dd scale[2];                // derivative walk: [comps] product of the pivots' mantissas
+    int scale_exp;              // and the sum of their exponents
     int pad;
 };
 
@@ -33,15 +41,18 @@ struct Problem {
     int n, comps, w, g, grid, threads;
     int na;                    // rows that vary within a unit: n (dense walk) or the
                                // active rows of the row-compacted walk (sparse_impl.cuh)
-    unsigned long long units;  // 2^(n-1-w) Gray units of 2^w terms each
-    double* as;                // row-scaled matrix (row-major, comps interleaved)
+    unsigned long long units;  // 2^(n-1-w) Gray units of 2^w terms each (the derivative walk
+                               // takes half of them, eff_units)
+    int deriv;                 // 1: the derivative walk runs if the matrix has a pivot column
+                               // (rb->pivot, set by the setup kernel); 0: the plain walk
     double* x0_hi;             // [comps][n] NW start vector, double-double
     double* x0_lo;
     double* de_hi;             // [comps][2^w/G][n][G] low-column subset sums
     double* de_lo;             // rounding residues of de_hi
     float* de32;               // SPB_PREC_FP32: de_hi rounded to float (else null)
     int f32;                   // 1: the FP32-product walk runs (tables include de32)
-    double* mt;                // [comps][n-1-w][n] high columns
+    double* mt;                // [comps][ntop][n] high columns
+    double* mt_lo;             // their low words (derivative walk)
     dd* partials;              // [comps][grid] per-CTA sums
     unsigned* ticket;          // last-CTA election counter (reset by the kernel)
     dd* result;                // [comps] grid total (rb->res; rb->corr for the refinement)
@@ -64,7 +75,6 @@ struct Problem {
     // raw_cap, and the walk appends every unit at or above it (raw_*).
     unsigned* pre_cnt;             // [kHistBins]
     int* list_bin;
-    int list_bin_init;             // written to *list_bin by setup_kernel (pick_list_bin may overwrite it)
     unsigned long long* raw_n;
     unsigned long long raw_cap;
     unsigned long long* raw_u;     // [raw_cap] unit index
@@ -81,6 +91,150 @@ struct Problem {
 // costs the walk an append.
 constexpr unsigned long long kRawCap = 1ull << 21;
 constexpr unsigned long long kRawTarget = 1ull << 14;
+constexpr int kListNone = 0x7f7f7f7f;  // a list bin above every bin
+
+// Derivative walk.  The permanent is linear in a column; expanded along
+// column c it is the sum over rows r of a_rc times the minor without r and c,
+// and one Nijenhuis-Wilf walk over the other n-1 columns (2^(n-2) subsets, half
+// of the plain walk's) evaluates all minors together: with every row divided
+// by its pivot a_rc,
+//   perm(A) = prod_r a_rc * (4((n-1)%2)-2) * sum_S (-1)^|S| q_S,
+//   q_S = sum_r prod_{r' != r} x_r'(S),
+// the derivative of prod_r (x_r + t) at t = 0.  The chain q <- q x + p, p <- p x
+// costs an add, a multiply and a fused multiply-add per row where the two
+// plain terms it stands for cost two adds and two multiplies: 3/4 of the FP64
+// instructions, with the same or a smaller rounding error.  The quotients are
+// kept in double-double wherever the plain walk holds exact entries (start
+// vector, subset sums, high columns).
+// Whether the derivative walk runs; the same for every thread of a call.
+__device__ __forceinline__ bool deriv_on(const Problem& pb) { return pb.deriv != 0 && pb.rb->pivot >= 0; }
+__device__ __forceinline__ int eff_ntop(const Problem& pb, bool deriv) { return pb.n - 1 - pb.w - (deriv ? 1 : 0); }
+__device__ __forceinline__ unsigned long long eff_units(const Problem& pb, bool deriv)
+{
+    return deriv ? pb.units >> 1 : pb.units;
+}
+
+// a + m, the sum normalised, low words added first: about 2^-105 off.
+__device__ __forceinline__ dd dd_step(dd a, double mh, double ml)
+{
+    const dd s = two_sum(a.hi, mh);
+    return fast_two_sum(s.hi, add_rn(s.lo, add_rn(a.lo, ml)));
+}
+
+// Pivot column of an n x n matrix whose rows are scaled to maxima in [0.5, 1);
+// mag(r, j) is entry (r, j)'s magnitude (complex: the larger of its parts).
+// The column whose smallest magnitude is largest; -1 when every column holds a
+// zero or a non-finite entry, or when dividing by the pivots could take products
+// of n row values out of the FP64 range (a row's absolute sum is below 2^7,
+// n <= 63; the exponents of those sums over the pivots are added up).  Called
+// by one full warp; every lane returns the same.
+template <class Mag>
+__device__ __forceinline__ int pick_pivot(int n, Mag mag)
+{
+    const int lane = threadIdx.x & 31;
+    double best = 0.0;
+    int col = -1;
+    for (int j = lane; j < n; j += 32) {
+        double lo = INFINITY;
+        int bits = 0;
+        bool ok = true;
+        for (int r = 0; r < n; ++r) {
+            const double m = mag(r, j);
+            const int em = (__double2hiint(m) >> 20) & 0x7ff;
+            ok = ok && em != 0 && em != 0x7ff;
+            bits += 1023 + 8 - em;
+            lo = fmin(lo, m);
+        }
+        if (ok && bits <= 960 && lo > best) {
+            best = lo;
+            col = j;
+        }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const double b = __shfl_xor_sync(0xffffffffu, best, off);
+        const int c = __shfl_xor_sync(0xffffffffu, col, off);
+        if (b > best || (b == best && c >= 0 && (col < 0 || c < col))) {
+            best = b;
+            col = c;
+        }
+    }
+    return col;
+}
+// The same on a row-major array of scaled entries, COMPS interleaved.
+template <int COMPS>
+__device__ __forceinline__ int pick_pivot(const double* a, int n)
+{
+    return pick_pivot(n, [&](int r, int j) {
+        const double* e = a + ((size_t)r * n + j) * COMPS;
+        return COMPS == 1 ? fabs(e[0]) : fmax(fabs(e[0]), fabs(e[COMPS - 1]));
+    });
+}
+
+struct ddc {
+    dd re, im;
+};
+__device__ __forceinline__ ddc ddc_mul(ddc a, ddc b)
+{
+    return {dd_add(dd_mul(a.re, b.re), dd_neg(dd_mul(a.im, b.im))),
+            dd_add(dd_mul(a.re, b.im), dd_mul(a.im, b.re))};
+}
+
+// Product of the n pivots as mantissa and exponent, formed by a full warp (every
+// lane returns it); get(r) is row r's pivot as {re, im}.
+struct DerivScale {
+    ddc v;
+    int e;
+};
+template <int COMPS, class Get>
+__device__ __forceinline__ DerivScale deriv_scale(int n, Get get)
+{
+    const int lane = threadIdx.x & 31;
+    DerivScale s{{{1.0, 0.0}, {0.0, 0.0}}, 0};
+    for (int r = lane; r < n; r += 32) {
+        const double2 d = get(r);
+        int e = 0;
+        if (COMPS == 1) {
+            const double m = frexp(d.x, &e);
+            s.v.re = dd_mul(s.v.re, dd{m, 0.0});
+        } else {
+            frexp(fmax(fabs(d.x), fabs(d.y)), &e);
+            s.v = ddc_mul(s.v, ddc{{ldexp(d.x, -e), 0.0}, {ldexp(d.y, -e), 0.0}});
+        }
+        s.e += e;
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const ddc o = {shfl_xor_dd(s.v.re, off), shfl_xor_dd(s.v.im, off)};
+        if (COMPS == 1) s.v.re = dd_mul(s.v.re, o.re);
+        else s.v = ddc_mul(s.v, o);
+        s.e += __shfl_xor_sync(0xffffffffu, s.e, off);
+    }
+    return s;
+}
+
+// x / d as a double-double (to about 2^-105), d not zero.
+__device__ __forceinline__ dd quotient(double x, double d)
+{
+    const double h = __ddiv_rn(x, d);
+    return dd{h, __ddiv_rn(__fma_rn(-h, d, x), d)};
+}
+
+// (xr + i xi) / (dr + i di) in double-double, to about 2^-102 of its magnitude.
+__device__ __forceinline__ ddc quotient_c(double xr, double xi, double dr, double di)
+{
+    auto prod = [](double a, double b) {
+        const double p = __dmul_rn(a, b);
+        return dd{p, __fma_rn(a, b, -p)};
+    };
+    auto div = [](dd a, dd b) {
+        const double h = __ddiv_rn(a.hi, b.hi);
+        const dd r = dd_add(a, dd_neg(dd_mul(dd{h, 0.0}, b)));
+        return fast_two_sum(h, __ddiv_rn(r.hi, b.hi));
+    };
+    const dd den = dd_add(prod(dr, dr), prod(di, di));
+    return {div(dd_add(prod(xr, dr), prod(xi, di)), den), div(dd_add(prod(xi, dr), dd_neg(prod(xr, di))), den)};
+}
 
 // Appends unit u (bound bin b) to the mode-1 list when b >= lbin.  The
 // appending lanes of a warp take their slots with one atomic (a leader
@@ -318,6 +472,77 @@ __device__ __forceinline__ double unit_sum_real(const double (&xh)[N], const dou
     return acc;
 }
 
+// The same for the derivative walk: sum_d (-1)^popc(d) q_d, one pass over the
+// rows per group (see deriv_on).  Twelve FP64 instructions per row and group
+// of four terms against two 16-byte shared loads; eight independent chains.
+// group_sum_deriv_rt (refine_impl.cuh) replays a group's operations.
+template <int N, int G, bool STATS = false>
+__device__ __forceinline__ double unit_sum_deriv(const double (&xh)[N], const double* __restrict__ s_de,
+                                                 int nq, double* s2 = nullptr)
+{
+    double acc = 0.0, sq[G];
+#pragma unroll
+    for (int i = 0; i < G; ++i) sq[i] = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < nq; ++k) {
+        const double* de = s_de + k * (N * G);
+        double p[G], q[G];
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+            double v[G];
+            if constexpr (G == 4) {
+                const double2 a = reinterpret_cast<const double2*>(de + r * 4)[0];
+                const double2 b = reinterpret_cast<const double2*>(de + r * 4)[1];
+                v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+            } else {
+#pragma unroll
+                for (int i = 0; i < G; ++i) v[i] = de[r * G + i];
+            }
+#pragma unroll
+            for (int i = 0; i < G; ++i) {
+                const double x = add_rn(xh[r], v[i]);
+                if (r == 0) {
+                    p[i] = x;
+                } else {
+                    q[i] = r == 1 ? add_rn(x, p[i]) : __fma_rn(q[i], x, p[i]);
+                    if (r + 1 < N) p[i] = mul_rn(p[i], x);
+                }
+            }
+        }
+        double gs;
+        if constexpr (G == 4) gs = sub_rn(sub_rn(q[0], q[1]), sub_rn(q[2], q[3]));  // + - - +
+        else if constexpr (G == 2) gs = sub_rn(q[0], q[1]);
+        else gs = q[0];
+        acc = (__popc(k) & 1) ? sub_rn(acc, gs) : add_rn(acc, gs);
+        if constexpr (STATS) {
+#pragma unroll
+            for (int i = 0; i < G; ++i) sq[i] = __fma_rn(q[i], q[i], sq[i]);
+        }
+    }
+    if constexpr (STATS) {
+        double t = 0.0;
+#pragma unroll
+        for (int i = 0; i < G; ++i) t += sq[i];
+        *s2 = t;
+    }
+    return acc;
+}
+
+// Upper bound of |term| over a unit: prod_r f_r, f_r = max |xh_r + DE[d][r]| with
+// bnd [2][n] the range of DE over d; for the derivative sum_r prod_{r' != r} f_r'.
+template <int N, bool D>
+__device__ __forceinline__ double unit_bound_real(const double (&xh)[N], const double* bnd)
+{
+    double p = 1.0, q = 0.0;
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+        const double f = fmax(fabs(add_rn(xh[r], bnd[r])), fabs(add_rn(xh[r], bnd[N + r])));
+        if (D) q = __fma_rn(q, f, p);
+        p = mul_rn(p, f);
+    }
+    return D ? q : p;
+}
+
 // First unit base of each thread, built cooperatively by its warp from the
 // NW start vector (x0h, x0l) and the high columns s_mt; every lane of the
 // warp calls this (it shuffles), whether it owns units or not.
@@ -331,9 +556,11 @@ __device__ __forceinline__ double unit_sum_real(const double (&xh)[N], const dou
 // lo words to the thread's shared slots s_lo[r * bd + tid].  Compared with
 // every lane adding all of its columns, this saves most of the double-double
 // adds when threads own few units (n <= 26).
-template <int N>
+// D: the derivative walk, whose high columns have low words (s_ml).
+template <int N, bool D>
 __device__ __forceinline__ void first_base_real(const double* __restrict__ x0h, const double* __restrict__ x0l,
-                                                const double* __restrict__ s_mt, double* s_lo, int ntop,
+                                                const double* __restrict__ s_mt, const double* __restrict__ s_ml,
+                                                double* s_lo, int ntop,
                                                 unsigned long long u0, unsigned long long u1, int tid, int bd,
                                                 double (&xh)[N])
 {
@@ -345,14 +572,15 @@ __device__ __forceinline__ void first_base_real(const double* __restrict__ x0h, 
     const unsigned long long ulo = __shfl_sync(full, u0, 0), uhi = __shfl_sync(full, u0, last);
     const int P = ulo == uhi ? -1 : 63 - __clzll(ulo ^ uhi);
     const unsigned long long gc = gray_of(ulo);
+    auto plus = [&](dd x, int i) { return D ? dd_step(x, s_mt[i], s_ml[i]) : dd_add_d(x, s_mt[i]); };
     dd c0 = {0.0, 0.0}, c1 = {0.0, 0.0};
     if (lane < N) {
         c0 = dd{x0h[lane], x0l[lane]};
         if (N > 32 && lane + 32 < N) c1 = dd{x0h[lane + 32], x0l[lane + 32]};
         for (int j = P + 1; j < ntop; ++j)
             if ((gc >> j) & 1ull) {
-                c0 = dd_add_d(c0, s_mt[j * N + lane]);
-                if (N > 32 && lane + 32 < N) c1 = dd_add_d(c1, s_mt[j * N + lane + 32]);
+                c0 = plus(c0, j * N + lane);
+                if (N > 32 && lane + 32 < N) c1 = plus(c1, j * N + lane + 32);
             }
     }
     const bool own = u0 < u1;
@@ -376,7 +604,7 @@ __device__ __forceinline__ void first_base_real(const double* __restrict__ x0h, 
             if ((g0 >> j) & 1ull) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                    if (r0 + k < N) x[k] = dd_add_d(x[k], s_mt[j * N + r0 + k]);
+                    if (r0 + k < N) x[k] = plus(x[k], j * N + r0 + k);
             }
 #pragma unroll
         for (int k = 0; k < 4; ++k)
@@ -387,26 +615,30 @@ __device__ __forceinline__ void first_base_real(const double* __restrict__ x0h, 
     }
 }
 
-template <int N>
-__global__ void __launch_bounds__(RealCfg<N>::kMaxThreads, 1) walk_real(Problem pb)
+template <int N, bool D>
+__device__ __forceinline__ void walk_real_body(const Problem& pb)
 {
     constexpr int G = RealCfg<N>::G;
     extern __shared__ __align__(16) double smem[];
     const int w = pb.w;
     const int terms = 1 << w;
     const int nq = terms / G;
-    const int ntop = N - 1 - w;
+    const int ntop = N - 1 - (D ? 1 : 0) - w;
     const int tid = threadIdx.x, bd = blockDim.x;
     double* s_de = smem;
     double* s_mt = s_de + terms * N;
-    double* s_lo = s_mt + (ntop > 0 ? ntop : 0) * N;
+    double* s_ml = s_mt + (ntop > 0 ? ntop : 0) * N;  // derivative walk: the high columns' low words
+    double* s_lo = s_ml + (D && ntop > 0 ? ntop : 0) * N;
     float* s_hist = reinterpret_cast<float*>(s_lo + N * bd);  // mode 1
     unsigned* s_cnt = reinterpret_cast<unsigned*>(s_hist + kHistBins);
     // DE range per row, [2][N] (min, max).  Two scalar loads per row: a paired
     // 16-byte load keeps more registers live and makes the n=32 walk spill.
     double* s_bnd = reinterpret_cast<double*>(s_cnt + kHistBins);
     for (int i = tid; i < terms * N; i += bd) s_de[i] = pb.de_hi[i];
-    for (int i = tid; i < ntop * N; i += bd) s_mt[i] = pb.mt[i];
+    for (int i = tid; i < ntop * N; i += bd) {
+        s_mt[i] = pb.mt[i];
+        if (D) s_ml[i] = pb.mt_lo[i];
+    }
     const int mode = pb.mode;
     if (mode != 0)
         for (int i = tid; i < 2 * N; i += bd) s_bnd[i] = pb.bnd[i];
@@ -417,7 +649,7 @@ __global__ void __launch_bounds__(RealCfg<N>::kMaxThreads, 1) walk_real(Problem 
     const unsigned long long T = (unsigned long long)gridDim.x * bd;
     const unsigned long long t = (unsigned long long)blockIdx.x * bd + tid;
     unsigned long long u0, u1;
-    balanced_range(pb.units, T, t, &u0, &u1);
+    balanced_range(eff_units(pb, D), T, t, &u0, &u1);
     // The scan only walks threads that own a unit at or above the threshold.
     if (mode == 2 && (int)pb.tmax[t] < pb.thr_bin) u1 = u0;
     dd tot[1] = {{0.0, 0.0}};
@@ -429,19 +661,14 @@ __global__ void __launch_bounds__(RealCfg<N>::kMaxThreads, 1) walk_real(Problem 
     // ones first (the refinement rebuilds bases in plain index order; the hi
     // words agree unless a row value lies within ~2^-100 of a rounding
     // midpoint, and then only that unit's correction carries one FP64 rounding).
-    first_base_real<N>(pb.x0_hi, pb.x0_lo, s_mt, s_lo, ntop, u0, u1, tid, bd, xh);
+    first_base_real<N, D>(pb.x0_hi, pb.x0_lo, s_mt, s_ml, s_lo, ntop, u0, u1, tid, bd, xh);
     if (u0 < u1) {
         unsigned long long u = u0;
         while (true) {
             int b = 0;
             if (mode != 0) {
-                // Upper bound of |term| over the unit: prod_r max |xh_r + DE[d][r]|;
-                // the scan recomputes it bit for bit to select the same units.
-                double ub = 1.0;
-#pragma unroll
-                for (int r = 0; r < N; ++r)
-                    ub = mul_rn(ub, fmax(fabs(add_rn(xh[r], s_bnd[r])), fabs(add_rn(xh[r], s_bnd[N + r]))));
-                b = hist_bin(ub);
+                // the scan recomputes the bound bit for bit to select the same units
+                b = hist_bin(unit_bound_real<N, D>(xh, s_bnd));
                 bmax = b > bmax ? b : bmax;
                 if (mode == 2 && b >= pb.thr_bin) {
                     unsigned long long k = atomicAdd(pb.list_n, 1ull);
@@ -454,11 +681,12 @@ __global__ void __launch_bounds__(RealCfg<N>::kMaxThreads, 1) walk_real(Problem 
                 }
             }
             if (mode == 0) {
-                double us = unit_sum_real<N, G>(xh, s_de, nq);
+                const double us = D ? unit_sum_deriv<N, G>(xh, s_de, nq) : unit_sum_real<N, G>(xh, s_de, nq);
                 tot[0] = dd_add_d(tot[0], (u & 1ull) ? -us : us);
             } else if (mode == 1) {
                 double sq;
-                double us = unit_sum_real<N, G, true>(xh, s_de, nq, &sq);
+                const double us = D ? unit_sum_deriv<N, G, true>(xh, s_de, nq, &sq)
+                                    : unit_sum_real<N, G, true>(xh, s_de, nq, &sq);
                 tot[0] = dd_add_d(tot[0], (u & 1ull) ? -us : us);
                 hc.add(b, sq, s_hist, s_cnt);  // actual sum of squared terms, keyed by the bound
                 raw_list_add(pb, lbin, u, b);
@@ -471,7 +699,9 @@ __global__ void __launch_bounds__(RealCfg<N>::kMaxThreads, 1) walk_real(Problem 
             for (int r = 0; r < N; ++r) {
                 double m = add ? col[r] : -col[r];
                 dd s = two_sum(xh[r], m);
-                dd z = fast_two_sum(s.hi, add_rn(s.lo, s_lo[r * bd + tid]));
+                double l = s_lo[r * bd + tid];
+                if (D) l = add ? add_rn(l, s_ml[j * N + r]) : sub_rn(l, s_ml[j * N + r]);
+                dd z = fast_two_sum(s.hi, add_rn(s.lo, l));
                 xh[r] = z.hi;
                 s_lo[r * bd + tid] = z.lo;
             }
@@ -484,6 +714,20 @@ __global__ void __launch_bounds__(RealCfg<N>::kMaxThreads, 1) walk_real(Problem 
         flush_hist(s_hist, s_cnt, pb);
     }
     if (mode != 2) grid_reduce<1>(tot, pb);
+}
+
+// The derivative walk where the matrix has a pivot column, else the plain
+// walk; the branch is the same for the whole grid.
+template <int N>
+__global__ void __launch_bounds__(RealCfg<N>::kMaxThreads, 1) walk_real(Problem pb)
+{
+    if constexpr (N >= kMinDerivReal) {
+        if (deriv_on(pb)) {
+            walk_real_body<N, true>(pb);
+            return;
+        }
+    }
+    walk_real_body<N, false>(pb);
 }
 
 // ------------------------------------------------------------- complex ----
@@ -559,25 +803,103 @@ __device__ __forceinline__ void unit_sum_complex(const double (&xr)[N], const do
     }
 }
 
-template <int N>
-__global__ void __launch_bounds__(ComplexCfg<N>::kMaxThreads, 1) walk_complex(Problem pb)
+// The derivative walk's complex terms (unit_sum_deriv): two at a time out of the
+// table's groups of G, so that p and q of each fit the registers beside x.
+// Ten FP64 instructions per row and term where the two plain terms it stands
+// for take twelve.
+template <int N, int G, bool STATS = false>
+__device__ __forceinline__ void unit_sum_complex_deriv(const double (&xr)[N], const double (&xi)[N],
+                                                       const double* __restrict__ s_de_re,
+                                                       const double* __restrict__ s_de_im, int nq,
+                                                       double& acc_re, double& acc_im, double* s2 = nullptr)
+{
+    static_assert(G % 2 == 0, "pairs of terms");
+    double ar = 0.0, ai = 0.0, sq[2] = {0.0, 0.0};
+#pragma unroll 1
+    for (int k = 0; k < nq * (G / 2); ++k) {
+        const double* dr = s_de_re + (k / (G / 2)) * (N * G) + 2 * (k % (G / 2));
+        const double* di = s_de_im + (k / (G / 2)) * (N * G) + 2 * (k % (G / 2));
+        double pr[2], pi[2], qr[2], qi[2];
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+            const double2 a = *reinterpret_cast<const double2*>(dr + r * G);
+            const double2 b = *reinterpret_cast<const double2*>(di + r * G);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const double yr = add_rn(xr[r], i ? a.y : a.x);
+                const double yi = add_rn(xi[r], i ? b.y : b.x);
+                if (r == 0) {
+                    pr[i] = yr;
+                    pi[i] = yi;
+                } else {
+                    if (r == 1) {
+                        qr[i] = add_rn(yr, pr[i]);
+                        qi[i] = add_rn(yi, pi[i]);
+                    } else {
+                        const double t = __fma_rn(-qi[i], yi, pr[i]);
+                        const double u = __fma_rn(qi[i], yr, pi[i]);
+                        qi[i] = __fma_rn(qr[i], yi, u);
+                        qr[i] = __fma_rn(qr[i], yr, t);
+                    }
+                    if (r + 1 < N) {
+                        const double t1 = mul_rn(pi[i], yi), t2 = mul_rn(pi[i], yr);
+                        pi[i] = __fma_rn(pr[i], yi, t2);
+                        pr[i] = __fma_rn(pr[i], yr, -t1);
+                    }
+                }
+            }
+        }
+        const double gr = sub_rn(qr[0], qr[1]), gi = sub_rn(qi[0], qi[1]);
+        if (__popc(k) & 1) { ar = sub_rn(ar, gr); ai = sub_rn(ai, gi); }
+        else { ar = add_rn(ar, gr); ai = add_rn(ai, gi); }
+        if constexpr (STATS) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) sq[i] = __fma_rn(qi[i], qi[i], __fma_rn(qr[i], qr[i], sq[i]));
+        }
+    }
+    acc_re = ar;
+    acc_im = ai;
+    if constexpr (STATS) *s2 = sq[0] + sq[1];
+}
+
+// Upper bound of |term| over a unit (unit_bound_real), with |x_r| <= |xtop_r| +
+// max_d |DE[d][r]| (triangle inequality), bnd [N] the latter.
+template <int N, bool D>
+__device__ __forceinline__ double unit_bound_complex(const double (&xr)[N], const double (&xi)[N], const double* bnd)
+{
+    double p = 1.0, q = 0.0;
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+        const double f = add_rn(__dsqrt_rn(__fma_rn(xr[r], xr[r], mul_rn(xi[r], xi[r]))), bnd[r]);
+        if (D) q = __fma_rn(q, f, p);
+        p = mul_rn(p, f);
+    }
+    return D ? q : p;
+}
+
+template <int N, bool D>
+__device__ __forceinline__ void walk_complex_body(const Problem& pb)
 {
     constexpr int G = ComplexCfg<N>::G;
     extern __shared__ __align__(16) double smem[];
     const int w = pb.w;
     const int terms = 1 << w;
     const int nq = terms / G;
-    const int ntop = N - 1 - w;
+    const int ntop = N - 1 - (D ? 1 : 0) - w;
     const int ntp = ntop > 0 ? ntop : 0;
     const int tid = threadIdx.x, bd = blockDim.x;
     double* s_de = smem;                        // [2][terms*N]
     double* s_mt = s_de + 2 * terms * N;        // [2][ntop*N]
-    double* s_lo = s_mt + 2 * ntp * N;          // [2][N][bd]
+    double* s_ml = s_mt + 2 * ntp * N;          // [2][ntop*N] low words (derivative walk)
+    double* s_lo = s_ml + (D ? 2 * ntp * N : 0);  // [2][N][bd]
     float* s_hist = reinterpret_cast<float*>(s_lo + 2 * N * bd);  // mode 1
     unsigned* s_cnt = reinterpret_cast<unsigned*>(s_hist + kHistBins);
     double* s_bnd = reinterpret_cast<double*>(s_cnt + kHistBins);  // [N]
     for (int i = tid; i < 2 * terms * N; i += bd) s_de[i] = pb.de_hi[i];
-    for (int i = tid; i < 2 * ntp * N; i += bd) s_mt[i] = pb.mt[i];
+    for (int i = tid; i < 2 * ntp * N; i += bd) {
+        s_mt[i] = pb.mt[i];
+        if (D) s_ml[i] = pb.mt_lo[i];
+    }
     const int mode = pb.mode;
     if (mode != 0)
         for (int i = tid; i < N; i += bd) s_bnd[i] = pb.bnd[i];
@@ -586,13 +908,15 @@ __global__ void __launch_bounds__(ComplexCfg<N>::kMaxThreads, 1) walk_complex(Pr
     __syncthreads();
     const double* s_mt_re = s_mt;
     const double* s_mt_im = s_mt + ntp * N;
+    // high column entry i (part 0, or at ntp * N + i part 1) added to x
+    auto plus = [&](dd x, int i) { return D ? dd_step(x, s_mt[i], s_ml[i]) : dd_add_d(x, s_mt[i]); };
     double* s_lo_re = s_lo;
     double* s_lo_im = s_lo + N * bd;
 
     const unsigned long long T = (unsigned long long)gridDim.x * bd;
     const unsigned long long t = (unsigned long long)blockIdx.x * bd + tid;
     unsigned long long u0, u1;
-    balanced_range(pb.units, T, t, &u0, &u1);
+    balanced_range(eff_units(pb, D), T, t, &u0, &u1);
     if (mode == 2 && (int)pb.tmax[t] < pb.thr_bin) u1 = u0;
     dd tot[2] = {{0.0, 0.0}, {0.0, 0.0}};
     HistCache hc;
@@ -616,8 +940,8 @@ __global__ void __launch_bounds__(ComplexCfg<N>::kMaxThreads, 1) walk_complex(Pr
 #pragma unroll
                     for (int k = 0; k < 2; ++k)
                         if (r0 + k < N) {
-                            a[k] = dd_add_d(a[k], s_mt_re[j * N + r0 + k]);
-                            b[k] = dd_add_d(b[k], s_mt_im[j * N + r0 + k]);
+                            a[k] = plus(a[k], j * N + r0 + k);
+                            b[k] = plus(b[k], (ntp + j) * N + r0 + k);
                         }
                 }
 #pragma unroll
@@ -633,12 +957,7 @@ __global__ void __launch_bounds__(ComplexCfg<N>::kMaxThreads, 1) walk_complex(Pr
         while (true) {
             int b = 0;
             if (mode != 0) {
-                // |x_r| <= |xtop_r| + max_d |DE[d][r]|  (triangle inequality)
-                double ub = 1.0;
-#pragma unroll
-                for (int r = 0; r < N; ++r)
-                    ub = mul_rn(ub, add_rn(__dsqrt_rn(__fma_rn(xr[r], xr[r], mul_rn(xi[r], xi[r]))), s_bnd[r]));
-                b = hist_bin(ub);
+                b = hist_bin(unit_bound_complex<N, D>(xr, xi, s_bnd));
                 bmax = b > bmax ? b : bmax;
                 if (mode == 2 && b >= pb.thr_bin) {
                     unsigned long long k = atomicAdd(pb.list_n, 1ull);
@@ -657,8 +976,13 @@ __global__ void __launch_bounds__(ComplexCfg<N>::kMaxThreads, 1) walk_complex(Pr
             }
             if (mode != 2) {
                 double ur, ui, sq = 0.0;
-                if (mode == 0) unit_sum_complex<N, G>(xr, xi, s_de, s_de + terms * N, nq, ur, ui);
-                else unit_sum_complex<N, G, true>(xr, xi, s_de, s_de + terms * N, nq, ur, ui, &sq);
+                if constexpr (D) {
+                    if (mode == 0) unit_sum_complex_deriv<N, G>(xr, xi, s_de, s_de + terms * N, nq, ur, ui);
+                    else unit_sum_complex_deriv<N, G, true>(xr, xi, s_de, s_de + terms * N, nq, ur, ui, &sq);
+                } else {
+                    if (mode == 0) unit_sum_complex<N, G>(xr, xi, s_de, s_de + terms * N, nq, ur, ui);
+                    else unit_sum_complex<N, G, true>(xr, xi, s_de, s_de + terms * N, nq, ur, ui, &sq);
+                }
                 if (u & 1ull) { ur = -ur; ui = -ui; }
                 tot[0] = dd_add_d(tot[0], ur);
                 tot[1] = dd_add_d(tot[1], ui);
@@ -674,12 +998,18 @@ __global__ void __launch_bounds__(ComplexCfg<N>::kMaxThreads, 1) walk_complex(Pr
             for (int r = 0; r < N; ++r) {
                 double mr = add ? s_mt_re[j * N + r] : -s_mt_re[j * N + r];
                 double mi = add ? s_mt_im[j * N + r] : -s_mt_im[j * N + r];
+                double lr = s_lo_re[r * bd + tid], li = s_lo_im[r * bd + tid];
+                if (D) {
+                    const double er = s_ml[j * N + r], ei = s_ml[(ntp + j) * N + r];
+                    lr = add ? add_rn(lr, er) : sub_rn(lr, er);
+                    li = add ? add_rn(li, ei) : sub_rn(li, ei);
+                }
                 dd s = two_sum(xr[r], mr);
-                dd z = fast_two_sum(s.hi, add_rn(s.lo, s_lo_re[r * bd + tid]));
+                dd z = fast_two_sum(s.hi, add_rn(s.lo, lr));
                 xr[r] = z.hi;
                 s_lo_re[r * bd + tid] = z.lo;
                 s = two_sum(xi[r], mi);
-                z = fast_two_sum(s.hi, add_rn(s.lo, s_lo_im[r * bd + tid]));
+                z = fast_two_sum(s.hi, add_rn(s.lo, li));
                 xi[r] = z.hi;
                 s_lo_im[r * bd + tid] = z.lo;
             }
@@ -692,6 +1022,20 @@ __global__ void __launch_bounds__(ComplexCfg<N>::kMaxThreads, 1) walk_complex(Pr
         flush_hist(s_hist, s_cnt, pb);
     }
     if (mode != 2) grid_reduce<2>(tot, pb);
+}
+
+// The derivative walk where the matrix has a pivot column, else the plain
+// walk; the branch is the same for the whole grid.
+template <int N>
+__global__ void __launch_bounds__(ComplexCfg<N>::kMaxThreads, 1) walk_complex(Problem pb)
+{
+    if constexpr (N >= kMinDerivComplex) {
+        if (deriv_on(pb)) {
+            walk_complex_body<N, true>(pb);
+            return;
+        }
+    }
+    walk_complex_body<N, false>(pb);
 }
 
 // Double-double refinement (dense_refine.cu), all stream-ordered after the

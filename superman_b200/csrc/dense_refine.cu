@@ -65,19 +65,53 @@ __device__ __forceinline__ void group_sum_complex_rt(const double* xr, const dou
     }
 }
 
+// The same for a pair of the derivative walk's terms (unit_sum_complex_deriv).
+__device__ __forceinline__ void pair_sum_complex_deriv_rt(const double* xr, const double* xi, const double* dr,
+                                                          const double* di, int n, int rs, double& gr, double& gi)
+{
+    double pr[2], pi[2], qr[2] = {0.0, 0.0}, qi[2] = {0.0, 0.0};
+    for (int r = 0; r < n; ++r)
+        for (int i = 0; i < 2; ++i) {
+            const double yr = add_rn(xr[r], dr[r * rs + i]), yi = add_rn(xi[r], di[r * rs + i]);
+            if (r == 0) {
+                pr[i] = yr;
+                pi[i] = yi;
+                continue;
+            }
+            if (r == 1) {
+                qr[i] = add_rn(yr, pr[i]);
+                qi[i] = add_rn(yi, pi[i]);
+            } else {
+                const double t = __fma_rn(-qi[i], yi, pr[i]);
+                const double u = __fma_rn(qi[i], yr, pi[i]);
+                qi[i] = __fma_rn(qr[i], yi, u);
+                qr[i] = __fma_rn(qr[i], yr, t);
+            }
+            const double t1 = mul_rn(pi[i], yi), t2 = mul_rn(pi[i], yr);
+            pi[i] = __fma_rn(pr[i], yi, t2);
+            pr[i] = __fma_rn(pr[i], yr, -t1);
+        }
+    gr = sub_rn(qr[0], qr[1]);
+    gi = sub_rn(qi[0], qi[1]);
+}
+
 // Unit base of unit u (component `part`) rebuilt from scratch in
 // double-double the way the walk builds a thread's first unit (x0 plus the
 // selected high columns in index order); the worker's threads take rows.
-__device__ __forceinline__ void unit_base(const Problem& pb, const double* mt_all, unsigned long long u, int part,
-                                          int lane, double* hi, double* lo, int stride = 32)
+// ml_all: the high columns' low words in the derivative walk, else null.
+__device__ __forceinline__ void unit_base(const Problem& pb, const double* mt_all, const double* ml_all,
+                                          unsigned long long u, int part, int lane, double* hi, double* lo,
+                                          int stride = 32)
 {
-    const int n = pb.n, ntop = n - 1 - pb.w;
+    const int n = pb.n, ntop = eff_ntop(pb, ml_all != nullptr);
     const unsigned long long g = gray_of(u);
-    const double* mt = mt_all + (size_t)part * (ntop > 0 ? ntop : 0) * n;
+    const size_t at = (size_t)part * (ntop > 0 ? ntop : 0) * n;
+    const double* mt = mt_all + at;
     for (int r = lane; r < n; r += stride) {
         dd x = {pb.x0_hi[part * n + r], pb.x0_lo[part * n + r]};
         for (int j = 0; j < ntop; ++j)
-            if ((g >> j) & 1ull) x = dd_add_d(x, mt[j * n + r]);
+            if ((g >> j) & 1ull)
+                x = ml_all ? dd_step(x, mt[j * n + r], ml_all[at + j * n + r]) : dd_add_d(x, mt[j * n + r]);
         hi[r] = x.hi;
         lo[r] = x.lo;
     }
@@ -86,10 +120,22 @@ __device__ __forceinline__ void unit_base(const Problem& pb, const double* mt_al
 // The walk's unit bound (dense_impl.cuh walk_real/walk_complex, and
 // sparse_impl.cuh walk_sparse when pb.na < pb.n) from the hi words of a unit
 // base (xh: [comps][n]): the same operations in the same order.
-__device__ double unit_bound_rt(const Problem& pb, const double* xh)
+__device__ double unit_bound_rt(const Problem& pb, const double* xh, bool deriv)
 {
     const int n = pb.n, na = pb.na;
     double ub = 1.0;
+    if (deriv) {
+        double q = 0.0;
+        for (int r = 0; r < n; ++r) {
+            const double xi = xh[kMaxN + r];  // (complex)
+            const double f = pb.comps == 2
+                                 ? add_rn(__dsqrt_rn(__fma_rn(xh[r], xh[r], mul_rn(xi, xi))), pb.bnd[r])
+                                 : fmax(fabs(add_rn(xh[r], pb.bnd[r])), fabs(add_rn(xh[r], pb.bnd[n + r])));
+            q = __fma_rn(q, f, ub);
+            ub = mul_rn(ub, f);
+        }
+        return q;
+    }
     if (pb.comps == 2) {
         for (int r = 0; r < n; ++r) {
             const double xr = xh[r], xi = xh[kMaxN + r];
@@ -135,14 +181,15 @@ __global__ void __launch_bounds__(128) list_units(Problem pb)
     }
     const unsigned long long T = (unsigned long long)pb.grid * pb.threads;
     const int lane = threadIdx.x & 31, n = pb.n, c = pb.comps;
-    const int ntop = n - 1 - pb.w, ntp = ntop > 0 ? ntop : 0;
+    const bool deriv = deriv_on(pb);
+    const int ntop = eff_ntop(pb, deriv), ntp = ntop > 0 ? ntop : 0;
     const unsigned long long warp = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
     double xh[2 * kMaxN], xl[2 * kMaxN];  // [comps][kMaxN], per lane
     for (unsigned long long t = warp; t < T; t += nwarps) {
         if ((int)pb.tmax[t] < thr) continue;  // warp-uniform
         unsigned long long u0, u1;
-        balanced_range(pb.units, T, t, &u0, &u1);
+        balanced_range(eff_units(pb, deriv), T, t, &u0, &u1);
         unsigned long long a, b;
         balanced_range(u1 - u0, 32, lane, &a, &b);
         a += u0;
@@ -151,16 +198,18 @@ __global__ void __launch_bounds__(128) list_units(Problem pb)
         const unsigned long long g0 = gray_of(a);
         for (int part = 0; part < c; ++part) {
             const double* mt = pb.mt + (size_t)part * ntp * n;
+            const double* ml = deriv ? pb.mt_lo + (size_t)part * ntp * n : nullptr;
             for (int r = 0; r < n; ++r) {
                 dd x = {pb.x0_hi[part * n + r], pb.x0_lo[part * n + r]};
                 for (int j = 0; j < ntop; ++j)
-                    if ((g0 >> j) & 1ull) x = dd_add_d(x, mt[j * n + r]);
+                    if ((g0 >> j) & 1ull)
+                        x = deriv ? dd_step(x, mt[j * n + r], ml[j * n + r]) : dd_add_d(x, mt[j * n + r]);
                 xh[part * kMaxN + r] = x.hi;
                 xl[part * kMaxN + r] = x.lo;
             }
         }
         for (unsigned long long u = a;;) {
-            if (hist_bin(unit_bound_rt(pb, xh)) >= thr) {
+            if (hist_bin(unit_bound_rt(pb, xh, deriv)) >= thr) {
                 const unsigned long long i = atomicAdd(pb.list_n, 1ull);
                 if (i < pb.list_cap) pb.list_u[i] = u;
             }
@@ -169,10 +218,13 @@ __global__ void __launch_bounds__(128) list_units(Problem pb)
             const bool add = (gray_of(u) >> j) & 1ull;
             for (int part = 0; part < c; ++part) {
                 const double* col = pb.mt + ((size_t)part * ntp + j) * n;
+                const double* cl = deriv ? pb.mt_lo + ((size_t)part * ntp + j) * n : nullptr;
                 for (int r = 0; r < n; ++r) {
                     const double m = add ? col[r] : -col[r];
                     dd s = two_sum(xh[part * kMaxN + r], m);
-                    dd z = fast_two_sum(s.hi, add_rn(s.lo, xl[part * kMaxN + r]));
+                    double l = xl[part * kMaxN + r];
+                    if (deriv) l = add ? add_rn(l, cl[r]) : sub_rn(l, cl[r]);
+                    dd z = fast_two_sum(s.hi, add_rn(s.lo, l));
                     xh[part * kMaxN + r] = z.hi;
                     xl[part * kMaxN + r] = z.lo;
                 }
@@ -188,6 +240,7 @@ __global__ void __launch_bounds__(128) list_units(Problem pb)
 __global__ void __launch_bounds__(32) pick_list_bin(Problem pb)
 {
     constexpr int kPer = kHistBins / 32;
+    if (eff_units(pb, deriv_on(pb)) <= pb.raw_cap / 2) return;  // every unit is listed (setup_kernel)
     const int lane = threadIdx.x;
     const unsigned full = 0xffffffffu;
     __shared__ unsigned s_pc[kHistPadded];
@@ -258,7 +311,7 @@ __global__ void __launch_bounds__(32) dd_threshold(Problem pb)
     }
     __syncwarp();
     const double mag = pb.comps == 1 ? fabs(rb->res[0].hi) : hypot(rb->res[0].hi, rb->res[1].hi);
-    const ThresholdPick t = pick_threshold_shared(pb, mag, s_h2, s_hc);
+    const ThresholdPick t = pick_threshold_shared(pb, deriv_on(pb), mag, s_h2, s_hc);
     if (lane == 0) {
         rb->thr = t.thr;
         rb->count = t.count;
@@ -399,17 +452,20 @@ __global__ void __launch_bounds__(512, 1) refine_real(Problem pb)
     const int nwarps = blockDim.x >> 5;
     const int wk = refine_worker_threads(count, terms, 2);  // threads per worker
     const int wl = threadIdx.x % wk, wid = threadIdx.x / wk, nwk = blockDim.x / wk;
-    const int ntp = n - 1 - pb.w > 0 ? n - 1 - pb.w : 0;
+    const bool deriv = deriv_on(pb);
+    const int ntop = eff_ntop(pb, deriv), ntp = ntop > 0 ? ntop : 0;
     double* s_dh = sm;
     double* s_dl = s_dh + terms * n;
     double* s_x = s_dl + terms * n;      // [nwarps][2n]
     double* s_g = s_x + nwarps * 2 * n;  // [nwarps][nq]
     double* s_mt = s_g + nwarps * nq;    // [ntp][n]
+    double* s_ml = s_mt + ntp * n;       // [ntp][n] low words, derivative walk only
     // CTAs without a unit skip the tables (they still join the grid reduction)
     if ((unsigned long long)blockIdx.x < count) {
         stage_rows(s_dh, pb.de_hi, 1, n, terms, G);  // [n][terms]
         stage_rows(s_dl, pb.de_lo, 1, n, terms, G);
         stage(s_mt, pb.mt, ntp * n);
+        if (deriv) stage(s_ml, pb.mt_lo, ntp * n);
     }
     __syncthreads();
     double* xw = s_x + wid * 2 * n;
@@ -424,14 +480,33 @@ __global__ void __launch_bounds__(512, 1) refine_real(Problem pb)
                 const double* src = pb.list_x + e * (2 * n);
                 for (int i = wl; i < 2 * n; i += wk) xw[i] = src[i];
             } else {
-                unit_base(pb, s_mt, pb.list_u[e], 0, wl, xw, xw + n, wk);
+                unit_base(pb, s_mt, deriv ? s_ml : nullptr, pb.list_u[e], 0, wl, xw, xw + n, wk);
             }
         }
         worker_sync(wk);
         dd acc = {0.0, 0.0};
         if (active) {
-            for (int q = wl; q < nq; q += wk) gw[q] = group_sum_real_rt(xw, s_dh + q * G, n, pb.na, G, terms);
-            if (terms >= 2 * wk) {
+            for (int q = wl; q < nq; q += wk)
+                gw[q] = deriv ? group_sum_deriv_rt(xw, s_dh + q * G, n, G, terms)
+                              : group_sum_real_rt(xw, s_dh + q * G, n, pb.na, G, terms);
+            if (deriv) {
+                // two terms at a time (one when the worker has no two each):
+                // the products p and derivatives q of each are separate chains
+                const int step = terms >= 2 * wk ? wk : 0;
+                for (int d = wl; d < terms; d += step ? 2 * wk : wk) {
+                    const int d2 = d + step;
+                    dd p1 = dd_add_fast(dd{xw[0], xw[n]}, dd{s_dh[d], s_dl[d]}), q1 = {1.0, 0.0};
+                    dd p2 = dd_add_fast(dd{xw[0], xw[n]}, dd{s_dh[d2], s_dl[d2]}), q2 = {1.0, 0.0};
+                    for (int r = 1; r < n; ++r) {
+                        const int k1 = r * terms + d, k2 = r * terms + d2;
+                        const dd x = {xw[r], xw[n + r]};
+                        deriv_step(p1, q1, dd_add_fast(x, dd{s_dh[k1], s_dl[k1]}));
+                        if (step) deriv_step(p2, q2, dd_add_fast(x, dd{s_dh[k2], s_dl[k2]}));
+                    }
+                    acc = (__popc(d) & 1) ? dd_add(acc, dd_neg(q1)) : dd_add(acc, q1);
+                    if (step) acc = (__popc(d2) & 1) ? dd_add(acc, dd_neg(q2)) : dd_add(acc, q2);
+                }
+            } else if (terms >= 2 * wk) {
                 for (int d = wl; d < terms; d += 2 * wk) {
                     const int d2 = d + wk;
                     dd p1 = dd_add_fast(dd{xw[0], xw[n]}, dd{s_dh[d], s_dl[d]});
@@ -510,17 +585,22 @@ __global__ void __launch_bounds__(512, 1) refine_complex(Problem pb)
     const int nwarps = blockDim.x >> 5;
     const int wk = refine_worker_threads(count, terms, 1);  // threads per worker
     const int wl = threadIdx.x % wk, wid = threadIdx.x / wk, nwk = blockDim.x / wk;
-    const int ntp = n - 1 - pb.w > 0 ? n - 1 - pb.w : 0;
+    const bool deriv = deriv_on(pb);
+    const int ntop = eff_ntop(pb, deriv), ntp = ntop > 0 ? ntop : 0;
+    // partial sums the walk forms in FP64: per group, in the derivative walk per pair
+    const int np = deriv ? terms / 2 : nq;
     double* s_dh = sm;                    // [2][terms*n]
     double* s_dl = s_dh + 2 * terms * n;  // [2][terms*n]
     double* s_x = s_dl + 2 * terms * n;   // [nwarps][4n]
-    double* s_g = s_x + nwarps * 4 * n;   // [nwarps][2*nq]
-    double* s_mt = s_g + nwarps * 2 * nq; // [2][ntp][n]
+    double* s_g = s_x + nwarps * 4 * n;   // [nwarps][2*np]
+    double* s_mt = s_g + nwarps * 2 * np; // [2][ntp][n]
+    double* s_ml = s_mt + 2 * ntp * n;    // [2][ntp][n] low words, derivative walk only
     // CTAs without a unit skip the tables (they still join the grid reduction)
     if ((unsigned long long)blockIdx.x < count) {
         stage_rows(s_dh, pb.de_hi, 2, n, terms, G);  // [2][n][terms]
         stage_rows(s_dl, pb.de_lo, 2, n, terms, G);
         stage(s_mt, pb.mt, 2 * ntp * n);
+        if (deriv) stage(s_ml, pb.mt_lo, 2 * ntp * n);
     }
     __syncthreads();
     const double* drh = s_dh;
@@ -528,7 +608,7 @@ __global__ void __launch_bounds__(512, 1) refine_complex(Problem pb)
     const double* drl = s_dl;
     const double* dil = s_dl + terms * n;
     double* xw = s_x + wid * 4 * n;  // xr hi, xr lo, xi hi, xi lo
-    double* gw = s_g + wid * 2 * nq;
+    double* gw = s_g + wid * 2 * np;
     dd corr_r = {0.0, 0.0}, corr_i = {0.0, 0.0};
     const unsigned long long round = (unsigned long long)gridDim.x * nwk;
     for (unsigned long long e0 = 0; e0 < count; e0 += round) {
@@ -539,30 +619,45 @@ __global__ void __launch_bounds__(512, 1) refine_complex(Problem pb)
                 const double* src = pb.list_x + e * (4 * n);
                 for (int i = wl; i < 4 * n; i += wk) xw[i] = src[i];
             } else {
-                unit_base(pb, s_mt, pb.list_u[e], 0, wl, xw, xw + n, wk);
-                unit_base(pb, s_mt, pb.list_u[e], 1, wl, xw + 2 * n, xw + 3 * n, wk);
+                unit_base(pb, s_mt, deriv ? s_ml : nullptr, pb.list_u[e], 0, wl, xw, xw + n, wk);
+                unit_base(pb, s_mt, deriv ? s_ml : nullptr, pb.list_u[e], 1, wl, xw + 2 * n, xw + 3 * n, wk);
             }
         }
         worker_sync(wk);
         dd ar = {0.0, 0.0}, ai = {0.0, 0.0};
         if (active) {
-            for (int q = wl; q < nq; q += wk)
-                group_sum_complex_rt(xw, xw + 2 * n, drh + q * G, dih + q * G, n, G, terms, gw[2 * q],
-                                     gw[2 * q + 1]);
+            for (int q = wl; q < np; q += wk) {
+                if (deriv)
+                    pair_sum_complex_deriv_rt(xw, xw + 2 * n, drh + 2 * q, dih + 2 * q, n, terms, gw[2 * q],
+                                              gw[2 * q + 1]);
+                else
+                    group_sum_complex_rt(xw, xw + 2 * n, drh + q * G, dih + q * G, n, G, terms, gw[2 * q],
+                                         gw[2 * q + 1]);
+            }
             for (int d = wl; d < terms; d += wk) {
                 int k = d;
                 dd pr = dd_add_fast(dd{xw[0], xw[n]}, dd{drh[k], drl[k]});
                 dd pi = dd_add_fast(dd{xw[2 * n], xw[3 * n]}, dd{dih[k], dil[k]});
+                dd qr = {1.0, 0.0}, qi = {0.0, 0.0};
                 for (int r = 1; r < n; ++r) {
                     k = r * terms + d;
                     dd yr = dd_add_fast(dd{xw[r], xw[n + r]}, dd{drh[k], drl[k]});
                     dd yi = dd_add_fast(dd{xw[2 * n + r], xw[3 * n + r]}, dd{dih[k], dil[k]});
+                    if (deriv) {  // q <- q y + p
+                        const dd tr = dd_add(dd_add_fast(dd_mul(qr, yr), dd_neg(dd_mul(qi, yi))), pr);
+                        qi = dd_add(dd_add_fast(dd_mul(qr, yi), dd_mul(qi, yr)), pi);
+                        qr = tr;
+                    }
                     // the products' sums unnormalised (dd_add_fast: about 2^-106 of
                     // |pr yr| + |pi yi| off, far inside what the refinement corrects)
                     dd nr = dd_add_fast(dd_mul(pr, yr), dd_neg(dd_mul(pi, yi)));
                     dd ni = dd_add_fast(dd_mul(pr, yi), dd_mul(pi, yr));
                     pr = nr;
                     pi = ni;
+                }
+                if (deriv) {
+                    pr = qr;
+                    pi = qi;
                 }
                 if (__popc(d) & 1) {
                     ar = dd_add(ar, dd_neg(pr));
@@ -578,7 +673,7 @@ __global__ void __launch_bounds__(512, 1) refine_complex(Problem pb)
         worker_sync(wk);
         if (active && wl == 0) {
             double fr = 0.0, fi = 0.0;
-            for (int q = 0; q < nq; ++q) {
+            for (int q = 0; q < np; ++q) {
                 if (__popc(q) & 1) {
                     fr = sub_rn(fr, gw[2 * q]);
                     fi = sub_rn(fi, gw[2 * q + 1]);
@@ -649,9 +744,13 @@ int launch_threshold(const Problem& pb, cudaStream_t s)
 
 size_t refine_smem_bytes(const Problem& pb, int threads)
 {
-    const size_t terms = (size_t)1 << pb.w, n = pb.n, c = pb.comps, nq = terms / pb.g;
+    // (the complex derivative walk keeps a partial sum per pair of terms)
+    const size_t terms = (size_t)1 << pb.w, n = pb.n, c = pb.comps;
+    const size_t nq = pb.deriv && c == 2 && pb.g > 2 ? terms / 2 : terms / pb.g;
     const size_t nwarps = threads / 32;
-    const size_t ntp = pb.n - 1 - pb.w > 0 ? pb.n - 1 - pb.w : 0;
+    // (whichever walk the matrix gets: see walk_smem_bytes)
+    size_t ntp = pb.n - 1 - pb.w > 0 ? pb.n - 1 - pb.w : 0;
+    if (pb.deriv && ntp > 2) ntp = 2 * (ntp - 1);
     return sizeof(double) * (2 * c * terms * n + nwarps * (2 * c * n + c * nq) + c * ntp * n);
 }
 

@@ -50,7 +50,7 @@ namespace dense {
 __global__ void setup_kernel(Problem pb, const double* __restrict__ a_in, int smem_tables);
 int launch_setup(const Problem& pb, const double* d_a, cudaStream_t s);
 int group_size(int n, int comps);
-int choose_unit_bits(int n, int comps, const spb_options* opt);
+void choose_walk(Problem* pb, const spb_options* opt, bool hint);
 size_t plan_layout(Problem* pb, char* base, size_t* in_offset);
 size_t walk_smem_bytes(const Problem& pb, int threads);
 int prepare_setup(int* limit);
@@ -71,14 +71,21 @@ void* g_scratch_ptr[64];
 cudaError_t g_scratch_err[64];
 int g_prepare_st[64];
 
-// perm = (4(n%2)-2) * total * 2^E, written as a double-double {hi, lo}.
+// perm = (4(nc%2)-2) * total * 2^E over nc walked columns, times the product
+// of the pivots in the derivative walk, written as a double-double {hi, lo}.
 __global__ void noalloc_finalize(spb::dense::Problem pb, double* out)
 {
     if (threadIdx.x == 0 && blockIdx.x == 0) {
-        const int e = *pb.exp_sum + 1;
-        const double sgn = (pb.n % 2) ? 1.0 : -1.0;
-        out[0] = sgn * ldexp(pb.result[0].hi, e);
-        out[1] = sgn * ldexp(pb.result[0].lo, e);
+        const bool deriv = spb::dense::deriv_on(pb);
+        int e = *pb.exp_sum + 1;
+        spb::dd v = pb.result[0];
+        if (deriv) {
+            v = spb::dd_mul(v, pb.rb->scale[0]);
+            e += pb.rb->scale_exp;
+        }
+        const double sgn = ((pb.n - (deriv ? 1 : 0)) % 2) ? 1.0 : -1.0;
+        out[0] = sgn * ldexp(v.hi, e);
+        out[1] = sgn * ldexp(v.lo, e);
     }
 }
 
@@ -143,7 +150,7 @@ extern "C" int spb_perm_dense_f64_noalloc(const double* d_a, int n, double* d_ou
     pb.n = n;
     pb.na = n;
     pb.comps = 1;
-    pb.w = choose_unit_bits(n, 1, &opt);
+    choose_walk(&pb, &opt, true);
     pb.g = group_size(n, 1);
     pb.units = 1ull << (n - 1 - pb.w);
     int threads = walk_max_threads(n, 1);
@@ -155,7 +162,8 @@ extern "C" int spb_perm_dense_f64_noalloc(const double* d_a, int n, double* d_ou
         return SPB_ERR_INVALID;
     }
     int blocks = sms < kNoAllocMaxBlocks ? sms : kNoAllocMaxBlocks;
-    unsigned long long max_blocks = (pb.units + threads - 1) / threads;
+    const unsigned long long units = pb.deriv ? pb.units >> 1 : pb.units;  // as the allocating call shapes it
+    unsigned long long max_blocks = (units + threads - 1) / threads;
     if ((unsigned long long)blocks > max_blocks) blocks = (int)max_blocks;
     if (blocks < 1) blocks = 1;
     pb.grid = blocks;

@@ -43,6 +43,31 @@ __device__ __forceinline__ double group_sum_real_rt(const double* xh, const doub
     return p0;
 }
 
+// One group of G terms of the derivative walk, bitwise identical to
+// unit_sum_deriv<N,G>'s group.
+__device__ __forceinline__ double group_sum_deriv_rt(const double* xh, const double* de, int n, int G, int rs)
+{
+    double p[4], q[4];
+    for (int i = 0; i < G; ++i) p[i] = add_rn(xh[0], de[i]);
+    for (int r = 1; r < n; ++r)
+        for (int i = 0; i < G; ++i) {
+            const double x = add_rn(xh[r], de[r * rs + i]);
+            q[i] = r == 1 ? add_rn(x, p[i]) : __fma_rn(q[i], x, p[i]);
+            p[i] = mul_rn(p[i], x);
+        }
+    if (G == 4) return sub_rn(sub_rn(q[0], q[1]), sub_rn(q[2], q[3]));
+    if (G == 2) return sub_rn(q[0], q[1]);
+    return q[0];
+}
+
+// (p, q) <- (p y, q y + p): one more factor x + t of the derivative's product.
+// q comes out unnormalised (dd_add_fast), which dd_mul takes.
+__device__ __forceinline__ void deriv_step(dd& p, dd& q, dd y)
+{
+    q = dd_add_fast(dd_mul(q, y), p);
+    p = dd_mul(p, y);
+}
+
 // The refinement bin: the lowest bin b such that the units below it, left in
 // FP64, have an expected rounding error sqrt(sum t^2 * k/12) * 2^-52 (k rounded
 // operations per term) within half the tolerance of the walk's magnitude
@@ -68,13 +93,19 @@ __host__ __device__ constexpr int hist_pad_index(int b)
 }
 constexpr int kHistPadded = 32 * (kHistBins / 32 + 1);
 
-__device__ __forceinline__ ThresholdPick pick_threshold_shared(const Problem& pb, double mag, const double* s_s2,
-                                                               const unsigned long long* s_cnt)
+__device__ __forceinline__ ThresholdPick pick_threshold_shared(const Problem& pb, bool deriv, double mag,
+                                                               const double* s_s2, const unsigned long long* s_cnt)
 {
     constexpr int kPer = kHistBins / 32;
     const int lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
-    const double k = pb.comps == 1 ? 2.0 * pb.n : 6.0 * pb.n;
+    // Rounded operations per term.  The real derivative walk counts six times
+    // as many variances as a term has roundings (2n): over permuted copies of
+    // U[0,1) matrices of n = 24 .. 32 the refined results spread by up to ten
+    // times the plain estimate, in either walk, and this keeps the derivative
+    // walk's spread at or below the plain walk's (n=31: 3.2e-13 without it,
+    // 1.3e-13 for the plain walk) for a few hundred refined units more.
+    const double k = pb.comps == 1 ? (deriv ? 12.0 : 2.0) * pb.n : 6.0 * pb.n;
     const double var_per_s2 = mul_rn(k / 12.0, 0x1p-104);
     const double half = mul_rn(0.5 * pb.tol, mag);
     const double budget = mag > 0.0 ? mul_rn(half, half) : 0.0;
@@ -117,7 +148,7 @@ __device__ __forceinline__ ThresholdPick pick_threshold_shared(const Problem& pb
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) first = min(first, __shfl_xor_sync(full, first, d));
     // b: the first bin >= b0 whose tail holds at most units/8 units.
-    const unsigned long long cap = pb.units / 8;
+    const unsigned long long cap = eff_units(pb, deriv) / 8;
     int bsel = kHistBins;
     unsigned long long tail = after;  // units in bins >= the current one, walking down
 #pragma unroll

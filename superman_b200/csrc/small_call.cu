@@ -8,7 +8,9 @@
 // kernels.  Here every CTA of a persistent grid (one per SM, launched
 // cooperatively so that all are resident) does the whole call:
 //   0. builds the tables the walk reads in its own shared memory from the
-//      matrix: row scaling by powers of two, the double-double NW start vector
+//      matrix: row scaling by powers of two, the pivot column and the rows'
+//      quotients by it (the derivative walk, dense_impl.cuh; the plain walk's
+//      entries when there is no pivot), the double-double NW start vector
 //      and subset-sum table, the high columns and the per-row bound ranges,
 //      with the operations of setup_kernel, so the values are the same;
 //      CTA 0 also zeroes the call's global accumulators; grid barrier;
@@ -59,22 +61,27 @@ __host__ __device__ constexpr size_t even(size_t v) { return (v + 1) & ~(size_t)
 // Shared-memory layout, in doubles from the dynamic base; every array
 // starts 16-byte aligned (the evaluators read the table with 16-byte loads).
 struct SmallLayout {
-    size_t a, x0h, x0l, dh, dl, mt, base, bnd, xw, hist, total;
+    size_t a, al, x0h, x0l, dh, dl, mt, ml, base, bnd, xw, hist, total;
     __host__ __device__ SmallLayout(int n, int w, int threads)
     {
         const size_t terms = (size_t)1 << w, ntop = n - 1 - w > 0 ? n - 1 - w : 0;
         const size_t warps = threads / 32;
-        a = 0;
-        x0h = even(a + (size_t)n * n);
+        x0h = 0;
         x0l = even(x0h + n);
         dh = even(x0l + n);
         dl = even(dh + terms * n);
         mt = even(dl + terms * n);
-        // [warps][n][33] the walk's unit bases (hi words); after the walk, the
-        // staged histogram (2 x kHistPadded doubles)
-        base = even(mt + ntop * n);
-        const size_t nb = warps * (size_t)n * 33 > 2 * (size_t)kHistPadded ? warps * (size_t)n * 33
-                                                                           : 2 * (size_t)kHistPadded;
+        // While the tables are built, [n][n] the scaled matrix, then the walked
+        // columns' entries or quotients, and their low words; in the walk,
+        // [warps][n][33] the unit bases (hi words); after it, the staged
+        // histogram (2 x kHistPadded doubles)
+        ml = even(mt + ntop * n);
+        base = even(ml + ntop * n);
+        size_t nb = warps * (size_t)n * 33;
+        if (nb < 2 * (size_t)kHistPadded) nb = 2 * (size_t)kHistPadded;
+        if (nb < 2 * even((size_t)n * n)) nb = 2 * even((size_t)n * n);
+        a = base;
+        al = a + even((size_t)n * n);
         bnd = even(base + nb);
         xw = even(bnd + 2 * (size_t)n);          // [2n] the refined unit's base, hi then lo
         hist = even(xw + 2 * (size_t)n);          // float[kHistBins] + unsigned[kHistBins]
@@ -125,22 +132,25 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
     cg::grid_group grid = cg::this_grid();
     extern __shared__ __align__(16) double smem[];
     __shared__ int s_exp[N];
+    __shared__ int s_pivot;
     __shared__ dd s_warp[32];
     __shared__ dd s_total;
     __shared__ int s_thr;
     __shared__ unsigned long long s_count;
     __shared__ double s_err;
     __shared__ int s_last;
-    const int w = pb.w, terms = 1 << w, nq = terms / G, ntop = N - 1 - w;
+    const int w = pb.w, terms = 1 << w, nq = terms / G;
     const int tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, wid = tid >> 5;
     const int mode = pb.mode;
     const SmallLayout L(N, w, bd);
     double* s_a = smem + L.a;
+    double* s_al = smem + L.al;
     double* s_x0h = smem + L.x0h;
     double* s_x0l = smem + L.x0l;
     double* s_dh = smem + L.dh;
     double* s_dl = smem + L.dl;
     double* s_mt = smem + L.mt;
+    double* s_ml = smem + L.ml;
     double* s_bnd = smem + L.bnd;
     float* s_hist = reinterpret_cast<float*>(smem + L.hist);
     unsigned* s_cnt = reinterpret_cast<unsigned*>(s_hist + kHistBins);
@@ -182,10 +192,48 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
             if (mx > 0.0 && isfinite(mx)) frexp(mx, &e);
             s_exp[r] = e;
         }
+        const int e = __shfl_sync(0xffffffffu, lane == 0 ? s_exp[r] : 0, 0);
+        if (lane < N) s_a[r * N + lane] = ldexp(s_a[r * N + lane], -e);
     }
     __syncthreads();
-    for (int i = tid; i < N * N; i += bd) s_a[i] = ldexp(s_a[i], -s_exp[i / N]);
-    __syncthreads();
+    // the pivot column, picked alike in every CTA
+    int pivot = -1;
+    if constexpr (N >= kMinDerivReal) {
+        if (wid == 0) {
+            const int pv = pb.deriv != 0 ? pick_pivot<1>(s_a, N) : -1;
+            if (lane == 0) s_pivot = pv;
+        }
+        __syncthreads();
+        pivot = s_pivot;
+    }
+    const bool deriv = N >= kMinDerivReal && pivot >= 0;
+    const int nc = N - (deriv ? 1 : 0), ntop = nc - 1 - w;
+    if (blockIdx.x == 0 && wid == 0) {
+        DerivScale sc{};
+        if (deriv) sc = deriv_scale<1>(N, [&](int r) { return make_double2(s_a[r * N + pivot], 0.0); });
+        if (lane == 0) {
+            pb.rb->pivot = pivot;
+            pb.rb->scale[0] = sc.v.re;
+            pb.rb->scale_exp = sc.e;
+        }
+    }
+    if (deriv) {
+        // row r's quotients by its pivot, packed into columns 0 .. n-2; a warp
+        // per row (it reads its row before it writes it)
+        if (blockIdx.x == 0) __syncthreads();  // deriv_scale has read the pivots
+        for (int r = wid; r < N; r += bd / 32) {
+            const double x = lane < N ? s_a[r * N + lane] : 0.0, d = s_a[r * N + pivot];
+            __syncwarp();
+            if (lane < N && lane != pivot) {
+                const dd v = quotient(x, d);
+                const int j = lane > pivot ? lane - 1 : lane;
+                s_a[r * N + j] = v.hi;
+                s_al[r * N + j] = v.lo;
+            }
+        }
+        __syncthreads();
+    }
+    auto plus = [&](dd x, int i) { return deriv ? dd_step(x, s_a[i], s_al[i]) : dd_add_d(x, s_a[i]); };
     // The NW start vector x0 (one row per lane of the CTA's last warp, n
     // dependent adds each) and the subset-sum table (the other warps, a row
     // each at a time) are built side by side.  A row's table is built level
@@ -198,9 +246,9 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
     if (wid == xwarp && lane < N) {
         const int r = lane;
         dd s = {0.0, 0.0};
-        for (int j = 0; j < N; ++j) s = dd_add_d(s, s_a[r * N + j]);
+        for (int j = 0; j < nc; ++j) s = plus(s, r * N + j);
         dd h = {-0.5 * s.hi, -0.5 * s.lo};  // exact halving
-        dd x = dd_add_d(h, s_a[r * N + (N - 1)]);
+        dd x = plus(h, r * N + nc - 1);
         s_x0h[r] = x.hi;
         s_x0l[r] = x.lo;
     }
@@ -226,11 +274,10 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
             for (int k = 0; k < w; ++k) {
                 __syncwarp();
                 const int half = 1 << k;
-                const double a0 = s_a[r0 * N + k], a1 = two ? s_a[r1 * N + k] : 0.0;
                 for (int e = lane; e < half; e += 32) {
-                    const dd v0 = dd_add_d(dd{s_dh[pos(e, r0)], s_dl[pos(e, r0)]}, a0);
+                    const dd v0 = plus(dd{s_dh[pos(e, r0)], s_dl[pos(e, r0)]}, r0 * N + k);
                     if (two) {
-                        const dd v1 = dd_add_d(dd{s_dh[pos(e, r1)], s_dl[pos(e, r1)]}, a1);
+                        const dd v1 = plus(dd{s_dh[pos(e, r1)], s_dl[pos(e, r1)]}, r1 * N + k);
                         s_dh[pos(half + e, r1)] = v1.hi;
                         s_dl[pos(half + e, r1)] = v1.lo;
                     }
@@ -253,6 +300,7 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
     for (int idx = tid; idx < ntop * N; idx += bd) {
         const int j = idx / N, r = idx % N;
         s_mt[idx] = s_a[r * N + (w + j)];
+        if (deriv) s_ml[idx] = s_al[r * N + (w + j)];
     }
     __syncthreads();
     if (!staged) grid.sync();  // the zeroed accumulators are visible before anyone adds to them
@@ -270,49 +318,51 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
     // owns units t, t + T, t + 2T, ... (T threads in the grid).
     const unsigned long long T = (unsigned long long)gridDim.x * bd;
     const unsigned long long t0 = (unsigned long long)blockIdx.x * bd + tid;
+    const unsigned long long units = eff_units(pb, deriv);
     double* s_base = smem + L.base + (size_t)wid * N * 33;  // [N][33]
     dd tot = {0.0, 0.0};
     int bin0 = -1, bin1 = -1;  // this thread's bins in the first two passes (listing reads the rest back)
     for (unsigned long long u = t0;; u += T) {
         const unsigned long long ub = u - (unsigned long long)lane;  // the warp's first unit
-        if (ub >= pb.units) break;  // the same in every lane of the warp
+        if (ub >= units) break;  // the same in every lane of the warp
         __syncwarp();               // the previous pass's bases are read
         if (lane < N) {
             const int r = lane;
             const unsigned long long g = gray_of(ub);
             dd x = {s_x0h[r], s_x0l[r]};
             for (int j = 0; j < ntop; ++j)
-                if ((g >> j) & 1ull) x = dd_add_d(x, s_mt[j * N + r]);
+                if ((g >> j) & 1ull)
+                    x = deriv ? dd_step(x, s_mt[j * N + r], s_ml[j * N + r]) : dd_add_d(x, s_mt[j * N + r]);
             s_base[r * 33] = x.hi;
-            for (int k = 1; k < 32 && ub + k < pb.units; ++k) {
+            for (int k = 1; k < 32 && ub + k < units; ++k) {
                 const unsigned long long v = ub + k;
                 const int j = __ffsll((long long)v) - 1;
+                const bool add = (gray_of(v) >> j) & 1ull;
                 const double c = s_mt[j * N + r];
-                const dd sm = two_sum(x.hi, ((gray_of(v) >> j) & 1ull) ? c : -c);
-                x = fast_two_sum(sm.hi, add_rn(sm.lo, x.lo));
+                const dd sm = two_sum(x.hi, add ? c : -c);
+                double l = x.lo;
+                if (deriv) l = add ? add_rn(l, s_ml[j * N + r]) : sub_rn(l, s_ml[j * N + r]);
+                x = fast_two_sum(sm.hi, add_rn(sm.lo, l));
                 s_base[r * 33 + k] = x.hi;
             }
         }
         __syncwarp();
         int b = -1;  // this lane's histogram bin in this pass (-1: no unit)
         double sq = 0.0;
-        if (u < pb.units) {
+        if (u < units) {
             double xh[N];
 #pragma unroll
             for (int r = 0; r < N; ++r) xh[r] = s_base[r * 33 + lane];
             if (mode == 0) {
-                const double us = unit_sum_real<N, G>(xh, s_dh, nq);
+                const double us = deriv ? unit_sum_deriv<N, G>(xh, s_dh, nq) : unit_sum_real<N, G>(xh, s_dh, nq);
                 tot = dd_add_d(tot, (u & 1ull) ? -us : us);
             } else {
-                double ubd = 1.0;
-#pragma unroll
-                for (int r = 0; r < N; ++r)
-                    ubd = mul_rn(ubd, fmax(fabs(add_rn(xh[r], s_bnd[r])), fabs(add_rn(xh[r], s_bnd[N + r]))));
-                b = hist_bin(ubd);
+                b = hist_bin(deriv ? unit_bound_real<N, true>(xh, s_bnd) : unit_bound_real<N, false>(xh, s_bnd));
                 pb.raw_b[u] = (unsigned short)b;
                 if (u == t0) bin0 = b;
                 else if (u == t0 + T) bin1 = b;
-                const double us = unit_sum_real<N, G, true>(xh, s_dh, nq, &sq);
+                const double us = deriv ? unit_sum_deriv<N, G, true>(xh, s_dh, nq, &sq)
+                                        : unit_sum_real<N, G, true>(xh, s_dh, nq, &sq);
                 tot = dd_add_d(tot, (u & 1ull) ? -us : us);
                 unit_value(pb)[u] = us;  // what the refinement corrects
             }
@@ -376,7 +426,7 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
         if (lane == 0) s_total = v;
         if (mode != 0) {
             const double mag = fabs(v.hi);
-            const ThresholdPick pk = pick_threshold_shared(pb, mag, s_h2, s_hc);
+            const ThresholdPick pk = pick_threshold_shared(pb, deriv, mag, s_h2, s_hc);
             if (lane == 0) {
                 s_thr = pk.thr;
                 s_count = pk.count;
@@ -404,7 +454,7 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
     // (they gather near the empty and the full subsets) spreads over the grid,
     // and each is refined by a whole CTA.
     const int thr = s_thr;
-    for (unsigned long long u = t0; u < pb.units; u += T) {
+    for (unsigned long long u = t0; u < units; u += T) {
         const int b = u == t0 ? bin0 : (u == t0 + T ? bin1 : (int)pb.raw_b[u]);
         if (b >= thr) {
             const unsigned long long k = atomicAdd(pb.list_n, 1ull);
@@ -431,7 +481,8 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
         for (int r = tid; r < N; r += bd) {
             dd x = {s_x0h[r], s_x0l[r]};
             for (int j = 0; j < ntop; ++j)
-                if ((g >> j) & 1ull) x = dd_add_d(x, s_mt[j * N + r]);
+                if ((g >> j) & 1ull)
+                    x = deriv ? dd_step(x, s_mt[j * N + r], s_ml[j * N + r]) : dd_add_d(x, s_mt[j * N + r]);
             xw[r] = x.hi;
             xw[N + r] = x.lo;
         }
@@ -440,10 +491,18 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
         // `per` threads, joined by shuffles
         dd acc = {0.0, 0.0};
         for (int d = tid / per; d < terms; d += bd / per) {
-            dd p = {1.0, 0.0};
-            for (int r = r0; r < r1; ++r)
-                p = dd_mul(p, dd_add_fast(dd{xw[r], xw[N + r]}, dd{s_dh[pos(d, r)], s_dl[pos(d, r)]}));
-            for (int off = 1; off < per; off <<= 1) p = dd_mul(p, shfl_xor_dd(p, off));
+            dd p = {1.0, 0.0}, q = {0.0, 0.0};
+            for (int r = r0; r < r1; ++r) {
+                const dd y = dd_add_fast(dd{xw[r], xw[N + r]}, dd{s_dh[pos(d, r)], s_dl[pos(d, r)]});
+                if (deriv) deriv_step(p, q, y);
+                else p = dd_mul(p, y);
+            }
+            for (int off = 1; off < per; off <<= 1) {
+                const dd po = shfl_xor_dd(p, off), qo = shfl_xor_dd(q, off);
+                if (deriv) q = dd_add(dd_mul(q, po), dd_mul(p, qo));
+                p = dd_mul(p, po);
+            }
+            if (deriv) p = q;
             if (sub == 0) acc = (__popc(d) & 1) ? dd_add(acc, dd_neg(p)) : dd_add(acc, p);
         }
         acc = block_sum_dd(acc, s_warp);

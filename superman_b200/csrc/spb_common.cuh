@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cmath>
+
 #include "superman_b200.h"
 
 #define SPB_CUDA_TRY(expr)                                                     \
@@ -99,13 +101,22 @@ __host__ __device__ __forceinline__ dd dd_add_fast(dd a, dd b)
     return {s.hi, add_rn(s.lo, add_rn(a.lo, b.lo))};
 }
 
-// (a.hi + a.lo) * (b.hi + b.lo) to ~2^-104 relative (Dekker product with FMA).
-__device__ __forceinline__ dd dd_mul(dd a, dd b)
+__host__ __device__ __forceinline__ double fma_rn(double a, double b, double c)
 {
-    double p = __dmul_rn(a.hi, b.hi);
-    double e = __fma_rn(a.hi, b.hi, -p);
-    e = __fma_rn(a.hi, b.lo, e);
-    e = __fma_rn(a.lo, b.hi, e);
+#ifdef __CUDA_ARCH__
+    return __fma_rn(a, b, c);
+#else
+    return std::fma(a, b, c);
+#endif
+}
+
+// (a.hi + a.lo) * (b.hi + b.lo) to ~2^-104 relative (Dekker product with FMA).
+__host__ __device__ __forceinline__ dd dd_mul(dd a, dd b)
+{
+    double p = mul_rn(a.hi, b.hi);
+    double e = fma_rn(a.hi, b.hi, -p);
+    e = fma_rn(a.hi, b.lo, e);
+    e = fma_rn(a.lo, b.hi, e);
     return fast_two_sum(p, e);
 }
 

@@ -1,0 +1,178 @@
+"""The derivative walk (rows divided by a pivot column, half the subsets) and
+the plain walk it falls back to when every column holds a zero: both against
+the exact permanent, at the smallest sizes, with the pivot at either end, with
+pivots far from the rows' maxima, and over each way units are listed for the
+double-double refinement."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from superman_b200 import _lib
+from superman_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+_exact = {}
+
+
+def EXACT(oracle, a):
+    """The oracle's exact value, kept per matrix (seconds each at n = 23)."""
+    k = a.tobytes()
+    if k not in _exact:
+        _exact[k] = oracle.exact_perm_complex(a) if np.iscomplexobj(a) else oracle.exact_perm(a)
+    return _exact[k]
+
+
+def full(r):
+    return r.permanent + r.permanent_lo
+
+
+def no_pivot(a, seed):
+    """One zero in every column, at different rows: no column can be divided by."""
+    a = a.copy()
+    n = a.shape[0]
+    a[np.random.default_rng(seed).permutation(n), np.arange(n)] = 0.0
+    return a
+
+
+def only_pivot(a, c, seed):
+    """Column c is the only one without a zero."""
+    b = no_pivot(a, seed)
+    b[:, c] = a[:, c] + 0.25
+    return b
+
+
+@pytest.mark.parametrize("small_call", [0, -1])
+@pytest.mark.parametrize("precision", ["fp64", "dd"])
+@pytest.mark.parametrize("n", [22, 23])
+def test_real_pivot_and_no_pivot(spb, oracle, n, precision, small_call):
+    u = W.dense_uniform(n, 40 + n)
+    for a in (u, no_pivot(u, n), only_pivot(u, 0, n), only_pivot(u, n - 1, n)):
+        r = spb.perm_dense(a, precision=precision, small_call=small_call, sparse_walk=1)
+        # FP64 products in an alternating sum: kappa sqrt(n/6) 2^-52, kappa about 2e2
+        assert oracle.rel_err(full(r), EXACT(oracle, a)) <= (4e-13 if precision == "fp64" else 2e-13)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "dd"])
+@pytest.mark.parametrize("n", [21, 22])
+def test_complex_pivot_and_no_pivot(spb, oracle, n, precision):
+    u = W.haar_block(n, 60 + n, N=64)
+    for a in (u, no_pivot(u, n), only_pivot(u, 0, n)):
+        er, ei = EXACT(oracle, a)
+        r = spb.perm_complex(a, precision=precision)
+        scale = float(np.prod(np.abs(a).sum(axis=1)))
+        assert abs(r.permanent - complex(float(er), float(ei))) <= 1e-14 * scale
+
+
+def test_pivots_far_from_the_row_maxima(spb, oracle):
+    """A small entry in every column: quotients up to 2^30 times the row's scale
+    keep the range (derivative walk).  Rows 2^-50 outside one entry: products of
+    quotients would reach 2^1100, and the plain walk runs."""
+    n = 23
+    u = W.dense_uniform(n, 5) + 0.5
+    one = np.eye(n, dtype=bool)
+    for a in (np.where(one, u * 2.0 ** -30, u), np.where(one, u, u * 2.0 ** -50)):
+        for small_call in (0, -1):
+            r = spb.perm_dense(a, precision="dd", small_call=small_call)
+            assert oracle.rel_err(full(r), EXACT(oracle, a)) <= 2e-13
+
+
+@pytest.mark.parametrize("pivot", [True, False])
+def test_refinement_listings_agree(spb, oracle, pivot):
+    """Many units refined (signed entries, tight tolerance): the first pass's
+    list, the fused call's list and the replay select the same units."""
+    a = np.random.default_rng(5).standard_normal((23, 23))
+    if not pivot:
+        a = no_pivot(a, 7)
+    kw = dict(precision="dd", rel_tol=1e-16, sparse_walk=1)
+    exact = EXACT(oracle, a)
+    rs = [spb.perm_dense(a, small_call=0, **kw), spb.perm_dense(a, small_call=-1, **kw),
+          spb.perm_dense(a, replay_listing=1, **kw)]
+    assert rs[0].refined_units == rs[1].refined_units == rs[2].refined_units > 0
+    for r in rs:
+        assert oracle.rel_err(full(r), exact) <= 1e-12
+
+
+def test_complex_refinement_listings_agree(spb, oracle):
+    rng = np.random.default_rng(8)
+    a = rng.standard_normal((22, 22)) + 1j * rng.standard_normal((22, 22))
+    er, ei = EXACT(oracle, a)
+    ex = complex(float(er), float(ei))
+    r1 = spb.perm_complex(a, precision="dd", rel_tol=1e-16)
+    r2 = spb.perm_complex(a, precision="dd", rel_tol=1e-16, replay_listing=1)
+    assert r1.refined_units == r2.refined_units > 0
+    assert abs(r1.permanent - ex) <= 1e-13 * abs(ex) and abs(r2.permanent - ex) <= 1e-13 * abs(ex)
+
+
+@pytest.mark.parametrize("n", [30, 31])
+def test_bound_pass_sizes(spb, n):
+    """n = 30 (2^20 units: every unit listed, the bound pass ends at once) and
+    31 (listed from the bound pass's bin): the transpose agrees."""
+    a = W.dense_uniform(n, 300 + n)
+    r1 = spb.perm_dense(a, precision="dd")
+    r2 = spb.perm_dense(np.ascontiguousarray(a.T), precision="dd")
+    assert r1.refined_units > 0
+    assert abs(full(r1) - full(r2)) <= 3e-13 * abs(full(r1))  # as the n = 32 transpose test
+
+
+@pytest.mark.parametrize("n", [10, 11, 12, 16, 18])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_batch_mixes_both_walks(spb, oracle, n, cplx):
+    """Matrices with and without a pivot in one launch, each on one warp or
+    (n >= 16, a launch this small) shared by the CTAs of a cluster."""
+    import torch
+    mats = []
+    for k in range(9):
+        u = W.haar_block(n, 900 + k, N=64) if cplx else W.dense_uniform(n, 900 + k)
+        mats.append(u if k % 3 == 0 else no_pivot(u, k) if k % 3 == 1 else only_pivot(u, k % n, k))
+    m = np.ascontiguousarray(np.stack(mats))
+    d = torch.from_numpy(m.view(np.float64)).cuda()
+    c = 2 if cplx else 1
+    out = torch.full((len(mats), c, 2), float("nan"), dtype=torch.float64, device="cuda")
+    _lib.check(_lib.lib().spb_perm_batch_dev(ctypes.c_void_p(d.data_ptr()), n, int(cplx), len(mats),
+                                             ctypes.c_void_p(out.data_ptr()), None))
+    torch.cuda.synchronize()
+    o = out.cpu().numpy()
+    for k, a in enumerate(mats):
+        scale = float(np.prod(np.abs(a).sum(axis=1)))
+        if cplx:
+            er, ei = EXACT(oracle, a)
+            assert abs(complex(o[k, 0, 0], o[k, 1, 0]) - complex(float(er), float(ei))) <= 1e-14 * scale
+        else:
+            assert oracle.rel_err(o[k, 0, 0], EXACT(oracle, a)) <= 1e-13
+
+
+@pytest.mark.parametrize("n,cplx", [(16, False), (19, False), (21, True), (24, False), (24, True)])
+def test_batch_split_is_the_same_as_alone(spb, n, cplx):
+    """A launch of few matrices splits each over a cluster, a launch of many
+    gives each a warp: the same units, so the same values to the
+    double-double sum's order."""
+    import torch
+    few, many = 2, 600 if n <= 21 else 470
+    u = [W.haar_block(n, 40 + k, N=64) if cplx else W.dense_uniform(n, 40 + k) for k in range(few)]
+    got = []
+    for count in (few, many):
+        m = np.ascontiguousarray(np.stack([u[k % few] for k in range(count)]))
+        d = torch.from_numpy(m.view(np.float64)).cuda()
+        out = torch.zeros((count, 2 if cplx else 1, 2), dtype=torch.float64, device="cuda")
+        _lib.check(_lib.lib().spb_perm_batch_dev(ctypes.c_void_p(d.data_ptr()), n, int(cplx), count,
+                                                 ctypes.c_void_p(out.data_ptr()), None))
+        torch.cuda.synchronize()
+        got.append(out.cpu().numpy())
+    for k in range(many):
+        a, b = got[0][k % few, :, 0], got[1][k, :, 0]
+        assert np.all(np.abs(a - b) <= 2.0 ** -52 * np.abs(a)), (k, a, b)
+
+
+def test_noalloc_without_a_pivot(spb):
+    import torch
+    a = no_pivot(W.dense_uniform(24, 3), 4)
+    d = torch.from_numpy(a).cuda()
+    out = torch.zeros(2, dtype=torch.float64, device="cuda")
+    _lib.check(_lib.lib().spb_perm_dense_f64_noalloc(ctypes.c_void_p(d.data_ptr()), 24,
+                                                     ctypes.c_void_p(out.data_ptr()), None))
+    torch.cuda.synchronize()
+    want = spb.perm_dense(a, small_call=-1, sparse_walk=1).permanent
+    assert abs(float(out[0]) - want) <= 1e-13 * abs(want)
