@@ -361,7 +361,7 @@ __device__ __forceinline__ uint32_t term_expanded(const int (&xt)[N], const int*
     long long W0, Q0;
     word_dual<N, G, 0>(xt, de, i, m, W0, Q0);
     if constexpr (rows_in_half(N, 2) > 0) {
-        if (m > 2 * half_rows(N)) {
+        if (m > 3 * half_rows(N)) {
             long long W1, Q1;
             word_dual<N, G, 1>(xt, de, i, m, W1, Q1);
             // Q0 W1 + W0 Q1, signed 128 bits (4K rows below (2^31)^4)
@@ -377,6 +377,37 @@ __device__ __forceinline__ uint32_t term_expanded(const int (&xt)[N], const int*
             p[1] = (uint32_t)(l0 >> 32);
             p[2] = (uint32_t)h0;
             p[3] = (uint32_t)(h0 >> 32);
+        } else if (m > 2 * half_rows(N)) {
+            // three halves (Bernoulli(0.5) columns at n = 36 mostly hold 11 to 14
+            // ones, two or three halves): (Q0 c + W0 q) d with the third half's
+            // product c (its sign moved to sg and q) and derivative q, and the
+            // fourth's product d: 96 bits, then one 32-bit factor
+            int c, q, d = 1;
+            half_any<N, G, 2>(xt, de, i, m, c, q);
+            if constexpr (rows_in_half(N, 3) > 0) d = half_plain<N, G, 3>(xt, de, i);
+            const int sc = c >> 31;
+            sg ^= (uint32_t)sc;
+            const uint32_t cm = (uint32_t)((c ^ sc) - sc);
+            const int qs = (q ^ sc) - sc;
+            const unsigned long long al = (unsigned long long)(uint32_t)Q0 * cm;
+            const long long ah = (Q0 >> 32) * (long long)cm + (long long)(al >> 32);
+            const long long bl = (long long)(uint32_t)W0 * (long long)qs;
+            const long long bh = (W0 >> 32) * (long long)qs + (bl >> 32);
+            const unsigned long long lo = (unsigned long long)(uint32_t)al + (uint32_t)bl;
+            const long long hi = ah + bh + (long long)(lo >> 32);  // 3K rows below 2^94
+            const uint32_t s = (uint32_t)(hi >> 63);
+            const unsigned long long l0 = (unsigned long long)((uint32_t)lo ^ s) + (s & 1u);
+            const unsigned long long h0 = ((unsigned long long)hi ^ (unsigned long long)(hi >> 63)) + (l0 >> 32);
+            const int sd = d >> 31;
+            sg ^= s ^ (uint32_t)sd;
+            const uint32_t dm = (uint32_t)((d ^ sd) - sd);
+            const unsigned long long t0 = (unsigned long long)(uint32_t)l0 * dm;
+            const unsigned long long t1 = (unsigned long long)(uint32_t)h0 * dm + (t0 >> 32);
+            const unsigned long long t2 = (h0 >> 32) * dm + (t1 >> 32);
+            p[0] = (uint32_t)t0;
+            p[1] = (uint32_t)t1;
+            p[2] = (uint32_t)t2;
+            p[3] = (uint32_t)(t2 >> 32);
         } else {
             const unsigned long long q = magnitude(Q0, sg);
             p[0] = (uint32_t)q;
@@ -434,11 +465,12 @@ __device__ __forceinline__ void shfl_add(uint32_t (&v)[L], int m)
 
 // Threads per CTA.  Plain walk: 512 (128 registers) keeps 4 limbs spill-free up
 // to n = 28; larger n or more limbs get 255 registers at 256 threads.  Expanded
-// walk, which holds fewer limbs at a time: 512 up to n = 36 (126 registers at
-// n = 36 with 5 limbs), 384 (168 registers) up to n = 44, then 256.
+// walk, which holds fewer limbs at a time: 512 up to n = 40 (126 registers at
+// n = 36 with 5 limbs; n = 37 and 38 spill, and still take 393 and 798 ms
+// against 436 and 854 at 384 threads), 384 (168 registers) up to n = 44, then 256.
 __host__ __device__ constexpr int bin_max_threads(int n, int limbs, bool x)
 {
-    if (x) return n <= 36 ? 512 : (n <= 44 ? 384 : 256);
+    if (x) return n <= 40 ? 512 : (n <= 44 ? 384 : 256);
     return (limbs <= 4 && n <= 28) ? 512 : 256;
 }
 
