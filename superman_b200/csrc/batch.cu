@@ -8,7 +8,10 @@
 // high columns in the warp's slice of shared memory, then its 32 lanes split
 // the Gray units of that matrix exactly as the threads of the big walk do
 // (same unit evaluators; the double-double unit bases live in registers), and
-// a warp reduction gives the double-double total.  The permanent of matrix m
+// a warp reduction gives the double-double total.  A matrix with a pivot column
+// (dense_impl.cuh) takes the derivative walk, half the subsets at 3/4 (complex
+// 5/6) of the FP64 instructions, the others the plain walk; the choice is the
+// warp's own.  The permanent of matrix m
 // is written as (hi, lo) per component: out[m*2*comps + 2*c + {0, 1}].
 //
 // Device pointers only, no allocation, no host synchronisation: the serving
@@ -25,12 +28,14 @@ namespace batch {
 
 constexpr int kWarpsPerCta = 4;
 
-template <int N, int C>
+// D: the derivative walk.
+template <int N, int C, bool D>
 struct Cfg {
-    static constexpr int W = (N - 1) < 5 ? (N - 1) : 5;  // low column bits per unit
+    static constexpr int NC = N - (D ? 1 : 0);           // walked columns
+    static constexpr int W = NC - 1 < 5 ? NC - 1 : 5;    // low column bits per unit
     static constexpr int G = C == 1 ? (W >= 2 ? 4 : (W == 1 ? 2 : 1)) : (W >= 1 ? 2 : 1);
     static constexpr int TERMS = 1 << W;
-    static constexpr int NTOP = N - 1 - W;
+    static constexpr int NTOP = NC - 1 - W;
     static constexpr int NTP = NTOP > 0 ? NTOP : 0;
     // Unit-base lo words: registers, except complex n >= 21, where hi and lo
     // of both parts (4n doubles) would spill; there they sit in a lane-private
@@ -38,13 +43,152 @@ struct Cfg {
     // per-unit traffic costs more than it saves wherever registers suffice.)
     static constexpr bool LO_SMEM = C == 2 && N >= 21;
     static constexpr int LO_DOUBLES = LO_SMEM ? 32 * N * C : 0;
-    // doubles per warp: DE table, high columns, x0 hi/lo, lo words, row
-    // exponents (as doubles), rounded up to 32 bytes: the unit evaluator reads
-    // the DE table with 16-byte vector loads, so every warp's slice must start
-    // aligned.
-    static constexpr int SMEM_DOUBLES = (TERMS * N * C + NTP * N * C + 2 * N * C + LO_DOUBLES + N + 3) / 4 * 4;
+    // doubles per warp: DE table, walked columns (with low words in the
+    // derivative walk), x0 hi/lo, lo words, row exponents (as doubles),
+    // rounded up to 32 bytes: the unit evaluator reads the DE table with
+    // 16-byte vector loads, so every warp's slice must start aligned.
+    static constexpr int SMEM_DOUBLES =
+        (TERMS * N * C + (D ? 2 : 1) * NC * N * C + 2 * N * C + LO_DOUBLES + N + 3) / 4 * 4;
     static_assert(SMEM_DOUBLES % 4 == 0, "per-warp shared slice must keep 32-byte alignment");
 };
+
+// Sizes that have a derivative walk, and the slice that holds either walk.
+// Below n = 11 the pivot and the quotients cost a matrix more than the walk saves
+// (4096 matrices on one B200, plain against derivative: n=8 real 25.6 and 27.7 us,
+// complex 60.7 and 64.0; n=12 real 52.4 and 46.2, n=14 complex 347 and 295).
+__host__ __device__ constexpr bool has_deriv(int n) { return n >= 11; }
+template <int N, int C>
+constexpr int slice_doubles()
+{
+    constexpr int p = Cfg<N, C, false>::SMEM_DOUBLES;
+    if constexpr (has_deriv(N)) {
+        constexpr int d = Cfg<N, C, true>::SMEM_DOUBLES;
+        return d > p ? d : p;
+    }
+    return p;
+}
+
+// One matrix, its rows' scaling exponents in s_exp: tables in the warp's slice,
+// the walk, the warp's total (in every lane).  pivot: the derivative walk's
+// column.
+template <int N, int C, bool D>
+__device__ __forceinline__ void walk_matrix(const double* __restrict__ A, const int* s_exp, int pivot, double* slice,
+                                            int lane, dd (&tot)[C])
+{
+    using Q = Cfg<N, C, D>;
+    constexpr int G = Q::G, TERMS = Q::TERMS, NTOP = Q::NTOP, NTP = Q::NTP, W = Q::W, NC = Q::NC;
+    double* s_de = slice;                    // [C][TERMS/G][N][G]
+    double* s_col = s_de + TERMS * N * C;    // [C][NC][N] walked columns: entries or quotients
+    double* s_cl = s_col + NC * N * C;       // their low words (derivative walk)
+    double* s_x0h = s_cl + (D ? NC * N * C : 0);  // [C][N]
+    double* s_x0l = s_x0h + N * C;           // [C][N]
+    double* s_lo = s_x0l + N * C;            // [C][N][32] lane-private lo words (LO_SMEM)
+    const double* s_mt = s_col + W * N;      // high columns of part c at + c * NC * N
+    const double* s_ml = s_cl + W * N;
+    for (int idx = lane; idx < NC * N; idx += 32) {
+        const int j = idx / N, r = idx % N, src = D && j >= pivot ? j + 1 : j;
+        const double* row = A + (size_t)r * N * C;
+        if constexpr (!D) {
+#pragma unroll
+            for (int c = 0; c < C; ++c) s_col[c * NC * N + idx] = ldexp(row[src * C + c], -s_exp[r]);
+        } else if constexpr (C == 1) {
+            const dd v = dense::quotient(ldexp(row[src], -s_exp[r]), ldexp(row[pivot], -s_exp[r]));
+            s_col[idx] = v.hi;
+            s_cl[idx] = v.lo;
+        } else {
+            const dense::ddc v = dense::quotient_c(
+                ldexp(row[2 * src], -s_exp[r]), ldexp(row[2 * src + 1], -s_exp[r]), ldexp(row[2 * pivot], -s_exp[r]),
+                ldexp(row[2 * pivot + 1], -s_exp[r]));
+            s_col[idx] = v.re.hi;
+            s_cl[idx] = v.re.lo;
+            s_col[NC * N + idx] = v.im.hi;
+            s_cl[NC * N + idx] = v.im.lo;
+        }
+    }
+    __syncwarp();
+    auto plus = [&](dd x, int i) { return D ? dense::dd_step(x, s_col[i], s_cl[i]) : dd_add_d(x, s_col[i]); };
+    // NW start vector (double-double)
+    for (int rr = lane; rr < N * C; rr += 32) {
+        const int r = rr / C, part = rr % C;
+        dd s = {0.0, 0.0};
+        for (int j = 0; j < NC; ++j) s = plus(s, (part * NC + j) * N + r);
+        dd h = {-0.5 * s.hi, -0.5 * s.lo};
+        dd x = plus(h, (part * NC + NC - 1) * N + r);
+        s_x0h[part * N + r] = x.hi;
+        s_x0l[part * N + r] = x.lo;
+    }
+    // low-column subset sums, grouped [part][d/G][r][d%G]
+    for (int idx = lane; idx < TERMS * N * C; idx += 32) {
+        const int part = idx / (TERMS * N), rem = idx % (TERMS * N);
+        const int d = rem / N, r = rem % N;
+        dd s = {0.0, 0.0};
+        for (int j = 0; j < W; ++j)
+            if ((d >> j) & 1) s = plus(s, (part * NC + j) * N + r);
+        s_de[part * TERMS * N + ((d / G) * N + r) * G + (d % G)] = s.hi;
+    }
+    __syncwarp();
+
+    unsigned long long u0, u1;
+    balanced_range(1ull << NTP, 32, lane, &u0, &u1);
+#pragma unroll
+    for (int c = 0; c < C; ++c) tot[c] = {0.0, 0.0};
+    if (u0 < u1) {
+        // unit base: hi words in registers; lo words in registers or in the
+        // lane's shared slot (element (c, r) at [(c * N + r) * 32 + lane])
+        double xh[C][N];
+        double xlr[Q::LO_SMEM ? 1 : C * N];
+        double* xl = Q::LO_SMEM ? s_lo + lane : xlr;
+        constexpr int LS = Q::LO_SMEM ? 32 : 1;  // stride between elements
+        const unsigned long long g0 = gray_of(u0);
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+#pragma unroll
+            for (int r = 0; r < N; ++r) {
+                dd x = {s_x0h[c * N + r], s_x0l[c * N + r]};
+                for (int j = 0; j < NTOP; ++j)
+                    if ((g0 >> j) & 1ull) x = plus(x, (c * NC + W + j) * N + r);
+                xh[c][r] = x.hi;
+                xl[(c * N + r) * LS] = x.lo;
+            }
+        unsigned long long u = u0;
+        while (true) {
+            if constexpr (C == 1) {
+                const double us = D ? dense::unit_sum_deriv<N, G>(xh[0], s_de, TERMS / G)
+                                    : dense::unit_sum_real<N, G>(xh[0], s_de, TERMS / G);
+                tot[0] = dd_add_d(tot[0], (u & 1ull) ? -us : us);
+            } else {
+                double ur, ui;
+                if constexpr (D)
+                    dense::unit_sum_complex_deriv<N, G>(xh[0], xh[C - 1], s_de, s_de + TERMS * N, TERMS / G, ur, ui);
+                else
+                    dense::unit_sum_complex<N, G>(xh[0], xh[C - 1], s_de, s_de + TERMS * N, TERMS / G, ur, ui);
+                if (u & 1ull) { ur = -ur; ui = -ui; }
+                tot[0] = dd_add_d(tot[0], ur);
+                tot[C - 1] = dd_add_d(tot[C - 1], ui);
+            }
+            if (++u >= u1) break;
+            const int j = __ffsll((long long)u) - 1;
+            const bool add = (gray_of(u) >> j) & 1ull;
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+#pragma unroll
+                for (int r = 0; r < N; ++r) {
+                    const double v = s_mt[(c * NC + j) * N + r];
+                    dd s = two_sum(xh[c][r], add ? v : -v);
+                    double l = xl[(c * N + r) * LS];
+                    if (D) {
+                        const double m = s_ml[(c * NC + j) * N + r];
+                        l = add ? add_rn(l, m) : sub_rn(l, m);
+                    }
+                    dd z = fast_two_sum(s.hi, add_rn(s.lo, l));
+                    xh[c][r] = z.hi;
+                    xl[(c * N + r) * LS] = z.lo;
+                }
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < C; ++c) tot[c] = warp_sum_dd(tot[c]);
+}
 
 // Matrix m of a batch starts at mats + m*N*N*C, or, with an offset table, at
 // mats + offs[m] * kOffsetUnit doubles (the serving loop's device pool).
@@ -59,16 +203,11 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) batch_walk(double* __restri
                                                                  const double* __restrict__ src,
                                                                  int count, double* __restrict__ out)
 {
-    using Q = Cfg<N, C>;
-    constexpr int G = Q::G, TERMS = Q::TERMS, NTOP = Q::NTOP, NTP = Q::NTP, W = Q::W;
+    constexpr int SLICE = slice_doubles<N, C>();
     extern __shared__ __align__(16) double smem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    double* s_de = smem + (size_t)wid * Q::SMEM_DOUBLES;  // [C][TERMS/G][N][G]
-    double* s_mt = s_de + TERMS * N * C;                  // [C][NTOP][N]
-    double* s_x0h = s_mt + NTP * N * C;                   // [C][N]
-    double* s_x0l = s_x0h + N * C;                        // [C][N]
-    double* s_lo = s_x0l + N * C;                         // [C][N][32] lane-private lo words (LO_SMEM)
-    int* s_exp = reinterpret_cast<int*>(s_lo + Q::LO_DOUBLES);  // [N]
+    double* slice = smem + (size_t)wid * SLICE;
+    int* s_exp = reinterpret_cast<int*>(slice + SLICE - N);  // [N], past either walk's arrays
 
     const int total_warps = gridDim.x * kWarpsPerCta;
     for (int m = blockIdx.x * kWarpsPerCta + wid; m < count; m += total_warps) {
@@ -87,90 +226,37 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) batch_walk(double* __restri
             s_exp[r] = e;
         }
         __syncwarp();
-        // NW start vector (double-double)
-        for (int rr = lane; rr < N * C; rr += 32) {
-            const int r = rr / C, part = rr % C;
-            dd s = {0.0, 0.0};
-            for (int j = 0; j < N; ++j) s = dd_add_d(s, ldexp(A[(r * N + j) * C + part], -s_exp[r]));
-            dd h = {-0.5 * s.hi, -0.5 * s.lo};
-            dd x = dd_add_d(h, ldexp(A[(r * N + (N - 1)) * C + part], -s_exp[r]));
-            s_x0h[part * N + r] = x.hi;
-            s_x0l[part * N + r] = x.lo;
-        }
-        // low-column subset sums, grouped [part][d/G][r][d%G]
-        for (int idx = lane; idx < TERMS * N * C; idx += 32) {
-            const int part = idx / (TERMS * N), rem = idx % (TERMS * N);
-            const int d = rem / N, r = rem % N;
-            dd s = {0.0, 0.0};
-            for (int j = 0; j < W; ++j)
-                if ((d >> j) & 1) s = dd_add_d(s, ldexp(A[(r * N + j) * C + part], -s_exp[r]));
-            s_de[part * TERMS * N + ((d / G) * N + r) * G + (d % G)] = s.hi;
-        }
-        // high columns [part][j][r]
-        if constexpr (NTP > 0)
-            for (int idx = lane; idx < NTP * N * C; idx += 32) {
-                const int part = idx / (NTP * N), rem = idx % (NTP * N);
-                const int j = rem / N, r = rem % N;
-                s_mt[idx] = ldexp(A[(r * N + (W + j)) * C + part], -s_exp[r]);
-            }
-        __syncwarp();
-
-        unsigned long long u0, u1;
-        balanced_range(1ull << NTP, 32, lane, &u0, &u1);
         dd tot[C];
-#pragma unroll
-        for (int c = 0; c < C; ++c) tot[c] = {0.0, 0.0};
-        if (u0 < u1) {
-            // unit base: hi words in registers; lo words in registers or in the
-            // lane's shared slot (element (c, r) at [(c * N + r) * 32 + lane])
-            double xh[C][N];
-            double xlr[Q::LO_SMEM ? 1 : C * N];
-            double* xl = Q::LO_SMEM ? s_lo + lane : xlr;
-            constexpr int LS = Q::LO_SMEM ? 32 : 1;  // stride between elements
-            const unsigned long long g0 = gray_of(u0);
-#pragma unroll
-            for (int c = 0; c < C; ++c)
-#pragma unroll
-                for (int r = 0; r < N; ++r) {
-                    dd x = {s_x0h[c * N + r], s_x0l[c * N + r]};
-                    for (int j = 0; j < NTOP; ++j)
-                        if ((g0 >> j) & 1ull) x = dd_add_d(x, s_mt[c * NTP * N + j * N + r]);
-                    xh[c][r] = x.hi;
-                    xl[(c * N + r) * LS] = x.lo;
-                }
-            unsigned long long u = u0;
-            while (true) {
-                if constexpr (C == 1) {
-                    double us = dense::unit_sum_real<N, G>(xh[0], s_de, TERMS / G);
-                    tot[0] = dd_add_d(tot[0], (u & 1ull) ? -us : us);
-                } else {
-                    double ur, ui;
-                    dense::unit_sum_complex<N, G>(xh[0], xh[C - 1], s_de, s_de + TERMS * N, TERMS / G, ur, ui);
-                    if (u & 1ull) { ur = -ur; ui = -ui; }
-                    tot[0] = dd_add_d(tot[0], ur);
-                    tot[C - 1] = dd_add_d(tot[C - 1], ui);
-                }
-                if (++u >= u1) break;
-                const int j = __ffsll((long long)u) - 1;
-                const bool add = (gray_of(u) >> j) & 1ull;
-#pragma unroll
-                for (int c = 0; c < C; ++c)
-#pragma unroll
-                    for (int r = 0; r < N; ++r) {
-                        const double v = s_mt[c * NTP * N + j * N + r];
-                        dd s = two_sum(xh[c][r], add ? v : -v);
-                        dd z = fast_two_sum(s.hi, add_rn(s.lo, xl[(c * N + r) * LS]));
-                        xh[c][r] = z.hi;
-                        xl[(c * N + r) * LS] = z.lo;
-                    }
-            }
+        int pivot = -1;
+        if constexpr (has_deriv(N)) {
+            pivot = dense::pick_pivot(N, [&](int r, int j) {
+                const double* e = A + ((size_t)r * N + j) * C;
+                return ldexp(C == 1 ? fabs(e[0]) : fmax(fabs(e[0]), fabs(e[C - 1])), -s_exp[r]);
+            });
+            if (pivot >= 0) walk_matrix<N, C, true>(A, s_exp, pivot, slice, lane, tot);
         }
-#pragma unroll
-        for (int c = 0; c < C; ++c) tot[c] = warp_sum_dd(tot[c]);
+        if (pivot < 0) walk_matrix<N, C, false>(A, s_exp, pivot, slice, lane, tot);
+        int es = 0;
+        for (int r = 0; r < N; ++r) es += s_exp[r];
+        bool odd = N % 2 != 0;  // perm = (4(nc%2)-2) * total over nc walked columns
+        if constexpr (has_deriv(N))
+            if (pivot >= 0) {  // times the product of the pivots
+                const dense::DerivScale sc = dense::deriv_scale<C>(N, [&](int r) {
+                    const double* d = A + ((size_t)r * N + pivot) * C;
+                    return make_double2(ldexp(d[0], -s_exp[r]), ldexp(d[C - 1], -s_exp[r]));
+                });
+                if constexpr (C == 1) {
+                    tot[0] = dd_mul(tot[0], sc.v.re);
+                } else {
+                    const dense::ddc t = dense::ddc_mul(dense::ddc{tot[0], tot[1]}, sc.v);
+                    tot[0] = t.re;
+                    tot[1] = t.im;
+                }
+                es += sc.e;
+                odd = !odd;
+            }
         if (lane == 0) {
-            int es = 0;
-            for (int r = 0; r < N; ++r) es += s_exp[r];
-            const double sgn = (N % 2) ? 1.0 : -1.0;
+            const double sgn = odd ? 1.0 : -1.0;
 #pragma unroll
             for (int c = 0; c < C; ++c) {
                 out[(size_t)m * 2 * C + 2 * c] = sgn * ldexp(tot[c].hi, es + 1);
@@ -185,7 +271,7 @@ template <int N, int C>
 int launch_n(double* mats, const unsigned* offs, const double* src, int count, double* out, int sms,
              cudaStream_t s)
 {
-    constexpr size_t smem = sizeof(double) * Cfg<N, C>::SMEM_DOUBLES * kWarpsPerCta;
+    constexpr size_t smem = sizeof(double) * slice_doubles<N, C>() * kWarpsPerCta;
     if (smem > 48 * 1024) {
         static cudaError_t attr = cudaFuncSetAttribute(batch_walk<N, C>,
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
