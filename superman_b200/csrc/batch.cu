@@ -17,19 +17,23 @@
 // Device pointers only, no allocation, no host synchronisation: the serving
 // loop captures one launch per batch shape in a CUDA graph, and the
 // decomposition path runs its independent pieces through it.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "batch.h"
 #include "dense_impl.cuh"
 #include "spb_common.cuh"
 
+namespace cg = cooperative_groups;
+
 namespace spb {
 namespace batch {
 
 constexpr int kWarpsPerCta = 4;
+constexpr int kMaxCluster = 8;  // CTAs that may share a matrix (the portable cluster size)
 
-// D: the derivative walk.
-template <int N, int C, bool D>
+// D: the derivative walk; T: threads that share the slice.
+template <int N, int C, bool D, int T>
 struct Cfg {
     static constexpr int NC = N - (D ? 1 : 0);           // walked columns
     static constexpr int W = NC - 1 < 5 ? NC - 1 : 5;    // low column bits per unit
@@ -39,17 +43,17 @@ struct Cfg {
     static constexpr int NTP = NTOP > 0 ? NTOP : 0;
     // Unit-base lo words: registers, except complex n >= 21, where hi and lo
     // of both parts (4n doubles) would spill; there they sit in a lane-private
-    // slot of the warp's shared slice.  (With 32 terms per unit the slot's
+    // slot of the shared slice.  (With 32 terms per unit the slot's
     // per-unit traffic costs more than it saves wherever registers suffice.)
     static constexpr bool LO_SMEM = C == 2 && N >= 21;
-    static constexpr int LO_DOUBLES = LO_SMEM ? 32 * N * C : 0;
-    // doubles per warp: DE table, walked columns (with low words in the
+    static constexpr int LO_DOUBLES = LO_SMEM ? T * N * C : 0;
+    // doubles per slice: DE table, walked columns (with low words in the
     // derivative walk), x0 hi/lo, lo words, row exponents (as doubles),
     // rounded up to 32 bytes: the unit evaluator reads the DE table with
-    // 16-byte vector loads, so every warp's slice must start aligned.
+    // 16-byte vector loads, so every slice must start aligned.
     static constexpr int SMEM_DOUBLES =
         (TERMS * N * C + (D ? 2 : 1) * NC * N * C + 2 * N * C + LO_DOUBLES + N + 3) / 4 * 4;
-    static_assert(SMEM_DOUBLES % 4 == 0, "per-warp shared slice must keep 32-byte alignment");
+    static_assert(SMEM_DOUBLES % 4 == 0, "shared slice must keep 32-byte alignment");
 };
 
 // Sizes that have a derivative walk, and the slice that holds either walk.
@@ -57,35 +61,49 @@ struct Cfg {
 // (4096 matrices on one B200, plain against derivative: n=8 real 25.6 and 27.7 us,
 // complex 60.7 and 64.0; n=12 real 52.4 and 46.2, n=14 complex 347 and 295).
 __host__ __device__ constexpr bool has_deriv(int n) { return n >= 11; }
-template <int N, int C>
+template <int N, int C, int T>
 constexpr int slice_doubles()
 {
-    constexpr int p = Cfg<N, C, false>::SMEM_DOUBLES;
+    constexpr int p = Cfg<N, C, false, T>::SMEM_DOUBLES;
     if constexpr (has_deriv(N)) {
-        constexpr int d = Cfg<N, C, true>::SMEM_DOUBLES;
+        constexpr int d = Cfg<N, C, true, T>::SMEM_DOUBLES;
         return d > p ? d : p;
     }
     return p;
 }
 
-// One matrix, its rows' scaling exponents in s_exp: tables in the warp's slice,
-// the walk, the warp's total (in every lane).  pivot: the derivative walk's
-// column.
-template <int N, int C, bool D>
+// The threads that share a matrix's tables: one warp, or (CTA) a whole CTA.
+template <bool CTA>
+struct Team {
+    static constexpr int kSize = CTA ? kWarpsPerCta * 32 : 32;
+    __device__ __forceinline__ static int rank() { return CTA ? threadIdx.x : (threadIdx.x & 31); }
+    __device__ __forceinline__ static void sync()
+    {
+        if (CTA) __syncthreads();
+        else __syncwarp();
+    }
+};
+
+// One matrix, its rows' scaling exponents in s_exp: tables in the team's slice,
+// then the walk over part `part` of `parts` teams' units; the warp's total (in
+// every lane).  pivot: the derivative walk's column.
+template <int N, int C, bool D, bool CTA>
 __device__ __forceinline__ void walk_matrix(const double* __restrict__ A, const int* s_exp, int pivot, double* slice,
-                                            int lane, dd (&tot)[C])
+                                            int part, int parts, dd (&tot)[C])
 {
-    using Q = Cfg<N, C, D>;
+    using TM = Team<CTA>;
+    const int rank = TM::rank();
+    using Q = Cfg<N, C, D, TM::kSize>;
     constexpr int G = Q::G, TERMS = Q::TERMS, NTOP = Q::NTOP, NTP = Q::NTP, W = Q::W, NC = Q::NC;
     double* s_de = slice;                    // [C][TERMS/G][N][G]
     double* s_col = s_de + TERMS * N * C;    // [C][NC][N] walked columns: entries or quotients
     double* s_cl = s_col + NC * N * C;       // their low words (derivative walk)
     double* s_x0h = s_cl + (D ? NC * N * C : 0);  // [C][N]
     double* s_x0l = s_x0h + N * C;           // [C][N]
-    double* s_lo = s_x0l + N * C;            // [C][N][32] lane-private lo words (LO_SMEM)
+    double* s_lo = s_x0l + N * C;            // [C][N][threads] thread-private lo words (LO_SMEM)
     const double* s_mt = s_col + W * N;      // high columns of part c at + c * NC * N
     const double* s_ml = s_cl + W * N;
-    for (int idx = lane; idx < NC * N; idx += 32) {
+    for (int idx = rank; idx < NC * N; idx += TM::kSize) {
         const int j = idx / N, r = idx % N, src = D && j >= pivot ? j + 1 : j;
         const double* row = A + (size_t)r * N * C;
         if constexpr (!D) {
@@ -105,10 +123,10 @@ __device__ __forceinline__ void walk_matrix(const double* __restrict__ A, const 
             s_cl[NC * N + idx] = v.im.lo;
         }
     }
-    __syncwarp();
+    TM::sync();
     auto plus = [&](dd x, int i) { return D ? dense::dd_step(x, s_col[i], s_cl[i]) : dd_add_d(x, s_col[i]); };
     // NW start vector (double-double)
-    for (int rr = lane; rr < N * C; rr += 32) {
+    for (int rr = rank; rr < N * C; rr += TM::kSize) {
         const int r = rr / C, part = rr % C;
         dd s = {0.0, 0.0};
         for (int j = 0; j < NC; ++j) s = plus(s, (part * NC + j) * N + r);
@@ -118,7 +136,7 @@ __device__ __forceinline__ void walk_matrix(const double* __restrict__ A, const 
         s_x0l[part * N + r] = x.lo;
     }
     // low-column subset sums, grouped [part][d/G][r][d%G]
-    for (int idx = lane; idx < TERMS * N * C; idx += 32) {
+    for (int idx = rank; idx < TERMS * N * C; idx += TM::kSize) {
         const int part = idx / (TERMS * N), rem = idx % (TERMS * N);
         const int d = rem / N, r = rem % N;
         dd s = {0.0, 0.0};
@@ -126,19 +144,20 @@ __device__ __forceinline__ void walk_matrix(const double* __restrict__ A, const 
             if ((d >> j) & 1) s = plus(s, (part * NC + j) * N + r);
         s_de[part * TERMS * N + ((d / G) * N + r) * G + (d % G)] = s.hi;
     }
-    __syncwarp();
+    TM::sync();
 
     unsigned long long u0, u1;
-    balanced_range(1ull << NTP, 32, lane, &u0, &u1);
+    balanced_range(1ull << NTP, (unsigned long long)parts * TM::kSize, (unsigned long long)part * TM::kSize + rank, &u0,
+                   &u1);
 #pragma unroll
     for (int c = 0; c < C; ++c) tot[c] = {0.0, 0.0};
     if (u0 < u1) {
         // unit base: hi words in registers; lo words in registers or in the
-        // lane's shared slot (element (c, r) at [(c * N + r) * 32 + lane])
+        // thread's shared slot (element (c, r) at [(c * N + r) * LS + rank])
         double xh[C][N];
         double xlr[Q::LO_SMEM ? 1 : C * N];
-        double* xl = Q::LO_SMEM ? s_lo + lane : xlr;
-        constexpr int LS = Q::LO_SMEM ? 32 : 1;  // stride between elements
+        double* xl = Q::LO_SMEM ? s_lo + rank : xlr;
+        constexpr int LS = Q::LO_SMEM ? TM::kSize : 1;  // stride between elements
         const unsigned long long g0 = gray_of(u0);
 #pragma unroll
         for (int c = 0; c < C; ++c)
@@ -197,35 +216,56 @@ __device__ __forceinline__ void walk_matrix(const double* __restrict__ A, const 
 // device's address space, at the same offsets), each warp first copies its
 // matrix from src into its place in mats, so every matrix crosses the host
 // link once, in coalesced reads that overlap the other warps' work.
-template <int N, int C>
+// SPLIT: a matrix is one CTA's, or shared by the CTAs of a cluster (part of the
+// units each, tables of its own); else one warp's.  A split matrix's total is
+// added up in the order of its warps, then its CTAs (through distributed shared
+// memory: no workspace, so the launch still allocates nothing).
+template <int N, int C, bool SPLIT>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) batch_walk(double* __restrict__ mats,
                                                                  const unsigned* __restrict__ offs,
                                                                  const double* __restrict__ src,
                                                                  int count, double* __restrict__ out)
 {
-    constexpr int SLICE = slice_doubles<N, C>();
+    using TM = Team<SPLIT>;
+    constexpr int SLICE = slice_doubles<N, C, TM::kSize>();
     extern __shared__ __align__(16) double smem[];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    double* slice = smem + (size_t)wid * SLICE;
+    __shared__ dd s_part[C][kWarpsPerCta];  // SPLIT: the CTA's warps' totals, then (first CTA) ...
+    __shared__ dd s_cta[C][kMaxCluster];    // ... the cluster's CTAs' totals
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, rank = TM::rank();
+    double* slice = smem + (SPLIT ? 0 : (size_t)wid * SLICE);
     int* s_exp = reinterpret_cast<int*>(slice + SLICE - N);  // [N], past either walk's arrays
+    cg::cluster_group cluster = cg::this_cluster();
+    const int parts = SPLIT ? (int)cluster.num_blocks() : 1, part = SPLIT ? (int)cluster.block_rank() : 0;
 
-    const int total_warps = gridDim.x * kWarpsPerCta;
-    for (int m = blockIdx.x * kWarpsPerCta + wid; m < count; m += total_warps) {
+    const int teams = SPLIT ? gridDim.x / parts : gridDim.x * kWarpsPerCta;
+    for (int m = SPLIT ? blockIdx.x / parts : blockIdx.x * kWarpsPerCta + wid; m < count; m += teams) {
         const size_t base = offs ? (size_t)offs[m] * kOffsetUnit : (size_t)m * N * N * C;
-        if (src) {
-            for (int i = lane; i < N * N * C; i += 32) mats[base + i] = src[base + i];
-            __syncwarp();  // orders the warp's writes before its reads below
-        }
         const double* A = mats + base;
+        if constexpr (SPLIT) {
+            // each CTA stages the matrix for itself; the first also brings a
+            // source matrix into its place
+            double* stage = slice + SLICE;
+            const double* from = src ? src + base : A;
+            for (int i = rank; i < N * N * C; i += TM::kSize) {
+                const double v = from[i];
+                stage[i] = v;
+                if (src && part == 0) mats[base + i] = v;
+            }
+            A = stage;
+            TM::sync();
+        } else if (src) {
+            for (int i = rank; i < N * N * C; i += TM::kSize) mats[base + i] = src[base + i];
+            TM::sync();  // orders the warp's writes before its reads below
+        }
         // row exponents: row max scaled into [0.5, 1)
-        for (int r = lane; r < N; r += 32) {
+        for (int r = rank; r < N; r += TM::kSize) {
             double mx = 0.0;
             for (int j = 0; j < N * C; ++j) mx = fmax(mx, fabs(A[r * N * C + j]));
             int e = 0;
             if (mx > 0.0 && isfinite(mx)) frexp(mx, &e);
             s_exp[r] = e;
         }
-        __syncwarp();
+        TM::sync();
         dd tot[C];
         int pivot = -1;
         if constexpr (has_deriv(N)) {
@@ -233,57 +273,124 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) batch_walk(double* __restri
                 const double* e = A + ((size_t)r * N + j) * C;
                 return ldexp(C == 1 ? fabs(e[0]) : fmax(fabs(e[0]), fabs(e[C - 1])), -s_exp[r]);
             });
-            if (pivot >= 0) walk_matrix<N, C, true>(A, s_exp, pivot, slice, lane, tot);
+            if (pivot >= 0) walk_matrix<N, C, true, SPLIT>(A, s_exp, pivot, slice, part, parts, tot);
         }
-        if (pivot < 0) walk_matrix<N, C, false>(A, s_exp, pivot, slice, lane, tot);
-        int es = 0;
-        for (int r = 0; r < N; ++r) es += s_exp[r];
-        bool odd = N % 2 != 0;  // perm = (4(nc%2)-2) * total over nc walked columns
-        if constexpr (has_deriv(N))
-            if (pivot >= 0) {  // times the product of the pivots
-                const dense::DerivScale sc = dense::deriv_scale<C>(N, [&](int r) {
-                    const double* d = A + ((size_t)r * N + pivot) * C;
-                    return make_double2(ldexp(d[0], -s_exp[r]), ldexp(d[C - 1], -s_exp[r]));
-                });
-                if constexpr (C == 1) {
-                    tot[0] = dd_mul(tot[0], sc.v.re);
-                } else {
-                    const dense::ddc t = dense::ddc_mul(dense::ddc{tot[0], tot[1]}, sc.v);
-                    tot[0] = t.re;
-                    tot[1] = t.im;
-                }
-                es += sc.e;
-                odd = !odd;
-            }
-        if (lane == 0) {
-            const double sgn = odd ? 1.0 : -1.0;
+        if (pivot < 0) walk_matrix<N, C, false, SPLIT>(A, s_exp, pivot, slice, part, parts, tot);
+        if constexpr (SPLIT) {
+            if (lane == 0)
 #pragma unroll
-            for (int c = 0; c < C; ++c) {
-                out[(size_t)m * 2 * C + 2 * c] = sgn * ldexp(tot[c].hi, es + 1);
-                out[(size_t)m * 2 * C + 2 * c + 1] = sgn * ldexp(tot[c].lo, es + 1);
+                for (int c = 0; c < C; ++c) s_part[c][wid] = tot[c];
+            __syncthreads();
+            if (threadIdx.x == 0)
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    dd v = s_part[c][0];
+                    for (int w = 1; w < kWarpsPerCta; ++w) v = dd_add(v, s_part[c][w]);
+                    *cluster.map_shared_rank(&s_cta[c][part], 0) = v;
+                }
+            cluster.sync();
+            if (part == 0)
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    tot[c] = s_cta[c][0];
+                    for (int b = 1; b < parts; ++b) tot[c] = dd_add(tot[c], s_cta[c][b]);
+                }
+        }
+        if (part == 0 && (!SPLIT || wid == 0)) {
+            int es = 0;
+            for (int r = 0; r < N; ++r) es += s_exp[r];
+            bool odd = N % 2 != 0;  // perm = (4(nc%2)-2) * total over nc walked columns
+            if constexpr (has_deriv(N))
+                if (pivot >= 0) {  // times the product of the pivots
+                    const dense::DerivScale sc = dense::deriv_scale<C>(N, [&](int r) {
+                        const double* d = A + ((size_t)r * N + pivot) * C;
+                        return make_double2(ldexp(d[0], -s_exp[r]), ldexp(d[C - 1], -s_exp[r]));
+                    });
+                    if constexpr (C == 1) {
+                        tot[0] = dd_mul(tot[0], sc.v.re);
+                    } else {
+                        const dense::ddc t = dense::ddc_mul(dense::ddc{tot[0], tot[1]}, sc.v);
+                        tot[0] = t.re;
+                        tot[1] = t.im;
+                    }
+                    es += sc.e;
+                    odd = !odd;
+                }
+            if (lane == 0) {
+                const double sgn = odd ? 1.0 : -1.0;
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    out[(size_t)m * 2 * C + 2 * c] = sgn * ldexp(tot[c].hi, es + 1);
+                    out[(size_t)m * 2 * C + 2 * c + 1] = sgn * ldexp(tot[c].lo, es + 1);
+                }
             }
         }
-        __syncwarp();
+        // the slice and the totals are rewritten for the next matrix (and no CTA
+        // of a cluster leaves while another may still write to it)
+        if (SPLIT) cluster.sync();
+        else __syncwarp();
     }
+}
+
+// CTAs per matrix: 0 for a warp per matrix, else a power of two up to
+// kMaxCluster.  A warp per matrix is the cheapest in total (its tables are built
+// once, its lanes never wait for another warp), so matrices are split only
+// while their warps would leave the chip idle (kBusyWarps warps per SM fill the
+// FP64 pipe to about 0.8), and only into parts of four units per thread.
+int choose_split(int n, int count, int sms)
+{
+    constexpr int kBusyWarps = 12;
+    const int nc = has_deriv(n) ? n - 1 : n, top = nc - 1 - (nc - 1 < 5 ? nc - 1 : 5);
+    const long long units = 1ll << top, have = (long long)count * kWarpsPerCta;
+    if (have > (long long)sms * kBusyWarps || units < 4ll * kWarpsPerCta * 32) return 0;
+    int c = 1;
+    while (c < kMaxCluster && have * 2 * c <= (long long)sms * kBusyWarps &&
+           units >= 4ll * kWarpsPerCta * 32 * 2 * c)
+        c *= 2;
+    return c;
+}
+
+template <int N, int C, bool SPLIT>
+int launch_split(double* mats, const unsigned* offs, const double* src, int count, double* out, int blocks,
+                 int cluster, cudaStream_t s)
+{
+    constexpr size_t smem =
+        sizeof(double) *
+        (SPLIT ? slice_doubles<N, C, kWarpsPerCta * 32>() + N * N * C : slice_doubles<N, C, 32>() * kWarpsPerCta);
+    if (smem > 48 * 1024) {
+        static cudaError_t attr = cudaFuncSetAttribute(batch_walk<N, C, SPLIT>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        SPB_CUDA_TRY(attr);
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kWarpsPerCta * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)cluster;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = cluster > 1 ? 1 : 0;
+    SPB_CUDA_TRY(cudaLaunchKernelEx(&cfg, batch_walk<N, C, SPLIT>, mats, offs, src, count, out));
+    return SPB_OK;
 }
 
 template <int N, int C>
 int launch_n(double* mats, const unsigned* offs, const double* src, int count, double* out, int sms,
              cudaStream_t s)
 {
-    constexpr size_t smem = sizeof(double) * slice_doubles<N, C>() * kWarpsPerCta;
-    if (smem > 48 * 1024) {
-        static cudaError_t attr = cudaFuncSetAttribute(batch_walk<N, C>,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        SPB_CUDA_TRY(attr);
+    // (four units for each thread of a CTA: n >= 16)
+    if constexpr (N >= 16) {
+        const int c = choose_split(N, count, sms);
+        if (c > 0) return launch_split<N, C, true>(mats, offs, src, count, out, count * c, c, s);
     }
     int blocks = (count + kWarpsPerCta - 1) / kWarpsPerCta;
     const int cap = sms * 8;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
-    batch_walk<N, C><<<blocks, kWarpsPerCta * 32, smem, s>>>(mats, offs, src, count, out);
-    SPB_CUDA_TRY(cudaGetLastError());
-    return SPB_OK;
+    return launch_split<N, C, false>(mats, offs, src, count, out, blocks, 1, s);
 }
 
 int dispatch(double* mats, const unsigned* offs, const double* src, int n, int is_complex, int count, double* out,
