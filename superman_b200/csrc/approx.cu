@@ -19,12 +19,25 @@
 //
 // B200 formulation.  One thread per sample stream; sample k always draws from
 // its own SplitMix64 stream seeded by (seed, k), and every floating-point
-// operation is an explicitly rounded add, multiply or divide, so a sample's
-// estimate does not depend on the launch shape, and the CPU restatement in the
-// oracle reproduces it bit for bit.  Per-thread state (scales, remaining
-// degrees, the propagation stack) lives in global memory laid out [i][thread],
-// so threads that work on the same row touch consecutive words.  Per-thread
-// sums of the estimates and of their squares are reduced deterministically.
+// operation is an explicitly rounded add, multiply or divide in the order above,
+// so a sample's estimate does not depend on the launch shape, and the CPU
+// restatement in the oracle reproduces it bit for bit.  Per-thread state
+// (scales, remaining degrees, the propagation stack) lives in global memory
+// laid out [i][thread]; the threads of a warp take the rows in step, so they
+// touch consecutive words and read the same pattern entries.  Per-thread sums of
+// the estimates and of their squares are reduced deterministically.
+//
+// A row's passes change nothing but its own scale and its columns', so the
+// other rows' scales that the columns' sums need are loaded once per row into
+// registers (scale_row_cached) and not once per pass: the sums before row i's
+// own entry as one number, those after it singly, in order.  The passes end
+// early for a warp whose rows' scales all repeat themselves (the rest would
+// repeat them too), and at once for rows already matched (nothing they compute
+// changes after the first pass).  What bounds it is the latency of the loads
+// and of the chains of short sums and reciprocals.  One B200, permutation plus three
+// entries per row, 2^18 samples: n=40 3.24 -> 2.25 ms, n=100 9.33 -> 7.48 ms, n=200
+// 16.1 -> 12.8 ms.  (Six CTAs per SM without spills: n=100 7.9 ms; the state in
+// shared memory with four lanes per sample: 10.1 ms.)
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -49,6 +62,7 @@ struct Pattern {
     const int* row;
     const float* rv0;  // host-scaled start
     const float* cv0;
+    const unsigned char* cached;  // [n] 1: scale_row_cached takes the row
 };
 
 __host__ __device__ __forceinline__ unsigned long long splitmix_next(unsigned long long& s)
@@ -68,20 +82,23 @@ __host__ __device__ __forceinline__ float uniform01(unsigned long long& s)
 
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float frecip(float a) { return __fdiv_rn(1.0f, a); }
+// 1 / a correctly rounded (the same bits as the division)
+__device__ __forceinline__ float frecip(float a) { return __frcp_rn(a); }
 
-// Strided per-thread arrays: element i of thread t at [i * T + t].
+// Strided per-thread arrays: element i of thread t at [i * T + t].  Count:
+// bytes where the degrees allow (a quarter of the traffic), else int.
+template <class Count>
 struct Lane {
     float* rv;
     float* cv;
-    int* re;  // remaining entries per row
-    int* ce;  // remaining entries per column
+    Count* re;  // remaining entries per row
+    Count* ce;  // remaining entries per column
     int* stk;
     unsigned long long T, t;
     __device__ __forceinline__ float& RV(int i) const { return rv[(size_t)i * T + t]; }
     __device__ __forceinline__ float& CV(int j) const { return cv[(size_t)j * T + t]; }
-    __device__ __forceinline__ int& RE(int i) const { return re[(size_t)i * T + t]; }
-    __device__ __forceinline__ int& CE(int j) const { return ce[(size_t)j * T + t]; }
+    __device__ __forceinline__ Count& RE(int i) const { return re[(size_t)i * T + t]; }
+    __device__ __forceinline__ Count& CE(int j) const { return ce[(size_t)j * T + t]; }
     __device__ __forceinline__ int& STK(int k) const { return stk[(size_t)k * T + t]; }
 };
 
@@ -90,7 +107,8 @@ struct Lane {
 // left with one entry is matched to it, which removes that column in turn.
 // Otherwise the same with rows and columns exchanged.  Returns true when a
 // line is left with no entry (no perfect matching remains).
-__device__ bool propagate(const Pattern& P, const Lane& L, int start, bool by_col)
+template <class Count>
+__device__ bool propagate(const Pattern& P, const Lane<Count>& L, int start, bool by_col)
 {
     const int* optr = by_col ? P.cptr : P.rptr;  // lines crossing a removed line
     const int* oidx = by_col ? P.row : P.col;
@@ -104,7 +122,7 @@ __device__ bool propagate(const Pattern& P, const Lane& L, int start, bool by_co
             const int i = oidx[q];
             float& si = by_col ? L.RV(i) : L.CV(i);
             if (si == 0.0f) continue;
-            int& cnt = by_col ? L.RE(i) : L.CE(i);
+            Count& cnt = by_col ? L.RE(i) : L.CE(i);
             const int k = --cnt;
             if (k == 0) return true;
             if (k != 1) continue;
@@ -122,49 +140,130 @@ __device__ bool propagate(const Pattern& P, const Lane& L, int start, bool by_co
     return false;
 }
 
+// The row's scaling passes with everything they read in registers: for a row
+// of at most kCols entries whose columns have at most kAfter entries below it
+// (Pattern::cached; uniform over the grid).  j[c], cv[c]: the row's columns and
+// their scales.  False when a sum vanishes.
+constexpr int kCols = 5, kAfter = 4;
+template <class Count>
+__device__ __forceinline__ bool scale_row_cached(const Pattern& P, const Lane<Count>& L, int i, int p0, int deg,
+                                                 float& ri, int (&j)[kCols], float (&cv)[kCols])
+{
+    float before[kCols], after[kCols][kAfter];
+#pragma unroll
+    for (int c = 0; c < kCols; ++c) {
+        j[c] = 0;
+        cv[c] = 0.0f;
+        if (c < deg) {
+            j[c] = P.col[p0 + c];
+            cv[c] = L.CV(j[c]);
+            int q = P.cptr[j[c]];
+            const int end = P.cptr[j[c] + 1];
+            before[c] = 0.0f;
+            for (; P.row[q] != i; ++q) before[c] = fadd(before[c], L.RV(P.row[q]));
+            ++q;
+#pragma unroll
+            for (int k = 0; k < kAfter; ++k) after[c][k] = q + k < end ? L.RV(P.row[q + k]) : 0.0f;
+        }
+    }
+    bool ok = true, done = false;
+    for (int it = 0; it < kBeta; ++it) {
+        float t = 0.0f;
+#pragma unroll
+        for (int c = 0; c < kCols; ++c)
+            if (c < deg) {
+                // (adding the zeros past the column's last entry changes nothing)
+                float s = fadd(before[c], ri);
+#pragma unroll
+                for (int k = 0; k < kAfter; ++k) s = fadd(s, after[c][k]);
+                if (cv[c] != 0.0f && !done) {
+                    if (s == 0.0f) ok = false;
+                    else cv[c] = frecip(s);
+                }
+                t = fadd(t, cv[c]);
+            }
+        if (!done) {
+            if (ri == 0.0f || t == 0.0f) {
+                ok = ok && ri == 0.0f;
+                done = true;
+            } else {
+                const float r = frecip(t);
+                done = r == ri;
+                ri = r;
+            }
+        }
+        if (__all_sync(__activemask(), done || !ok)) break;
+    }
+#pragma unroll
+    for (int c = 0; c < kCols; ++c)
+        if (c < deg) L.CV(j[c]) = cv[c];
+    L.RV(i) = ri;
+    return ok;
+}
+
 // One sample's estimate (0 when the drawn partial matching cannot be
 // completed).
-__device__ double sample_estimate(const Pattern& P, const Lane& L, unsigned long long seed, unsigned long long k)
+template <class Count>
+__device__ __forceinline__ double sample_estimate(const Pattern& P, const Lane<Count>& L, unsigned long long seed, unsigned long long k)
 {
     const int n = P.n;
     for (int i = 0; i < n; ++i) {
-        L.RE(i) = P.rptr[i + 1] - P.rptr[i];
-        L.CE(i) = P.cptr[i + 1] - P.cptr[i];
+        L.RE(i) = (Count)(P.rptr[i + 1] - P.rptr[i]);
+        L.CE(i) = (Count)(P.cptr[i + 1] - P.cptr[i]);
         L.RV(i) = P.rv0[i];
         L.CV(i) = P.cv0[i];
     }
     unsigned long long rng = seed ^ (k * 0xD1B54A32D192ED03ull);
     double est = 1.0;
     for (int i = 0; i < n; ++i) {
-        for (int it = 0; it < kBeta; ++it) {
-            for (int p = P.rptr[i]; p < P.rptr[i + 1]; ++p) {
-                const int j = P.col[p];
-                if (L.CV(j) == 0.0f) continue;
-                float s = 0.0f;
-                for (int q = P.cptr[j]; q < P.cptr[j + 1]; ++q) s = fadd(s, L.RV(P.row[q]));
-                if (s == 0.0f) return 0.0;
-                L.CV(j) = frecip(s);
-            }
-            if (L.RV(i) != 0.0f) {
-                float s = 0.0f;
-                for (int p = P.rptr[i]; p < P.rptr[i + 1]; ++p) s = fadd(s, L.CV(P.col[p]));
-                if (s == 0.0f) return 0.0;
-                L.RV(i) = frecip(s);
-            }
-        }
-        const float ri = L.RV(i);
-        if (ri == 0.0f) continue;  // matched by propagation
-        const float u = uniform01(rng);
-        float run = 0.0f, prob = 0.0f;
+        const int p0 = P.rptr[i], deg = P.rptr[i + 1] - p0;
+        float ri = L.RV(i), run = 0.0f, prob = 0.0f;
         int chosen = -1;
-        for (int p = P.rptr[i]; p < P.rptr[i + 1]; ++p) {
-            const int j = P.col[p];
-            const float cj = L.CV(j);
-            if (cj == 0.0f) continue;
-            prob = fmul(ri, cj);
-            run = fadd(run, prob);
-            chosen = j;
-            if (run > u) break;  // else, rounding left the total below u: the last column
+        if (P.cached[i]) {
+            int j[kCols];
+            float cv[kCols];
+            if (!scale_row_cached(P, L, i, p0, deg, ri, j, cv)) return 0.0;
+            if (ri == 0.0f) continue;  // matched by propagation
+            const float u = uniform01(rng);
+            bool open = true;
+#pragma unroll
+            for (int c = 0; c < kCols; ++c)
+                if (c < deg && open && cv[c] != 0.0f) {
+                    prob = fmul(ri, cv[c]);
+                    run = fadd(run, prob);
+                    chosen = j[c];
+                    open = !(run > u);  // else, rounding left the total below u: the last column
+                }
+        } else {
+            for (int it = 0; it < kBeta; ++it) {
+                for (int p = p0; p < p0 + deg; ++p) {
+                    const int j = P.col[p];
+                    if (L.CV(j) == 0.0f) continue;
+                    float s = 0.0f;
+                    for (int q = P.cptr[j]; q < P.cptr[j + 1]; ++q) s = fadd(s, L.RV(P.row[q]));
+                    if (s == 0.0f) return 0.0;
+                    L.CV(j) = frecip(s);
+                }
+                if (ri == 0.0f) break;  // nothing changes from here on
+                float s = 0.0f;
+                for (int p = p0; p < p0 + deg; ++p) s = fadd(s, L.CV(P.col[p]));
+                if (s == 0.0f) return 0.0;
+                const float r = frecip(s);
+                const bool same = r == ri;  // the remaining passes would repeat this one
+                L.RV(i) = ri = r;
+                if (same) break;
+            }
+            if (ri == 0.0f) continue;  // matched by propagation
+            const float u = uniform01(rng);
+            for (int p = p0; p < p0 + deg; ++p) {
+                const int j = P.col[p];
+                const float cj = L.CV(j);
+                if (cj == 0.0f) continue;
+                prob = fmul(ri, cj);
+                run = fadd(run, prob);
+                chosen = j;
+                if (run > u) break;  // else, rounding left the total below u: the last column
+            }
         }
         if (chosen < 0) return 0.0;
         est = __dmul_rn(est, __ddiv_rn(1.0, (double)prob));
@@ -182,10 +281,13 @@ struct Sums {
     double* per_sample;      // optional: estimates of samples [first, first + count)
 };
 
-__global__ void __launch_bounds__(128, 8) rasmussen_kernel(Pattern P, Lane L0, unsigned long long first,
-                                                        unsigned long long count, unsigned long long seed, Sums S)
+constexpr int kCtasPerSm = 8;  // 64 registers a thread
+template <class Count>
+__global__ void __launch_bounds__(128, kCtasPerSm) rasmussen_kernel(Pattern P, Lane<Count> L0, unsigned long long first,
+                                                                    unsigned long long count,
+                                                                    unsigned long long seed, Sums S)
 {
-    Lane L = L0;
+    Lane<Count> L = L0;
     L.T = (unsigned long long)gridDim.x * blockDim.x;
     L.t = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
     double s1 = 0.0, s2 = 0.0;
@@ -309,11 +411,26 @@ int run(const int* cptrs, const int* rows, int n, unsigned long long first, unsi
     SPB_CUDA_TRY(cudaSetDevice(ctx->device));
     cudaStream_t stream = call_stream(ctx, &opt);
 
-    // Launch shape: 8 CTAs of 128 threads per SM (the sampler is latency-bound;
-    // 64 registers a thread let all of them be resident), fewer when the per-thread
-    // state (5n words) would pass 2 GB or there are fewer samples.
+    // rows scale_row_cached takes, and the widest line
+    std::vector<unsigned char> cached(n, 0);
+    int most = 0;
+    for (int i = 0; i < n; ++i) {
+        const int deg = rptr[i + 1] - rptr[i];
+        most = std::max(most, std::max(deg, cptr[i + 1] - cptr[i]));
+        bool ok = deg <= kCols;
+        for (int p = rptr[i]; p < rptr[i + 1] && ok; ++p) {
+            const int* end = row.data() + cptr[col[p] + 1];
+            ok = end - std::lower_bound((const int*)row.data() + cptr[col[p]], end, i) - 1 <= kAfter;
+        }
+        cached[i] = ok ? 1 : 0;
+    }
+    const bool bytes = most <= 255;
+
+    // Launch shape: kCtasPerSm CTAs of 128 threads per SM (the sampler is
+    // latency-bound; their registers let all of them be resident), fewer when the
+    // per-thread state (up to 5n words) would pass 2 GB or there are fewer samples.
     const int threads = 128;
-    unsigned long long T = (unsigned long long)ctx->sm_count * 8 * threads;
+    unsigned long long T = (unsigned long long)ctx->sm_count * kCtasPerSm * threads;
     const unsigned long long cap = (2ull << 30) / (20ull * (unsigned long long)n);
     if (T > cap) T = cap;
     if (T > count) T = count;
@@ -327,9 +444,10 @@ int run(const int* cptrs, const int* rows, int n, unsigned long long first, unsi
     auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
     const size_t o_rp = take(sizeof(int) * (nn + 1)), o_cl = take(sizeof(int) * nz);
     const size_t o_cp = take(sizeof(int) * (nn + 1)), o_rw = take(sizeof(int) * nz);
-    const size_t o_r0 = take(sizeof(float) * nn), o_c0 = take(sizeof(float) * nn);
+    const size_t o_r0 = take(sizeof(float) * nn), o_c0 = take(sizeof(float) * nn), o_ca = take(nn);
     const size_t o_rv = take(sizeof(float) * nn * T), o_cv = take(sizeof(float) * nn * T);
-    const size_t o_re = take(sizeof(int) * nn * T), o_ce = take(sizeof(int) * nn * T);
+    const size_t cb = bytes ? sizeof(unsigned char) : sizeof(int);
+    const size_t o_re = take(cb * nn * T), o_ce = take(cb * nn * T);
     const size_t o_sk = take(sizeof(int) * nn * T);
     const size_t o_pt = take(sizeof(double) * 2 * blocks), o_tk = take(sizeof(unsigned) * 4);
     const size_t o_tt = take(sizeof(double) * 2);
@@ -342,10 +460,8 @@ int run(const int* cptrs, const int* rows, int n, unsigned long long first, unsi
     Pattern P{n,
               reinterpret_cast<int*>(base + o_rp), reinterpret_cast<int*>(base + o_cl),
               reinterpret_cast<int*>(base + o_cp), reinterpret_cast<int*>(base + o_rw),
-              reinterpret_cast<float*>(base + o_r0), reinterpret_cast<float*>(base + o_c0)};
-    Lane L{reinterpret_cast<float*>(base + o_rv), reinterpret_cast<float*>(base + o_cv),
-           reinterpret_cast<int*>(base + o_re), reinterpret_cast<int*>(base + o_ce),
-           reinterpret_cast<int*>(base + o_sk), 0, 0};
+              reinterpret_cast<float*>(base + o_r0), reinterpret_cast<float*>(base + o_c0),
+              reinterpret_cast<unsigned char*>(base + o_ca)};
     Sums S{reinterpret_cast<double*>(base + o_pt), reinterpret_cast<unsigned*>(base + o_tk),
            reinterpret_cast<double*>(base + o_tt), h_per_sample ? reinterpret_cast<double*>(base + o_ps) : nullptr};
     SPB_CUDA_TRY(cudaEventRecord(ctx->ev_call0, stream));
@@ -357,9 +473,18 @@ int run(const int* cptrs, const int* rows, int n, unsigned long long first, unsi
     }
     SPB_CUDA_TRY(cudaMemcpyAsync(base + o_r0, rv.data(), sizeof(float) * nn, cudaMemcpyHostToDevice, stream));
     SPB_CUDA_TRY(cudaMemcpyAsync(base + o_c0, cv.data(), sizeof(float) * nn, cudaMemcpyHostToDevice, stream));
+    SPB_CUDA_TRY(cudaMemcpyAsync(base + o_ca, cached.data(), nn, cudaMemcpyHostToDevice, stream));
     SPB_CUDA_TRY(cudaMemsetAsync(S.ticket, 0, sizeof(unsigned) * 4, stream));
     SPB_CUDA_TRY(cudaEventRecord(ctx->ev_begin, stream));
-    rasmussen_kernel<<<blocks, threads, 0, stream>>>(P, L, first, count, seed, S);
+    auto launch = [&](auto c) {
+        using Count = decltype(c);
+        Lane<Count> L{reinterpret_cast<float*>(base + o_rv), reinterpret_cast<float*>(base + o_cv),
+                      reinterpret_cast<Count*>(base + o_re), reinterpret_cast<Count*>(base + o_ce),
+                      reinterpret_cast<int*>(base + o_sk), 0, 0};
+        rasmussen_kernel<Count><<<blocks, threads, 0, stream>>>(P, L, first, count, seed, S);
+    };
+    if (bytes) launch((unsigned char)0);
+    else launch(0);
     SPB_CUDA_TRY(cudaGetLastError());
     SPB_CUDA_TRY(cudaEventRecord(ctx->ev_end, stream));
     double tot[2] = {0.0, 0.0};
