@@ -36,9 +36,10 @@
 // The host picks the line (column, or row by transposing) with the fewest
 // ones.  Sigma = sum_S (-1)^|S| term = 2^(n-2) * (+-) perm(A) (+ for even n).
 // On one B200 at 1965 MHz, Bernoulli(0.5) entries with the identity: n=36
-// 203.0 -> 134.1 ms, n=32 11.25 -> 7.62 ms, n=28 0.668 -> 0.521 ms.  Bound, as the
-// plain walk, by the instructions it issues: with 32-bit words as there (a sign
-// and a magnitude per word) n=36 took 146 ms at 16 warps per SM and 183 ms at 8.
+// 203.4 -> 120 ms with 12 ones in the line, 140 ms with 14.
+// Bound, as the plain walk, by the instructions it issues: with 32-bit words as
+// there (a sign and a magnitude per word) n=36 took 146 ms at 16 warps per SM and
+// 183 ms at 8, one term at a time with these 64-bit words 134 ms.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -234,40 +235,61 @@ __host__ __device__ constexpr int expand_limbs_after(int n, int g, int L)
     return l < L ? l : L;
 }
 
+// Terms evaluated side by side.  Two share each table load (8 bytes: with the
+// branches on m the loads of separate terms are not merged) and give the
+// scheduler two chains; four would not fit the registers.  One term at a time
+// spent a table load per row (the load pipe 40 % busy): n=36 141.6 -> 122.7 ms,
+// n=33 15.4 -> 13.9 ms, n=30 1.91 -> 1.64 ms.
+constexpr int kPair = 2;
+
+// Row r's values of terms i and i + 1.
+__device__ __forceinline__ void row_values(int xt, const int* __restrict__ de, int (&x)[kPair])
+{
+    const int2 d = *reinterpret_cast<const int2*>(de);
+    x[0] = xt + d.x;
+    x[1] = xt + d.y;
+}
+
 // Half h: the product p of its rows' values.
 template <int N, int G, int h>
-__device__ __forceinline__ int half_plain(const int (&xt)[N], const int* __restrict__ de, int i)
+__device__ __forceinline__ void half_plain(const int (&xt)[N], const int* __restrict__ de, int i, int (&p)[kPair])
 {
     constexpr int r0 = h * half_rows(N), rows = rows_in_half(N, h);
-    int p = 1;
 #pragma unroll
     for (int k = 0; k < rows; ++k) {
-        const int x = xt[r0 + k] + de[(r0 + k) * G + i];
-        p = k == 0 ? x : p * x;
+        int x[kPair];
+        row_values(xt[r0 + k], de + (r0 + k) * G + i, x);
+#pragma unroll
+        for (int t = 0; t < kPair; ++t) p[t] = k == 0 ? x[t] : p[t] * x[t];
     }
-    return p;
 }
 
 // The same with its derivative q over the rows below m.  ALL: all of them are.
 template <int N, int G, int h, bool ALL>
-__device__ __forceinline__ void half_dual(const int (&xt)[N], const int* __restrict__ de, int i, int m, int& p, int& q)
+__device__ __forceinline__ void half_dual(const int (&xt)[N], const int* __restrict__ de, int i, int m, int (&p)[kPair],
+                                          int (&q)[kPair])
 {
     constexpr int r0 = h * half_rows(N), rows = rows_in_half(N, h);
 #pragma unroll
     for (int k = 0; k < rows; ++k) {
-        const int x = xt[r0 + k] + de[(r0 + k) * G + i];
-        if (k == 0) {
-            p = x;
-            q = 1;  // the half holds a row below m
-        } else {
-            q = ALL && k == 1 ? x + p : q * x + (ALL || r0 + k < m ? p : 0);
-            p *= x;
+        int x[kPair];
+        row_values(xt[r0 + k], de + (r0 + k) * G + i, x);
+#pragma unroll
+        for (int t = 0; t < kPair; ++t) {
+            if (k == 0) {
+                p[t] = x[t];
+                q[t] = 1;  // the half holds a row below m
+            } else {
+                q[t] = ALL && k == 1 ? x[t] + p[t] : q[t] * x[t] + (ALL || r0 + k < m ? p[t] : 0);
+                p[t] *= x[t];
+            }
         }
     }
 }
 
 template <int N, int G, int h>
-__device__ __forceinline__ void half_any(const int (&xt)[N], const int* __restrict__ de, int i, int m, int& p, int& q)
+__device__ __forceinline__ void half_any(const int (&xt)[N], const int* __restrict__ de, int i, int m, int (&p)[kPair],
+                                         int (&q)[kPair])
 {
     if (m >= h * half_rows(N) + rows_in_half(N, h)) half_dual<N, G, h, true>(xt, de, i, m, p, q);
     else half_dual<N, G, h, false>(xt, de, i, m, p, q);
@@ -275,32 +297,43 @@ __device__ __forceinline__ void half_any(const int (&xt)[N], const int* __restri
 
 // Word g: the product W of its rows, its derivative Q when it holds rows below m.
 template <int N, int G, int g>
-__device__ __forceinline__ long long word_plain(const int (&xt)[N], const int* __restrict__ de, int i)
+__device__ __forceinline__ void word_plain(const int (&xt)[N], const int* __restrict__ de, int i, long long (&W)[kPair])
 {
-    const long long a = half_plain<N, G, 2 * g>(xt, de, i);
-    if constexpr (rows_in_half(N, 2 * g + 1) == 0) return a;
-    else return a * (long long)half_plain<N, G, 2 * g + 1>(xt, de, i);
+    int a[kPair], b[kPair];
+    half_plain<N, G, 2 * g>(xt, de, i, a);
+    if constexpr (rows_in_half(N, 2 * g + 1) > 0) half_plain<N, G, 2 * g + 1>(xt, de, i, b);
+#pragma unroll
+    for (int t = 0; t < kPair; ++t) {
+        if constexpr (rows_in_half(N, 2 * g + 1) > 0) W[t] = (long long)a[t] * b[t];
+        else W[t] = a[t];
+    }
 }
 template <int N, int G, int g>
-__device__ __forceinline__ void word_dual(const int (&xt)[N], const int* __restrict__ de, int i, int m, long long& W,
-                                          long long& Q)
+__device__ __forceinline__ void word_dual(const int (&xt)[N], const int* __restrict__ de, int i, int m,
+                                          long long (&W)[kPair], long long (&Q)[kPair])
 {
-    int pa, qa;
+    int pa[kPair], qa[kPair];
     half_any<N, G, 2 * g>(xt, de, i, m, pa, qa);
     if constexpr (rows_in_half(N, 2 * g + 1) == 0) {
-        W = pa;
-        Q = qa;
+#pragma unroll
+        for (int t = 0; t < kPair; ++t) {
+            W[t] = pa[t];
+            Q[t] = qa[t];
+        }
     } else {
-        int pb, qb;
+        int pb[kPair], qb[kPair];
         if (m > (2 * g + 1) * half_rows(N)) {
             half_any<N, G, 2 * g + 1>(xt, de, i, m, pb, qb);
             // at most 2K (n-1)^(2K-1) < 2^63: 2K <= n rows, (n-1)^(2K) < 2^62
-            Q = (long long)qa * pb + (long long)pa * qb;
+#pragma unroll
+            for (int t = 0; t < kPair; ++t) Q[t] = (long long)qa[t] * pb[t] + (long long)pa[t] * qb[t];
         } else {
-            pb = half_plain<N, G, 2 * g + 1>(xt, de, i);
-            Q = (long long)qa * pb;
+            half_plain<N, G, 2 * g + 1>(xt, de, i, pb);
+#pragma unroll
+            for (int t = 0; t < kPair; ++t) Q[t] = (long long)qa[t] * pb[t];
         }
-        W = (long long)pa * pb;
+#pragma unroll
+        for (int t = 0; t < kPair; ++t) W[t] = (long long)pa[t] * pb[t];
     }
 }
 
@@ -337,90 +370,116 @@ __device__ __forceinline__ void fold64(uint32_t (&p)[L], unsigned long long w)
     for (int l = 0; l < nb + 2 && l < L; ++l) p[l] = r[l];
 }
 
-// Words g, g+1, ... of a term, none with rows of the expanded column.
+// Words g, g+1, ... of two terms, none with rows of the expanded column.
 template <int N, int L, int G, int g>
 __device__ __forceinline__ void plain_words(const int (&xt)[N], const int* __restrict__ de, int i,
-                                            uint32_t (&p)[L], uint32_t& sg)
+                                            uint32_t (&p)[kPair][L], uint32_t (&sg)[kPair])
 {
     if constexpr (rows_in_half(N, 2 * g) > 0) {
-        fold64<L, expand_limbs_after(N, g - 1, L)>(p, magnitude(word_plain<N, G, g>(xt, de, i), sg));
+        long long W[kPair];
+        word_plain<N, G, g>(xt, de, i, W);
+#pragma unroll
+        for (int t = 0; t < kPair; ++t) fold64<L, expand_limbs_after(N, g - 1, L)>(p[t], magnitude(W[t], sg[t]));
         plain_words<N, L, G, g + 1>(xt, de, i, p, sg);
     }
 }
 
-// |sum_{r < m} prod_{r' != r} x'_r'| mod 2^(32L) for one term into p; returns
-// a word whose bit 31 is its sign.  1 <= m <= kExpandHalves * K.  The branches
-// on m are the same for every thread of the grid.
+// |Q0 W1 + W0 Q1|, 128 bits (4K rows below (2^31)^4), into p; the sign to sg.
+template <int L>
+__device__ __forceinline__ void join_words(long long W0, long long Q0, long long W1, long long Q1, uint32_t (&p)[L],
+                                           uint32_t& sg)
+{
+    const unsigned long long a = (unsigned long long)Q0 * (unsigned long long)W1;
+    const unsigned long long b = (unsigned long long)W0 * (unsigned long long)Q1;
+    const unsigned long long lo = a + b;
+    const long long hi = (long long)((unsigned long long)__mul64hi(Q0, W1) + (unsigned long long)__mul64hi(W0, Q1) +
+                                     (lo < a ? 1ull : 0ull));
+    const unsigned long long s = (unsigned long long)(hi >> 63);
+    sg ^= (uint32_t)s;
+    const unsigned long long l0 = (lo ^ s) - s, h0 = ((unsigned long long)hi ^ s) + (s && l0 == 0 ? 1ull : 0ull);
+    p[0] = (uint32_t)l0;
+    p[1] = (uint32_t)(l0 >> 32);
+    p[2] = (uint32_t)h0;
+    p[3] = (uint32_t)(h0 >> 32);
+}
+
+// |(Q0 c + W0 q) d| with a half's product c and derivative q and another's
+// product d: 96 bits (3K rows below 2^94), then one 32-bit factor.
+template <int L>
+__device__ __forceinline__ void join_half(long long W0, long long Q0, int c, int q, int d, uint32_t (&p)[L],
+                                          uint32_t& sg)
+{
+    const int sc = c >> 31;  // c's sign moves to sg and q
+    sg ^= (uint32_t)sc;
+    const uint32_t cm = (uint32_t)((c ^ sc) - sc);
+    const int qs = (q ^ sc) - sc;
+    const unsigned long long al = (unsigned long long)(uint32_t)Q0 * cm;
+    const long long ah = (Q0 >> 32) * (long long)cm + (long long)(al >> 32);
+    const long long bl = (long long)(uint32_t)W0 * (long long)qs;
+    const long long bh = (W0 >> 32) * (long long)qs + (bl >> 32);
+    const unsigned long long lo = (unsigned long long)(uint32_t)al + (uint32_t)bl;
+    const long long hi = ah + bh + (long long)(lo >> 32);
+    const uint32_t s = (uint32_t)(hi >> 63);
+    const unsigned long long l0 = (unsigned long long)((uint32_t)lo ^ s) + (s & 1u);
+    const unsigned long long h0 = ((unsigned long long)hi ^ (unsigned long long)(hi >> 63)) + (l0 >> 32);
+    const int sd = d >> 31;
+    sg ^= s ^ (uint32_t)sd;
+    const uint32_t dm = (uint32_t)((d ^ sd) - sd);
+    const unsigned long long t0 = (unsigned long long)(uint32_t)l0 * dm;
+    const unsigned long long t1 = (unsigned long long)(uint32_t)h0 * dm + (t0 >> 32);
+    const unsigned long long t2 = (h0 >> 32) * dm + (t1 >> 32);
+    p[0] = (uint32_t)t0;
+    p[1] = (uint32_t)t1;
+    p[2] = (uint32_t)t2;
+    p[3] = (uint32_t)(t2 >> 32);
+}
+
+// |sum_{r < m} prod_{r' != r} x'_r'| mod 2^(32L) for terms i and i + 1 into p;
+// bit 31 of sg[t] is term t's sign.  1 <= m <= kExpandHalves * K.  The branches
+// on m are the same for every thread of the grid.  Bernoulli(0.5) columns at
+// n = 36 mostly hold 11 to 14 ones, two or three halves.
 template <int N, int L, int G>
-__device__ __forceinline__ uint32_t term_expanded(const int (&xt)[N], const int* __restrict__ de, int i, int m,
-                                                  uint32_t (&p)[L])
+__device__ __forceinline__ void terms_expanded(const int (&xt)[N], const int* __restrict__ de, int i, int m,
+                                               uint32_t (&p)[kPair][L], uint32_t (&sg)[kPair])
 {
 #pragma unroll
-    for (int l = 0; l < L; ++l) p[l] = 0u;
-    uint32_t sg = 0u;
-    long long W0, Q0;
+    for (int t = 0; t < kPair; ++t) {
+#pragma unroll
+        for (int l = 0; l < L; ++l) p[t][l] = 0u;
+        sg[t] = 0u;
+    }
+    long long W0[kPair], Q0[kPair];
     word_dual<N, G, 0>(xt, de, i, m, W0, Q0);
-    if constexpr (rows_in_half(N, 2) > 0) {
-        if (m > 3 * half_rows(N)) {
-            long long W1, Q1;
+    if (rows_in_half(N, 2) > 0 && m > 3 * half_rows(N)) {
+        if constexpr (rows_in_half(N, 2) > 0) {
+            long long W1[kPair], Q1[kPair];
             word_dual<N, G, 1>(xt, de, i, m, W1, Q1);
-            // Q0 W1 + W0 Q1, signed 128 bits (4K rows below (2^31)^4)
-            const unsigned long long a = (unsigned long long)Q0 * (unsigned long long)W1;
-            const unsigned long long b = (unsigned long long)W0 * (unsigned long long)Q1;
-            const unsigned long long lo = a + b;
-            const long long hi = (long long)((unsigned long long)__mul64hi(Q0, W1) +
-                                             (unsigned long long)__mul64hi(W0, Q1) + (lo < a ? 1ull : 0ull));
-            const unsigned long long s = (unsigned long long)(hi >> 63);
-            sg ^= (uint32_t)s;
-            const unsigned long long l0 = (lo ^ s) - s, h0 = ((unsigned long long)hi ^ s) + (s && l0 == 0 ? 1ull : 0ull);
-            p[0] = (uint32_t)l0;
-            p[1] = (uint32_t)(l0 >> 32);
-            p[2] = (uint32_t)h0;
-            p[3] = (uint32_t)(h0 >> 32);
-        } else if (m > 2 * half_rows(N)) {
-            // three halves (Bernoulli(0.5) columns at n = 36 mostly hold 11 to 14
-            // ones, two or three halves): (Q0 c + W0 q) d with the third half's
-            // product c (its sign moved to sg and q) and derivative q, and the
-            // fourth's product d: 96 bits, then one 32-bit factor
-            int c, q, d = 1;
+#pragma unroll
+            for (int t = 0; t < kPair; ++t) join_words<L>(W0[t], Q0[t], W1[t], Q1[t], p[t], sg[t]);
+        }
+    } else if (rows_in_half(N, 2) > 0 && m > 2 * half_rows(N)) {
+        if constexpr (rows_in_half(N, 2) > 0) {
+            int c[kPair], q[kPair], d[kPair] = {1, 1};
             half_any<N, G, 2>(xt, de, i, m, c, q);
-            if constexpr (rows_in_half(N, 3) > 0) d = half_plain<N, G, 3>(xt, de, i);
-            const int sc = c >> 31;
-            sg ^= (uint32_t)sc;
-            const uint32_t cm = (uint32_t)((c ^ sc) - sc);
-            const int qs = (q ^ sc) - sc;
-            const unsigned long long al = (unsigned long long)(uint32_t)Q0 * cm;
-            const long long ah = (Q0 >> 32) * (long long)cm + (long long)(al >> 32);
-            const long long bl = (long long)(uint32_t)W0 * (long long)qs;
-            const long long bh = (W0 >> 32) * (long long)qs + (bl >> 32);
-            const unsigned long long lo = (unsigned long long)(uint32_t)al + (uint32_t)bl;
-            const long long hi = ah + bh + (long long)(lo >> 32);  // 3K rows below 2^94
-            const uint32_t s = (uint32_t)(hi >> 63);
-            const unsigned long long l0 = (unsigned long long)((uint32_t)lo ^ s) + (s & 1u);
-            const unsigned long long h0 = ((unsigned long long)hi ^ (unsigned long long)(hi >> 63)) + (l0 >> 32);
-            const int sd = d >> 31;
-            sg ^= s ^ (uint32_t)sd;
-            const uint32_t dm = (uint32_t)((d ^ sd) - sd);
-            const unsigned long long t0 = (unsigned long long)(uint32_t)l0 * dm;
-            const unsigned long long t1 = (unsigned long long)(uint32_t)h0 * dm + (t0 >> 32);
-            const unsigned long long t2 = (h0 >> 32) * dm + (t1 >> 32);
-            p[0] = (uint32_t)t0;
-            p[1] = (uint32_t)t1;
-            p[2] = (uint32_t)t2;
-            p[3] = (uint32_t)(t2 >> 32);
-        } else {
-            const unsigned long long q = magnitude(Q0, sg);
-            p[0] = (uint32_t)q;
-            p[1] = (uint32_t)(q >> 32);
-            fold64<L, 2>(p, magnitude(word_plain<N, G, 1>(xt, de, i), sg));
+            if constexpr (rows_in_half(N, 3) > 0) half_plain<N, G, 3>(xt, de, i, d);
+#pragma unroll
+            for (int t = 0; t < kPair; ++t) join_half<L>(W0[t], Q0[t], c[t], q[t], d[t], p[t], sg[t]);
         }
     } else {
-        const unsigned long long q = magnitude(Q0, sg);
-        p[0] = (uint32_t)q;
-        p[1] = (uint32_t)(q >> 32);
+#pragma unroll
+        for (int t = 0; t < kPair; ++t) {
+            const unsigned long long q = magnitude(Q0[t], sg[t]);
+            p[t][0] = (uint32_t)q;
+            p[t][1] = (uint32_t)(q >> 32);
+        }
+        if constexpr (rows_in_half(N, 2) > 0) {
+            long long W1[kPair];
+            word_plain<N, G, 1>(xt, de, i, W1);
+#pragma unroll
+            for (int t = 0; t < kPair; ++t) fold64<L, 2>(p[t], magnitude(W1[t], sg[t]));
+        }
     }
     plain_words<N, L, G, 2>(xt, de, i, p, sg);
-    return sg;
 }
 
 // Sum over one unit: sum_d (-1)^popc(d) prod_r (xt_r + DEI[d][r]), or with X
@@ -430,10 +489,6 @@ __device__ __forceinline__ void unit_sum_bin(const int (&xt)[N], const int* __re
                                              uint32_t (&acc)[L])
 {
     constexpr int G = 4;
-    auto term = [&](const int* de, int i, uint32_t (&p)[L]) {
-        if constexpr (X) return term_expanded<N, L, G>(xt, de, i, m, p);
-        else return term_product<N, L, G>(xt, de, i, p);
-    };
 #pragma unroll
     for (int l = 0; l < L; ++l) acc[l] = 0u;
 #pragma unroll 1
@@ -442,14 +497,25 @@ __device__ __forceinline__ void unit_sum_bin(const int (&xt)[N], const int* __re
         // signs: the product's (bit 31 of the returned word) and the group
         // pattern + - - + relative to popc(q); an all-ones mask subtracts
         const uint32_t flip = (__popc(q) & 1) ? 0x80000000u : 0u;
+        if constexpr (X) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {  // + - then - +
+                uint32_t p[kPair][L], sg[kPair];
+                terms_expanded<N, L, G>(xt, de, 2 * h, m, p, sg);
+                const uint32_t f = flip ^ (h ? 0x80000000u : 0u);
+                limb_add_masked<L>(acc, p[0], (uint32_t)((int32_t)(sg[0] ^ f) >> 31));
+                limb_add_masked<L>(acc, p[1], (uint32_t)((int32_t)(sg[1] ^ f ^ 0x80000000u) >> 31));
+            }
+            continue;
+        }
         uint32_t p[L];
-        uint32_t sg = term(de, 0, p);
+        uint32_t sg = term_product<N, L, G>(xt, de, 0, p);
         limb_add_masked<L>(acc, p, (uint32_t)((int32_t)(sg ^ flip) >> 31));
-        sg = term(de, 1, p);
+        sg = term_product<N, L, G>(xt, de, 1, p);
         limb_add_masked<L>(acc, p, (uint32_t)((int32_t)(sg ^ flip ^ 0x80000000u) >> 31));
-        sg = term(de, 2, p);
+        sg = term_product<N, L, G>(xt, de, 2, p);
         limb_add_masked<L>(acc, p, (uint32_t)((int32_t)(sg ^ flip ^ 0x80000000u) >> 31));
-        sg = term(de, 3, p);
+        sg = term_product<N, L, G>(xt, de, 3, p);
         limb_add_masked<L>(acc, p, (uint32_t)((int32_t)(sg ^ flip) >> 31));
     }
 }
