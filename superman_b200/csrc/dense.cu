@@ -323,8 +323,9 @@ int group_size(int n, int comps)
     return ComplexGroup(n);
 }
 
-// bits: walked columns less one, n-1 or, for the derivative walk, n-2.
-int choose_unit_bits(int n, int comps, const spb_options* opt, int bits)
+// bits: walked columns less one, n-1 or, for the derivative walk, n-2; entry:
+// bytes of a table entry in the walk's shared memory, 8 or (FP32 products) 4.
+int choose_unit_bits(int n, int comps, const spb_options* opt, int bits, size_t entry)
 {
     int w;
     if (opt && opt->unit_bits > 0) {
@@ -332,7 +333,7 @@ int choose_unit_bits(int n, int comps, const spb_options* opt, int bits)
     } else {
         // Table budget 64 KB per part; keep >= 2^16 units when n allows.
         w = 8;
-        while (w > 2 && ((size_t)1 << w) * n * 8 * comps > (size_t)64 * 1024) --w;
+        while (w > 2 && ((size_t)1 << w) * n * entry * comps > (size_t)64 * 1024) --w;
         while (w > 2 && bits - w < 16) --w;
     }
     if (w > n - 1) w = n - 1;
@@ -342,20 +343,43 @@ int choose_unit_bits(int n, int comps, const spb_options* opt, int bits)
     return w;
 }
 
-int choose_unit_bits(int n, int comps, const spb_options* opt) { return choose_unit_bits(n, comps, opt, n - 1); }
+int choose_unit_bits(int n, int comps, const spb_options* opt) { return choose_unit_bits(n, comps, opt, n - 1, sizeof(double)); }
 
 // Whether the derivative walk may run, and the unit width to go with it: on
 // dense matrices of its sizes, where the units leave it a column to expand, and
 // not with FP32 products (n=27 complex 592 -> 541 us, but the error of a Haar
-// block against exact went from 2.6e-6 to 6.2e-6).  The setup kernel decides by the matrix (rb->pivot); `hint` false
-// (a host matrix known to have a zero in every column) only sizes the units
-// for the plain walk, which then runs.
-void choose_walk(Problem* pb, const spb_options* opt, bool hint)
+// block against exact went from 2.6e-6 to 6.2e-6).  The setup kernel decides by
+// the matrix (rb->pivot); `hint` false (a host matrix known to have a zero in
+// every column) only sizes the units for the plain walk, which then runs.
+//
+// The whole-GPU walks give every thread whole units, so a few units per thread
+// leave some threads waiting for others with one more (n=28: 2^18 units of 2^8
+// terms, 3.46 per thread, four rounds).  The width is narrowed by up to two bits
+// where the evener split outweighs the base updates of more units, which cost
+// about 6 terms each, 15 of the FP32 walk's (fitted to widths 5 to 8; wall times
+// with the wider and the taken width: real n=28 493 -> 450 us, complex n=26
+// 396 -> 369 us, with double-double 583 -> 414 us).
+void choose_walk(Problem* pb, const spb_options* opt, bool hint, int sms)
 {
+    const double unit_terms = pb->f32 ? 15.0 : 6.0;
     const int n = pb->n;
     pb->deriv = pb->na == n && !pb->f32 && n >= (pb->comps == 1 ? kMinDerivReal : kMinDerivComplex) ? 1 : 0;
-    pb->w = choose_unit_bits(n, pb->comps, opt, n - 1 - (pb->deriv && hint ? 1 : 0));
+    const int bits = n - 1 - (pb->deriv && hint ? 1 : 0);
+    pb->w = choose_unit_bits(n, pb->comps, opt, bits, pb->f32 ? sizeof(float) : sizeof(double));
     if (pb->w > n - 2) pb->deriv = 0;
+    const double threads =
+        (double)sms * (pb->f32 ? walk_f32_max_threads(n, pb->comps) : walk_max_threads(n, pb->comps));
+    if (opt->unit_bits > 0 || std::ldexp(1.0, bits - pb->w) < threads) return;
+    double best = 0.0;
+    const int w0 = pb->w;
+    for (int w = w0; w >= w0 - 2 && w >= 4; --w) {
+        const double per = std::ldexp(1.0, bits - w) / threads, terms = std::ldexp(1.0, w);
+        const double eff = per / std::ceil(per) * terms / (terms + unit_terms);
+        if (eff > best * 1.02) {
+            best = eff;
+            pb->w = w;
+        }
+    }
 }
 
 // Sizes the scratch arena and fills the device pointers of *pb.
@@ -484,7 +508,7 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
             }
         }
     }
-    choose_walk(&pb, &opt, hint);
+    choose_walk(&pb, &opt, hint, ctx->sm_count);
     if (plan && plan->na < n) {
         if (comps != 1 || plan->na < 1 || plan->na > kMaxActive || plan->w < 2 || plan->w > n - 2) {
             spb_set_error("row-compacted walk: bad plan (n=%d, active rows %d, w=%d)", n, plan->na, plan->w);

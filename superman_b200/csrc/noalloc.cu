@@ -50,7 +50,7 @@ namespace dense {
 __global__ void setup_kernel(Problem pb, const double* __restrict__ a_in, int smem_tables);
 int launch_setup(const Problem& pb, const double* d_a, cudaStream_t s);
 int group_size(int n, int comps);
-void choose_walk(Problem* pb, const spb_options* opt, bool hint);
+void choose_walk(Problem* pb, const spb_options* opt, bool hint, int sms);
 size_t plan_layout(Problem* pb, char* base, size_t* in_offset);
 size_t walk_smem_bytes(const Problem& pb, int threads);
 int prepare_setup(int* limit);
@@ -150,7 +150,7 @@ extern "C" int spb_perm_dense_f64_noalloc(const double* d_a, int n, double* d_ou
     pb.n = n;
     pb.na = n;
     pb.comps = 1;
-    choose_walk(&pb, &opt, true);
+    choose_walk(&pb, &opt, true, sms);
     pb.g = group_size(n, 1);
     pb.units = 1ull << (n - 1 - pb.w);
     int threads = walk_max_threads(n, 1);
