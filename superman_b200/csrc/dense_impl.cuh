@@ -543,8 +543,8 @@ __device__ __forceinline__ double unit_bound_real(const double (&xh)[N], const d
     return D ? q : p;
 }
 
-// First unit base of each thread, built cooperatively by its warp from the
-// NW start vector (x0h, x0l) and the high columns s_mt; every lane of the
+// First unit base of each thread (one component), built cooperatively by its
+// warp from the NW start vector (x0h, x0l) and the high columns s_mt; every lane of the
 // warp calls this (it shuffles), whether it owns units or not.
 // The lanes' first units u0 lie in one range [ulo, uhi] (balanced_range is
 // monotonic in the thread index), so the Gray bits above P, the highest bit
@@ -558,7 +558,7 @@ __device__ __forceinline__ double unit_bound_real(const double (&xh)[N], const d
 // adds when threads own few units (n <= 26).
 // D: the derivative walk, whose high columns have low words (s_ml).
 template <int N, bool D>
-__device__ __forceinline__ void first_base_real(const double* __restrict__ x0h, const double* __restrict__ x0l,
+__device__ __forceinline__ void first_base(const double* __restrict__ x0h, const double* __restrict__ x0l,
                                                 const double* __restrict__ s_mt, const double* __restrict__ s_ml,
                                                 double* s_lo, int ntop,
                                                 unsigned long long u0, unsigned long long u1, int tid, int bd,
@@ -661,7 +661,7 @@ __device__ __forceinline__ void walk_real_body(const Problem& pb)
     // ones first (the refinement rebuilds bases in plain index order; the hi
     // words agree unless a row value lies within ~2^-100 of a rounding
     // midpoint, and then only that unit's correction carries one FP64 rounding).
-    first_base_real<N, D>(pb.x0_hi, pb.x0_lo, s_mt, s_ml, s_lo, ntop, u0, u1, tid, bd, xh);
+    first_base<N, D>(pb.x0_hi, pb.x0_lo, s_mt, s_ml, s_lo, ntop, u0, u1, tid, bd, xh);
     if (u0 < u1) {
         unsigned long long u = u0;
         while (true) {
@@ -908,8 +908,6 @@ __device__ __forceinline__ void walk_complex_body(const Problem& pb)
     __syncthreads();
     const double* s_mt_re = s_mt;
     const double* s_mt_im = s_mt + ntp * N;
-    // high column entry i (part 0, or at ntp * N + i part 1) added to x
-    auto plus = [&](dd x, int i) { return D ? dd_step(x, s_mt[i], s_ml[i]) : dd_add_d(x, s_mt[i]); };
     double* s_lo_re = s_lo;
     double* s_lo_im = s_lo + N * bd;
 
@@ -922,37 +920,10 @@ __device__ __forceinline__ void walk_complex_body(const Problem& pb)
     HistCache hc;
     const int lbin = mode == 1 ? __ldcg(pb.list_bin) : 0;
     int bmax = 0;
+    double xr[N], xi[N];
+    first_base<N, D>(pb.x0_hi, pb.x0_lo, s_mt_re, s_ml, s_lo_re, ntop, u0, u1, tid, bd, xr);
+    first_base<N, D>(pb.x0_hi + N, pb.x0_lo + N, s_mt_im, s_ml + ntp * N, s_lo_im, ntop, u0, u1, tid, bd, xi);
     if (u0 < u1) {
-        double xr[N], xi[N];
-        const unsigned long long g0 = gray_of(u0);
-        // Two rows (four add chains) at a time, the same operations per row.
-#pragma unroll
-        for (int r0 = 0; r0 < N; r0 += 2) {
-            dd a[2], b[2];
-#pragma unroll
-            for (int k = 0; k < 2; ++k)
-                if (r0 + k < N) {
-                    a[k] = dd{pb.x0_hi[r0 + k], pb.x0_lo[r0 + k]};
-                    b[k] = dd{pb.x0_hi[N + r0 + k], pb.x0_lo[N + r0 + k]};
-                }
-            for (int j = 0; j < ntop; ++j)
-                if ((g0 >> j) & 1ull) {
-#pragma unroll
-                    for (int k = 0; k < 2; ++k)
-                        if (r0 + k < N) {
-                            a[k] = plus(a[k], j * N + r0 + k);
-                            b[k] = plus(b[k], (ntp + j) * N + r0 + k);
-                        }
-                }
-#pragma unroll
-            for (int k = 0; k < 2; ++k)
-                if (r0 + k < N) {
-                    xr[r0 + k] = a[k].hi;
-                    xi[r0 + k] = b[k].hi;
-                    s_lo_re[(r0 + k) * bd + tid] = a[k].lo;
-                    s_lo_im[(r0 + k) * bd + tid] = b[k].lo;
-                }
-        }
         unsigned long long u = u0;
         while (true) {
             int b = 0;
