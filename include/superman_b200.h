@@ -91,11 +91,9 @@ typedef struct spb_options {
                               fused kernel (tables, walk, threshold and
                               refinement); < 0: as separate kernels        */
     int skip_timing;       /* 1: the dense entry points skip their device
-                              timing (no elapsed-time queries; the replayed
-                              fused call records no events); kernel_s and
-                              device_s in spb_result are then 0.  About 6 us
-                              less per call, for callers that time calls
-                              themselves                                    */
+                              timing (n > 26: no events around the kernels, a
+                              few us less per call); kernel_s and device_s in
+                              spb_result are then 0                         */
 } spb_options;
 
 typedef struct spb_result {
@@ -106,7 +104,11 @@ typedef struct spb_result {
     double elapsed_s;      /* wall time of the whole call                   */
     double kernel_s;       /* device time of the Gray-walk kernels          */
     double device_s;       /* device time of the whole call on its stream:
-                              input copy (if any), kernels, result copy     */
+                              input copy (if any), kernels, result copy.
+                              Dense calls of n <= 26 take both times from
+                              the kernels' own stamps of the device's clock
+                              (from the first kernel's start to the result
+                              in host memory), larger ones from events      */
     double err_est;        /* estimated relative error (statistical); for
                               spb_perm_approx the relative standard error */
     uint64_t gray_steps;   /* Gray steps of the Nijenhuis-Wilf formula,

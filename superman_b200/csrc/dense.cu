@@ -53,6 +53,7 @@ namespace dense {
 //   4 warps: 0, 1 tables (part 0, 1), 2 start values, 3 high columns.
 __global__ void __launch_bounds__(128) setup_kernel(Problem pb, const double* __restrict__ a_in, int smem_tables)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) pb.rb->stamp[0] = global_ns();
     const int n = pb.n, c = pb.comps, w = pb.w, G = pb.g;
     const int tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, wid = tid >> 5, r = blockIdx.x;
     const int terms = 1 << w;
@@ -276,8 +277,7 @@ size_t small_call_smem_bytes(int n, int w, int threads);
 int launch_small_call(const Problem& pb, const double* d_a, const double* a_stage, int blocks, int threads,
                       Readback* rb_host, int dev, int sms, cudaStream_t s, bool* launched);
 int launch_small_call_graph(DeviceContext* ctx, const Problem& pb, const double* d_a, const double* a_stage,
-                            int blocks, int threads, Readback* rb_host, bool timed, cudaStream_t s,
-                            bool* launched);
+                            int blocks, int threads, Readback* rb_host, cudaStream_t s, bool* launched);
 
 // The staged matrix plus, when they fit, one row's subset-sum tables: the setup
 // kernel's dynamic shared-memory limit is raised to the maximum once per
@@ -586,6 +586,10 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
     constexpr size_t kStageOff = 256;
     static_assert(sizeof(Readback) <= kStageOff, "readback fits before the staging area");
     const size_t a_bytes = sizeof(double) * n * n * comps;
+    // device times: events around the kernels, or (small calls) the kernels' own
+    // stamps; none with skip_timing
+    const bool events = !opt.skip_timing && (n > kStampedMaxN || !ctx->pinned_dev);
+    auto record = [&](cudaEvent_t ev) { return events ? cudaEventRecord(ev, stream) : cudaSuccess; };
     if ((st = ensure_pinned(ctx, kStageOff + a_bytes)) != SPB_OK) return out->status = st;
     Readback* hrb = static_cast<Readback*>(ctx->pinned);
     // The refinement list is sized before the walk for the threshold's cap
@@ -612,39 +616,40 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
     // device can address it (no copy after the kernel), and takes a host
     // matrix from the pinned staging area itself (no copy before it: a copy
     // engine takes several microseconds to start for 4.6 KB).  A launch asked
-    // for again is replayed as a CUDA graph (events and kernel; the kernel
-    // alone with skip_timing).
+    // for again is replayed as a CUDA graph.
     const bool fused_fits = small_candidate && pb.units <= kRawCap &&
                             small_call_smem_bytes(n, pb.w, threads) <= ctx->smem_optin;
     Readback* mapped = static_cast<Readback*>(ctx->pinned_dev);
     const double* a_stage = nullptr;  // device address of the staged host matrix
-    if (fused_fits && mapped && !a_on_device) {
+    // The plain walk's setup kernel, whose CTAs need a row each, reads a host
+    // matrix from the staging area too, where it lies (with the derivative walk
+    // every CTA needs the whole matrix: 195 KB at n=29 took it 15 us longer over
+    // the host link than the copy).
+    const bool map_in = mapped && !a_on_device && !pb.deriv;
+    if (mapped && !a_on_device && (fused_fits || map_in)) {
         std::memcpy(static_cast<char*>(ctx->pinned) + kStageOff, a, a_bytes);
         a_stage = reinterpret_cast<const double*>(static_cast<char*>(ctx->pinned_dev) + kStageOff);
     }
     bool fused = false, graphed = false;
     if (fused_fits && mapped) {
-        if ((st = launch_small_call_graph(ctx, pb, d_a, a_stage, blocks, threads, mapped, !opt.skip_timing, stream,
-                                          &fused)) != SPB_OK)
+        if ((st = launch_small_call_graph(ctx, pb, d_a, a_stage, blocks, threads, mapped, stream, &fused)) != SPB_OK)
             return out->status = st;
         graphed = fused;
     }
     if (!graphed) {
-        SPB_CUDA_TRY(cudaEventRecord(ctx->ev_call0, stream));
+        SPB_CUDA_TRY(record(ctx->ev_call0));
         if (!a_on_device && !a_stage)
             SPB_CUDA_TRY(cudaMemcpyAsync(d_in, a, a_bytes, cudaMemcpyHostToDevice, stream));
         if (fused_fits) {
-            SPB_CUDA_TRY(cudaEventRecord(ctx->ev_begin, stream));
+            SPB_CUDA_TRY(record(ctx->ev_begin));
             if ((st = launch_small_call(pb, d_a, a_stage, blocks, threads, mapped, ctx->device, ctx->sm_count,
                                         stream, &fused)) != SPB_OK)
                 return out->status = st;
             if (fused) {
-                SPB_CUDA_TRY(cudaEventRecord(ctx->ev_end, stream));
-                SPB_CUDA_TRY(cudaEventRecord(ctx->ev_call1, stream));
+                SPB_CUDA_TRY(record(ctx->ev_end));
+                SPB_CUDA_TRY(record(ctx->ev_call1));
             }
         }
-        // the fused call did not run: the separate kernels read the matrix at d_in
-        if (!fused && a_stage) SPB_CUDA_TRY(cudaMemcpyAsync(d_in, a, a_bytes, cudaMemcpyHostToDevice, stream));
     }
     if (fused) {
         if (!mapped) SPB_CUDA_TRY(cudaMemcpyAsync(hrb, pb.rb, sizeof(Readback), cudaMemcpyDeviceToHost, stream));
@@ -659,12 +664,9 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
         }
     }
     if (!fused) {
-    // after a replayed fused call whose count check failed, the call's device
-    // span is timed from here (the graph records no ev_call0)
-    if (graphed) SPB_CUDA_TRY(cudaEventRecord(ctx->ev_call0, stream));
-    if ((st = launch_setup(pb, d_a, stream)) != SPB_OK) return out->status = st;
+    if ((st = launch_setup(pb, a_stage ? a_stage : d_a, stream)) != SPB_OK) return out->status = st;
     SPB_CUDA_TRY(cudaGetLastError());
-    SPB_CUDA_TRY(cudaEventRecord(ctx->ev_begin, stream));
+    SPB_CUDA_TRY(record(ctx->ev_begin));
     launches = 2;
     if (dd_mode && pb.na == n && pb.units > pb.raw_cap / 2) {
         // Size the first pass's unit list from a bound-only pass (about 1.5 %
@@ -674,29 +676,33 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
         if ((st = launch_bound_pass(pb, blocks, stream)) != SPB_OK) return out->status = st;
         launches += 2;
     }
+    // the call's last kernel, the FP64 or FP32 walk or the refinement, fills
+    // the host's copy of the readback
+    pb.rb_host = dd_mode ? nullptr : mapped;
     st = pb.f32 ? launch_walk_f32(pb, blocks, threads, smem, stream) : launch_walk(pb, blocks, threads, smem, stream);
     if (st != SPB_OK) return out->status = st;
-    SPB_CUDA_TRY(cudaEventRecord(ctx->ev_end, stream));
+    SPB_CUDA_TRY(record(ctx->ev_end));
 
     // Double-double: threshold, listing and refinement follow the walk on the
     // stream; the host reads everything back once.
     auto enqueue_refinement = [&]() -> int {
         int r;
         if ((r = launch_listing(pb, stream)) != SPB_OK) return r;
-        if ((r = launch_refine(pb, blocks, stream)) != SPB_OK) return r;
-        SPB_CUDA_TRY(cudaEventRecord(ctx->ev_ref1, stream));
+        if ((r = launch_refine(pb, blocks, mapped, stream)) != SPB_OK) return r;
+        SPB_CUDA_TRY(record(ctx->ev_ref1));
         launches += 2;
         return SPB_OK;
     };
-    auto read_back = [&]() -> int {
-        SPB_CUDA_TRY(cudaEventRecord(ctx->ev_call1, stream));
-        SPB_CUDA_TRY(cudaMemcpyAsync(hrb, pb.rb, sizeof(Readback), cudaMemcpyDeviceToHost, stream));
+    auto read_back = [&](bool published) -> int {
+        SPB_CUDA_TRY(record(ctx->ev_call1));
+        if (!(mapped && published))
+            SPB_CUDA_TRY(cudaMemcpyAsync(hrb, pb.rb, sizeof(Readback), cudaMemcpyDeviceToHost, stream));
         SPB_CUDA_TRY(cudaStreamSynchronize(stream));
         return SPB_OK;
     };
     bool refined = false;
     if (dd_mode) {
-        SPB_CUDA_TRY(cudaEventRecord(ctx->ev_ref0, stream));
+        SPB_CUDA_TRY(record(ctx->ev_ref0));
         if ((st = launch_threshold(pb, stream)) != SPB_OK) return out->status = st;
         launches += 1;
         if (!opt.replay_listing) {
@@ -704,7 +710,7 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
             refined = true;
         }
     }
-    if ((st = read_back()) != SPB_OK) return out->status = st;
+    if ((st = read_back(!dd_mode || refined)) != SPB_OK) return out->status = st;
     const dd res0[2] = {hrb->res[0], hrb->res[1]};
     res[0] = res0[0];
     res[1] = res0[1];
@@ -719,10 +725,10 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
                 return out->status = st;
             pb.list_u = static_cast<unsigned long long*>(ctx->list);
             pb.list_cap = count;
-            SPB_CUDA_TRY(cudaEventRecord(ctx->ev_ref0, stream));
+            SPB_CUDA_TRY(record(ctx->ev_ref0));
             SPB_CUDA_TRY(cudaMemsetAsync(pb.list_n, 0, sizeof(unsigned long long), stream));
             if ((st = enqueue_refinement()) != SPB_OK) return out->status = st;
-            if ((st = read_back()) != SPB_OK) return out->status = st;
+            if ((st = read_back(true)) != SPB_OK) return out->status = st;
             ok = hrb->list_n == count;
         }
         if (!ok) {
@@ -736,14 +742,14 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
             pb.list_u = static_cast<unsigned long long*>(ctx->list);
             pb.list_x = reinterpret_cast<double*>(static_cast<char*>(ctx->list) +
                                                   align_up(count * sizeof(unsigned long long), 256));
-            SPB_CUDA_TRY(cudaEventRecord(ctx->ev_ref0, stream));
+            SPB_CUDA_TRY(record(ctx->ev_ref0));
             SPB_CUDA_TRY(cudaMemsetAsync(pb.list_n, 0, sizeof(unsigned long long), stream));
             if (count > 0 && (st = launch_walk(pb, blocks, threads, smem, stream)) != SPB_OK)
                 return out->status = st;
-            if ((st = launch_refine(pb, blocks, stream)) != SPB_OK) return out->status = st;
-            SPB_CUDA_TRY(cudaEventRecord(ctx->ev_ref1, stream));
+            if ((st = launch_refine(pb, blocks, mapped, stream)) != SPB_OK) return out->status = st;
+            SPB_CUDA_TRY(record(ctx->ev_ref1));
             launches += count > 0 ? 2 : 1;
-            if ((st = read_back()) != SPB_OK) return out->status = st;
+            if ((st = read_back(true)) != SPB_OK) return out->status = st;
             if (hrb->list_n != count) {
                 spb_set_error("refinement listed %llu units, histogram counted %llu",
                               (unsigned long long)hrb->list_n, (unsigned long long)count);
@@ -753,16 +759,19 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
         for (int cc = 0; cc < comps; ++cc) res[cc] = dd_add(res0[cc], hrb->corr[cc]);
         out->refined_units = count;
         float mr = 0.f;
-        if (!opt.skip_timing) SPB_CUDA_TRY(cudaEventElapsedTime(&mr, ctx->ev_ref0, ctx->ev_ref1));
+        if (events) SPB_CUDA_TRY(cudaEventElapsedTime(&mr, ctx->ev_ref0, ctx->ev_ref1));
         ms_refine = mr;
     }
     }  // separate kernels
     float ms = 0.f, ms_call = 0.f;
-    if (!opt.skip_timing) {
+    if (events) {
         SPB_CUDA_TRY(cudaEventElapsedTime(&ms, ctx->ev_begin, ctx->ev_end));
-        // a replayed fused call is one kernel, which copies its own input
-        if (graphed && fused) ms_call = ms;
-        else SPB_CUDA_TRY(cudaEventElapsedTime(&ms_call, ctx->ev_call0, ctx->ev_call1));
+        SPB_CUDA_TRY(cudaEventElapsedTime(&ms_call, ctx->ev_call0, ctx->ev_call1));
+    } else if (!opt.skip_timing) {
+        const unsigned long long* t = hrb->stamp;
+        const unsigned long long end = dd_mode || fused ? t[3] : t[2];
+        ms = (float)(1e-6 * (double)(end - (fused ? t[0] : t[1])));
+        ms_call = (float)(1e-6 * (double)(t[3] - t[0]));
     }
 
     // FP32 products: estimated relative error of the result from the sum of

@@ -33,7 +33,20 @@ struct Readback {
     dd scale[2];                // derivative walk: [comps] product of the pivots' mantissas
     int scale_exp;              // and the sum of their exponents
     int pad;
+    // Nanosecond stamps of the device's global timer: the call's first kernel
+    // begins, the walk begins, the walk ends, the readback is complete.  Calls of
+    // up to kStampedMaxN take their device times from them: events around the
+    // kernels and the queries of their times cost such a call 5 to 12 us.
+    unsigned long long stamp[4];
 };
+constexpr int kStampedMaxN = 26;
+
+__device__ __forceinline__ unsigned long long global_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
 
 // Device-side description of one permanent: sizes plus pointers into the
 // scratch arena written by setup_kernel.
@@ -58,6 +71,9 @@ struct Problem {
     dd* result;                // [comps] grid total (rb->res; rb->corr for the refinement)
     int* exp_sum;              // sum of the row scaling exponents (&rb->exp_sum)
     Readback* rb;
+    Readback* rb_host;         // the device's address of the host's page-locked copy of *rb; the
+                               // call's last kernel fills it (null in the others, and where the
+                               // host copies the readback itself)
     double tol;                // SPB_PREC_DD: relative tolerance of the threshold
     // Double-double refinement (SPB_PREC_DD); unused when mode == 0.
     int mode;                  // 0 walk, 1 walk + unit-bound histogram, 2 scan only
@@ -371,6 +387,21 @@ __device__ __forceinline__ dd lane_sum_dd(const dd* p, int count, int lane)
     return v;
 }
 
+// Copies the finished readback to the host's page-locked copy (mapped into
+// the device's address space), reading it through L2: its fields were
+// written by other CTAs and kernels.  The host then needs no copy after the call.
+__device__ __forceinline__ void publish(const Problem& pb, Readback* host)
+{
+    if (!host) return;
+    pb.rb->stamp[3] = global_ns();
+    __threadfence();
+    const unsigned long long* src = reinterpret_cast<const unsigned long long*>(pb.rb);
+    unsigned long long* dst = reinterpret_cast<unsigned long long*>(host);
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(Readback) / sizeof(unsigned long long)); ++i) dst[i] = __ldcg(src + i);
+}
+static_assert(sizeof(Readback) % sizeof(unsigned long long) == 0, "readback copied in 8-byte words");
+
 // Warp -> block -> grid double-double reduction of C components.  The last
 // CTA to finish (ticket election) sums the per-CTA partials in index order,
 // so the result does not depend on CTA completion order.
@@ -409,7 +440,11 @@ __device__ __forceinline__ void grid_reduce(dd (&tot)[C], const Problem& pb)
             v = warp_sum_dd(v);
             if (lane == 0) pb.result[c] = v;
         }
-        if (lane == 0) *pb.ticket = 0u;
+        if (lane == 0) {
+            *pb.ticket = 0u;
+            if (pb.result == pb.rb->res) pb.rb->stamp[2] = global_ns();  // the walk's end
+            publish(pb, pb.rb_host);
+        }
     }
 }
 
@@ -559,10 +594,10 @@ __device__ __forceinline__ double unit_bound_real(const double (&xh)[N], const d
 // D: the derivative walk, whose high columns have low words (s_ml).
 template <int N, bool D>
 __device__ __forceinline__ void first_base(const double* __restrict__ x0h, const double* __restrict__ x0l,
-                                                const double* __restrict__ s_mt, const double* __restrict__ s_ml,
-                                                double* s_lo, int ntop,
-                                                unsigned long long u0, unsigned long long u1, int tid, int bd,
-                                                double (&xh)[N])
+                                           const double* __restrict__ s_mt, const double* __restrict__ s_ml,
+                                           double* s_lo, int ntop,
+                                           unsigned long long u0, unsigned long long u1, int tid, int bd,
+                                           double (&xh)[N])
 {
     const unsigned full = 0xffffffffu;
     const int lane = tid & 31;
@@ -721,6 +756,7 @@ __device__ __forceinline__ void walk_real_body(const Problem& pb)
 template <int N>
 __global__ void __launch_bounds__(RealCfg<N>::kMaxThreads, 1) walk_real(Problem pb)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) pb.rb->stamp[1] = global_ns();
     if constexpr (N >= kMinDerivReal) {
         if (deriv_on(pb)) {
             walk_real_body<N, true>(pb);
@@ -1000,6 +1036,7 @@ __device__ __forceinline__ void walk_complex_body(const Problem& pb)
 template <int N>
 __global__ void __launch_bounds__(ComplexCfg<N>::kMaxThreads, 1) walk_complex(Problem pb)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) pb.rb->stamp[1] = global_ns();
     if constexpr (N >= kMinDerivComplex) {
         if (deriv_on(pb)) {
             walk_complex_body<N, true>(pb);
@@ -1027,7 +1064,7 @@ __global__ void __launch_bounds__(ComplexCfg<N>::kMaxThreads, 1) walk_complex(Pr
 // replays the listing with the walk's own bases (pb.list_x) when the host
 // finds the count check failed.
 int launch_threshold(const Problem& pb, cudaStream_t s);
-int launch_refine(const Problem& pb, int blocks, cudaStream_t s);
+int launch_refine(const Problem& pb, int blocks, Readback* rb_host, cudaStream_t s);  // rb_host: Problem::rb_host
 int launch_bound_pass(const Problem& pb, int blocks, cudaStream_t s);
 int launch_listing(const Problem& pb, cudaStream_t s);
 // Dynamic shared memory of the refinement at `threads` threads per CTA: both

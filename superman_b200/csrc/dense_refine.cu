@@ -445,7 +445,10 @@ __device__ __forceinline__ void worker_sync(int wk)
 __global__ void __launch_bounds__(512, 1) refine_real(Problem pb)
 {
     const unsigned long long count = refine_count(pb);
-    if (count == 0) return;
+    if (count == 0) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) publish(pb, pb.rb_host);
+        return;
+    }
     extern __shared__ __align__(16) double sm[];
     __shared__ dd s_red[16];
     const int n = pb.n, G = pb.g, terms = 1 << pb.w, nq = terms / G;
@@ -578,7 +581,10 @@ __global__ void __launch_bounds__(512, 1) refine_real(Problem pb)
 __global__ void __launch_bounds__(512, 1) refine_complex(Problem pb)
 {
     const unsigned long long count = refine_count(pb);
-    if (count == 0) return;
+    if (count == 0) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) publish(pb, pb.rb_host);
+        return;
+    }
     extern __shared__ __align__(16) double sm[];
     __shared__ dd s_red[2][16];
     const int n = pb.n, G = pb.g, terms = 1 << pb.w, nq = terms / G;
@@ -754,7 +760,7 @@ size_t refine_smem_bytes(const Problem& pb, int threads)
     return sizeof(double) * (2 * c * terms * n + nwarps * (2 * c * n + c * nq) + c * ntp * n);
 }
 
-int launch_refine(const Problem& pb, int blocks, cudaStream_t s)
+int launch_refine(const Problem& pb, int blocks, Readback* rb_host, cudaStream_t s)
 {
     // 512 threads (16 warps per SM hide the double-double latency chains)
     // when their per-warp buffers fit next to the tables, else 256.
@@ -795,6 +801,7 @@ int launch_refine(const Problem& pb, int blocks, cudaStream_t s)
     }
     Problem pr = pb;
     pr.result = pb.rb->corr;
+    pr.rb_host = rb_host;
     kern<<<blocks, threads, smem, s>>>(pr);
     SPB_CUDA_TRY(cudaGetLastError());
     return SPB_OK;

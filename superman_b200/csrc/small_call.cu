@@ -105,20 +105,6 @@ __device__ __forceinline__ dd block_sum_dd(dd v, dd* s_warp)
     return v;
 }
 
-// Copies the finished readback to the host's page-locked copy (mapped into
-// the device's address space), reading it through L2: its fields were
-// written by other CTAs.  The host then needs no copy after the kernel.
-__device__ __forceinline__ void publish(const Problem& pb, Readback* host)
-{
-    if (!host) return;
-    __threadfence();
-    const unsigned long long* src = reinterpret_cast<const unsigned long long*>(pb.rb);
-    unsigned long long* dst = reinterpret_cast<unsigned long long*>(host);
-#pragma unroll
-    for (int i = 0; i < (int)(sizeof(Readback) / sizeof(unsigned long long)); ++i) dst[i] = __ldcg(src + i);
-}
-static_assert(sizeof(Readback) % sizeof(unsigned long long) == 0, "readback copied in 8-byte words");
-
 // The walk's FP64 value of each unit, kept for the refinement in the space
 // of the separate kernels' unit list (pb.raw_u, kRawCap entries of 8 bytes,
 // unused by this call; units <= kRawCap here).
@@ -142,6 +128,7 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
     const int w = pb.w, terms = 1 << w, nq = terms / G;
     const int tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, wid = tid >> 5;
     const int mode = pb.mode;
+    if (blockIdx.x == 0 && tid == 0) pb.rb->stamp[0] = global_ns();
     const SmallLayout L(N, w, bd);
     double* s_a = smem + L.a;
     double* s_al = smem + L.al;
@@ -160,7 +147,11 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
     // (a_stage, mapped): the grid copies it to a_in first, one element per
     // thread, and meets at a barrier, which also publishes the zeroed
     // accumulators; a device matrix is read where it is.
-    const bool staged = a_stage != nullptr;  // the same in every CTA
+    // A grid small enough to fetch the staged matrix once per CTA does so
+    // without the copy and its barrier; the FP64 mode then needs no barrier
+    // before the walk at all (it adds to nothing global).
+    const bool direct = a_stage != nullptr && gridDim.x * (N * N * 8) <= 64 * 1024;
+    const bool staged = a_stage != nullptr && !direct;  // the same in every CTA
     if (blockIdx.x == 0) {
         if (tid < 4) pb.ticket[tid] = 0u;
         if (mode != 0)
@@ -176,7 +167,8 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
         grid.sync();
         for (int i = tid; i < N * N; i += bd) s_a[i] = __ldcg(a_in + i);
     } else {
-        for (int i = tid; i < N * N; i += bd) s_a[i] = a_in[i];
+        const double* a = direct ? a_stage : a_in;
+        for (int i = tid; i < N * N; i += bd) s_a[i] = a[i];
     }
     if (mode != 0)
         for (int i = tid; i < kHistBins; i += bd) { s_hist[i] = 0.0f; s_cnt[i] = 0u; }
@@ -303,7 +295,7 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
         if (deriv) s_ml[idx] = s_al[r * N + (w + j)];
     }
     __syncthreads();
-    if (!staged) grid.sync();  // the zeroed accumulators are visible before anyone adds to them
+    if (!staged && mode != 0) grid.sync();  // the zeroed accumulators are visible before anyone adds to them
 
     // ---- 1. the walk, one unit per thread and pass, evaluated as walk_real
     // evaluates it.  In each pass the warp builds its 32 unit bases
@@ -615,15 +607,12 @@ int launch_small_call(const Problem& pb, const double* d_a, const double* a_stag
 }
 
 // ---- the call as a CUDA graph --------------------------------------------
-// A call issues the events around it and the cooperative launch: several
-// microseconds of host time, during which the device waits for the launch.
-// Replayed as one graph (the kernel between two events) it costs one graph
-// launch.  A
-// graph is built for a launch (the kernel's Problem, its matrix, staging and
-// readback addresses, the shape) the second time that launch is asked for,
-// and kept in a small per-context cache; a matrix given on the device is
-// part of the launch, so a caller that passes a new device pointer each time
-// keeps the direct path.
+// Replayed as a graph a cooperative launch costs the host less than issued
+// anew.  A graph is built for a launch (the kernel's Problem, its matrix,
+// staging and readback addresses, the shape) the second time that launch is
+// asked for, and kept in a small per-context cache; a matrix given on the
+// device is part of the launch, so a caller that passes a new device pointer
+// each time keeps the direct path.
 namespace {
 
 struct SmallGraph {
@@ -636,7 +625,6 @@ struct SmallGraph {
     const double* stage = nullptr;  // device address of the page-locked staging (host input) or null
     Readback* rb_host = nullptr;
     int blocks = 0, threads = 0;
-    bool timed = true;  // the graph records the context's events around the kernel
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
 };
@@ -662,13 +650,13 @@ void release_cache(void* p)
 }
 
 bool same_launch(const SmallGraph& g, const Problem& pb, const double* a, const double* stage, Readback* rb_host,
-                 int blocks, int threads, bool timed)
+                 int blocks, int threads)
 {
     return g.valid && std::memcmp(&g.pb, &pb, sizeof(Problem)) == 0 && g.a == a && g.stage == stage &&
-           g.rb_host == rb_host && g.blocks == blocks && g.threads == threads && g.timed == timed;
+           g.rb_host == rb_host && g.blocks == blocks && g.threads == threads;
 }
 
-// Captures events and kernel on the context's own stream.  Any error ends
+// Captures the kernel on the context's own stream.  Any error ends
 // the capture and leaves the entry marked failed.
 void build(DeviceContext* ctx, SmallGraph& g, SmallKernel kern, size_t smem)
 {
@@ -683,11 +671,7 @@ void build(DeviceContext* ctx, SmallGraph& g, SmallKernel kern, size_t smem)
     const double* as = g.stage;
     Readback* h = g.rb_host;
     void* args[] = {&p, &a, &as, &h};
-    cudaError_t e = cudaSuccess;
-    if (g.timed) e = cudaEventRecordWithFlags(ctx->ev_begin, cs, cudaEventRecordExternal);
-    if (e == cudaSuccess)
-        e = cudaLaunchCooperativeKernel((const void*)kern, dim3(g.blocks), dim3(g.threads), args, smem, cs);
-    if (e == cudaSuccess && g.timed) e = cudaEventRecordWithFlags(ctx->ev_end, cs, cudaEventRecordExternal);
+    cudaError_t e = cudaLaunchCooperativeKernel((const void*)kern, dim3(g.blocks), dim3(g.threads), args, smem, cs);
     cudaGraph_t graph = nullptr;
     const cudaError_t e2 = cudaStreamEndCapture(cs, &graph);
     if (e == cudaSuccess) e = e2;
@@ -708,13 +692,10 @@ void build(DeviceContext* ctx, SmallGraph& g, SmallKernel kern, size_t smem)
 // The fused call through a cached graph, on stream s.  The kernel reads its
 // matrix at d_a; with host input, a_stage (the device address of the
 // page-locked staging that holds it) is copied there by the kernel first.
-// When timed, the graph also records the context's events ev_begin and
-// ev_end around the kernel, which is then the whole call on the device (the
-// matrix copy is its first step).  *launched tells whether it ran; when it
+// *launched tells whether it ran; when it
 // did not, nothing was enqueued.
 int launch_small_call_graph(DeviceContext* ctx, const Problem& pb, const double* d_a, const double* a_stage,
-                            int blocks, int threads, Readback* rb_host, bool timed, cudaStream_t s,
-                            bool* launched)
+                            int blocks, int threads, Readback* rb_host, cudaStream_t s, bool* launched)
 {
     *launched = false;
     SmallKernel kern = small_kernel(pb.n);
@@ -729,7 +710,7 @@ int launch_small_call_graph(DeviceContext* ctx, const Problem& pb, const double*
     SmallGraphCache* c = static_cast<SmallGraphCache*>(ctx->small_graphs);
     SmallGraph* g = nullptr;
     for (SmallGraph& x : c->e)
-        if (same_launch(x, pb, d_a, a_stage, rb_host, blocks, threads, timed)) g = &x;
+        if (same_launch(x, pb, d_a, a_stage, rb_host, blocks, threads)) g = &x;
     if (!g) {  // first sight of this launch: remember it, run it directly
         SmallGraph* lru = &c->e[0];
         for (SmallGraph& x : c->e)
@@ -739,7 +720,6 @@ int launch_small_call_graph(DeviceContext* ctx, const Problem& pb, const double*
         lru->pb = pb;
         lru->a = d_a;
         lru->stage = a_stage;
-        lru->timed = timed;
         lru->rb_host = rb_host;
         lru->blocks = blocks;
         lru->threads = threads;
