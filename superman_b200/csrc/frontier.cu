@@ -45,22 +45,51 @@ namespace frontier {
 namespace {
 
 constexpr int kThreads = 1024;
+constexpr int kMaxCluster = 8;  // the portable cluster size
 constexpr size_t kSmem = sizeof(double2) * 2 << kNarrow;  // 64 KB
+
+// What the host reads: the total, and the device's global timer (ns) as the
+// kernel began and ended.
+struct Outcome {
+    dd total;
+    unsigned long long begin, end;
+};
 
 struct Tables {
     double2* t[2][2];    // [half][parity]: step s of a half writes parity s & 1
     dd* partials;        // [grid]
     unsigned* ticket;    // last-CTA election
-    dd* result;          // page-locked host memory, mapped
+    unsigned long long* begin;
+    Outcome* out;        // page-locked host memory, mapped
 };
 
-// acc + a * t in double-double: the product to ~2^-106, its sum as dd_add.
-__device__ __forceinline__ dd mul_add(dd acc, double a, double2 t)
+__device__ __forceinline__ unsigned long long global_ns()
 {
-    const double p = __dmul_rn(a, t.x);
-    const double e = __fma_rn(a, t.y, __fma_rn(a, t.x, -p));
-    return dd_add(acc, fast_two_sum(p, e));
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
 }
+
+// A double-double sum of products a * t: the high words by TwoSum in order, all
+// rounding errors and low words in one FP64 sum beside it (they are 2^-53 of the
+// high words, so its own rounding is of the order of the result's).  The chain
+// from entry to entry is one addition, not a normalised double-double one.
+struct Sum {
+    double hi = 0.0, lo = 0.0;
+    __device__ __forceinline__ void add(double a, double2 t)
+    {
+        const double p = __dmul_rn(a, t.x);
+        const double e = __fma_rn(a, t.y, __fma_rn(a, t.x, -p));
+        const dd s = two_sum(hi, p);
+        hi = s.hi;
+        lo = add_rn(lo, add_rn(s.lo, e));
+    }
+    __device__ __forceinline__ double2 value() const
+    {
+        const dd v = fast_two_sum(hi, lo);
+        return make_double2(v.hi, v.lo);
+    }
+};
 
 // State `idx` of the table after step `st`, from the table before it.  Four
 // entries' states are loaded before the first is added, so a state waits for
@@ -75,7 +104,7 @@ __device__ __forceinline__ double2 advance(const Plan& P, const Step& st, const 
         const unsigned low = (m & (0u - m)) - 1u;
         full = (full & low) | ((full & ~low) << 1) | (low + 1u);
     }
-    dd acc = {0.0, 0.0};
+    Sum acc;
     if (__popc(full) == st.used) {
         for (int e0 = 0; e0 < st.entries; e0 += 4) {
             double2 t[4];
@@ -90,17 +119,24 @@ __device__ __forceinline__ double2 advance(const Plan& P, const Step& st, const 
             }
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-                if (e0 + k < st.entries) acc = mul_add(acc, P.val[st.entry + e0 + k], t[k]);
+                if (e0 + k < st.entries) acc.add(P.val[st.entry + e0 + k], t[k]);
         }
     }
-    return make_double2(acc.hi, acc.lo);
+    return acc.value();
 }
 
 __device__ __forceinline__ dd dd_mul_dd(double2 a, double2 b) { return dd_mul(dd{a.x, a.y}, dd{b.x, b.y}); }
 
+// COOP: the grid is launched cooperatively, else it is one cluster, whose
+// barrier is several times cheaper and whose launch needs no residency check.
+template <bool COOP>
 __global__ void __launch_bounds__(kThreads, 1) expand_rows(const __grid_constant__ Plan A, const Tables T)
 {
-    cg::grid_group grid = cg::this_grid();
+    auto sync_all = [] {
+        if constexpr (COOP) cg::this_grid().sync();
+        else cg::this_cluster().sync();
+    };
+    if (blockIdx.x == 0 && threadIdx.x == 0) *T.begin = global_ns();
     // The plan's used part goes to shared memory at once: read in place, every
     // step's first look at its row missed the constant cache anew (about 2 us
     // a step).
@@ -140,7 +176,7 @@ __global__ void __launch_bounds__(kThreads, 1) expand_rows(const __grid_constant
             }
         }
     }
-    grid.sync();
+    sync_all();
     // the remaining steps, one of each half at a time, over the whole grid
     const int wf = P.nf - P.hf, wb = P.nb - P.hb, wide = wf > wb ? wf : wb;
     const unsigned g = blockIdx.x * kThreads + tid, G = gridDim.x * kThreads;
@@ -152,7 +188,7 @@ __global__ void __launch_bounds__(kThreads, 1) expand_rows(const __grid_constant
             const unsigned at = h ? i - cf : i;
             __stcg(T.t[h][s & 1] + at, advance<true>(P, P.step[(h ? P.nf : 0) + s], T.t[h][(s + 1) & 1], at));
         }
-        grid.sync();
+        sync_all();
     }
     // the cut: front set M meets the back set of the other open columns
     const double2* front = T.t[0][(P.nf + 1) & 1];
@@ -182,19 +218,19 @@ __global__ void __launch_bounds__(kThreads, 1) expand_rows(const __grid_constant
         for (unsigned b = lane; b < gridDim.x; b += 32)
             v = dd_add(v, dd{__ldcg(&T.partials[b].hi), __ldcg(&T.partials[b].lo)});
         v = warp_sum_dd(v);
-        if (lane == 0) *T.result = v;
+        if (lane == 0) *T.out = Outcome{v, __ldcg(T.begin), global_ns()};
     }
 }
 
 }  // namespace
 
-// Fitted on one B200 to kernel times of 31 us (n=20, 20 narrow steps of 7 open
-// columns at most), 52 us (n=24, 12), 61 us (n=26, 13), 128 us (n=30, 19) and 229 us
-// (n=34, 20 and 10.5 million states).
+// Fitted on one B200 to kernel times of 15 us (n=20, 10 narrow steps a half), 20 us
+// (n=30, 15), 38 us (n=20, 10 and 3 wide), 59 us (n=34, 9 and 10), 109 us (n=30, 11
+// wide, 4.4 million states) and 205 us (n=34, 13 wide, 10.5 million).
 double expansion_seconds(const Plan& p)
 {
     const int wide = std::max(p.nf - p.hf, p.nb - p.hb);
-    return 20e-6 + 1.0e-6 * std::max(p.hf, p.hb) + 4e-6 * wide + 14e-12 * p.states;
+    return 7e-6 + 0.9e-6 * std::max(p.hf, p.hb) + 4e-6 * wide + 13e-12 * p.states;
 }
 
 int run(const Plan& p, const spb_options* opt, spb_result* out, DeviceContext* own_ctx, bool* launched)
@@ -219,24 +255,33 @@ int run(const Plan& p, const spb_options* opt, spb_result* out, DeviceContext* o
     }
     int blocks = (int)std::min((double)ctx->sm_count, std::ceil(most / kThreads));
     if (blocks < 2) blocks = 2;
+    // One cluster while a step's states give its threads two each at most,
+    // above that the whole GPU.
+    const bool coop = most > 2.0 * kMaxCluster * kThreads;
+    if (!coop) {
+        int c = 2;
+        while (c < blocks && c < kMaxCluster) c *= 2;
+        blocks = c;
+    }
     static std::mutex mu;
     static signed char fits[64];  // per device: 1 a CTA per SM stays resident, -1 not
     {
         std::lock_guard<std::mutex> lk2(mu);
         signed char& f = fits[ctx->device & 63];
         if (f == 0) {
-            int coop = 0, per_sm = 0;
-            SPB_CUDA_TRY(cudaFuncSetAttribute(expand_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
-            SPB_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
-            SPB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, expand_rows, kThreads, kSmem));
-            f = coop && per_sm >= 1 && ctx->sm_count >= 2 ? 1 : -1;
+            int can = 0, per_sm = 0;
+            SPB_CUDA_TRY(cudaFuncSetAttribute(expand_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
+            SPB_CUDA_TRY(cudaFuncSetAttribute(expand_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
+            SPB_CUDA_TRY(cudaDeviceGetAttribute(&can, cudaDevAttrCooperativeLaunch, ctx->device));
+            SPB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, expand_rows<true>, kThreads, kSmem));
+            f = can && per_sm >= 1 && ctx->sm_count >= 2 ? 1 : -1;
         }
         if (f < 0) return SPB_OK;
     }
 
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
-    const size_t o_tick = take(sizeof(unsigned));
+    const size_t o_tick = take(sizeof(unsigned)), o_begin = take(sizeof(unsigned long long));
     const size_t o_part = take(sizeof(dd) * blocks);
     size_t o_t[2][2];
     for (int h = 0; h < 2; ++h)
@@ -246,7 +291,7 @@ int run(const Plan& p, const spb_options* opt, spb_result* out, DeviceContext* o
             o_t[h][q] = take(sizeof(double2) << w);
         }
     if ((st = ensure_scratch(ctx, off)) != SPB_OK) return out->status = st;
-    if ((st = ensure_pinned(ctx, sizeof(dd))) != SPB_OK) return out->status = st;
+    if ((st = ensure_pinned(ctx, sizeof(Outcome))) != SPB_OK) return out->status = st;
     if (!ctx->pinned_dev) return SPB_OK;
     char* base = static_cast<char*>(ctx->scratch);
     Tables t{};
@@ -254,25 +299,36 @@ int run(const Plan& p, const spb_options* opt, spb_result* out, DeviceContext* o
         for (int q = 0; q < 2; ++q) t.t[h][q] = reinterpret_cast<double2*>(base + o_t[h][q]);
     t.ticket = reinterpret_cast<unsigned*>(base + o_tick);
     t.partials = reinterpret_cast<dd*>(base + o_part);
-    t.result = static_cast<dd*>(ctx->pinned_dev);
+    t.begin = reinterpret_cast<unsigned long long*>(base + o_begin);
+    t.out = static_cast<Outcome*>(ctx->pinned_dev);
 
-    const bool timed = !opt->skip_timing;
-    if (timed) SPB_CUDA_TRY(cudaEventRecord(ctx->ev_begin, stream));
-    Plan plan = p;
-    void* args[] = {&plan, &t};
-    SPB_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)expand_rows, dim3(blocks), dim3(kThreads), args, kSmem, stream));
-    if (timed) SPB_CUDA_TRY(cudaEventRecord(ctx->ev_end, stream));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at{};
+    if (coop) {
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+    } else {
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)blocks;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    }
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    SPB_CUDA_TRY(cudaLaunchKernelEx(&cfg, coop ? expand_rows<true> : expand_rows<false>, p, t));
     SPB_CUDA_TRY(cudaStreamSynchronize(stream));
     *launched = true;
-    float ms = 0.f;
-    if (timed) SPB_CUDA_TRY(cudaEventElapsedTime(&ms, ctx->ev_begin, ctx->ev_end));
-    const dd res = *static_cast<const dd*>(ctx->pinned);
+    const Outcome o = *static_cast<const Outcome*>(ctx->pinned);
+    const dd res = o.total;
     out->value = std::ldexp(res.hi, p.exp_sum);
     out->value_lo = std::ldexp(res.lo, p.exp_sum);
     // every state carries a few roundings of 2^-104 per row, and no partial
     // sum exceeds the product of the rows' absolute sums
     out->err_est = res.hi != 0.0 ? 4.0 * p.n * 0x1p-104 * p.abs_bound / std::fabs(res.hi) : 0.0;
-    out->kernel_s = out->device_s = ms * 1e-3;
+    out->kernel_s = out->device_s = opt->skip_timing ? 0.0 : 1e-9 * (double)(o.end - o.begin);
     out->gray_steps = (uint64_t)p.n << (p.n - 1);
     out->launches = 1;
     out->active_rows = p.width;

@@ -186,15 +186,12 @@ bool plan_expansion(const double* a, int n, const spb_options& opt, frontier::Pl
     return frontier::make_plan(a, n, plan);
 }
 
-// Estimated wall time of the walk the automatic mode would take: FP64-pipe
-// operations at 1.3e13 a second, on top of what the call costs before its
-// first term (n=20: 132 us of wall time, 51 of them kernels, for the
-// row-compacted walk's five launches; 45 us for a fused dense call).
-double walk_seconds(int n, bool compacted, const Choice& ch)
-{
-    if (compacted) return 110e-6 + ch.cost / 1.3e13;
-    return (n <= 26 ? 40e-6 : 75e-6) + 1.5 * n * std::ldexp(1.0, n - 1) / 1.3e13;
-}
+// Estimated wall times of the walks: FP64-pipe operations at 1.3e13 a second, on
+// top of what a call costs before its first term (n=20: 132 us of wall time, 51 of
+// them kernels, for the row-compacted walk's five launches; 45 us for a fused
+// dense call, 75 us for a dense call of separate kernels).
+double dense_seconds(int n) { return (n <= 26 ? 40e-6 : 75e-6) + 1.5 * n * std::ldexp(1.0, n - 1) / 1.3e13; }
+constexpr double kCompactedSeconds = 110e-6;
 
 }  // namespace
 
@@ -203,20 +200,24 @@ int run_real_host(const double* a, int n, const spb_options* opt, spb_result* ou
     if (a && n >= 1 && n <= kMaxN && opt->sparse_walk != SPB_SPARSE_WALK_NEVER) {
         bool has_zero = false;
         for (size_t i = 0; i < (size_t)n * n && !has_zero; ++i) has_zero = a[i] == 0.0;
-        // The expansion where it is the faster call: at once when it takes
-        // less than any walk's launches do, else by both estimates.
+        // The expansion where it is the faster call (20 us of planning and
+        // launch besides): at once when the walks could not be faster, or by no
+        // more than it takes to plan one (30 to 70 us), else by the estimates.
         frontier::Plan fp;
-        const bool expand = has_zero && out && plan_expansion(a, n, *opt, &fp);
+        bool expand = has_zero && out && plan_expansion(a, n, *opt, &fp);
         const double te = expand ? frontier::expansion_seconds(fp) + 20e-6 : INFINITY;
+        const bool at_once = te < std::min(kCompactedSeconds, dense_seconds(n) + 25e-6);
         Choice ch;
-        const bool compacted = has_zero && te > 50e-6 && plan_compacted(a, n, opt->sparse_walk, *opt, &ch);
-        if (expand && (te <= 50e-6 || te < walk_seconds(n, compacted, ch))) {
+        bool compacted = has_zero && !at_once && plan_compacted(a, n, opt->sparse_walk, *opt, &ch);
+        if (expand && !at_once) expand = te < (compacted ? kCompactedSeconds + ch.cost / 1.3e13 : dense_seconds(n));
+        if (expand) {
             std::memset(out, 0, sizeof(*out));
             bool launched = false;
             const int st = frontier::run(fp, opt, out, ctx, &launched);
             if (st != SPB_OK || launched) return st;
+            if (at_once) compacted = plan_compacted(a, n, opt->sparse_walk, *opt, &ch);
         }
-        if (compacted || (te <= 50e-6 && plan_compacted(a, n, opt->sparse_walk, *opt, &ch))) {
+        if (compacted) {
             std::vector<double> ap((size_t)n * n);
             for (int i = 0; i < n; ++i)
                 for (int j = 0; j < n; ++j) ap[(size_t)i * n + j] = a[(size_t)ch.rows[i] * n + ch.cols[j]];
