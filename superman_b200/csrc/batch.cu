@@ -20,6 +20,8 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <cmath>
+
 #include "batch.h"
 #include "dense_impl.cuh"
 #include "spb_common.cuh"
@@ -81,6 +83,11 @@ struct Team {
     {
         if (CTA) __syncthreads();
         else __syncwarp();
+    }
+    // sync, and whether v holds for any of the threads
+    __device__ __forceinline__ static bool any(bool v)
+    {
+        return CTA ? __syncthreads_or(v) != 0 : __any_sync(0xffffffffu, v) != 0;
     }
 };
 
@@ -258,15 +265,24 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) batch_walk(double* __restri
             TM::sync();  // orders the warp's writes before its reads below
         }
         // row exponents: row max scaled into [0.5, 1)
+        bool any = false;  // a nonzero (or NaN) entry
         for (int r = rank; r < N; r += TM::kSize) {
             double mx = 0.0;
-            for (int j = 0; j < N * C; ++j) mx = fmax(mx, fabs(A[r * N * C + j]));
+            for (int j = 0; j < N * C; ++j) {
+                const double v = A[r * N * C + j];
+                mx = fmax(mx, fabs(v));
+                any |= v != 0.0;
+            }
             int e = 0;
             if (mx > 0.0 && isfinite(mx)) frexp(mx, &e);
             s_exp[r] = e;
         }
-        TM::sync();
+        // A matrix of zeros (the serving loop fills its batches up with them)
+        // takes no walk, which would be the plain one, the slower.
+        any = TM::any(any);
         dd tot[C];
+#pragma unroll
+        for (int c = 0; c < C; ++c) tot[c] = {0.0, 0.0};
         int pivot = -1;
         if constexpr (has_deriv(N)) {
             pivot = dense::pick_pivot(N, [&](int r, int j) {
@@ -275,7 +291,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) batch_walk(double* __restri
             });
             if (pivot >= 0) walk_matrix<N, C, true, SPLIT>(A, s_exp, pivot, slice, part, parts, tot);
         }
-        if (pivot < 0) walk_matrix<N, C, false, SPLIT>(A, s_exp, pivot, slice, part, parts, tot);
+        if (pivot < 0 && any) walk_matrix<N, C, false, SPLIT>(A, s_exp, pivot, slice, part, parts, tot);
         if constexpr (SPLIT) {
             if (lane == 0)
 #pragma unroll
@@ -333,21 +349,36 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) batch_walk(double* __restri
 }
 
 // CTAs per matrix: 0 for a warp per matrix, else a power of two up to
-// kMaxCluster.  A warp per matrix is the cheapest in total (its tables are built
-// once, its lanes never wait for another warp), so matrices are split only
-// while their warps would leave the chip idle (kBusyWarps warps per SM fill the
-// FP64 pipe to about 0.8), and only into parts of four units per thread.
+// kMaxCluster, by the walks that the busiest SM is given.  An SM's FP64 pipe is
+// 0.6 busy with one CTA of four warps and little busier with more, so what counts
+// is how evenly the parts fill the SMs: `rounds` CTAs of 1/c of a matrix, where a
+// warp per matrix hands them out four matrices at a time.  Every CTA builds
+// tables of its own: kTables of the walk at n=16, where the whole is 8 us of the
+// pipe, less in proportion at larger n.  Clusters of 4 and 8 leave some SMs of a
+// GPC over.  4096 matrices or more are a warp each; on one B200 the choice takes
+// 1024 x n=20 from 1448 us (a warp each) to 1248 us, 700 x n=22 from 6324 to
+// 3851 us, complex 24488 to 12531 us, 16 x n=16 from 33 to 27 us (one CTA each,
+// four).
 int choose_split(int n, int count, int sms)
 {
-    constexpr int kBusyWarps = 12;
+    constexpr double kTables = 0.43, kShared = 0.92;  // kShared: a round's time beside other CTAs
     const int nc = has_deriv(n) ? n - 1 : n, top = nc - 1 - (nc - 1 < 5 ? nc - 1 : 5);
-    const long long units = 1ll << top, have = (long long)count * kWarpsPerCta;
-    if (have > (long long)sms * kBusyWarps || units < 4ll * kWarpsPerCta * 32) return 0;
-    int c = 1;
-    while (c < kMaxCluster && have * 2 * c <= (long long)sms * kBusyWarps &&
-           units >= 4ll * kWarpsPerCta * 32 * 2 * c)
-        c *= 2;
-    return c;
+    const double tables = kTables * 16.0 / n * std::ldexp(1.0, 16 - n);
+    auto cost = [&](double ctas, double on, double work) {
+        const double rounds = std::ceil(ctas / on);
+        return rounds * work * (rounds > 1.0 ? kShared : 1.0);
+    };
+    double best = cost(std::ceil((double)count / kWarpsPerCta), sms, kWarpsPerCta);
+    int split = 0;
+    for (int c = 1; c <= kMaxCluster && (1ll << top) >= (long long)c * kWarpsPerCta * 32; c *= 2) {
+        const double on = sms * (c == 8 ? 13.0 / 16.0 : c == 4 ? 15.0 / 16.0 : 1.0);
+        const double t = cost((double)count * c, on, 1.0 / c + tables);
+        if (t < best) {
+            best = t;
+            split = c;
+        }
+    }
+    return split;
 }
 
 template <int N, int C, bool SPLIT>
@@ -361,6 +392,11 @@ int launch_split(double* mats, const unsigned* offs, const double* src, int coun
         static cudaError_t attr = cudaFuncSetAttribute(batch_walk<N, C, SPLIT>,
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         SPB_CUDA_TRY(attr);
+    }
+    if constexpr (!SPLIT) {
+        batch_walk<N, C, false><<<blocks, kWarpsPerCta * 32, smem, s>>>(mats, offs, src, count, out);
+        SPB_CUDA_TRY(cudaGetLastError());
+        return SPB_OK;
     }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(blocks);
@@ -381,7 +417,7 @@ template <int N, int C>
 int launch_n(double* mats, const unsigned* offs, const double* src, int count, double* out, int sms,
              cudaStream_t s)
 {
-    // (four units for each thread of a CTA: n >= 16)
+    // (four units or more for each thread of a CTA)
     if constexpr (N >= 16) {
         const int c = choose_split(N, count, sms);
         if (c > 0) return launch_split<N, C, true>(mats, offs, src, count, out, count * c, c, s);

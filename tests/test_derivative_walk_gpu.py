@@ -166,6 +166,36 @@ def test_batch_split_is_the_same_as_alone(spb, n, cplx):
         assert np.all(np.abs(a - b) <= 2.0 ** -52 * np.abs(a)), (k, a, b)
 
 
+@pytest.mark.parametrize("n,cplx", [(16, False), (16, True), (17, False), (18, True)])
+def test_batch_counts_around_the_split(spb, n, cplx):
+    """Launches of 1 to 2400 matrices, i.e. clusters of eight, four and two CTAs,
+    a CTA each (with more CTAs than SMs, too) and a warp each: the same units, so
+    the same values to the double-double sum's order; a matrix of zeros, which
+    takes no walk, gives 0 in each."""
+    import torch
+    few = 3
+    u = [W.haar_block(n, 60 + k, N=64) if cplx else W.dense_uniform(n, 60 + k) for k in range(few)]
+    first = None
+    for count in (1, 5, 20, 100, 600, 2400):
+        m = np.ascontiguousarray(np.stack([u[k % few] for k in range(count)]))
+        m[count // 2] *= 0.0 if count > 1 else 1.0
+        d = torch.from_numpy(m.view(np.float64)).cuda()
+        out = torch.full((count, 2 if cplx else 1, 2), 7.0, dtype=torch.float64, device="cuda")
+        _lib.check(_lib.lib().spb_perm_batch_dev(ctypes.c_void_p(d.data_ptr()), n, int(cplx), count,
+                                                 ctypes.c_void_p(out.data_ptr()), None))
+        torch.cuda.synchronize()
+        o = out.cpu().numpy()
+        if count > 1:
+            assert np.all(o[count // 2] == 0.0)
+        for k in range(count):
+            if count > 1 and k == count // 2:
+                continue
+            if k < few and (first is None or k not in first):
+                first = {**(first or {}), k: o[k, :, 0]}
+            a = first[k % few]
+            assert np.all(np.abs(a - o[k, :, 0]) <= 2.0 ** -52 * np.abs(a)), (count, k)
+
+
 def test_noalloc_without_a_pivot(spb):
     import torch
     a = no_pivot(W.dense_uniform(24, 3), 4)
