@@ -14,7 +14,7 @@
 //        of one shape into a free slot: H2D copy of the slot's offset table,
 //        then batch_walk, whose warps each copy their matrix from the pinned
 //        mirror into its reserved device location and compute its permanent
-//        there, then D2H of the results, all on the small stream;
+//        there, then D2H of the results, all on the slot's stream;
 //        replayed from one CUDA graph per (shape, padded count, slot) once
 //        that key has been used kGraphAfterUses times.  Completion is
 //        detected with an event per slot, so up to `slots` batches are in
@@ -61,11 +61,14 @@ constexpr int kMaxN = batch::kMaxN;           // batch kernel limit (24)
 constexpr size_t kUnit = batch::kOffsetUnit * sizeof(double);  // pool granule, 256 B
 constexpr int kGraphAfterUses = 3;            // uses of a key before its graph is captured
 
-// Mid-size shapes are batched when at least this many requests of the shape
-// are queued: one warp per matrix takes about 2^(n-21) * 1.5 ms at n > 20,
-// a whole-GPU call about 0.1 ms, so batching pays from ~16 * 2^(n-21)
-// requests on.
-inline size_t mid_batch_min(int n) { return (size_t)16 << (n > 21 ? n - 21 : 0); }
+// Mid-size shapes are batched when at least this many requests of the shape are
+// queued.  A batch of up to 15 takes 95 us (real n=21) to 490 us (n=24), complex
+// 240 us to 1.6 ms, beside other shapes' batches on their own streams; a
+// whole-GPU call 45 to 80 us, complex 85 to 140 us, and shares nothing.  Bursts of
+// mixed sizes on one B200, against batching from 16, 32, 64, 128 queued requests
+// on: 512 of n = 8..24 7.7 -> 5.9 ms, 1024 of n = 16..24 25 -> 13.2 ms, 128 of
+// n = 8..24 2.35 -> 2.05 ms.
+inline size_t mid_batch_min(int n) { return n <= 21 ? 3 : (n == 22 ? 4 : (n == 23 ? 6 : 9)); }
 
 // Host-side double-double product (Dekker with exact FMA).
 inline dd dd_mul_host(dd a, dd b)
@@ -156,6 +159,7 @@ struct Slot {
     unsigned* h_offs = nullptr;
     double* d_out = nullptr;
     double* h_out = nullptr;
+    cudaStream_t stream = nullptr;
     cudaEvent_t ev = nullptr;
     bool busy = false;
     int n = 0, comps = 1, count = 0;
@@ -194,7 +198,6 @@ private:
 
     spb_server_config cfg;
     int device = 0;
-    cudaStream_t small_stream = nullptr;
     std::vector<Slot> slots;
     std::map<GraphKey, cudaGraphExec_t> graphs;
     std::map<GraphKey, int> key_uses;
@@ -243,11 +246,11 @@ int Server::start()
     int st0 = SPB_OK;
     if (!get_context(device, &st0)) return st0;  // device checks, kernel set-up of the shared context
     SPB_CUDA_TRY(cudaSetDevice(device));
-    // Batches go on the highest-priority stream: when SMs free up between
-    // whole-GPU walks, a waiting batch is scheduled before the next walk.
+    // Batches go on streams of the highest priority: when SMs free up between
+    // whole-GPU walks, a waiting batch is scheduled before the next walk.  A
+    // stream per slot, because a shape's queue seldom fills the chip.
     int prio_lo = 0, prio_hi = 0;
     SPB_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi));
-    SPB_CUDA_TRY(cudaStreamCreateWithPriority(&small_stream, cudaStreamNonBlocking, prio_hi));
     // device pool: admitted matrices, plus one zero matrix for padding
     // the zero block sits after the requests' part, outside the allocator
     zero_units = (sizeof(double) * kMaxN * kMaxN * 2 + kUnit - 1) / kUnit;
@@ -274,6 +277,7 @@ int Server::start()
             spb_set_error("spb_server_create: could not allocate %d batch slots", cfg.slots);
             return SPB_ERR_OOM;
         }
+        SPB_CUDA_TRY(cudaStreamCreateWithPriority(&s.stream, cudaStreamNonBlocking, prio_hi));
         SPB_CUDA_TRY(cudaEventCreateWithFlags(&s.ev, cudaEventDisableTiming));
     }
     for (int k = 0; k < cfg.large_workers; ++k) {
@@ -299,10 +303,12 @@ Server::~Server()
         if (t.joinable()) t.join();
     for (DeviceContext* ctx : large_ctx) destroy_context(ctx);
     cudaSetDevice(device);
-    if (small_stream) cudaStreamSynchronize(small_stream);
+    for (auto& s : slots)
+        if (s.stream) cudaStreamSynchronize(s.stream);
     for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
     for (auto& s : slots) {
         if (s.ev) cudaEventDestroy(s.ev);
+        if (s.stream) cudaStreamDestroy(s.stream);
         if (s.d_offs) cudaFree(s.d_offs);
         if (s.d_out) cudaFree(s.d_out);
         if (s.h_offs) cudaFreeHost(s.h_offs);
@@ -310,7 +316,6 @@ Server::~Server()
     }
     if (d_pool) cudaFree(d_pool);
     if (h_pool) cudaFreeHost(h_pool);
-    if (small_stream) cudaStreamDestroy(small_stream);
 }
 
 void Server::enqueue(uint64_t id, const Request& r)
@@ -592,12 +597,12 @@ int Server::launch_slot(int si, int n, int comps, std::vector<uint64_t>& ids)
     const bool graphs_on = cfg.use_graphs >= 0;
     auto enqueue_chain = [&]() -> int {
         SPB_CUDA_TRY(cudaMemcpyAsync(s.d_offs, s.h_offs, sizeof(unsigned) * bucket, cudaMemcpyHostToDevice,
-                                     small_stream));
+                                     s.stream));
         const int r = batch::launch_gathered(h_pool_dev, d_pool, s.d_offs, n, comps == 2, bucket, s.d_out,
-                                             small_stream);
+                                             s.stream);
         if (r != SPB_OK) return r;
         SPB_CUDA_TRY(cudaMemcpyAsync(s.h_out, s.d_out, (size_t)bucket * 2 * comps * sizeof(double),
-                                     cudaMemcpyDeviceToHost, small_stream));
+                                     cudaMemcpyDeviceToHost, s.stream));
         return SPB_OK;
     };
     const GraphKey key{n, comps, bucket, si};
@@ -608,9 +613,9 @@ int Server::launch_slot(int si, int n, int comps, std::vector<uint64_t>& ids)
             // The key's earlier plain launches set the kernel's attributes
             // outside any capture; capture the copy-walk-copy chain.
             cudaGraph_t g = nullptr;
-            SPB_CUDA_TRY(cudaStreamBeginCapture(small_stream, cudaStreamCaptureModeThreadLocal));
+            SPB_CUDA_TRY(cudaStreamBeginCapture(s.stream, cudaStreamCaptureModeThreadLocal));
             int rc = enqueue_chain();
-            cudaError_t ce = cudaStreamEndCapture(small_stream, &g);
+            cudaError_t ce = cudaStreamEndCapture(s.stream, &g);
             if (rc != SPB_OK) return rc;
             SPB_CUDA_TRY(ce);
             cudaGraphExec_t ge = nullptr;
@@ -621,14 +626,14 @@ int Server::launch_slot(int si, int n, int comps, std::vector<uint64_t>& ids)
             std::lock_guard<std::mutex> lk(mu);
             ++st.graphs_captured;
         }
-        SPB_CUDA_TRY(cudaGraphLaunch(it->second, small_stream));
+        SPB_CUDA_TRY(cudaGraphLaunch(it->second, s.stream));
         std::lock_guard<std::mutex> lk(mu);
         ++st.graph_launches;
     } else {
         const int rc = enqueue_chain();
         if (rc != SPB_OK) return rc;
     }
-    SPB_CUDA_TRY(cudaEventRecord(s.ev, small_stream));
+    SPB_CUDA_TRY(cudaEventRecord(s.ev, s.stream));
     s.busy = true;
     s.n = n;
     s.comps = comps;
