@@ -1,4 +1,5 @@
-// Many small permanents in one launch: one warp per matrix.
+// Many small permanents in one launch: one warp per matrix, a CTA or a cluster
+// each where there are too few matrices for that (choose_split).
 //
 // The whole-GPU walk (dense_impl.cuh) spreads one permanent over every SM;
 // for n <= 24 a permanent is too small for that (2^(n-1) terms, a few
@@ -38,7 +39,13 @@ constexpr int kMaxCluster = 8;  // CTAs that may share a matrix (the portable cl
 template <int N, int C, bool D, int T>
 struct Cfg {
     static constexpr int NC = N - (D ? 1 : 0);           // walked columns
-    static constexpr int W = NC - 1 < 5 ? NC - 1 : 5;    // low column bits per unit
+    // low column bits per unit.  A unit's base costs about 10 operations per row,
+    // a tenth of a real unit's work at 32 terms, 6 % of a complex one's.  Real
+    // matrices of n >= 18 take 64 terms (three CTAs per SM stay, the registers'
+    // limit): 4096 x n=20 4825 -> 4533 us, 1500 x n=24 34.6 -> 32.3 ms, errors as
+    // before.  Complex ones would leave room for one CTA per SM.
+    static constexpr int LOW = C == 1 && N >= 18 ? 6 : 5;
+    static constexpr int W = NC - 1 < LOW ? NC - 1 : LOW;
     static constexpr int G = C == 1 ? (W >= 2 ? 4 : (W == 1 ? 2 : 1)) : (W >= 1 ? 2 : 1);
     static constexpr int TERMS = 1 << W;
     static constexpr int NTOP = NC - 1 - W;
@@ -355,14 +362,13 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) batch_walk(double* __restri
 // warp per matrix hands them out four matrices at a time.  Every CTA builds
 // tables of its own: kTables of the walk at n=16, where the whole is 8 us of the
 // pipe, less in proportion at larger n.  Clusters of 4 and 8 leave some SMs of a
-// GPC over.  4096 matrices or more are a warp each; on one B200 the choice takes
-// 1024 x n=20 from 1448 us (a warp each) to 1248 us, 700 x n=22 from 6324 to
-// 3851 us, complex 24488 to 12531 us, 16 x n=16 from 33 to 27 us (one CTA each,
-// four).
-int choose_split(int n, int count, int sms)
+// GPC over.  4096 matrices or more are a warp each; on one B200 (all with 32 terms
+// per unit) the choice takes 1024 x n=20 from 1448 us (a warp each) to 1248 us,
+// 700 x n=22 from 6324 to 3851 us, complex 24488 to 12531 us, 16 x n=16 from 33
+// to 27 us (one CTA each, four).  top: high column bits, 2^top units.
+int choose_split(int n, int top, int count, int sms)
 {
     constexpr double kTables = 0.43, kShared = 0.92;  // kShared: a round's time beside other CTAs
-    const int nc = has_deriv(n) ? n - 1 : n, top = nc - 1 - (nc - 1 < 5 ? nc - 1 : 5);
     const double tables = kTables * 16.0 / n * std::ldexp(1.0, 16 - n);
     auto cost = [&](double ctas, double on, double work) {
         const double rounds = std::ceil(ctas / on);
@@ -417,9 +423,8 @@ template <int N, int C>
 int launch_n(double* mats, const unsigned* offs, const double* src, int count, double* out, int sms,
              cudaStream_t s)
 {
-    // (four units or more for each thread of a CTA)
     if constexpr (N >= 16) {
-        const int c = choose_split(N, count, sms);
+        const int c = choose_split(N, Cfg<N, C, has_deriv(N), 32>::NTOP, count, sms);
         if (c > 0) return launch_split<N, C, true>(mats, offs, src, count, out, count * c, c, s);
     }
     int blocks = (count + kWarpsPerCta - 1) / kWarpsPerCta;
