@@ -53,7 +53,7 @@ namespace dense {
 //   4 warps: 0, 1 tables (part 0, 1), 2 start values, 3 high columns.
 __global__ void __launch_bounds__(128) setup_kernel(Problem pb, const double* __restrict__ a_in, int smem_tables)
 {
-    if (blockIdx.x == 0 && threadIdx.x == 0) pb.rb->stamp[0] = global_ns();
+    if (pb.timed && blockIdx.x == 0 && threadIdx.x == 0) pb.rb->stamp[0] = global_ns();
     const int n = pb.n, c = pb.comps, w = pb.w, G = pb.g;
     const int tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, wid = tid >> 5, r = blockIdx.x;
     const int terms = 1 << w;
@@ -589,6 +589,7 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
     // device times: events around the kernels, or (small calls) the kernels' own
     // stamps; none with skip_timing
     const bool events = !opt.skip_timing && (n > kStampedMaxN || !ctx->pinned_dev);
+    pb.timed = !events && !opt.skip_timing ? 1 : 0;
     auto record = [&](cudaEvent_t ev) { return events ? cudaEventRecord(ev, stream) : cudaSuccess; };
     if ((st = ensure_pinned(ctx, kStageOff + a_bytes)) != SPB_OK) return out->status = st;
     Readback* hrb = static_cast<Readback*>(ctx->pinned);

@@ -13,8 +13,9 @@ constexpr int kMaxN = 63;
 // Smallest n of the derivative walk in whole-GPU calls.  Below, picking the
 // pivot and dividing by it cost the call more than the walk saves (FP64 calls
 // on one B200, plain against derivative: real n=20 43.6 and 47.1 us, n=22 51.0 and
-// 52.0, n=24 75.5 and 70.5; complex n=21 95.4 and 97.4, n=23 133.5 and 130.9).
-constexpr int kMinDerivReal = 23, kMinDerivComplex = 22;
+// 52.0, n=23 with double-double 45.6 and 48.2 of device time, n=24 75.5 and 70.5; complex n=21
+// 95.4 and 97.4, n=23 133.5 and 130.9).
+constexpr int kMinDerivReal = 24, kMinDerivComplex = 22;
 
 // Everything the host reads back after a call, contiguous so that one copy
 // brings it over: a call costs one host round trip, the double-double
@@ -74,6 +75,7 @@ struct Problem {
     Readback* rb_host;         // the device's address of the host's page-locked copy of *rb; the
                                // call's last kernel fills it (null in the others, and where the
                                // host copies the readback itself)
+    int timed;                 // the kernels stamp their times
     double tol;                // SPB_PREC_DD: relative tolerance of the threshold
     // Double-double refinement (SPB_PREC_DD); unused when mode == 0.
     int mode;                  // 0 walk, 1 walk + unit-bound histogram, 2 scan only
@@ -393,7 +395,7 @@ __device__ __forceinline__ dd lane_sum_dd(const dd* p, int count, int lane)
 __device__ __forceinline__ void publish(const Problem& pb, Readback* host)
 {
     if (!host) return;
-    pb.rb->stamp[3] = global_ns();
+    if (pb.timed) pb.rb->stamp[3] = global_ns();
     __threadfence();
     const unsigned long long* src = reinterpret_cast<const unsigned long long*>(pb.rb);
     unsigned long long* dst = reinterpret_cast<unsigned long long*>(host);
@@ -442,7 +444,7 @@ __device__ __forceinline__ void grid_reduce(dd (&tot)[C], const Problem& pb)
         }
         if (lane == 0) {
             *pb.ticket = 0u;
-            if (pb.result == pb.rb->res) pb.rb->stamp[2] = global_ns();  // the walk's end
+            if (pb.timed && pb.result == pb.rb->res) pb.rb->stamp[2] = global_ns();  // the walk's end
             publish(pb, pb.rb_host);
         }
     }
@@ -756,7 +758,7 @@ __device__ __forceinline__ void walk_real_body(const Problem& pb)
 template <int N>
 __global__ void __launch_bounds__(RealCfg<N>::kMaxThreads, 1) walk_real(Problem pb)
 {
-    if (blockIdx.x == 0 && threadIdx.x == 0) pb.rb->stamp[1] = global_ns();
+    if (pb.timed && blockIdx.x == 0 && threadIdx.x == 0) pb.rb->stamp[1] = global_ns();
     if constexpr (N >= kMinDerivReal) {
         if (deriv_on(pb)) {
             walk_real_body<N, true>(pb);
@@ -1036,7 +1038,7 @@ __device__ __forceinline__ void walk_complex_body(const Problem& pb)
 template <int N>
 __global__ void __launch_bounds__(ComplexCfg<N>::kMaxThreads, 1) walk_complex(Problem pb)
 {
-    if (blockIdx.x == 0 && threadIdx.x == 0) pb.rb->stamp[1] = global_ns();
+    if (pb.timed && blockIdx.x == 0 && threadIdx.x == 0) pb.rb->stamp[1] = global_ns();
     if constexpr (N >= kMinDerivComplex) {
         if (deriv_on(pb)) {
             walk_complex_body<N, true>(pb);

@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
     const int w = pb.w, terms = 1 << w, nq = terms / G;
     const int tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, wid = tid >> 5;
     const int mode = pb.mode;
-    if (blockIdx.x == 0 && tid == 0) pb.rb->stamp[0] = global_ns();
+    if (pb.timed && blockIdx.x == 0 && tid == 0) pb.rb->stamp[0] = global_ns();
     const SmallLayout L(N, w, bd);
     double* s_a = smem + L.a;
     double* s_al = smem + L.al;

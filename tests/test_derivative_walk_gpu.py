@@ -18,7 +18,7 @@ _exact = {}
 
 
 def EXACT(oracle, a):
-    """The oracle's exact value, kept per matrix (seconds each at n = 23)."""
+    """The oracle's exact value, kept per matrix (seconds each at n = 24)."""
     k = a.tobytes()
     if k not in _exact:
         _exact[k] = oracle.exact_perm_complex(a) if np.iscomplexobj(a) else oracle.exact_perm(a)
@@ -46,7 +46,7 @@ def only_pivot(a, c, seed):
 
 @pytest.mark.parametrize("small_call", [0, -1])
 @pytest.mark.parametrize("precision", ["fp64", "dd"])
-@pytest.mark.parametrize("n", [22, 23])
+@pytest.mark.parametrize("n", [23, 24])
 def test_real_pivot_and_no_pivot(spb, oracle, n, precision, small_call):
     u = W.dense_uniform(n, 40 + n)
     for a in (u, no_pivot(u, n), only_pivot(u, 0, n), only_pivot(u, n - 1, n)):
@@ -70,7 +70,7 @@ def test_pivots_far_from_the_row_maxima(spb, oracle):
     """A small entry in every column: quotients up to 2^30 times the row's scale
     keep the range (derivative walk).  Rows 2^-50 outside one entry: products of
     quotients would reach 2^1100, and the plain walk runs."""
-    n = 23
+    n = 24
     u = W.dense_uniform(n, 5) + 0.5
     one = np.eye(n, dtype=bool)
     for a in (np.where(one, u * 2.0 ** -30, u), np.where(one, u, u * 2.0 ** -50)):
@@ -83,7 +83,7 @@ def test_pivots_far_from_the_row_maxima(spb, oracle):
 def test_refinement_listings_agree(spb, oracle, pivot):
     """Many units refined (signed entries, tight tolerance): the first pass's
     list, the fused call's list and the replay select the same units."""
-    a = np.random.default_rng(5).standard_normal((23, 23))
+    a = np.random.default_rng(5).standard_normal((24, 24))
     if not pivot:
         a = no_pivot(a, 7)
     kw = dict(precision="dd", rel_tol=1e-16, sparse_walk=1)
