@@ -51,9 +51,9 @@ WORKLOADS = {
     "approx100": ("approx", 100, 5, "sampling_pattern_perm_plus3_n100_seed5_4Msamples"),
 }
 
-# DRAM bytes (read + write) per walk_real<32> launch, from one ncu capture of
-# this workload (dram__bytes_read.sum + dram__bytes_write.sum).
-NCU_TRAFFIC = {"dense32": 199424}
+# DRAM bytes (read + write) per walk_real<32> launch, the mean of two launches in
+# one ncu capture of this workload (dram__bytes_read.sum + dram__bytes_write.sum).
+NCU_TRAFFIC = {"dense32": 435584}
 
 
 def env_int(name, default):
@@ -431,8 +431,7 @@ def ours_arm(args, wl):
     steps_per_perm = n * 2 ** (n - 1)
     value = world * steps_per_perm / (ms_dev * 1e-3)
     e2e = world * steps_per_perm / (ms_e2e * 1e-3)
-    fp64_per_row = 2 if comps == 1 else 6  # DADD+DMUL (real); 2 DADD+2 DMUL+2 DFMA (complex)
-    alg = fp64_per_row * steps_per_perm  # FP64 pipe instructions per walk launch
+    alg = walk_work(n, comps == 2)  # FP64 pipe instructions per walk launch
     achieved = alg / walk_dev
     roofline = {"bound": "fp64", "achieved": achieved / 1e12, "peak": peak.value / 1e12,
                 "unit": "T FP64-pipe inst/s", "frac": achieved / peak.value,
@@ -532,10 +531,20 @@ SERVE_WORKLOADS = {
 SERVE_BATCH_MAX_N = 24
 
 
-def serve_work(n, cplx):
-    """FP64 pipe instructions of one permanent: per row per Gray step 2 (real:
-    DADD + DMUL) or 6 (complex: 2 DADD, 2 DMUL, 2 DFMA), n*2^(n-1) steps."""
+def walk_work(n, cplx, batched=False):
+    """FP64 pipe instructions of one permanent of a matrix without zeros.  The
+    plain walk takes 2^(n-1) subsets at 2 per row (real: DADD + DMUL) or 6
+    (complex: 2 DADD, 2 DMUL, 2 DFMA); the derivative walk, which runs from n = 24
+    (complex 22; in batches 11) on, 2^(n-2) subsets at 3 (DADD, DMUL, DFMA) or
+    10 (2 DADD, 2 DMUL, 6 DFMA)."""
+    if n >= (11 if batched else 22 if cplx else 24):
+        return (10 if cplx else 3) * n * 2 ** (n - 2)
     return (6 if cplx else 2) * n * 2 ** (n - 1)
+
+
+def serve_work(n, cplx):
+    """walk_work on the path the serving loop gives the size (batches to n = 20)."""
+    return walk_work(n, cplx, batched=n <= 20)
 
 
 def serve_sample(stream):
@@ -767,7 +776,7 @@ def other_arm(args, wl):
                 step()
             torch.cuda.synchronize()  # device-wide: the launches run on the library's default stream
             t = (time.perf_counter() - t0) / args.steps
-        alg = count * 2 * n * 2 ** (n - 1)
+        alg = count * walk_work(n, False, batched=True)
         got = d_out.cpu().numpy()[0::2]
         want0 = S.perm_dense(mats[0]).permanent
         assert abs(got[0] - want0) <= 1e-13 * abs(want0)
@@ -850,18 +859,21 @@ def other_arm(args, wl):
         # what the call copies: the start vector, the doubled low-column
         # table and the high columns in (its width rule), the limbs out
         wb = 8
-        while wb > 2 and ((1 << wb) * n * 4 > 32 * 1024 or n - 1 - wb < 16):
+        while wb > 2 and ((1 << wb) * n * 4 > 32 * 1024 or n - 2 - wb < 16):
             wb -= 1
-        h2d = 4 * n + 4 * (1 << wb) * n + (n - 1 - wb) * n
+        h2d = 4 * n + 4 * (1 << wb) * n + (n - 2 - wb) * n
         # limbs read back: the Bregman-Minc bound rule of the call
         nz = a != 0
         def side(m):
             rs_ = m.sum(axis=1)
             return sum(math.lgamma(r + 1) / math.log(2) / r for r in rs_) if rs_.min() > 0 else 0.0
-        bits = min(side(nz), side(nz.T)) + (n - 1) + 2
+        bits = min(side(nz), side(nz.T)) + (n - 2) + 2
         limbs = 4 if bits <= 128 else 5 if bits <= 160 else 6 if bits <= 192 else 10 if bits <= 320 else 12
         steps = n * 2 ** (n - 1)  # the integer NW walk: 2^(n-1) subsets of n rows
-        alg = 2 * steps  # one integer add + one multiply per row per subset
+        # the expanded walk: 2^(n-2) subsets, one integer add + one multiply per
+        # row, one multiply-add more per row of the line with the fewest ones
+        m = min(int(nz.sum(axis=0).min()), int(nz.sum(axis=1).min()))
+        alg = (2 * n + m) * 2 ** (n - 2)
         line = {"metric": "ryser_gray_steps_per_s", "value": steps / t, "unit": "gray-steps/s (NW, n*2^(n-1))",
                 "n_gpus": 1, "steps": args.steps, "warmup": args.warmup, "ms_per_step": dt * 1e3,
                 "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "int32/multi-limb",
@@ -869,7 +881,7 @@ def other_arm(args, wl):
                 "config": {"workload": desc, "n": n, "seed": seed, "permanent": str(rs[0].permanent),
                            "plain_ryser_equivalent_steps_per_s": n * 2 ** n / t},
                 "roofline": {"bound": "int", "achieved": alg / t / 1e12, "peak": peak.value / 1e12,
-                             "unit": "T int32 ops/s (add+mul per row-update) vs IMAD pipe",
+                             "unit": "T int32 ops/s (row adds, products, derivative) vs IMAD pipe",
                              "frac": alg / t / peak.value, "traffic": None},
                 "e2e": {"value": steps / statistics.mean(walls), "unit": "gray-steps/s (NW, n*2^(n-1))",
                         "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": 4 * limbs,
@@ -889,16 +901,11 @@ def other_arm(args, wl):
         with ClockSampler(0) as clk:
             ts = [step() for _ in range(args.steps)]
         t = statistics.mean(ts)
-        # roofline of the dominant kernel: the pieces' walks, 2 FP64 instructions
-        # per active row per Gray step, over their kernel time
-        _lib.check(L.spb_measure_pipe_peak(0, 0, ctypes.byref(peak)))
+        # the pieces are expanded row by row (a chain of dependent steps): no
+        # pipe or memory rate bounds them, so the line has no roofline
         _, pieces = S.plan_pieces(a)
-        alg, kt, nas = 0, 0.0, []
-        for _, pc in pieces:
-            rr = S.perm_dense(pc, precision=args.precision)
-            alg += 2 * rr.active_rows * 2 ** (pc.shape[0] - 1)
-            kt += rr.kernel_s
-            nas.append(rr.active_rows)
+        rs = [S.perm_dense(pc, precision=args.precision) for _, pc in pieces]
+        launched = sum(r.launches for r in rs)
         # the same matrix as one request of the serving loop: decomposed there,
         # its pieces run as independent requests on two whole-GPU workers
         from superman_b200.serving import Server
@@ -928,10 +935,9 @@ def other_arm(args, wl):
                            "permanent": repr(out.permanent),
                            "rel_err_vs_exact": err, "precision": args.precision,
                            "timing": "host wall clock around spb_perm_pipeline (pruning, decomposition, GPU pieces)"},
-                "roofline": {"bound": "fp64", "achieved": alg / kt / 1e12, "peak": peak.value / 1e12,
-                             "unit": "T FP64-pipe inst/s", "frac": alg / kt / peak.value, "traffic": None,
-                             "kernel": f"row-compacted walk of the {len(pieces)} pieces, active rows {nas}",
-                             "algorithmic_per_permanent": alg},
+                "roofline": None,
+                "kernels": {"kernel_us": [r.kernel_s * 1e6 for r in rs],
+                            "open_columns_or_active_rows": [r.active_rows for r in rs]},
                 "served": {"latency_ms_mean": statistics.mean(lat) * 1e3, "requests": len(lat),
                            "burst_of_8_perms_per_s": burst / t_burst,
                            "permanent": repr(served_val),
@@ -940,7 +946,7 @@ def other_arm(args, wl):
                 "e2e": {"value": 1.0 / t, "unit": "perms/s", "h2d_bytes_per_step": n * n * 8,
                         "d2h_bytes_per_step": 16 * max(1, len(pieces)),
                         "timing": "host wall clock around the public call"},
-                "clocks": clk.summary(), "gpu_launches": 5 * len(pieces)}
+                "clocks": clk.summary(), "gpu_launches": launched * args.steps}
     if not args.no_cpu_baseline:
         cores = os.cpu_count() or 1
         import tempfile
