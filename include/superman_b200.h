@@ -208,8 +208,8 @@ SPB_API int spb_perm_dense_c128(const double* a, int n, const spb_options* opt, 
 SPB_API int spb_perm_dense_c128_dev(const double* d_a, int n, const spb_options* opt,
                             spb_result* out);
 
-/* Permanents of `count` n x n matrices in one launch, one warp per matrix
- * (1 <= n <= 24).  d_mats: device, count consecutive row-major matrices
+/* Permanents of `count` n x n matrices in one launch, one warp per matrix or,
+ * of few matrices, a CTA or a cluster each (1 <= n <= 24).  d_mats: device, count consecutive row-major matrices
  * (is_complex: interleaved re/im, 2*n*n doubles each); d_out: device,
  * 2 doubles per component per matrix, the permanent as a double-double
  * (hi, lo).  Asynchronous on `stream` (NULL = default stream); allocates
@@ -242,7 +242,7 @@ SPB_API int spb_perm_binary(const uint8_t* a, int n, const spb_options* opt, uin
  * (NULL = the default stream); read d_out after synchronising.
  * Precision is that of SPB_PREC_FP64 (FP64 row sums and products,
  * double-double sums, no double-double refinement): about 1e-13 relative at
- * n=24 and 3e-12 at n=32 on U[0,1) entries, so lo is not a double-double
+ * n=24 and 1e-12 at n=32 on U[0,1) entries, so lo is not a double-double
  * accurate correction.  Working memory is one fixed 256 KiB device array per
  * GPU inside the library, so n is limited to 1..40 (larger n:
  * SPB_ERR_INVALID).  The first call on a device looks up that array's address
@@ -338,12 +338,13 @@ SPB_API int spb_decompose(const double* a, int n, int* count, int* sizes, double
  * entries is pruned and decomposed on the host as the reference's main flow
  * does (spb_plan_pieces), and its pieces run as independent requests.
  * Small matrices (n <= 20) are packed per (n, real/complex) into batched
- * launches (one warp per matrix; a batch shape used a few times is captured
+ * launches (spb_perm_batch_dev's kernel; a batch shape used a few times is captured
  * once in a CUDA graph and replayed); mid-size ones (21 <= n <= batch_max_n)
  * are batched when enough of one shape are queued and otherwise run like the
  * large ones; large ones run the whole-GPU walk on large_workers streams with
  * their own working memory, so batches and whole-GPU calls overlap on the
- * device.  A request's result does not depend on what it was batched with. */
+ * device.  A request's result does not depend on what it was batched with,
+ * but for the order of its double-double sum. */
 typedef struct spb_server_config {
     int device;
     int batch_max_n;      /* n <= this may go through batched launches (1..24; 0 = 24) */

@@ -12,7 +12,7 @@
 // Precision: the FP64 walk (the allocating entry points' SPB_PREC_FP64: FP64
 // row sums and products, double-double sums, no double-double refinement of
 // dominant units).  On U[0,1) inputs that is about 1e-13 relative at n=24 and
-// 3e-12 at n=32; the error grows with the cancellation of Ryser's sum.
+// 1e-12 at n=32; the error grows with the cancellation of Ryser's sum.
 //
 // Working memory: g_noalloc_scratch below, kNoAllocScratchBytes (256 KiB) per
 // GPU that loads this library, held until the process exits.  It holds the

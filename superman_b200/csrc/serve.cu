@@ -27,12 +27,13 @@
 //        and short kernels of one call overlap the walk of another; matrices
 //        are copied from the mirror into the pool on that context's stream
 //        (real matrices with zeros go through the host entry, whose planner
-//        may pick the row-compacted walk).
+//        may pick the row-compacted walk or the row-by-row expansion).
 //   poll / wait ─► result with admission and completion timestamps.
 //
-// A request's result depends only on its own matrix: the batch kernel gives
-// each matrix its own warp, tables and reduction (padding entries read a
-// zero matrix and are discarded), and the whole-GPU walk's result does not
+// A request's result depends only on its own matrix (and, in the order of its
+// double-double sum, on the size of its batch): the batch kernel gives each
+// matrix its own warp, CTA or cluster, tables and reduction (padding entries read
+// a zero matrix and are discarded), and the whole-GPU walk's result does not
 // depend on what else runs.
 #include <cuda_runtime.h>
 
