@@ -91,10 +91,14 @@ struct Team {
         if (CTA) __syncthreads();
         else __syncwarp();
     }
-    // sync, and whether v holds for any of the threads
+    // sync, and whether v holds for any of the threads (a warp's vote orders no
+    // memory by itself)
     __device__ __forceinline__ static bool any(bool v)
     {
-        return CTA ? __syncthreads_or(v) != 0 : __any_sync(0xffffffffu, v) != 0;
+        if (CTA) return __syncthreads_or(v) != 0;
+        v = __any_sync(0xffffffffu, v) != 0;
+        __syncwarp();
+        return v;
     }
 };
 

@@ -67,6 +67,19 @@ def test_batch_complex(spb, oracle, n):
         assert err <= 1e-12
 
 
+@pytest.mark.parametrize("n,count", [(11, 6000), (16, 6000)])
+def test_batch_rows_scaled_by_powers_of_two(spb, n, count):
+    """Rows of a matrix, and matrices a warp takes one after the other, whose
+    scaling exponents all differ: every lane reads the exponents the others
+    wrote for this matrix.  Scaling by powers of two changes no bit of the rest."""
+    u = W.dense_uniform(n, seed=n) + 0.125
+    want = run_batch(np.stack([u] * count), False)[0]
+    rng = np.random.default_rng(n)
+    e = rng.integers(-30, 31, size=(count, n))
+    got = run_batch(u * np.exp2(e)[:, :, None], False)
+    assert np.array_equal(got, want * np.exp2(e.sum(axis=1)))
+
+
 def test_batch_empty_and_invalid(spb):
     import torch
     L = _lib.lib()
