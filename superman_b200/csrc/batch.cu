@@ -255,6 +255,10 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) batch_walk(double* __restri
     cg::cluster_group cluster = cg::this_cluster();
     const int parts = SPLIT ? (int)cluster.num_blocks() : 1, part = SPLIT ? (int)cluster.block_rank() : 0;
 
+    // A CTA's shared memory may be written by another of its cluster only once it
+    // has started: each arrives here and waits before the first such write.
+    if constexpr (SPLIT) cluster.barrier_arrive();
+    bool started = false;
     const int teams = SPLIT ? gridDim.x / parts : gridDim.x * kWarpsPerCta;
     for (int m = SPLIT ? blockIdx.x / parts : blockIdx.x * kWarpsPerCta + wid; m < count; m += teams) {
         const size_t base = offs ? (size_t)offs[m] * kOffsetUnit : (size_t)m * N * N * C;
@@ -308,6 +312,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) batch_walk(double* __restri
 #pragma unroll
                 for (int c = 0; c < C; ++c) s_part[c][wid] = tot[c];
             __syncthreads();
+            if (!started) cluster.barrier_wait();  // long since complete: no CTA is waited for
+            started = true;
             if (threadIdx.x == 0)
 #pragma unroll
                 for (int c = 0; c < C; ++c) {

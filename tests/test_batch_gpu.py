@@ -67,11 +67,13 @@ def test_batch_complex(spb, oracle, n):
         assert err <= 1e-12
 
 
-@pytest.mark.parametrize("n,count", [(11, 6000), (16, 6000)])
+@pytest.mark.parametrize("n,count", [(11, 6000), (16, 6000), (17, 1), (17, 9), (17, 30), (18, 60), (18, 200)])
 def test_batch_rows_scaled_by_powers_of_two(spb, n, count):
     """Rows of a matrix, and matrices a warp takes one after the other, whose
     scaling exponents all differ: every lane reads the exponents the others
-    wrote for this matrix.  Scaling by powers of two changes no bit of the rest."""
+    wrote for this matrix.  Scaling by powers of two changes no bit of the rest.  The
+    small counts share a matrix among the CTAs of a cluster of eight, four or two,
+    whose totals meet in the first one's shared memory, or give it one CTA."""
     u = W.dense_uniform(n, seed=n) + 0.125
     want = run_batch(np.stack([u] * count), False)[0]
     rng = np.random.default_rng(n)
