@@ -239,8 +239,17 @@ __device__ __forceinline__ dd quotient(double x, double d)
 }
 
 // (xr + i xi) / (dr + i di) in double-double, to about 2^-102 of its magnitude.
+// Both are first scaled by the power of two that takes the divisor's larger
+// part to [0.5, 1): of a divisor below 2^-460 the squares and their errors
+// would leave the FP64 range.
 __device__ __forceinline__ ddc quotient_c(double xr, double xi, double dr, double di)
 {
+    int e = 0;
+    frexp(fmax(fabs(dr), fabs(di)), &e);
+    dr = ldexp(dr, -e);
+    di = ldexp(di, -e);
+    xr = ldexp(xr, -e);
+    xi = ldexp(xi, -e);
     auto prod = [](double a, double b) {
         const double p = __dmul_rn(a, b);
         return dd{p, __fma_rn(a, b, -p)};

@@ -79,6 +79,29 @@ def test_pivots_far_from_the_row_maxima(spb, oracle):
             assert oracle.rel_err(full(r), EXACT(oracle, a)) <= 2e-13
 
 
+@pytest.mark.parametrize("exp", [-300, -600])
+@pytest.mark.parametrize("n", [11, 22])
+def test_complex_tiny_pivot(spb, oracle, n, exp):
+    """One entry of 2^-300 or 2^-600 in the only column without a zero: its
+    square leaves the FP64 range, its quotients do not.  n = 11 as a batch of one,
+    n = 22 as a whole-GPU call."""
+    import torch
+    a = only_pivot(W.haar_block(n, 5 + n, N=64), 3, n)
+    a[n // 2, 3] *= 2.0 ** exp
+    er, ei = EXACT(oracle, a)
+    if n <= 20:
+        d = torch.from_numpy(a.view(np.float64)).cuda()
+        out = torch.zeros(4, dtype=torch.float64, device="cuda")
+        _lib.check(_lib.lib().spb_perm_batch_dev(ctypes.c_void_p(d.data_ptr()), n, 1, 1,
+                                                 ctypes.c_void_p(out.data_ptr()), None))
+        torch.cuda.synchronize()
+        got = complex(float(out[0]), float(out[2]))
+    else:
+        got = spb.perm_complex(a, precision="fp64").permanent
+    scale = float(np.prod(np.abs(a).sum(axis=1)))
+    assert abs(got - complex(float(er), float(ei))) <= 1e-14 * scale
+
+
 @pytest.mark.parametrize("pivot", [True, False])
 def test_refinement_listings_agree(spb, oracle, pivot):
     """Many units refined (signed entries, tight tolerance): the first pass's
