@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) batch_walk(double* __restri
         for (int c = 0; c < C; ++c) tot[c] = {0.0, 0.0};
         int pivot = -1;
         if constexpr (has_deriv(N)) {
-            pivot = dense::pick_pivot(N, [&](int r, int j) {
+            pivot = dense::pick_pivot(N, false, [&](int r, int j) {
                 const double* e = A + ((size_t)r * N + j) * C;
                 return ldexp(C == 1 ? fabs(e[0]) : fmax(fabs(e[0]), fabs(e[C - 1])), -s_exp[r]);
             });

@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(128) setup_kernel(Problem pb, const double* __
         if (lane == 0) *pb.exp_sum = es;
     }
     if (pb.deriv != 0 && wid == 0) {
-        const int pv = c == 1 ? pick_pivot<1>(s_mat, n) : pick_pivot<2>(s_mat, n);
+        const int pv = c == 1 ? pick_pivot<1>(s_mat, n, pb.mode != 0) : pick_pivot<2>(s_mat, n, pb.mode != 0);
         if (lane == 0) s_pivot = pv;
     }
     __syncthreads();

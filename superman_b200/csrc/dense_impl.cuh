@@ -142,14 +142,19 @@ __device__ __forceinline__ dd dd_step(dd a, double mh, double ml)
 // Pivot column of an n x n matrix whose rows are scaled to maxima in [0.5, 1);
 // mag(r, j) is entry (r, j)'s magnitude (complex: the larger of its parts).
 // The column whose smallest magnitude is largest; -1 when every column holds a
-// zero or a non-finite entry, or when dividing by the pivots could take products
-// of n row values out of the FP64 range (a row's absolute sum is below 2^7,
-// n <= 63; the exponents of those sums over the pivots are added up).  Called
-// by one full warp; every lane returns the same.
+// zero or a non-finite entry, or when dividing by the pivots could take what the
+// walk forms out of the FP64 range.  A row value of the walk is below n, n over
+// its pivot after the division, so a term is below n 2^bits, with `bits` the
+// pivots' exponents and log2 n added up over the rows.  Without refinement
+// (`squares` false) terms are only added up, 2^62 of them at most: 900 bits.  The
+// refinement sums their squares and squares the total: 420 bits (terms below
+// 2^426, squares 2^852, their sum 2^914, the total's square 2^976).  Called by
+// one full warp; every lane returns the same.
 template <class Mag>
-__device__ __forceinline__ int pick_pivot(int n, Mag mag)
+__device__ __forceinline__ int pick_pivot(int n, bool squares, Mag mag)
 {
     const int lane = threadIdx.x & 31;
+    const int log2n = 32 - __clz(n), most = squares ? 420 : 900;
     double best = 0.0;
     int col = -1;
     for (int j = lane; j < n; j += 32) {
@@ -160,10 +165,10 @@ __device__ __forceinline__ int pick_pivot(int n, Mag mag)
             const double m = mag(r, j);
             const int em = (__double2hiint(m) >> 20) & 0x7ff;
             ok = ok && em != 0 && em != 0x7ff;
-            bits += 1023 + 8 - em;
+            bits += 1023 + log2n - em;
             lo = fmin(lo, m);
         }
-        if (ok && bits <= 960 && lo > best) {
+        if (ok && bits <= most && lo > best) {
             best = lo;
             col = j;
         }
@@ -181,9 +186,9 @@ __device__ __forceinline__ int pick_pivot(int n, Mag mag)
 }
 // The same on a row-major array of scaled entries, COMPS interleaved.
 template <int COMPS>
-__device__ __forceinline__ int pick_pivot(const double* a, int n)
+__device__ __forceinline__ int pick_pivot(const double* a, int n, bool squares)
 {
-    return pick_pivot(n, [&](int r, int j) {
+    return pick_pivot(n, squares, [&](int r, int j) {
         const double* e = a + ((size_t)r * n + j) * COMPS;
         return COMPS == 1 ? fabs(e[0]) : fmax(fabs(e[0]), fabs(e[COMPS - 1]));
     });

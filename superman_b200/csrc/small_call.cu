@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
     int pivot = -1;
     if constexpr (N >= kMinDerivReal) {
         if (wid == 0) {
-            const int pv = pb.deriv != 0 ? pick_pivot<1>(s_a, N) : -1;
+            const int pv = pb.deriv != 0 ? pick_pivot<1>(s_a, N, mode != 0) : -1;
             if (lane == 0) s_pivot = pv;
         }
         __syncthreads();

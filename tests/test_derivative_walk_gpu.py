@@ -79,6 +79,52 @@ def test_pivots_far_from_the_row_maxima(spb, oracle):
             assert oracle.rel_err(full(r), EXACT(oracle, a)) <= 2e-13
 
 
+def two_permutations(n, background, seed):
+    """Two permutations of entries near 1 over a small background."""
+    rng = np.random.default_rng(seed)
+    a = background * (0.5 + rng.random((n, n)))
+    p = rng.permutation(n)
+    for s in (0, 1):
+        a[np.arange(n), np.roll(p, s)] = 0.5 + rng.random(n)
+    return a
+
+
+@pytest.mark.parametrize("small_call", [0, -1])
+@pytest.mark.parametrize("background", [1e-3, 1e-4, 1e-5, 1e-6, 1e-7, 1e-8, 1e-9])
+def test_wide_range_is_refined(spb, oracle, background, small_call):
+    """Quotients by entries of the background reach 2^13 to 2^33, products of
+    them 2^360 to 2^800: the refinement, which squares them, still has finite
+    sums to choose its units by, whichever walk that takes.  (These matrices
+    hardly cancel: only a tight tolerance asks for refined units.)"""
+    a = two_permutations(24, background, 7)
+    r = spb.perm_dense(a, precision="dd", small_call=small_call, rel_tol=1e-16)
+    assert 0.0 < r.err_est <= 1e-16 and r.refined_units > 0
+    assert oracle.rel_err(full(r), EXACT(oracle, a)) <= 1e-15  # a few times the tolerance and full's rounding
+
+
+@pytest.mark.parametrize("background", [1e-3, 1e-5, 1e-6, 1e-7])
+def test_wide_range_is_refined_n28(spb, background):
+    a = two_permutations(28, background, 8)
+    r = [spb.perm_dense(np.ascontiguousarray(m), precision="dd", rel_tol=1e-16) for m in (a, a.T)]
+    for x in r:
+        assert 0.0 < x.err_est <= 1e-16 and x.refined_units > 0
+    assert abs(full(r[0]) - full(r[1])) <= 2e-15 * abs(full(r[0]))
+
+
+@pytest.mark.parametrize("background", [1e-6, 1e-8])
+def test_wide_range_is_refined_complex(spb, oracle, background):
+    n = 22
+    rng = np.random.default_rng(9)
+    a = two_permutations(n, background, 9) * np.exp(2j * np.pi * rng.random((n, n)))
+    er, ei = EXACT(oracle, a)
+    ex = complex(float(er), float(ei))
+    r = spb.perm_complex(a, precision="dd", rel_tol=1e-16)
+    # (the plain walk at this size meets the cap of an eighth of the units, and
+    # the rest leaves 1.1e-15 by the estimate)
+    assert 0.0 < r.err_est <= 2e-15 and r.refined_units > 0
+    assert abs(r.permanent - ex) <= 4.0 * r.err_est * abs(ex)
+
+
 @pytest.mark.parametrize("exp", [-300, -600])
 @pytest.mark.parametrize("n", [11, 22])
 def test_complex_tiny_pivot(spb, oracle, n, exp):
