@@ -25,6 +25,7 @@
 
 #include "batch.h"
 #include "dense_impl.cuh"
+#include "per_device.h"
 #include "spb_common.cuh"
 
 namespace cg = cooperative_groups;
@@ -405,9 +406,13 @@ int launch_split(double* mats, const unsigned* offs, const double* src, int coun
         sizeof(double) *
         (SPLIT ? slice_doubles<N, C, kWarpsPerCta * 32>() + N * N * C : slice_doubles<N, C, 32>() * kWarpsPerCta);
     if (smem > 48 * 1024) {
-        static cudaError_t attr = cudaFuncSetAttribute(batch_walk<N, C, SPLIT>,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        SPB_CUDA_TRY(attr);
+        static OncePerDevice<cudaError_t> ready;
+        int dev = 0;
+        SPB_CUDA_TRY(cudaGetDevice(&dev));
+        SPB_CUDA_TRY(ready(dev, [] {
+            return cudaFuncSetAttribute(batch_walk<N, C, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)smem);
+        }));
     }
     if constexpr (!SPLIT) {
         batch_walk<N, C, false><<<blocks, kWarpsPerCta * 32, smem, s>>>(mats, offs, src, count, out);
