@@ -209,10 +209,11 @@ SPB_API int spb_perm_dense_c128_dev(const double* d_a, int n, const spb_options*
                             spb_result* out);
 
 /* Permanents of `count` n x n matrices in one launch, one warp per matrix or,
- * of few matrices, a CTA or a cluster each (1 <= n <= 24).  d_mats: device, count consecutive row-major matrices
- * (is_complex: interleaved re/im, 2*n*n doubles each); d_out: device,
- * 2 doubles per component per matrix, the permanent as a double-double
- * (hi, lo).  Asynchronous on `stream` (NULL = default stream); allocates
+ * of few matrices, a CTA or a cluster each (1 <= n <= 24); a permanent's bits
+ * do not depend on how many others are launched with it.  d_mats: device, count
+ * consecutive row-major matrices (is_complex: interleaved re/im, 2*n*n doubles
+ * each); d_out: device, 2 doubles per component per matrix, the permanent as a
+ * double-double (hi, lo).  Asynchronous on `stream` (NULL = default stream); allocates
  * nothing.  Batched counterpart of the dense drivers above for the many
  * small permanents a serving queue or a decomposition produces; the
  * reference runs each of them through its own chunk loop and launches
@@ -343,8 +344,7 @@ SPB_API int spb_decompose(const double* a, int n, int* count, int* sizes, double
  * are batched when enough of one shape are queued and otherwise run like the
  * large ones; large ones run the whole-GPU walk on large_workers streams with
  * their own working memory, so batches and whole-GPU calls overlap on the
- * device.  A request's result does not depend on what it was batched with,
- * but for the order of its double-double sum. */
+ * device.  A request's result does not depend on what it was batched with. */
 typedef struct spb_server_config {
     int device;
     int batch_max_n;      /* n <= this may go through batched launches (1..24; 0 = 24) */

@@ -9,7 +9,8 @@
 // high columns in the warp's slice of shared memory, then its 32 lanes split
 // the Gray units of that matrix exactly as the threads of the big walk do
 // (same unit evaluators; the double-double unit bases live in registers), and
-// a warp reduction gives the double-double total.  A matrix with a pivot column
+// their sums are added up in double-double, in one order whatever the launch's
+// split (kLeaves).  A matrix with a pivot column
 // (dense_impl.cuh) takes the derivative walk, half the subsets at 3/4 (complex
 // 5/6) of the FP64 instructions, the others the plain walk; the choice is the
 // warp's own.  The permanent of matrix m
@@ -103,6 +104,56 @@ struct Team {
     }
 };
 
+// The order of a matrix's sum (n >= 16, where launches differ in how they split a
+// matrix).  Its units fall into kLeaves runs of equal length (fewer where there
+// are fewer units); a run's unit sums are added one after the other, the runs'
+// sums pairwise as a binary tree over the runs in their order.  A thread owns a
+// power of two of neighbouring runs, a warp's, a CTA's and a cluster's threads
+// neighbouring ranges, so every split adds up the same tree, and a permanent's
+// bits do not depend on how many matrices are launched with it.  (A row value
+// carried from unit to unit and one built anew differ by 2^-100: the bits agree
+// unless one lies that close to a rounding boundary.)  A thread's
+// own levels of the tree (five of them, one warp per matrix) cost little: 4096 x
+// n=16 293 -> 297 us against sums in each split's own order, n=17 568 -> 576 us,
+// n=20 4635 -> 4645 us, 148 x n=24 3205 -> 3236 us.
+constexpr int kLeaves = kMaxCluster * kWarpsPerCta * 32;
+
+template <int C>
+struct RunTree {
+    dd level[C][6];  // sums of 2^l runs, waiting for their neighbours
+    // Adds the thread's run number i, whose sum is tot; the sum of all runs so far
+    // is then in tot when i + 1 is a power of two, else tot is to start at zero.
+    __device__ __forceinline__ void add(unsigned i, bool last, dd (&tot)[C])
+    {
+        int l = 0;
+        for (; (i >> l) & 1u; ++l)
+#pragma unroll
+            for (int c = 0; c < C; ++c) tot[c] = dd_add(level[c][l], tot[c]);
+        if (last) return;
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            level[c][l] = tot[c];
+            tot[c] = {0.0, 0.0};
+        }
+    }
+};
+
+// Neighbouring lanes first (dd_add gives both of them the same bits).
+__device__ __forceinline__ dd warp_tree_dd(dd v)
+{
+#pragma unroll
+    for (int m = 1; m <= 16; m <<= 1) v = dd_add(v, shfl_xor_dd(v, m));
+    return v;
+}
+
+// The sum of count (a power of two) values, pairwise in order; v is overwritten.
+__device__ __forceinline__ dd tree_dd(dd* v, int count)
+{
+    for (int step = 1; step < count; step *= 2)
+        for (int i = 0; i + step < count; i += 2 * step) v[i] = dd_add(v[i], v[i + step]);
+    return v[0];
+}
+
 // One matrix, its rows' scaling exponents in s_exp: tables in the team's slice,
 // then the walk over part `part` of `parts` teams' units; the warp's total (in
 // every lane).  pivot: the derivative walk's column.
@@ -170,6 +221,8 @@ __device__ __forceinline__ void walk_matrix(const double* __restrict__ A, const 
                    &u1);
 #pragma unroll
     for (int c = 0; c < C; ++c) tot[c] = {0.0, 0.0};
+    constexpr unsigned long long UNITS = 1ull << NTP, RUN = UNITS > kLeaves ? UNITS / kLeaves : 1;
+    RunTree<C> tree;
     if (u0 < u1) {
         // unit base: hi words in registers; lo words in registers or in the
         // thread's shared slot (element (c, r) at [(c * N + r) * LS + rank])
@@ -204,6 +257,7 @@ __device__ __forceinline__ void walk_matrix(const double* __restrict__ A, const 
                 tot[0] = dd_add_d(tot[0], ur);
                 tot[C - 1] = dd_add_d(tot[C - 1], ui);
             }
+            if (N >= 16 && ((u + 1) & (RUN - 1)) == 0) tree.add((unsigned)((u - u0) / RUN), u + 1 >= u1, tot);
             if (++u >= u1) break;
             const int j = __ffsll((long long)u) - 1;
             const bool add = (gray_of(u) >> j) & 1ull;
@@ -225,7 +279,7 @@ __device__ __forceinline__ void walk_matrix(const double* __restrict__ A, const 
         }
     }
 #pragma unroll
-    for (int c = 0; c < C; ++c) tot[c] = warp_sum_dd(tot[c]);
+    for (int c = 0; c < C; ++c) tot[c] = warp_tree_dd(tot[c]);
 }
 
 // Matrix m of a batch starts at mats + m*N*N*C, or, with an offset table, at
@@ -236,9 +290,8 @@ __device__ __forceinline__ void walk_matrix(const double* __restrict__ A, const 
 // matrix from src into its place in mats, so every matrix crosses the host
 // link once, in coalesced reads that overlap the other warps' work.
 // SPLIT: a matrix is one CTA's, or shared by the CTAs of a cluster (part of the
-// units each, tables of its own); else one warp's.  A split matrix's total is
-// added up in the order of its warps, then its CTAs (through distributed shared
-// memory: no workspace, so the launch still allocates nothing).
+// units each, tables of its own); else one warp's.  A split matrix's CTAs meet in
+// distributed shared memory (no workspace, so the launch still allocates nothing).
 template <int N, int C, bool SPLIT>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) batch_walk(double* __restrict__ mats,
                                                                  const unsigned* __restrict__ offs,
@@ -317,17 +370,16 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) batch_walk(double* __restri
             started = true;
             if (threadIdx.x == 0)
 #pragma unroll
-                for (int c = 0; c < C; ++c) {
-                    dd v = s_part[c][0];
-                    for (int w = 1; w < kWarpsPerCta; ++w) v = dd_add(v, s_part[c][w]);
-                    *cluster.map_shared_rank(&s_cta[c][part], 0) = v;
-                }
+                for (int c = 0; c < C; ++c)
+                    *cluster.map_shared_rank(&s_cta[c][part], 0) = tree_dd(s_part[c], kWarpsPerCta);
             cluster.sync();
-            if (part == 0)
+            if (part == 0 && wid == 0)
 #pragma unroll
                 for (int c = 0; c < C; ++c) {
-                    tot[c] = s_cta[c][0];
-                    for (int b = 1; b < parts; ++b) tot[c] = dd_add(tot[c], s_cta[c][b]);
+                    dd v[kMaxCluster];
+#pragma unroll
+                    for (int b = 0; b < kMaxCluster; ++b) v[b] = b < parts ? s_cta[c][b] : dd{0.0, 0.0};
+                    tot[c] = tree_dd(v, kMaxCluster);  // (adding the zeros changes nothing)
                 }
         }
         if (part == 0 && (!SPLIT || wid == 0)) {
@@ -373,7 +425,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) batch_walk(double* __restri
 // warp per matrix hands them out four matrices at a time.  Every CTA builds
 // tables of its own: kTables of the walk at n=16, where the whole is 8 us of the
 // pipe, less in proportion at larger n.  Clusters of 4 and 8 leave some SMs of a
-// GPC over.  4096 matrices or more are a warp each; on one B200 (all with 32 terms
+// GPC over.  On one B200 (all with 32 terms
 // per unit) the choice takes 1024 x n=20 from 1448 us (a warp each) to 1248 us,
 // 700 x n=22 from 6324 to 3851 us, complex 24488 to 12531 us, 16 x n=16 from 33
 // to 27 us (one CTA each, four).  top: high column bits, 2^top units.

@@ -30,11 +30,11 @@
 //        may pick the row-compacted walk or the row-by-row expansion).
 //   poll / wait ─► result with admission and completion timestamps.
 //
-// A request's result depends only on its own matrix (and, in the order of its
-// double-double sum, on the size of its batch): the batch kernel gives each
-// matrix its own warp, CTA or cluster, tables and reduction (padding entries read
-// a zero matrix and are discarded), and the whole-GPU walk's result does not
-// depend on what else runs.
+// A request's result depends only on its own matrix and on whether it was batched
+// (mid-size ones): the batch kernel gives each matrix its own warp, CTA or cluster
+// and tables, and adds its sum up in one order whatever the batch's size (padding
+// entries read a zero matrix and are discarded), and the whole-GPU walk's result
+// does not depend on what else runs.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -1,6 +1,6 @@
-"""Batched small permanents (spb_perm_batch_dev, one warp per matrix) through
-the C ABI: each matrix of a batch against the exact oracle and against the
-single-matrix entry point."""
+"""Batched small permanents (spb_perm_batch_dev: a warp, a CTA or a cluster per
+matrix) through the C ABI: each matrix of a batch against the exact oracle and
+against the single-matrix entry point."""
 import ctypes
 
 import numpy as np
@@ -12,7 +12,7 @@ from superman_b200 import workloads as W
 pytestmark = pytest.mark.gpu
 
 
-def run_batch(mats, is_complex):
+def run_batch(mats, is_complex, low=False):
     import torch
     mats = np.ascontiguousarray(mats)
     count, n = mats.shape[0], mats.shape[1]
@@ -25,6 +25,8 @@ def run_batch(mats, is_complex):
                                              ctypes.c_void_p(d_out.data_ptr()), None))
     torch.cuda.synchronize()
     o = d_out.cpu().numpy().reshape(count, comps, 2)
+    if low:
+        return o
     if is_complex:
         return o[:, 0, 0] + 1j * o[:, 1, 0]
     return o[:, 0, 0]
@@ -80,6 +82,29 @@ def test_batch_rows_scaled_by_powers_of_two(spb, n, count):
     e = rng.integers(-30, 31, size=(count, n))
     got = run_batch(u * np.exp2(e)[:, :, None], False)
     assert np.array_equal(got, want * np.exp2(e.sum(axis=1)))
+
+
+@pytest.mark.parametrize("n,cplx,counts", [(16, False, (5, 60, 100, 2400)), (16, True, (5, 60, 100, 2400)),
+                                           (17, False, (9, 30, 60, 100, 600, 4096)),
+                                           (20, False, (9, 60, 200, 1024, 4096)), (21, True, (9, 60, 200, 1024)),
+                                           (23, False, (9, 60, 200, 592))])
+def test_batch_bits_do_not_depend_on_the_count(spb, n, cplx, counts):
+    """A matrix split over clusters of eight, four or two CTAs, on one CTA and on
+    one warp: the same bits, high word and low.  With a pivot column, without one
+    (a zero in every column) and signed."""
+    rng = np.random.default_rng(n)
+    u = W.haar_block(n, 70, N=64) if cplx else W.dense_uniform(n, 70)
+    z = u.copy()
+    z[rng.permutation(n), np.arange(n)] = 0.0
+    g = rng.standard_normal((n, n)) + (1j * rng.standard_normal((n, n)) if cplx else 0.0)
+    some = [u, z, g]
+    want = None
+    for count in counts:
+        o = run_batch(np.stack([some[k % 3] for k in range(count)]), cplx, low=True)
+        if want is None:
+            want = o[:3]
+            assert np.any(want[:, :, 1] != 0.0)
+        assert np.array_equal(o, want[np.arange(count) % 3])
 
 
 def test_batch_empty_and_invalid(spb):

@@ -216,8 +216,7 @@ def test_batch_mixes_both_walks(spb, oracle, n, cplx):
 @pytest.mark.parametrize("n,cplx", [(16, False), (19, False), (21, True), (24, False), (24, True)])
 def test_batch_split_is_the_same_as_alone(spb, n, cplx):
     """A launch of few matrices splits each over a cluster, a launch of many
-    gives each a warp: the same units, so the same values to the
-    double-double sum's order."""
+    gives each a warp: the same values."""
     import torch
     few, many = 2, 600 if n <= 21 else 470
     u = [W.haar_block(n, 40 + k, N=64) if cplx else W.dense_uniform(n, 40 + k) for k in range(few)]
@@ -238,9 +237,8 @@ def test_batch_split_is_the_same_as_alone(spb, n, cplx):
 @pytest.mark.parametrize("n,cplx", [(16, False), (16, True), (17, False), (18, True)])
 def test_batch_counts_around_the_split(spb, n, cplx):
     """Launches of 1 to 2400 matrices, i.e. clusters of eight, four and two CTAs,
-    a CTA each (with more CTAs than SMs, too) and a warp each: the same units, so
-    the same values to the double-double sum's order; a matrix of zeros, which
-    takes no walk, gives 0 in each."""
+    a CTA each (with more CTAs than SMs, too) and a warp each: the same values; a
+    matrix of zeros, which takes no walk, gives 0 in each."""
     import torch
     few = 3
     u = [W.haar_block(n, 60 + k, N=64) if cplx else W.dense_uniform(n, 60 + k) for k in range(few)]

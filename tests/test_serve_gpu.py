@@ -83,7 +83,7 @@ def test_same_matrix_alone_and_in_batch(spb):
         r_mix = srv.wait(t_mix)
         for t in others + more:
             srv.wait(t)
-    assert r_mix["permanent"] == r_alone["permanent"]  # bit-identical: own warp, own reduction
+    assert r_mix["permanent"] == r_alone["permanent"]  # bit-identical: one order of its sum
 
 
 def test_admission_refuses_beyond_budget(spb):
