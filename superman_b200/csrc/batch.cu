@@ -114,8 +114,8 @@ struct Team {
 // carried from unit to unit and one built anew differ by 2^-100: the bits agree
 // unless one lies that close to a rounding boundary.)  A thread's
 // own levels of the tree (five of them, one warp per matrix) cost little: 4096 x
-// n=16 293 -> 297 us against sums in each split's own order, n=17 568 -> 576 us,
-// n=20 4635 -> 4645 us, 148 x n=24 3205 -> 3236 us.
+// n=16 292 -> 297 us against sums in each split's own order, n=17 567 -> 574 us,
+// n=20 4532 -> 4548 us, 148 x n=24 3213 -> 3228 us.
 constexpr int kLeaves = kMaxCluster * kWarpsPerCta * 32;
 
 template <int C>

@@ -345,13 +345,49 @@ int choose_unit_bits(int n, int comps, const spb_options* opt, int bits, size_t 
 
 int choose_unit_bits(int n, int comps, const spb_options* opt) { return choose_unit_bits(n, comps, opt, n - 1, sizeof(double)); }
 
+size_t walk_smem_bytes(const Problem& pb, int threads);
+
+// The walk's threads per CTA: `wanted` of them, or, with 0, as many as their
+// per-thread lo vectors leave room for next to the tables (64 at the least).
+int walk_threads(const Problem& pb, int wanted, int most, size_t limit)
+{
+    auto smem_for = [&](int th) { return pb.f32 ? walk_f32_smem_bytes(pb, th) : walk_smem_bytes(pb, th); };
+    int threads = wanted > 0 ? wanted : most;
+    while (wanted <= 0 && threads > 64 && smem_for(threads) > limit) threads -= 32;
+    if (threads > most) threads = most;
+    threads = (threads / 32) * 32;
+    return threads < 32 ? 32 : threads;
+}
+
+void choose_width(Problem* pb, const spb_options* opt, int sms);
+
 // Whether the derivative walk may run, and the unit width to go with it: on
 // dense matrices of its sizes, where the units leave it a column to expand, and
 // not with FP32 products (n=27 complex 592 -> 541 us, but the error of a Haar
 // block against exact went from 2.6e-6 to 6.2e-6).  The setup kernel decides by
-// the matrix (rb->pivot); `hint` false (a host matrix known to have a zero in
-// every column) only sizes the units for the plain walk, which then runs.
-//
+// the matrix (rb->pivot); `hint` false: a host matrix known to have a zero in
+// every column, which takes the plain walk.  So do calls whose own launch shape
+// leaves no room beside the tables for the derivative walk's low words, or only
+// for fewer threads than the plain walk has: a matrix without a pivot would pay
+// for words that it does not use.
+void choose_walk(Problem* pb, const spb_options* opt, bool hint, int sms, size_t limit)
+{
+    const int n = pb->n;
+    pb->g = group_size(n, pb->comps);
+    pb->deriv = hint && pb->na == n && !pb->f32 && n >= (pb->comps == 1 ? kMinDerivReal : kMinDerivComplex) ? 1 : 0;
+    choose_width(pb, opt, sms);
+    if (!pb->deriv) return;
+    Problem plain = *pb;
+    plain.deriv = 0;
+    choose_width(&plain, opt, sms);
+    const int most = walk_max_threads(n, pb->comps);
+    const int td = walk_threads(*pb, opt->threads_per_block, most, limit);
+    if (pb->w > n - 2 || td < walk_threads(plain, opt->threads_per_block, most, limit) ||
+        walk_smem_bytes(*pb, td) > limit ||
+        (pb->mode != 0 && refine_smem_bytes(*pb, 256) + 2048 > limit))
+        *pb = plain;
+}
+
 // The whole-GPU walks give every thread whole units, so a few units per thread
 // leave some threads waiting for others with one more (n=28: 2^18 units of 2^8
 // terms, 3.46 per thread, four rounds).  The width is narrowed by up to two bits
@@ -359,14 +395,12 @@ int choose_unit_bits(int n, int comps, const spb_options* opt) { return choose_u
 // about 6 terms each, 15 of the FP32 walk's (fitted to widths 5 to 8; wall times
 // with the wider and the taken width: real n=28 493 -> 450 us, complex n=26
 // 396 -> 369 us, with double-double 583 -> 414 us).
-void choose_walk(Problem* pb, const spb_options* opt, bool hint, int sms)
+void choose_width(Problem* pb, const spb_options* opt, int sms)
 {
     const double unit_terms = pb->f32 ? 15.0 : 6.0;
     const int n = pb->n;
-    pb->deriv = pb->na == n && !pb->f32 && n >= (pb->comps == 1 ? kMinDerivReal : kMinDerivComplex) ? 1 : 0;
-    const int bits = n - 1 - (pb->deriv && hint ? 1 : 0);
+    const int bits = n - 1 - (pb->deriv ? 1 : 0);
     pb->w = choose_unit_bits(n, pb->comps, opt, bits, pb->f32 ? sizeof(float) : sizeof(double));
-    if (pb->w > n - 2) pb->deriv = 0;
     const double threads =
         (double)sms * (pb->f32 ? walk_f32_max_threads(n, pb->comps) : walk_max_threads(n, pb->comps));
     if (opt->unit_bits > 0 || std::ldexp(1.0, bits - pb->w) < threads) return;
@@ -454,9 +488,9 @@ size_t walk_smem_bytes(const Problem& pb, int threads)
     if (pb.na < n) return sparse_smem_bytes(n, pb.na, pb.w, threads);
     size_t terms = (size_t)1 << pb.w;
     // high columns: n-1-w, or with the derivative walk n-2-w with their low
-    // words; the call must fit whichever walk the matrix gets
+    // words; the call must fit whichever walk the matrix gets (choose_walk)
     int ntop = n - 1 - pb.w;
-    if (pb.deriv && 2 * (ntop - 1) > ntop) ntop = 2 * (ntop - 1);
+    if (pb.deriv && !deriv_low_far(n, c) && 2 * (ntop - 1) > ntop) ntop = 2 * (ntop - 1);
     return sizeof(double) * (terms * n * c + (size_t)(ntop > 0 ? ntop : 0) * n * c +
                              (size_t)n * c * threads) +
            kHistSmemBytes + bound_smem_bytes(n);
@@ -508,7 +542,9 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
             }
         }
     }
-    choose_walk(&pb, &opt, hint, ctx->sm_count);
+    const bool dd_mode = opt.precision == SPB_PREC_DD;
+    pb.mode = dd_mode ? 1 : 0;
+    choose_walk(&pb, &opt, hint, ctx->sm_count, ctx->smem_optin);
     if (plan && plan->na < n) {
         if (comps != 1 || plan->na < 1 || plan->na > kMaxActive || plan->w < 2 || plan->w > n - 2) {
             spb_set_error("row-compacted walk: bad plan (n=%d, active rows %d, w=%d)", n, plan->na, plan->w);
@@ -518,22 +554,13 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
         pb.w = plan->w;
         pb.deriv = 0;
     }
-    pb.g = group_size(n, comps);
     pb.units = 1ull << (n - 1 - pb.w);
     // the units the launch is shaped for: half of them in the derivative walk
-    const unsigned long long units = pb.deriv && hint ? pb.units >> 1 : pb.units;
+    const unsigned long long units = pb.deriv ? pb.units >> 1 : pb.units;
 
     auto smem_for = [&](int th) { return pb.f32 ? walk_f32_smem_bytes(pb, th) : walk_smem_bytes(pb, th); };
-    int threads = opt.threads_per_block > 0 ? opt.threads_per_block : 0;
     const int max_threads = pb.f32 ? walk_f32_max_threads(n, comps) : (pb.na < n ? 512 : walk_max_threads(n, comps));
-    if (threads == 0) {
-        threads = max_threads;
-        // fit the per-thread lo vectors next to the tables
-        while (threads > 64 && smem_for(threads) > ctx->smem_optin) threads -= 32;
-    }
-    if (threads > max_threads) threads = max_threads;
-    threads = (threads / 32) * 32;
-    if (threads < 32) threads = 32;
+    int threads = walk_threads(pb, opt.threads_per_block, max_threads, ctx->smem_optin);
     size_t smem = smem_for(threads);
     if (smem > ctx->smem_optin) {
         spb_set_error("dense n=%d: %zu B shared memory exceeds the %zu B limit", n, smem, ctx->smem_optin);
@@ -563,8 +590,6 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
     if (blocks < 1) blocks = 1;
     pb.grid = blocks;
     pb.threads = threads;
-    const bool dd_mode = opt.precision == SPB_PREC_DD;
-    pb.mode = dd_mode ? 1 : 0;
     if (dd_mode && pb.na == n) {
         // the refinement stages both table words of every part (256 threads
         // at the least): refuse before any launch when they cannot fit

@@ -124,6 +124,14 @@ constexpr int kListNone = 0x7f7f7f7f;  // a list bin above every bin
 // instructions, with the same or a smaller rounding error.  The quotients are
 // kept in double-double wherever the plain walk holds exact entries (start
 // vector, subset sums, high columns).
+// Where the high columns' low words lie during the walk: beside the columns in
+// shared memory, or, at sizes whose tables and per-thread words leave no room
+// there without taking threads from the CTA, in global memory.  They are read
+// once per unit of 64 or 128 terms, mostly the same column by all threads.  One
+// B200: real n=40 2292 ms with the words in shared memory and 480 threads, 2198 ms
+// here with 512 (plain walk 3014 ms); complex n=37 994 ms with 224 threads, 804 ms
+// with 256 (1045 ms).
+__host__ __device__ constexpr bool deriv_low_far(int n, int comps) { return n >= (comps == 1 ? 40 : 37); }
 // Whether the derivative walk runs; the same for every thread of a call.
 __device__ __forceinline__ bool deriv_on(const Problem& pb) { return pb.deriv != 0 && pb.rb->pivot >= 0; }
 __device__ __forceinline__ int eff_ntop(const Problem& pb, bool deriv) { return pb.n - 1 - pb.w - (deriv ? 1 : 0); }
@@ -678,8 +686,10 @@ __device__ __forceinline__ void walk_real_body(const Problem& pb)
     const int tid = threadIdx.x, bd = blockDim.x;
     double* s_de = smem;
     double* s_mt = s_de + terms * N;
-    double* s_ml = s_mt + (ntop > 0 ? ntop : 0) * N;  // derivative walk: the high columns' low words
-    double* s_lo = s_ml + (D && ntop > 0 ? ntop : 0) * N;
+    constexpr bool kFar = deriv_low_far(N, 1);
+    const int ntp = ntop > 0 ? ntop : 0;
+    double* s_ml = kFar ? pb.mt_lo : s_mt + ntp * N;  // derivative walk: the high columns' low words
+    double* s_lo = s_mt + (D && !kFar ? 2 : 1) * ntp * N;
     float* s_hist = reinterpret_cast<float*>(s_lo + N * bd);  // mode 1
     unsigned* s_cnt = reinterpret_cast<unsigned*>(s_hist + kHistBins);
     // DE range per row, [2][N] (min, max).  Two scalar loads per row: a paired
@@ -688,7 +698,7 @@ __device__ __forceinline__ void walk_real_body(const Problem& pb)
     for (int i = tid; i < terms * N; i += bd) s_de[i] = pb.de_hi[i];
     for (int i = tid; i < ntop * N; i += bd) {
         s_mt[i] = pb.mt[i];
-        if (D) s_ml[i] = pb.mt_lo[i];
+        if (D && !kFar) s_ml[i] = pb.mt_lo[i];
     }
     const int mode = pb.mode;
     if (mode != 0)
@@ -942,15 +952,16 @@ __device__ __forceinline__ void walk_complex_body(const Problem& pb)
     const int tid = threadIdx.x, bd = blockDim.x;
     double* s_de = smem;                        // [2][terms*N]
     double* s_mt = s_de + 2 * terms * N;        // [2][ntop*N]
-    double* s_ml = s_mt + 2 * ntp * N;          // [2][ntop*N] low words (derivative walk)
-    double* s_lo = s_ml + (D ? 2 * ntp * N : 0);  // [2][N][bd]
+    constexpr bool kFar = deriv_low_far(N, 2);
+    double* s_ml = kFar ? pb.mt_lo : s_mt + 2 * ntp * N;  // [2][ntop*N] low words (derivative walk)
+    double* s_lo = s_mt + (D && !kFar ? 4 : 2) * ntp * N;  // [2][N][bd]
     float* s_hist = reinterpret_cast<float*>(s_lo + 2 * N * bd);  // mode 1
     unsigned* s_cnt = reinterpret_cast<unsigned*>(s_hist + kHistBins);
     double* s_bnd = reinterpret_cast<double*>(s_cnt + kHistBins);  // [N]
     for (int i = tid; i < 2 * terms * N; i += bd) s_de[i] = pb.de_hi[i];
     for (int i = tid; i < 2 * ntp * N; i += bd) {
         s_mt[i] = pb.mt[i];
-        if (D) s_ml[i] = pb.mt_lo[i];
+        if (D && !kFar) s_ml[i] = pb.mt_lo[i];
     }
     const int mode = pb.mode;
     if (mode != 0)

@@ -462,13 +462,14 @@ __global__ void __launch_bounds__(512, 1) refine_real(Problem pb)
     double* s_x = s_dl + terms * n;      // [nwarps][2n]
     double* s_g = s_x + nwarps * 2 * n;  // [nwarps][nq]
     double* s_mt = s_g + nwarps * nq;    // [ntp][n]
-    double* s_ml = s_mt + ntp * n;       // [ntp][n] low words, derivative walk only
+    // [ntp][n] low words, derivative walk only
+    double* s_ml = deriv_low_far(n, 1) ? pb.mt_lo : s_mt + ntp * n;
     // CTAs without a unit skip the tables (they still join the grid reduction)
     if ((unsigned long long)blockIdx.x < count) {
         stage_rows(s_dh, pb.de_hi, 1, n, terms, G);  // [n][terms]
         stage_rows(s_dl, pb.de_lo, 1, n, terms, G);
         stage(s_mt, pb.mt, ntp * n);
-        if (deriv) stage(s_ml, pb.mt_lo, ntp * n);
+        if (deriv && !deriv_low_far(n, 1)) stage(s_ml, pb.mt_lo, ntp * n);
     }
     __syncthreads();
     double* xw = s_x + wid * 2 * n;
@@ -600,13 +601,14 @@ __global__ void __launch_bounds__(512, 1) refine_complex(Problem pb)
     double* s_x = s_dl + 2 * terms * n;   // [nwarps][4n]
     double* s_g = s_x + nwarps * 4 * n;   // [nwarps][2*np]
     double* s_mt = s_g + nwarps * 2 * np; // [2][ntp][n]
-    double* s_ml = s_mt + 2 * ntp * n;    // [2][ntp][n] low words, derivative walk only
+    // [2][ntp][n] low words, derivative walk only
+    double* s_ml = deriv_low_far(n, 2) ? pb.mt_lo : s_mt + 2 * ntp * n;
     // CTAs without a unit skip the tables (they still join the grid reduction)
     if ((unsigned long long)blockIdx.x < count) {
         stage_rows(s_dh, pb.de_hi, 2, n, terms, G);  // [2][n][terms]
         stage_rows(s_dl, pb.de_lo, 2, n, terms, G);
         stage(s_mt, pb.mt, 2 * ntp * n);
-        if (deriv) stage(s_ml, pb.mt_lo, 2 * ntp * n);
+        if (deriv && !deriv_low_far(n, 2)) stage(s_ml, pb.mt_lo, 2 * ntp * n);
     }
     __syncthreads();
     const double* drh = s_dh;
@@ -756,7 +758,7 @@ size_t refine_smem_bytes(const Problem& pb, int threads)
     const size_t nwarps = threads / 32;
     // (whichever walk the matrix gets: see walk_smem_bytes)
     size_t ntp = pb.n - 1 - pb.w > 0 ? pb.n - 1 - pb.w : 0;
-    if (pb.deriv && ntp > 2) ntp = 2 * (ntp - 1);
+    if (pb.deriv && !deriv_low_far(pb.n, pb.comps) && ntp > 2) ntp = 2 * (ntp - 1);
     return sizeof(double) * (2 * c * terms * n + nwarps * (2 * c * n + c * nq) + c * ntp * n);
 }
 

@@ -49,8 +49,8 @@ namespace dense {
 // Defined in dense.cu.
 __global__ void setup_kernel(Problem pb, const double* __restrict__ a_in, int smem_tables);
 int launch_setup(const Problem& pb, const double* d_a, cudaStream_t s);
-int group_size(int n, int comps);
-void choose_walk(Problem* pb, const spb_options* opt, bool hint, int sms);
+void choose_walk(Problem* pb, const spb_options* opt, bool hint, int sms, size_t limit);
+int walk_threads(const Problem& pb, int wanted, int most, size_t limit);
 size_t plan_layout(Problem* pb, char* base, size_t* in_offset);
 size_t walk_smem_bytes(const Problem& pb, int threads);
 int prepare_setup(int* limit);
@@ -150,12 +150,9 @@ extern "C" int spb_perm_dense_f64_noalloc(const double* d_a, int n, double* d_ou
     pb.n = n;
     pb.na = n;
     pb.comps = 1;
-    choose_walk(&pb, &opt, true, sms);
-    pb.g = group_size(n, 1);
+    choose_walk(&pb, &opt, true, sms, smem_budget);
     pb.units = 1ull << (n - 1 - pb.w);
-    int threads = walk_max_threads(n, 1);
-    while (threads > 64 && walk_smem_bytes(pb, threads) > smem_budget) threads -= 32;
-    threads = (threads / 32) * 32;
+    const int threads = walk_threads(pb, 0, walk_max_threads(n, 1), smem_budget);
     const size_t smem = walk_smem_bytes(pb, threads);
     if (smem > smem_budget) {
         spb_set_error("spb_perm_dense_f64_noalloc: n=%d needs %zu B shared memory", n, smem);

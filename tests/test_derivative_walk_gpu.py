@@ -263,6 +263,21 @@ def test_batch_counts_around_the_split(spb, n, cplx):
             assert np.all(np.abs(a - o[k, :, 0]) <= 2.0 ** -52 * np.abs(a)), (count, k)
 
 
+def test_launch_shapes_that_only_the_plain_walk_fits(spb):
+    """Shapes whose shared memory holds the plain walk but not the derivative
+    walk's low words beside it: accepted, on the plain walk (real n=24 with 2^10
+    terms at 128 threads 228160 B against 230272 B of 228352; complex n=24 with 2^8
+    terms, whose refinement takes 218752 B against 229888 B)."""
+    a = W.dense_uniform(24, 12)
+    want = spb.perm_dense(a).permanent
+    r = spb.perm_dense(a, unit_bits=10, threads_per_block=128, small_call=-1)
+    assert abs(r.permanent - want) <= 1e-12 * abs(want)
+    c = W.haar_block(24, 13, N=64)
+    want = spb.perm_complex(c, precision="dd").permanent
+    r = spb.perm_complex(c, precision="dd", unit_bits=8)
+    assert abs(r.permanent - want) <= 1e-12 * abs(want)
+
+
 def test_noalloc_without_a_pivot(spb):
     import torch
     a = no_pivot(W.dense_uniform(24, 3), 4)
