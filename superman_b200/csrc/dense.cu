@@ -323,9 +323,8 @@ int group_size(int n, int comps)
     return ComplexGroup(n);
 }
 
-// bits: walked columns less one, n-1 or, for the derivative walk, n-2; entry:
-// bytes of a table entry in the walk's shared memory, 8 or (FP32 products) 4.
-int choose_unit_bits(int n, int comps, const spb_options* opt, int bits, size_t entry)
+// bits: walked columns less one, n-1 or, for the derivative walk, n-2.
+int choose_unit_bits(int n, int comps, const spb_options* opt, int bits)
 {
     int w;
     if (opt && opt->unit_bits > 0) {
@@ -333,7 +332,7 @@ int choose_unit_bits(int n, int comps, const spb_options* opt, int bits, size_t 
     } else {
         // Table budget 64 KB per part; keep >= 2^16 units when n allows.
         w = 8;
-        while (w > 2 && ((size_t)1 << w) * n * entry * comps > (size_t)64 * 1024) --w;
+        while (w > 2 && ((size_t)1 << w) * n * 8 * comps > (size_t)64 * 1024) --w;
         while (w > 2 && bits - w < 16) --w;
     }
     if (w > n - 1) w = n - 1;
@@ -343,7 +342,7 @@ int choose_unit_bits(int n, int comps, const spb_options* opt, int bits, size_t 
     return w;
 }
 
-int choose_unit_bits(int n, int comps, const spb_options* opt) { return choose_unit_bits(n, comps, opt, n - 1, sizeof(double)); }
+int choose_unit_bits(int n, int comps, const spb_options* opt) { return choose_unit_bits(n, comps, opt, n - 1); }
 
 size_t walk_smem_bytes(const Problem& pb, int threads);
 
@@ -392,23 +391,24 @@ void choose_walk(Problem* pb, const spb_options* opt, bool hint, int sms, size_t
 // leave some threads waiting for others with one more (n=28: 2^18 units of 2^8
 // terms, 3.46 per thread, four rounds).  The width is narrowed by up to two bits
 // where the evener split outweighs the base updates of more units, which cost
-// about 6 terms each, 15 of the FP32 walk's (fitted to widths 5 to 8; wall times
-// with the wider and the taken width: real n=28 493 -> 450 us, complex n=26
-// 396 -> 369 us, with double-double 583 -> 414 us).
+// about 6 terms each (fitted to widths 5 to 8; wall times with the wider and the
+// taken width: real n=28 493 -> 450 us, complex n=26 396 -> 369 us, with
+// double-double 583 -> 414 us).  FP32 products keep the width of their double
+// table: with twice the terms, which a float table has room for, complex n=27
+// takes 545 us for 569, but the error over 96 Haar blocks grows from 2.0e-5 to
+// 2.5e-5 (root mean square).
 void choose_width(Problem* pb, const spb_options* opt, int sms)
 {
-    const double unit_terms = pb->f32 ? 15.0 : 6.0;
     const int n = pb->n;
     const int bits = n - 1 - (pb->deriv ? 1 : 0);
-    pb->w = choose_unit_bits(n, pb->comps, opt, bits, pb->f32 ? sizeof(float) : sizeof(double));
-    const double threads =
-        (double)sms * (pb->f32 ? walk_f32_max_threads(n, pb->comps) : walk_max_threads(n, pb->comps));
-    if (opt->unit_bits > 0 || std::ldexp(1.0, bits - pb->w) < threads) return;
+    pb->w = choose_unit_bits(n, pb->comps, opt, bits);
+    const double threads = (double)sms * walk_max_threads(n, pb->comps);
+    if (pb->f32 || opt->unit_bits > 0 || std::ldexp(1.0, bits - pb->w) < threads) return;
     double best = 0.0;
     const int w0 = pb->w;
     for (int w = w0; w >= w0 - 2 && w >= 4; --w) {
         const double per = std::ldexp(1.0, bits - w) / threads, terms = std::ldexp(1.0, w);
-        const double eff = per / std::ceil(per) * terms / (terms + unit_terms);
+        const double eff = per / std::ceil(per) * terms / (terms + 6.0);
         if (eff > best * 1.02) {
             best = eff;
             pb->w = w;

@@ -73,3 +73,13 @@ def test_f32_refused_beyond_the_bound(spb):
     with pytest.raises(spb.SupermanError) as e:
         spb.perm_dense(W.dense_uniform(16, 2), precision="fp32")
     assert e.value.status == _lib.SPB_ERR_ACCURACY
+
+
+@pytest.mark.parametrize("n,cplx,bits", [(27, True, 7), (25, True, 7), (26, True, 7), (28, False, 8)])
+def test_f32_unit_width_is_the_double_tables(spb, n, cplx, bits):
+    """The terms of a unit share one FP32 rounding of its base, so the width
+    belongs to the accuracy: the default is what 64 KB of doubles hold."""
+    a = W.haar_block(n, 2, N=64) if cplx else W.dense_uniform(n, 2)
+    f = spb.perm_complex if cplx else spb.perm_dense
+    r, s = f(a, precision="fp32", rel_tol=1.0), f(a, precision="fp32", rel_tol=1.0, unit_bits=bits)
+    assert (r.permanent, r.permanent_lo) == (s.permanent, s.permanent_lo)
