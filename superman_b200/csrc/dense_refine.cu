@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(512, 1) refine_real(Problem pb)
 {
     const unsigned long long count = refine_count(pb);
     if (count == 0) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) publish(pb, pb.rb_host);
+        if (blockIdx.x == 0 && threadIdx.x < 32) publish(pb, pb.rb_host);
         return;
     }
     extern __shared__ __align__(16) double sm[];
@@ -583,7 +583,7 @@ __global__ void __launch_bounds__(512, 1) refine_complex(Problem pb)
 {
     const unsigned long long count = refine_count(pb);
     if (count == 0) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) publish(pb, pb.rb_host);
+        if (blockIdx.x == 0 && threadIdx.x < 32) publish(pb, pb.rb_host);
         return;
     }
     extern __shared__ __align__(16) double sm[];

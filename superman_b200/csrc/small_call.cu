@@ -184,9 +184,11 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
             if (mx > 0.0 && isfinite(mx)) frexp(mx, &e);
             s_exp[r] = e;
         }
-        const int e = __shfl_sync(0xffffffffu, lane == 0 ? s_exp[r] : 0, 0);
-        if (lane < N) s_a[r * N + lane] = ldexp(s_a[r * N + lane], -e);
     }
+    __syncthreads();
+    // (all threads at once: a warp scaling its own rows waits for one frexp
+    // after the other)
+    for (int i = tid; i < N * N; i += bd) s_a[i] = ldexp(s_a[i], -s_exp[i / N]);
     __syncthreads();
     // the pivot column, picked alike in every CTA
     int pivot = -1;
@@ -225,7 +227,8 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
         }
         __syncthreads();
     }
-    auto plus = [&](dd x, int i) { return deriv ? dd_step(x, s_a[i], s_al[i]) : dd_add_d(x, s_a[i]); };
+    auto low = [&](int i) { return deriv ? s_al[i] : 0.0; };
+    auto plus = [&](dd x, double h, double l) { return deriv ? dd_step(x, h, l) : dd_add_d(x, h); };
     // The NW start vector x0 (one row per lane of the CTA's last warp, n
     // dependent adds each) and the subset-sum table (the other warps, a row
     // each at a time) are built side by side.  A row's table is built level
@@ -238,9 +241,9 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
     if (wid == xwarp && lane < N) {
         const int r = lane;
         dd s = {0.0, 0.0};
-        for (int j = 0; j < nc; ++j) s = plus(s, r * N + j);
+        for (int j = 0; j < nc; ++j) s = plus(s, s_a[r * N + j], low(r * N + j));
         dd h = {-0.5 * s.hi, -0.5 * s.lo};  // exact halving
-        dd x = plus(h, r * N + nc - 1);
+        dd x = plus(h, s_a[r * N + nc - 1], low(r * N + nc - 1));
         s_x0h[r] = x.hi;
         s_x0l[r] = x.lo;
     }
@@ -266,10 +269,13 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
             for (int k = 0; k < w; ++k) {
                 __syncwarp();
                 const int half = 1 << k;
+                // (read once per level: the table's stores may alias them)
+                const double a0 = s_a[r0 * N + k], m0 = low(r0 * N + k);
+                const double a1 = two ? s_a[r1 * N + k] : 0.0, m1 = two ? low(r1 * N + k) : 0.0;
                 for (int e = lane; e < half; e += 32) {
-                    const dd v0 = plus(dd{s_dh[pos(e, r0)], s_dl[pos(e, r0)]}, r0 * N + k);
+                    const dd v0 = plus(dd{s_dh[pos(e, r0)], s_dl[pos(e, r0)]}, a0, m0);
                     if (two) {
-                        const dd v1 = plus(dd{s_dh[pos(e, r1)], s_dl[pos(e, r1)]}, r1 * N + k);
+                        const dd v1 = plus(dd{s_dh[pos(e, r1)], s_dl[pos(e, r1)]}, a1, m1);
                         s_dh[pos(half + e, r1)] = v1.hi;
                         s_dl[pos(half + e, r1)] = v1.lo;
                     }
@@ -427,14 +433,16 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
         }
     }
     __syncthreads();
-    if (blockIdx.x == 0 && tid == 0) {
-        pb.rb->res[0] = s_total;
-        pb.rb->corr[0] = dd{0.0, 0.0};
-        if (mode != 0) {
-            pb.rb->thr = s_thr;
-            pb.rb->count = s_count;
-            pb.rb->err = s_err;
-            pb.rb->from_list = 1;
+    if (blockIdx.x == 0 && wid == 0) {
+        if (lane == 0) {
+            pb.rb->res[0] = s_total;
+            pb.rb->corr[0] = dd{0.0, 0.0};
+            if (mode != 0) {
+                pb.rb->thr = s_thr;
+                pb.rb->count = s_count;
+                pb.rb->err = s_err;
+                pb.rb->from_list = 1;
+            }
         }
         if (mode == 0 || s_thr >= kHistBins) publish(pb, rb_host);
     }
@@ -490,8 +498,8 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
                 else p = dd_mul(p, y);
             }
             for (int off = 1; off < per; off <<= 1) {
-                const dd po = shfl_xor_dd(p, off), qo = shfl_xor_dd(q, off);
-                if (deriv) q = dd_add(dd_mul(q, po), dd_mul(p, qo));
+                const dd po = shfl_xor_dd(p, off);
+                if (deriv) q = dd_add(dd_mul(q, po), dd_mul(p, shfl_xor_dd(q, off)));
                 p = dd_mul(p, po);
             }
             if (deriv) p = q;
@@ -520,8 +528,8 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
         if (lane == 0) {
             pb.rb->corr[0] = v;
             *pb.ticket = 0u;
-            publish(pb, rb_host);
         }
+        publish(pb, rb_host);
     }
 }
 
