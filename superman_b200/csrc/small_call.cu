@@ -152,6 +152,11 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
     // before the walk at all (it adds to nothing global).
     const bool direct = a_stage != nullptr && gridDim.x * (N * N * 8) <= 64 * 1024;
     const bool staged = a_stage != nullptr && !direct;  // the same in every CTA
+    // The double-double mode's barrier, where the staging has none: behind the
+    // tables, which hide the fetching of the matrix (1 us of 30 at n=13), but before them at the derivative walk's sizes.  There a
+    // barrier right in front of the walk made two calls of three take its slow
+    // pace (a matrix on the device, n=24 67 or 76 us, n=26 149 or 180 us).
+    constexpr bool kEarly = N >= kMinDerivReal;
     if (blockIdx.x == 0) {
         if (tid < 4) pb.ticket[tid] = 0u;
         if (mode != 0)
@@ -167,6 +172,7 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
         grid.sync();
         for (int i = tid; i < N * N; i += bd) s_a[i] = __ldcg(a_in + i);
     } else {
+        if (kEarly && mode != 0) grid.sync();
         const double* a = direct ? a_stage : a_in;
         for (int i = tid; i < N * N; i += bd) s_a[i] = a[i];
     }
@@ -301,7 +307,8 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
         if (deriv) s_ml[idx] = s_al[r * N + (w + j)];
     }
     __syncthreads();
-    if (!staged && mode != 0) grid.sync();  // the zeroed accumulators are visible before anyone adds to them
+    // the zeroed accumulators are visible before anyone adds to them
+    if (!kEarly && !staged && mode != 0) grid.sync();
 
     // ---- 1. the walk, one unit per thread and pass, evaluated as walk_real
     // evaluates it.  In each pass the warp builds its 32 unit bases
