@@ -393,7 +393,9 @@ void choose_walk(Problem* pb, const spb_options* opt, bool hint, int sms, size_t
 // where the evener split outweighs the base updates of more units, which cost
 // about 6 terms each (fitted to widths 5 to 8; wall times with the wider and the
 // taken width: real n=28 493 -> 450 us, complex n=26 396 -> 369 us, with
-// double-double 583 -> 414 us).  FP32 products keep the width of their double
+// double-double 583 -> 414 us).  Not at the fused call's sizes, where units are
+// dealt out in passes and each pass builds bases anew (real n=26 without a pivot,
+// double-double, 213 us with 2^6 terms, 187 us with 2^8).  FP32 products keep the width of their double
 // table: with twice the terms, which a float table has room for, complex n=27
 // takes 545 us for 569, but the error over 96 Haar blocks grows from 2.0e-5 to
 // 2.5e-5 (root mean square).
@@ -403,7 +405,7 @@ void choose_width(Problem* pb, const spb_options* opt, int sms)
     const int bits = n - 1 - (pb->deriv ? 1 : 0);
     pb->w = choose_unit_bits(n, pb->comps, opt, bits);
     const double threads = (double)sms * walk_max_threads(n, pb->comps);
-    if (pb->f32 || opt->unit_bits > 0 || std::ldexp(1.0, bits - pb->w) < threads) return;
+    if (pb->f32 || (pb->comps == 1 && n <= kSmallCallMaxN) || opt->unit_bits > 0 || std::ldexp(1.0, bits - pb->w) < threads) return;
     double best = 0.0;
     const int w0 = pb->w;
     for (int w = w0; w >= w0 - 2 && w >= 4; --w) {

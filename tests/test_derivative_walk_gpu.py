@@ -278,6 +278,14 @@ def test_launch_shapes_that_only_the_plain_walk_fits(spb):
     assert abs(r.permanent - want) <= 1e-12 * abs(want)
 
 
+def test_fused_call_keeps_its_unit_width(spb):
+    """n = 26 without a pivot: 2^8 terms a unit, the fused call's 2^17 units in two
+    passes (narrower units would take more, each with bases of its own)."""
+    a = no_pivot(W.dense_uniform(26, 2), 2)
+    r, s = (spb.perm_dense(a, precision="dd", sparse_walk=1, unit_bits=b) for b in (0, 8))
+    assert (r.permanent, r.permanent_lo, r.refined_units) == (s.permanent, s.permanent_lo, s.refined_units)
+
+
 def test_noalloc_without_a_pivot(spb):
     import torch
     a = no_pivot(W.dense_uniform(24, 3), 4)
