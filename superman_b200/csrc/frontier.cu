@@ -227,11 +227,13 @@ __global__ void __launch_bounds__(kThreads, 1) expand_rows(const __grid_constant
 // Fitted on one B200 to kernel times of 15 us (n=20, 10 narrow steps a half), 20 us
 // (n=30, 15), 38 us (n=20, 10 and 3 wide), 59 us (n=34, 9 and 10), 109 us (n=30, 11
 // wide, 4.4 million states) and 205 us (n=34, 13 wide, 10.5 million).
+constexpr double kLaunch = 7e-6, kState = 13e-12;
 double expansion_seconds(const Plan& p)
 {
     const int wide = std::max(p.nf - p.hf, p.nb - p.hb);
-    return 7e-6 + 0.9e-6 * std::max(p.hf, p.hb) + 4e-6 * wide + 13e-12 * p.states;
+    return kLaunch + 0.9e-6 * std::max(p.hf, p.hb) + 4e-6 * wide + kState * p.states;
 }
+double expansion_states(double seconds) { return (seconds - kLaunch) / kState; }
 
 int run(const Plan& p, const spb_options* opt, spb_result* out, DeviceContext* own_ctx, bool* launched)
 {

@@ -46,8 +46,12 @@ static_assert(kMaxWidth <= 24 && offsetof(Plan, bit) % 4 == 0 && offsetof(Plan, 
               "the kernel copies the plan in 4-byte words");
 
 // Plans the expansion of the row-major n x n matrix a (finite entries).
-// False when a plan does not fit the limits above.
-bool make_plan(const double* a, int n, Plan* plan);
+// False when a plan does not fit the limits above or visits more states than
+// max_states (given up after an order of either orientation).
+bool make_plan(const double* a, int n, Plan* plan, double max_states = 1e300);
+
+// States that take the kernel `seconds`, whatever the plan.
+double expansion_states(double seconds);
 
 // Estimated device time of the expansion, in seconds.
 double expansion_seconds(const Plan& plan);

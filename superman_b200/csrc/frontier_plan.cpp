@@ -102,7 +102,7 @@ bool simulate(const std::vector<uint64_t>& line, const std::vector<uint64_t>& cr
 
 }  // namespace
 
-bool make_plan(const double* a, int n, Plan* p)
+bool make_plan(const double* a, int n, Plan* p, double max_states)
 {
     if (n < 2 || n > kMaxRows) return false;
     std::memset(p, 0, sizeof(*p));
@@ -116,7 +116,7 @@ bool make_plan(const double* a, int n, Plan* p)
     // the lines with the fewest entries of each orientation as starts
     constexpr int kStarts = 4;
     std::vector<int> order, best_order;
-    double best = std::ldexp(1.0, kMaxWidth + 4);
+    double best = std::min(max_states, std::ldexp(1.0, kMaxWidth + 4));
     bool transpose = false;
     for (int o = 0; o < 2; ++o) {
         // (a start past the limit leaves no order: the rest rarely differ by

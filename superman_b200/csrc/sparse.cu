@@ -169,8 +169,9 @@ bool plan_compacted(const double* a, int n, int mode, const spb_options& opt, Ch
 // size from which that mode looks for a compacted walk; below it a fused dense
 // call takes 20-40 us), and on finite entries: the walks turn any non-finite
 // entry into NaN, the expansion only those that a perfect matching uses.  A
-// zero column keeps the dense walk.
-bool plan_expansion(const double* a, int n, const spb_options& opt, frontier::Plan* plan)
+// zero column keeps the dense walk.  max_states: where the states alone would take
+// longer than any walk.
+bool plan_expansion(const double* a, int n, const spb_options& opt, double max_states, frontier::Plan* plan)
 {
     if (opt.sparse_walk != SPB_SPARSE_WALK_AUTO || n < 20 || n > kMaxN || opt.precision == SPB_PREC_FP32 ||
         opt.unit_bits > 0 || opt.threads_per_block > 0 || opt.blocks > 0 || opt.replay_listing)
@@ -183,15 +184,15 @@ bool plan_expansion(const double* a, int n, const spb_options& opt, frontier::Pl
         }
         if (!any) return false;
     }
-    return frontier::make_plan(a, n, plan);
+    return frontier::make_plan(a, n, plan, max_states);
 }
 
-// Estimated wall times of the walks: FP64-pipe operations at 1.3e13 a second, on
-// top of what a call costs before its first term (n=20: 132 us of wall time, 51 of
-// them kernels, for the row-compacted walk's five launches; 45 us for a fused
-// dense call, 75 us for a dense call of separate kernels).
-double dense_seconds(int n) { return (n <= 26 ? 40e-6 : 75e-6) + 1.5 * n * std::ldexp(1.0, n - 1) / 1.3e13; }
-constexpr double kCompactedSeconds = 110e-6;
+// Estimated wall times from the plan on, one B200.  Dense walk without a pivot: 52 us
+// at n=20, 59 at 22, 85 at 24, 190 at 26.  Row-compacted walk: 75 us at n=20, 27 of
+// them kernels; its planning takes 30 us there, 60 at n=26, 90 at n=28.  The
+// expansion: its kernel and 38 us.
+double dense_seconds(int n) { return (n <= 26 ? 50e-6 : 75e-6) + 2.1 * n * std::ldexp(1.0, n - 1) / 1.3e13; }
+constexpr double kCompactedSeconds = 60e-6, kCompactedPlan = 35e-6, kExpansionCall = 38e-6;
 
 }  // namespace
 
@@ -200,13 +201,17 @@ int run_real_host(const double* a, int n, const spb_options* opt, spb_result* ou
     if (a && n >= 1 && n <= kMaxN && opt->sparse_walk != SPB_SPARSE_WALK_NEVER) {
         bool has_zero = false;
         for (size_t i = 0; i < (size_t)n * n && !has_zero; ++i) has_zero = a[i] == 0.0;
-        // The expansion where it is the faster call (20 us of planning and
-        // launch besides): at once when the walks could not be faster, or by no
-        // more than it takes to plan one (30 to 70 us), else by the estimates.
+        // The expansion where it is the faster call: at once when no walk could
+        // be faster with the compacted one's planning before it, else, that
+        // planning done, by the estimates.  (Without the planning in them, and 20 us
+        // for the call, patterns with 17 to 19 open columns took it too early: n=20
+        // with ten more per row 175 us for 120, n=23 with seven 213 us for 155.)
         frontier::Plan fp;
-        bool expand = has_zero && out && plan_expansion(a, n, *opt, &fp);
-        const double te = expand ? frontier::expansion_seconds(fp) + 20e-6 : INFINITY;
-        const bool at_once = te < std::min(kCompactedSeconds, dense_seconds(n) + 25e-6);
+        const double longest = kCompactedPlan + kCompactedSeconds + dense_seconds(n);
+        bool expand = has_zero && out &&
+                      plan_expansion(a, n, *opt, frontier::expansion_states(longest - kExpansionCall), &fp);
+        const double te = expand ? frontier::expansion_seconds(fp) + kExpansionCall : INFINITY;
+        const bool at_once = te < kCompactedPlan + std::min(kCompactedSeconds, dense_seconds(n));
         Choice ch;
         bool compacted = has_zero && !at_once && plan_compacted(a, n, opt->sparse_walk, *opt, &ch);
         if (expand && !at_once) expand = te < (compacted ? kCompactedSeconds + ch.cost / 1.3e13 : dense_seconds(n));

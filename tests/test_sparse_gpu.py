@@ -71,6 +71,18 @@ def test_sparse_dd_refinement_signed(spb, oracle):
     assert oracle.rel_err(r2.permanent, exact) <= 1e-12
 
 
+@pytest.mark.parametrize("n,extra,seed,expansion", [(20, 10, 3, False), (23, 7, 3, False), (24, 6, 3, False),
+                                                    (20, 3, 3, True), (28, 4, 3, True), (30, 5, 3, True)])
+def test_sparse_auto_takes_the_faster_route(spb, n, extra, seed, expansion):
+    """The expansion (one launch) where few columns are open, the compacted walk
+    (two) where 17 to 19 of n = 20 to 24 are and the expansion takes longer."""
+    a = W.sparse_perm_plus(n, seed, extra=extra)
+    r = spb.perm_sparse(a)
+    assert r.active_rows < n and (r.launches == 1) == expansion
+    d = spb.perm_sparse(a, walk="always", precision="dd")
+    assert abs(r.permanent - d.permanent) <= 1e-12 * abs(d.permanent)
+
+
 def test_sparse_csc_input_matches_dense_input(spb):
     a = W.sparse_perm_plus(24, 11)
     r1 = spb.perm_sparse(a)
