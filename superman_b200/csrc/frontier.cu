@@ -293,8 +293,8 @@ int run(const Plan& p, const spb_options* opt, spb_result* out, DeviceContext* o
             for (int s = q; s < (h ? p.nb : p.nf); s += 2) w = std::max(w, (int)p.step[(h ? p.nf : 0) + s].ka);
             o_t[h][q] = take(sizeof(double2) << w);
         }
-    if ((st = ensure_scratch(ctx, off)) != SPB_OK) return out->status = st;
-    if ((st = ensure_pinned(ctx, sizeof(Outcome))) != SPB_OK) return out->status = st;
+    // no room for the tables (up to 256 MiB): a walk needs far less
+    if (ensure_scratch(ctx, off) != SPB_OK || ensure_pinned(ctx, sizeof(Outcome)) != SPB_OK) return SPB_OK;
     if (!ctx->pinned_dev) return SPB_OK;
     char* base = static_cast<char*>(ctx->scratch);
     Tables t{};
@@ -321,7 +321,12 @@ int run(const Plan& p, const spb_options* opt, spb_result* out, DeviceContext* o
     }
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    SPB_CUDA_TRY(cudaLaunchKernelEx(&cfg, coop ? expand_rows<true> : expand_rows<false>, p, t));
+    // (refused launches, a grid that cannot be resident beside what else runs,
+    // leave no kernel behind)
+    if (cudaLaunchKernelEx(&cfg, coop ? expand_rows<true> : expand_rows<false>, p, t) != cudaSuccess) {
+        cudaGetLastError();
+        return SPB_OK;
+    }
     SPB_CUDA_TRY(cudaStreamSynchronize(stream));
     *launched = true;
     const Outcome o = *static_cast<const Outcome*>(ctx->pinned);
@@ -329,8 +334,9 @@ int run(const Plan& p, const spb_options* opt, spb_result* out, DeviceContext* o
     out->value = std::ldexp(res.hi, p.exp_sum);
     out->value_lo = std::ldexp(res.lo, p.exp_sum);
     // every state carries a few roundings of 2^-104 per row, and no partial
-    // sum exceeds the product of the rows' absolute sums
-    out->err_est = res.hi != 0.0 ? 4.0 * p.n * 0x1p-104 * p.abs_bound / std::fabs(res.hi) : 0.0;
+    // sum exceeds the product of the rows' absolute sums; a sum that cancels
+    // to zero has no relative error
+    out->err_est = res.hi != 0.0 ? 4.0 * p.n * 0x1p-104 * p.abs_bound / std::fabs(res.hi) : HUGE_VAL;
     out->kernel_s = out->device_s = opt->skip_timing ? 0.0 : 1e-9 * (double)(o.end - o.begin);
     out->gray_steps = (uint64_t)p.n << (p.n - 1);
     out->launches = 1;

@@ -56,8 +56,11 @@ double expansion_states(double seconds);
 // Estimated device time of the expansion, in seconds.
 double expansion_seconds(const Plan& plan);
 
+// Whether the nonzeros of the n x n matrix a hold a perfect matching, n <= 63.
+bool has_matching(const double* a, int n);
+
 // Runs the plan; *launched is false when its tables could not be allocated or
-// the grid cannot be resident, in which case nothing ran.
+// its launch was refused, in which case nothing ran and a walk can.
 int run(const Plan& plan, const spb_options* opt, spb_result* out, DeviceContext* own_ctx, bool* launched);
 
 }  // namespace frontier

@@ -100,7 +100,35 @@ bool simulate(const std::vector<uint64_t>& line, const std::vector<uint64_t>& cr
     return true;
 }
 
+// Augments a matching of rows to columns from row r (columns of `seen` tried).
+bool augment(const std::vector<uint64_t>& line, int r, uint64_t* seen, std::vector<int>* row_of)
+{
+    while (uint64_t m = line[r] & ~*seen) {
+        const int c = __builtin_ctzll(m);
+        *seen |= 1ull << c;
+        if ((*row_of)[c] < 0 || augment(line, (*row_of)[c], seen, row_of)) {
+            (*row_of)[c] = r;
+            return true;
+        }
+    }
+    return false;
+}
+
 }  // namespace
+
+bool has_matching(const double* a, int n)
+{
+    std::vector<uint64_t> line(n, 0);
+    for (int r = 0; r < n; ++r)
+        for (int c = 0; c < n; ++c)
+            if (a[(size_t)r * n + c] != 0.0) line[r] |= 1ull << c;
+    std::vector<int> row_of(n, -1);
+    for (int r = 0; r < n; ++r) {
+        uint64_t seen = 0;
+        if (!augment(line, r, &seen, &row_of)) return false;
+    }
+    return true;
+}
 
 bool make_plan(const double* a, int n, Plan* p, double max_states)
 {

@@ -219,6 +219,7 @@ int run_real_host(const double* a, int n, const spb_options* opt, spb_result* ou
             std::memset(out, 0, sizeof(*out));
             bool launched = false;
             const int st = frontier::run(fp, opt, out, ctx, &launched);
+            if (launched && out->value == 0.0 && !frontier::has_matching(a, n)) out->err_est = 0.0;  // zero exactly
             if (st != SPB_OK || launched) return st;
             if (at_once) compacted = plan_compacted(a, n, opt->sparse_walk, *opt, &ch);
         }
