@@ -91,9 +91,10 @@ typedef struct spb_options {
                               fused kernel (tables, walk, threshold and
                               refinement); < 0: as separate kernels        */
     int skip_timing;       /* 1: the dense entry points skip their device
-                              timing (n > 26: no events around the kernels, a
-                              few us less per call); kernel_s and device_s in
-                              spb_result are then 0                         */
+                              timing; kernel_s and device_s in spb_result are
+                              then 0.  Up to n = 26 that saves nothing (the
+                              kernels stamp their own times), above it the
+                              events around the kernels, 10 to 25 us a call  */
 } spb_options;
 
 typedef struct spb_result {
@@ -107,8 +108,9 @@ typedef struct spb_result {
                               input copy (if any), kernels, result copy.
                               Dense calls of n <= 26 take both times from
                               the kernels' own stamps of the device's clock
-                              (from the first kernel's start to the result
-                              in host memory), larger ones from events      */
+                              (from the start of the first kernel, which
+                              fetches a host matrix, to the result in host
+                              memory), larger ones from events              */
     double err_est;        /* estimated relative error (statistical); for
                               spb_perm_approx the relative standard error */
     uint64_t gray_steps;   /* Gray steps of the Nijenhuis-Wilf formula,

@@ -53,7 +53,7 @@ namespace dense {
 //   4 warps: 0, 1 tables (part 0, 1), 2 start values, 3 high columns.
 __global__ void __launch_bounds__(128) setup_kernel(Problem pb, const double* __restrict__ a_in, int smem_tables)
 {
-    if (pb.timed && blockIdx.x == 0 && threadIdx.x == 0) pb.rb->stamp[0] = global_ns();
+    if (pb.timed == 1 && blockIdx.x == 0 && threadIdx.x == 0) pb.rb->stamp[0] = global_ns();
     const int n = pb.n, c = pb.comps, w = pb.w, G = pb.g;
     const int tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, wid = tid >> 5, r = blockIdx.x;
     const int terms = 1 << w;
@@ -256,6 +256,18 @@ __global__ void __launch_bounds__(128) setup_kernel(Problem pb, const double* __
         for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         if (lane == 0) pb.bnd[r] = __longlong_as_double((long long)mx) * (1.0 + 0x1p-50);
     }
+}
+
+// Brings a staged matrix (page-locked host memory) to the device, `count`
+// doubles, as the first kernel of a call that takes its device time from stamps.
+// Bound by the host link's round trip, and no slower than the copy it stands for
+// (complex n=22 79 us a call with either), where events around copy and kernels,
+// the other way to time them, cost such a call 20 us (101 us).
+__global__ void __launch_bounds__(256) fetch_kernel(Problem pb, const double* __restrict__ from, double* to, int count)
+{
+    if (pb.timed && blockIdx.x == 0 && threadIdx.x == 0) pb.rb->stamp[0] = global_ns();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < count) to[i] = from[i];
 }
 
 }  // namespace dense
@@ -613,13 +625,23 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
     constexpr size_t kStageOff = 256;
     static_assert(sizeof(Readback) <= kStageOff, "readback fits before the staging area");
     const size_t a_bytes = sizeof(double) * n * n * comps;
-    // device times: events around the kernels, or (small calls) the kernels' own
-    // stamps; none with skip_timing
-    const bool events = !opt.skip_timing && (n > kStampedMaxN || !ctx->pinned_dev);
-    pb.timed = !events && !opt.skip_timing ? 1 : 0;
-    auto record = [&](cudaEvent_t ev) { return events ? cudaEventRecord(ev, stream) : cudaSuccess; };
     if ((st = ensure_pinned(ctx, kStageOff + a_bytes)) != SPB_OK) return out->status = st;
     Readback* hrb = static_cast<Readback*>(ctx->pinned);
+    Readback* mapped = static_cast<Readback*>(ctx->pinned_dev);
+    const bool fused_fits = small_candidate && pb.units <= kRawCap &&
+                            small_call_smem_bytes(n, pb.w, threads) <= ctx->smem_optin;
+    // The plain walk's setup kernel, whose CTAs need a row each, reads a host
+    // matrix from the staging area too, where it lies.  With the derivative walk
+    // every CTA needs the whole matrix (195 KB at n=29 took it 15 us longer over
+    // the host link than a copy): small calls fetch it with a kernel of its own,
+    // so that the call's device time holds the fetching, larger ones copy it.
+    const bool fetch = mapped && !a_on_device && !fused_fits && pb.deriv && n <= kStampedMaxN;
+    const bool stage_in = mapped && !a_on_device && (fused_fits || !pb.deriv || fetch);
+    // device times: the kernels' own stamps in small calls, else events around
+    // the kernels; none with skip_timing
+    const bool events = !opt.skip_timing && (n > kStampedMaxN || !mapped);
+    pb.timed = events || opt.skip_timing ? 0 : (fetch ? 2 : 1);
+    auto record = [&](cudaEvent_t ev) { return events ? cudaEventRecord(ev, stream) : cudaSuccess; };
     // The refinement list is sized before the walk for the threshold's cap
     // (1/8 of the units), up to 2^21 units; a larger count is met after the
     // readback with a larger list.
@@ -645,16 +667,8 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
     // matrix from the pinned staging area itself (no copy before it: a copy
     // engine takes several microseconds to start for 4.6 KB).  A launch asked
     // for again is replayed as a CUDA graph.
-    const bool fused_fits = small_candidate && pb.units <= kRawCap &&
-                            small_call_smem_bytes(n, pb.w, threads) <= ctx->smem_optin;
-    Readback* mapped = static_cast<Readback*>(ctx->pinned_dev);
     const double* a_stage = nullptr;  // device address of the staged host matrix
-    // The plain walk's setup kernel, whose CTAs need a row each, reads a host
-    // matrix from the staging area too, where it lies (with the derivative walk
-    // every CTA needs the whole matrix: 195 KB at n=29 took it 15 us longer over
-    // the host link than the copy).
-    const bool map_in = mapped && !a_on_device && !pb.deriv;
-    if (mapped && !a_on_device && (fused_fits || map_in)) {
+    if (stage_in) {
         std::memcpy(static_cast<char*>(ctx->pinned) + kStageOff, a, a_bytes);
         a_stage = reinterpret_cast<const double*>(static_cast<char*>(ctx->pinned_dev) + kStageOff);
     }
@@ -692,10 +706,15 @@ int run(const double* a, bool a_on_device, int n, int comps, const spb_options* 
         }
     }
     if (!fused) {
-    if ((st = launch_setup(pb, a_stage ? a_stage : d_a, stream)) != SPB_OK) return out->status = st;
+    if (fetch) {
+        const int count = n * n * comps;
+        fetch_kernel<<<(count + 255) / 256, 256, 0, stream>>>(pb, a_stage, d_in, count);
+        SPB_CUDA_TRY(cudaGetLastError());
+    }
+    if ((st = launch_setup(pb, a_stage && !fetch ? a_stage : d_a, stream)) != SPB_OK) return out->status = st;
     SPB_CUDA_TRY(cudaGetLastError());
     SPB_CUDA_TRY(record(ctx->ev_begin));
-    launches = 2;
+    launches = fetch ? 3 : 2;
     if (dd_mode && pb.na == n && pb.units > pb.raw_cap / 2) {
         // Size the first pass's unit list from a bound-only pass (about 1.5 %
         // of a dense walk).  The row-compacted walk has few terms per unit, so

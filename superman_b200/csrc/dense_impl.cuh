@@ -75,7 +75,7 @@ struct Problem {
     Readback* rb_host;         // the device's address of the host's page-locked copy of *rb; the
                                // call's last kernel fills it (null in the others, and where the
                                // host copies the readback itself)
-    int timed;                 // the kernels stamp their times
+    int timed;                 // nonzero: the kernels stamp their times (2: fetch_kernel takes the first)
     double tol;                // SPB_PREC_DD: relative tolerance of the threshold
     // Double-double refinement (SPB_PREC_DD); unused when mode == 0.
     int mode;                  // 0 walk, 1 walk + unit-bound histogram, 2 scan only

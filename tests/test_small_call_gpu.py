@@ -1,9 +1,12 @@
 """The fused small-matrix call (one cooperative kernel for real 4 <= n <= 26:
 tables, walk, threshold and double-double refinement) against the same call
 made of separate kernels, and against the exact value."""
+import ctypes
+
 import numpy as np
 import pytest
 
+from superman_b200 import _lib
 from superman_b200 import workloads as W
 from conftest import load_golden
 
@@ -145,3 +148,25 @@ def test_skip_timing_complex(spb):
     u = spb.perm_complex(c, precision="dd", skip_timing=1)
     assert abs(u.permanent - t.permanent) <= 1e-14 * abs(t.permanent)
     assert u.kernel_s == 0.0 and t.kernel_s > 0.0
+
+
+@pytest.mark.parametrize("n,cplx", [(24, False), (22, True), (25, True)])
+def test_device_time_covers_the_input_copy(spb, n, cplx):
+    """A call whose matrix is copied to the device before its first kernel (the
+    separate kernels with a pivot column) counts that copy in device_s, the same
+    call on a matrix already there has none."""
+    import torch
+    a = W.haar_block(n, 3, N=64) if cplx else W.dense_uniform(n, 3)
+    f = np.ascontiguousarray(a).view(np.float64)
+    d = torch.from_numpy(f).cuda()
+    torch.cuda.synchronize()
+    L, o, r = _lib.lib(), _lib.default_options(small_call=-1), _lib.spb_result()
+    host, dev = (L.spb_perm_dense_c128, L.spb_perm_dense_c128_dev) if cplx else \
+                (L.spb_perm_dense_f64, L.spb_perm_dense_f64_dev)
+    t = [[], []]
+    for _ in range(20):
+        _lib.check(host(f.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), n, ctypes.byref(o), ctypes.byref(r)))
+        t[0].append(r.device_s)
+        _lib.check(dev(ctypes.c_void_p(d.data_ptr()), n, ctypes.byref(o), ctypes.byref(r)))
+        t[1].append(r.device_s)
+    assert np.median(t[0]) >= np.median(t[1]) + 0.5e-6, (np.median(t[0]), np.median(t[1]))
