@@ -202,9 +202,10 @@ __device__ __forceinline__ bool scale_row_cached(const Pattern& P, const Lane<Co
 }
 
 // One sample's estimate (0 when the drawn partial matching cannot be
-// completed).
-template <class Count>
-__device__ __forceinline__ double sample_estimate(const Pattern& P, const Lane<Count>& L, unsigned long long seed, unsigned long long k)
+// completed).  CACHED: the kernel has the cached rows' path.
+template <class Count, bool CACHED>
+__device__ __forceinline__ double sample_estimate(const Pattern& P, const Lane<Count>& L, unsigned long long seed,
+                                                  unsigned long long k)
 {
     const int n = P.n;
     for (int i = 0; i < n; ++i) {
@@ -219,7 +220,7 @@ __device__ __forceinline__ double sample_estimate(const Pattern& P, const Lane<C
         const int p0 = P.rptr[i], deg = P.rptr[i + 1] - p0;
         float ri = L.RV(i), run = 0.0f, prob = 0.0f;
         int chosen = -1;
-        if (P.cached[i]) {
+        if (CACHED && P.cached[i]) {
             int j[kCols];
             float cv[kCols];
             if (!scale_row_cached(P, L, i, p0, deg, ri, j, cv)) return 0.0;
@@ -282,7 +283,7 @@ struct Sums {
 };
 
 constexpr int kCtasPerSm = 8;  // 64 registers a thread
-template <class Count>
+template <class Count, bool CACHED>
 __global__ void __launch_bounds__(128, kCtasPerSm) rasmussen_kernel(Pattern P, Lane<Count> L0, unsigned long long first,
                                                                     unsigned long long count,
                                                                     unsigned long long seed, Sums S)
@@ -292,7 +293,7 @@ __global__ void __launch_bounds__(128, kCtasPerSm) rasmussen_kernel(Pattern P, L
     L.t = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
     double s1 = 0.0, s2 = 0.0;
     for (unsigned long long k = L.t; k < count; k += L.T) {
-        const double e = sample_estimate(P, L, seed, first + k);
+        const double e = sample_estimate<Count, CACHED>(P, L, seed, first + k);
         if (S.per_sample) S.per_sample[k] = e;
         s1 += e;
         s2 = __fma_rn(e, e, s2);
@@ -425,6 +426,13 @@ int run(const int* cptrs, const int* rows, int n, unsigned long long first, unsi
         cached[i] = ok ? 1 : 0;
     }
     const bool bytes = most <= 255;
+    // With the cached path in it the kernel spills, which rows that don't take it
+    // pay for (up to 1.4 times the time): it stays out unless half of the rows do.
+    // Against one kernel for all without either path (1.0), with and without the
+    // cached path: n=100, three more per row (0.8 of the rows cached) 1.24 and 1.11,
+    // four (0.6) 1.18 and 1.09, five (0.1) 1.04 and 1.11, eight 0.96 and 1.07, 15 0.76
+    // and 1.04; all entries, n=30, 4.0 and 5.2.
+    const bool most_cached = 2 * std::count(cached.begin(), cached.end(), (unsigned char)1) >= n;
 
     // Launch shape: kCtasPerSm CTAs of 128 threads per SM (the sampler is
     // latency-bound; their registers let all of them be resident), fewer when the
@@ -481,7 +489,8 @@ int run(const int* cptrs, const int* rows, int n, unsigned long long first, unsi
         Lane<Count> L{reinterpret_cast<float*>(base + o_rv), reinterpret_cast<float*>(base + o_cv),
                       reinterpret_cast<Count*>(base + o_re), reinterpret_cast<Count*>(base + o_ce),
                       reinterpret_cast<int*>(base + o_sk), 0, 0};
-        rasmussen_kernel<Count><<<blocks, threads, 0, stream>>>(P, L, first, count, seed, S);
+        if (most_cached) rasmussen_kernel<Count, true><<<blocks, threads, 0, stream>>>(P, L, first, count, seed, S);
+        else rasmussen_kernel<Count, false><<<blocks, threads, 0, stream>>>(P, L, first, count, seed, S);
     };
     if (bytes) launch((unsigned char)0);
     else launch(0);

@@ -42,6 +42,25 @@ def test_samples_bit_exact_vs_oracle(spb, oracle, name, first):
     assert (got > 0).any()
 
 
+@pytest.mark.parametrize("name", ["extra4", "extra5", "extra8", "full", "one_full_row", "n300_full"])
+def test_samples_bit_exact_on_either_kernel(spb, oracle, name):
+    """Patterns on both sides of the rule that picks the kernel (half of the rows
+    with at most five entries whose columns have at most four below), and lines of
+    more than 255 entries, whose counts need more than a byte."""
+    n = 300 if name == "n300_full" else 40
+    a = (W.sparse_perm_plus(n, 6, extra=int(name[5:]) if name.startswith("extra") else 3) != 0).astype(np.uint8)
+    if name == "full":
+        a[:] = 1
+    elif "full" in name:
+        a[7, :] = 1
+        a[:, 9] = 1
+    count = 400 if n == 300 else 2000
+    got = spb.approx_samples(a, 11, count, seed=5)
+    want = oracle.rasmussen_samples(a, 11, count, seed=5)
+    assert np.array_equal(got, want), np.flatnonzero(got != want)[:5]
+    assert (got > 0).any()
+
+
 @pytest.mark.parametrize("n,seed", [(12, 1), (16, 2), (20, 3)])
 def test_mean_matches_exact(spb, oracle, n, seed):
     a = W.binary_bernoulli(n, seed)
