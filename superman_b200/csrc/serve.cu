@@ -63,13 +63,19 @@ constexpr size_t kUnit = batch::kOffsetUnit * sizeof(double);  // pool granule, 
 constexpr int kGraphAfterUses = 3;            // uses of a key before its graph is captured
 
 // Mid-size shapes are batched when at least this many requests of the shape are
-// queued.  A batch of up to 15 takes 95 us (real n=21) to 490 us (n=24), complex
-// 240 us to 1.6 ms, beside other shapes' batches on their own streams; a
-// whole-GPU call 45 to 80 us, complex 85 to 140 us, and shares nothing.  Bursts of
-// mixed sizes on one B200, against batching from 16, 32, 64, 128 queued requests
-// on: 512 of n = 8..24 7.7 -> 5.9 ms, 1024 of n = 16..24 25 -> 13.2 ms, 128 of
-// n = 8..24 2.35 -> 2.05 ms.
-inline size_t mid_batch_min(int n) { return n <= 21 ? 3 : (n == 22 ? 4 : (n == 23 ? 6 : 9)); }
+// queued.  A batch forms its products in FP64.  Where whole-GPU calls refine them
+// (or the server runs FP32), fewer requests than its time alone asks for must not
+// change what a request gets: 16 of n=21, twice as many per row more.  A server in
+// FP64 loses nothing by a batch, and real ones pay earlier: bursts of 9, 12 and 24
+// requests took 183, 194 and 345 us batched and 221, 562 and 495 us as whole-GPU
+// calls at n=21, 380, 395 and 623 against 408, 494 and 738 us at n=23, but 575, 615
+// and 1212 against 619, 520 and 1017 us at n=24; complex ones (n=22 573, 641, 1006
+// against 426, 550, 1048 us) do not.
+inline size_t mid_batch_min(int n, int comps, int precision)
+{
+    if (precision == SPB_PREC_FP64 && comps == 1) return n <= 22 ? 9 : (n == 23 ? 12 : 32);
+    return (size_t)16 << (n > 21 ? n - 21 : 0);
+}
 
 // Host-side double-double product (Dekker with exact FMA).
 inline dd dd_mul_host(dd a, dd b)
@@ -646,7 +652,7 @@ int Server::launch_slot(int si, int n, int comps, std::vector<uint64_t>& ids)
 // Starts one batch if a slot is free and a shape is due: its queue holds a
 // full batch, its oldest request waited max_wait_s, or (force) the batch side
 // of the GPU is idle, in which case waiting would only add latency.  A
-// mid-size shape with fewer than mid_batch_min(n) queued requests goes to the
+// mid-size shape with fewer than mid_batch_min queued requests goes to the
 // whole-GPU workers once its oldest request has waited max_wait_s.
 bool Server::launch_ready(bool force)
 {
@@ -662,7 +668,7 @@ bool Server::launch_ready(bool force)
         for (int c = 0; c < 2; ++c)
             for (int k = kSmallN + 1; k <= cfg.batch_max_n; ++k) {
                 auto& q = small_q[c][k];
-                if (q.empty() || q.size() >= mid_batch_min(k)) continue;
+                if (q.empty() || q.size() >= mid_batch_min(k, c + 1, cfg.precision)) continue;
                 if (now - reqs.at(q.front()).t_submit < cfg.max_wait_s) continue;
                 st.mid_to_large += q.size();
                 for (uint64_t id : q) large_q.push_back(id);
@@ -677,7 +683,7 @@ bool Server::launch_ready(bool force)
             for (int k = 1; k <= cfg.batch_max_n; ++k) {
                 auto& q = small_q[c][k];
                 if (q.empty()) continue;
-                if (k > kSmallN && q.size() < mid_batch_min(k)) continue;
+                if (k > kSmallN && q.size() < mid_batch_min(k, c + 1, cfg.precision)) continue;
                 const double t = reqs.at(q.front()).t_submit;
                 if ((int)q.size() >= cfg.max_batch) { oldest = -1; bc = c; bn = k; }
                 else if (t < oldest) { oldest = t; bc = c; bn = k; }

@@ -224,6 +224,24 @@ def test_mid_size_requests_take_the_favoured_path(spb):
         assert abs(r["permanent"] - want) <= REL_TOL * abs(want)
 
 
+def test_refined_requests_are_not_batched_early(spb):
+    """A double-double server refines what it can: ten requests of n=22 and of n=24
+    run as whole-GPU calls and give their bits.  In FP64 the ten of n=22 are one
+    batch (which refines nothing)."""
+    for n in (22, 24):
+        mats = [W.dense_uniform(n, 90 + k) for k in range(10)]
+        with Server(precision="dd", max_wait_s=1e-3) as srv:
+            rs = [srv.wait(t, timeout_s=60) for t in srv.submit_many(mats)]
+            st = srv.stats()
+        assert st["mid_to_large"] == 10 and st["batched_requests"] == 0
+        for a, r in zip(mats, rs):
+            want = spb.perm_dense(a, precision="dd")
+            assert abs(r["permanent"] - want.permanent) <= 2e-15 * abs(want.permanent)
+    with Server(precision="fp64", max_wait_s=1e-2) as srv:
+        rs = [srv.wait(t, timeout_s=60) for t in srv.submit_many([W.dense_uniform(22, 90 + k) for k in range(10)])]
+        assert srv.stats()["batched_requests"] == 10
+
+
 def test_admission_counts_device_pool_bytes(spb):
     """Admission reserves each request's matrix in the device pool until it
     completes: a pool of 64 KiB takes eight 32 x 32 real matrices (8 KiB
