@@ -42,13 +42,12 @@ static int pick_limbs(double perm_bits, int shift)
 // Rewrites the matrix for the expanded walk: the line with the fewest ones
 // becomes the last column (a row by transposing, which keeps the permanent) and
 // the rows with a one in it come first.  Returns their number m, or 0 when the
-// plain walk runs: n < 4 (no two walk columns besides the expanded one), an
-// empty line (permanent 0) or more ones than the kernel's halves hold.
-// Where it applies the expanded walk is the faster one at every n and m: it
-// takes half the subsets and at most 3/2 of the operations per subset.
+// plain walk runs: an empty line (permanent 0), more ones than the kernel's halves
+// hold, or n < kMinExpand.  From there on the expanded walk is the faster one at
+// every m: it takes half the subsets and at most 3/2 of the operations per subset.
 static int expand(std::vector<uint8_t>* m, int n)
 {
-    if (n < 4) return 0;
+    if (n < kMinExpand) return 0;
     int best = n + 1, line = 0;  // line < n: column, else row line - n
     for (int l = 0; l < 2 * n; ++l) {
         int c = 0;

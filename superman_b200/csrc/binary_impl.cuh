@@ -204,6 +204,10 @@ __device__ __forceinline__ void limb_add_masked(uint32_t (&a)[L], const uint32_t
 // takes a sign and a magnitude per 2K rows instead of one per K.  The words
 // with rows of the expanded column carry the derivative q beside the product.
 constexpr int kExpandHalves = 4;  // halves that may hold rows of the expanded column
+// Smallest n of the expanded walk.  Below, a call waits for its launch and copies
+// and the longer chain of a term only adds to it (wall time, plain and expanded:
+// n=12 61.4 and 65.1 us, n=16 63.5 and 67.2, n=21 70.6 and 73.4, n=23 90.1 and 80.0).
+constexpr int kMinExpand = 22;
 
 // Rows per half: the largest K with (n-1)^K < 2^31 and K (n-1)^(K-1) < 2^31 (the
 // half's product and its derivative; row values are at most n-1 in magnitude).

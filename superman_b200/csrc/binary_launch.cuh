@@ -41,7 +41,7 @@ int launch_bin_nx(const Problem& pb, int blocks, int threads, size_t smem, cudaS
 template <int N, int L>
 int launch_bin_n(const Problem& pb, int blocks, int threads, size_t smem, cudaStream_t s, int* per_sm)
 {
-    if constexpr (N >= 4)
+    if constexpr (N >= kMinExpand)
         if (pb.m > 0) return launch_bin_nx<N, L, true>(pb, blocks, threads, smem, s, per_sm);
     return launch_bin_nx<N, L, false>(pb, blocks, threads, smem, s, per_sm);
 }

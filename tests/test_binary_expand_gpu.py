@@ -22,10 +22,12 @@ def with_column_ones(n, m, seed, p):
     return a
 
 
-# rows per half: 9 at n = 10 and 11, 8 at 12 .. 15, 7 at 16 .. 22
+# rows per half: 7 at n = 22, 6 at 23 .. 36; below n = 22 the plain walk runs
 @pytest.mark.parametrize("n,m", [(4, 1), (4, 4), (5, 2), (9, 9), (10, 8), (10, 9), (10, 10), (12, 8), (12, 9),
                                  (16, 7), (16, 8), (16, 14), (16, 15), (16, 16), (17, 6), (20, 1), (20, 13),
-                                 (20, 14), (20, 15), (20, 20), (22, 20), (22, 21), (22, 22)])
+                                 (20, 14), (20, 15), (20, 20), (22, 1), (22, 7), (22, 8), (22, 14), (22, 15),
+                                 (22, 20), (22, 21), (22, 22), (23, 6), (23, 7), (23, 12), (23, 13), (23, 18),
+                                 (23, 19), (23, 23), (24, 24), (25, 24), (25, 25)])
 def test_expanded_words_bit_exact(spb, oracle, n, m):
     a = with_column_ones(n, m, 100 * n + m, 0.95)
     want = oracle.binary_u128(a)
@@ -33,7 +35,7 @@ def test_expanded_words_bit_exact(spb, oracle, n, m):
     assert spb.perm_binary(a.T.copy()).permanent == want  # the line is a row
 
 
-@pytest.mark.parametrize("n", [16, 21, 24, 25])
+@pytest.mark.parametrize("n", [16, 21, 22, 24, 25])
 def test_all_ones_around_the_last_half(spb, n):
     """m = n: within four halves up to n = 24 (6 rows a half there), the plain
     walk past it, and the launch shapes the options allow."""
