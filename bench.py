@@ -531,13 +531,18 @@ SERVE_WORKLOADS = {
 SERVE_BATCH_MAX_N = 24
 
 
-def walk_work(n, cplx, batched=False):
-    """FP64 pipe instructions of one permanent of a matrix without zeros.  The
-    plain walk takes 2^(n-1) subsets at 2 per row (real: DADD + DMUL) or 6
-    (complex: 2 DADD, 2 DMUL, 2 DFMA); the derivative walk, which runs from n = 24
-    (complex 22; in batches 11) on, 2^(n-2) subsets at 3 (DADD, DMUL, DFMA) or
-    10 (2 DADD, 2 DMUL, 6 DFMA)."""
-    if n >= (11 if batched else 22 if cplx else 24):
+# Smallest n of the derivative walk: kMinDerivReal and kMinDerivComplex
+# (dense_impl.cuh), has_deriv (batch.cu).
+MIN_DERIV = {"real": 24, "complex": 22, "batch": 11}
+
+
+def walk_work(n, cplx, batched=False, pivot=True):
+    """FP64 pipe instructions of one permanent.  The plain walk takes 2^(n-1)
+    subsets at 2 per row (real: DADD + DMUL) or 6 (complex: 2 DADD, 2 DMUL, 2
+    DFMA); the derivative walk, from MIN_DERIV on for a matrix with a pivot column
+    (one without zeros, as every workload here has), 2^(n-2) subsets at 3 (DADD,
+    DMUL, DFMA) or 10 (2 DADD, 2 DMUL, 6 DFMA)."""
+    if pivot and n >= MIN_DERIV["batch" if batched else "complex" if cplx else "real"]:
         return (10 if cplx else 3) * n * 2 ** (n - 2)
     return (6 if cplx else 2) * n * 2 ** (n - 1)
 

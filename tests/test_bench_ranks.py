@@ -63,3 +63,19 @@ def test_reference_arm_other_ranks_idle(monkeypatch, capsys):
     args = argparse.Namespace(gpus=2, steps=1, warmup=1)
     assert bench.reference_arm(args, "dense32") == 0
     assert not called and capsys.readouterr().out == ""
+
+
+def test_bench_counts_the_walks_that_run():
+    """The sizes from which bench.py counts the derivative walk are the kernels'."""
+    import re
+    sys.path.insert(0, ROOT)
+    import bench
+    csrc = os.path.join(ROOT, "superman_b200", "csrc")
+    dense = open(os.path.join(csrc, "dense_impl.cuh")).read()
+    batch = open(os.path.join(csrc, "batch.cu")).read()
+    want = {"real": int(re.search(r"kMinDerivReal = (\d+)", dense)[1]),
+            "complex": int(re.search(r"kMinDerivComplex = (\d+)", dense)[1]),
+            "batch": int(re.search(r"has_deriv\(int n\) \{ return n >= (\d+)", batch)[1])}
+    assert bench.MIN_DERIV == want
+    assert bench.walk_work(30, False) == 3 * 30 * 2 ** 28
+    assert bench.walk_work(30, False, pivot=False) == 2 * 30 * 2 ** 29
