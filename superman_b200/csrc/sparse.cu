@@ -189,10 +189,13 @@ bool plan_expansion(const double* a, int n, const spb_options& opt, double max_s
 
 // Estimated wall times from the plan on, one B200.  Dense walk without a pivot: 52 us
 // at n=20, 59 at 22, 85 at 24, 190 at 26.  Row-compacted walk: 75 us at n=20, 27 of
-// them kernels; its planning takes 30 us there, 60 at n=26, 90 at n=28.  The
-// expansion: its kernel and 38 us.
-double dense_seconds(int n) { return (n <= 26 ? 50e-6 : 75e-6) + 2.1 * n * std::ldexp(1.0, n - 1) / 1.3e13; }
-constexpr double kCompactedSeconds = 60e-6, kCompactedPlan = 35e-6, kExpansionCall = 38e-6;
+// them kernels; at n=28 and 30 its kernels took a third of the dense walk's or more.
+// Its planning takes 30 us at n=20, 60 at n=26, 90 at n=28.  The expansion: its
+// kernel and 38 us.
+double walk_seconds(int n) { return 2.1 * n * std::ldexp(1.0, n - 1) / 1.3e13; }
+double dense_seconds(int n) { return (n <= 26 ? 50e-6 : 75e-6) + walk_seconds(n); }
+double compacted_plan(int n) { return 35e-6 + 10e-6 * std::max(0, n - 24); }
+constexpr double kCompactedSeconds = 60e-6, kExpansionCall = 38e-6;
 
 }  // namespace
 
@@ -207,11 +210,12 @@ int run_real_host(const double* a, int n, const spb_options* opt, spb_result* ou
         // for the call, patterns with 17 to 19 open columns took it too early: n=20
         // with ten more per row 175 us for 120, n=23 with seven 213 us for 155.)
         frontier::Plan fp;
-        const double longest = kCompactedPlan + kCompactedSeconds + dense_seconds(n);
+        const double longest = compacted_plan(n) + kCompactedSeconds + dense_seconds(n);
         bool expand = has_zero && out &&
                       plan_expansion(a, n, *opt, frontier::expansion_states(longest - kExpansionCall), &fp);
         const double te = expand ? frontier::expansion_seconds(fp) + kExpansionCall : INFINITY;
-        const bool at_once = te < kCompactedPlan + std::min(kCompactedSeconds, dense_seconds(n));
+        const bool at_once =
+            te < compacted_plan(n) + std::min(kCompactedSeconds + 0.25 * walk_seconds(n), dense_seconds(n));
         Choice ch;
         bool compacted = has_zero && !at_once && plan_compacted(a, n, opt->sparse_walk, *opt, &ch);
         if (expand && !at_once) expand = te < (compacted ? kCompactedSeconds + ch.cost / 1.3e13 : dense_seconds(n));
