@@ -99,12 +99,13 @@ __device__ __forceinline__ ThresholdPick pick_threshold_shared(const Problem& pb
     constexpr int kPer = kHistBins / 32;
     const int lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
-    // Rounded operations per term.  The real derivative walk counts six times
-    // as many variances as a term has roundings (2n): over permuted copies of
-    // U[0,1) matrices of n = 24 .. 32 the refined results spread by up to ten
-    // times the plain estimate, in either walk, and this keeps the derivative
-    // walk's spread at or below the plain walk's (n=31: 3.2e-13 without it,
-    // 1.3e-13 for the plain walk) for a few hundred refined units more.
+    // Rounded operations per term, 2n real and 6n complex.  The real derivative
+    // walk takes six times as many: a margin, since roundings that a unit's products
+    // share are not independent.  Over permuted copies of U[0,1) matrices of n = 24
+    // .. 32 the refined results spread by up to ten times the plain estimate, in
+    // either walk; with the margin the derivative walk's spread is at or below the
+    // plain walk's (n=31: 3.2e-13 without it, 1.3e-13 for the plain walk) for a few
+    // hundred refined units more.  err_est holds the margin too.
     const double k = pb.comps == 1 ? (deriv ? 12.0 : 2.0) * pb.n : 6.0 * pb.n;
     const double var_per_s2 = mul_rn(k / 12.0, 0x1p-104);
     const double half = mul_rn(0.5 * pb.tol, mag);

@@ -1,6 +1,8 @@
-"""Parity of the sparse entry point spb_perm_sparse_f64 (row-compacted walk)
-with the oracle: exact CRT permanents, and the exact n=40 sparse fixture
-through its decomposition pieces."""
+"""Parity of the sparse entry point spb_perm_sparse_f64 with the oracle: exact
+CRT permanents, and the exact n=40 sparse fixture through its decomposition
+pieces.  walk="always" is the row-compacted walk; in automatic mode these patterns
+take the row-by-row expansion from n = 20 on (its own tests: test_expand_rows_gpu),
+except where a launch shape is given."""
 import numpy as np
 import pytest
 
@@ -102,8 +104,8 @@ def test_sparse_deterministic_and_shape_invariant(spb, oracle):
 
 
 def test_sparse_n40_pieces_sum_to_exact(spb, oracle):
-    """The decomposition pieces of the n=40 fixture, each on the compacted
-    walk, sum to its exact permanent."""
+    """The decomposition pieces of the n=40 fixture, each expanded row by row,
+    sum to its exact permanent."""
     from conftest import load_golden
     from test_host_pipeline import decompose
     a, exact, _ = load_golden("sparse_n40_s5")
