@@ -149,8 +149,10 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
     // accumulators; a device matrix is read where it is.
     // A grid small enough to fetch the staged matrix once per CTA does so
     // without the copy and its barrier; the FP64 mode then needs no barrier
-    // before the walk at all (it adds to nothing global).
-    const bool direct = a_stage != nullptr && gridDim.x * (N * N * 8) <= 64 * 1024;
+    // before the walk at all (it adds to nothing global).  Up to 16 KB over the
+    // host link together, n = 15; n = 16's 32 KB took a double-double call 37.4 us,
+    // the staged one 31.3.
+    const bool direct = a_stage != nullptr && gridDim.x * (N * N * 8) <= 16 * 1024;
     const bool staged = a_stage != nullptr && !direct;  // the same in every CTA
     // The double-double mode's barrier, where the staging has none: behind the
     // tables, which hide the fetching of the matrix (1 us of 30 at n=13), but before them at the derivative walk's sizes.  There a
