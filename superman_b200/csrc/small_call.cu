@@ -155,7 +155,8 @@ __global__ void __launch_bounds__(kSmallCallThreads, 1) small_call_real(Problem 
     const bool direct = a_stage != nullptr && gridDim.x * (N * N * 8) <= 16 * 1024;
     const bool staged = a_stage != nullptr && !direct;  // the same in every CTA
     // The double-double mode's barrier, where the staging has none: behind the
-    // tables, which hide the fetching of the matrix (1 us of 30 at n=13), but before them at the derivative walk's sizes.  There a
+    // tables, which hide the fetching of the matrix (1 us of 30 at n=13), but
+    // before them at the derivative walk's sizes.  There a
     // barrier right in front of the walk made two calls of three take its slow
     // pace (a matrix on the device, n=24 67 or 76 us, n=26 149 or 180 us).
     constexpr bool kEarly = N >= kMinDerivReal;
