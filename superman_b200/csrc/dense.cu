@@ -417,7 +417,9 @@ void choose_width(Problem* pb, const spb_options* opt, int sms)
     const int bits = n - 1 - (pb->deriv ? 1 : 0);
     pb->w = choose_unit_bits(n, pb->comps, opt, bits);
     const double threads = (double)sms * walk_max_threads(n, pb->comps);
-    if (pb->f32 || (pb->comps == 1 && n <= kSmallCallMaxN) || opt->unit_bits > 0 || std::ldexp(1.0, bits - pb->w) < threads) return;
+    if (pb->f32 || (pb->comps == 1 && n <= kSmallCallMaxN) || opt->unit_bits > 0 ||
+        std::ldexp(1.0, bits - pb->w) < threads)
+        return;
     double best = 0.0;
     const int w0 = pb->w;
     for (int w = w0; w >= w0 - 2 && w >= 4; --w) {
